@@ -129,7 +129,7 @@ typedef struct {
     uint64_t record_bytes;    /* bytes of bucket records written */
     uint64_t gpu_launches;    /* kernels launched by the last tg_job_run */
     double phase2_count_ms;   /* part of phase2_ms: the shared-memory counting kernel(s) */
-    double phase2_keys_ms;    /* part of phase2_ms: bin histogram, group plan, key array */
+    double phase2_keys_ms;    /* part of phase2_ms: bin offsets, group plan, packed records */
     uint64_t groups;          /* phase-2 groups (runs of minimizer bins counted in one table) */
     double lex_ms;            /* device time: FASTA/FASTQ lexing of the feeds */
     uint64_t fastx_bytes;     /* FASTA/FASTQ bytes fed (before lexing) */

@@ -5,10 +5,10 @@
 //   k_pack      ASCII stream -> 2-bit codes + validity bits
 //   (k_lex_*    FASTA/FASTQ bytes -> the stream, when fed as files)
 //   k_cut_seq   minimizers, chain starts, forced splits -> record descriptors
-//               per CTA, k-mer instances per bin (one host sync here)
-//   k_scan_*    bin counts -> key offsets
+//               per CTA, k-mers and packed records per bin (one host sync here)
+//   k_scan*     bin counts -> k-mer and packed record offsets
 //   k_plan      groups of whole bins per segment (a run of bins of one sample)
-//   k_keys      every canonical k-mer key at its bin's cursor
+//   k_recs      every record with its bases at its group's cursor
 //   k_count     per group: keys into a shared-memory table, ci/cx, compaction
 //               (again for groups split by key hash)
 //   k_fb_*      (rare) key ranges that overflowed shared memory, global tables
@@ -96,9 +96,9 @@ uint32_t next_pow2_u32(uint64_t v) {
 }
 
 // Layout of the small device counter buffer ctx->misc (byte offsets).
-constexpr size_t MISC_CUT_STATS = 0;    // u64[3]: k-mers, records, runs (k_cut)
-constexpr size_t MISC_BASES = 24;       // u64: ACGT bases (k_pack)
-constexpr size_t MISC_OVERFLOW = 32;    // u32: descriptor list overflow (k_cut)
+constexpr size_t MISC_CUT_STATS = 0;    // u64[4]: k-mers, records, runs, extra packed records (k_cut)
+constexpr size_t MISC_BASES = 32;       // u64: ACGT bases (k_pack)
+constexpr size_t MISC_OVERFLOW = 40;    // u32: descriptor list overflow (k_cut)
 constexpr size_t MISC_DIGEST = 64;      // u64[4]: result digest (tg_job_result_digest)
 constexpr size_t MISC_NDESC = 256;      // u32[C]: descriptors per Phase-1 CTA
 constexpr size_t MISC_BYTES = MISC_NDESC + 4 * 65536;
@@ -204,7 +204,7 @@ struct SpillStore {
     std::vector<tgh::Bytes> bytes;
     std::vector<std::vector<uint64_t>> desc;
     std::vector<uint64_t> n_bytes, n_desc;
-    std::vector<uint64_t> hist;
+    std::vector<uint64_t> hist, rec_hist;  // k-mers and packed records per bin
     uint64_t kmers = 0, records = 0, runs = 0, bases = 0, chunks = 0, spilled_bytes = 0;
     std::string path(uint32_t b, const char* what) const {
         return dir + "/tuna_spill_" + std::to_string(b) + "." + what;
@@ -231,6 +231,7 @@ struct tg_job {
     bool ran = false;
     // layout of the last run
     uint32_t p1_bits = 0, n_cta = 0;
+    int bin_bits = BIN_BITS;       // log2 of the bins
     uint64_t chunk = 0, desc_cap = 0, packed_words = 0;
     // results
     uint64_t n_out = 0;
@@ -763,10 +764,10 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
             CK(ctx->ensure(ctx->hist, kmers_off + (size_t)p1 * 8), "alloc histograms");
             CK(cudaMemsetAsync(ctx->hist.as<uint8_t>() + kmers_off, 0, (size_t)p1 * 8, ctx->st), "memset");
         } else {
-            CK(ctx->ensure(ctx->hist, (size_t)4 << BIN_BITS), "alloc bin histogram");
-            CK(cudaMemsetAsync(ctx->hist.p, 0, (size_t)4 << BIN_BITS, ctx->st), "memset");
+            CK(ctx->ensure(ctx->hist, (size_t)8 << j->bin_bits), "alloc bin histogram");
+            CK(cudaMemsetAsync(ctx->hist.p, 0, (size_t)8 << j->bin_bits, ctx->st), "memset");
         }
-        CK(cudaMemsetAsync(ctx->misc.as<uint8_t>() + MISC_CUT_STATS, 0, 24, ctx->st), "memset");
+        CK(cudaMemsetAsync(ctx->misc.as<uint8_t>() + MISC_CUT_STATS, 0, 32, ctx->st), "memset");
         CK(cudaMemsetAsync(ctx->misc.as<uint8_t>() + MISC_OVERFLOW, 0, 4, ctx->st), "memset");
         CutParams P{};
         P.packed = ctx->packed.as<uint32_t>();
@@ -780,7 +781,7 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
         P.desc_cap = cap;
         P.n_desc = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_NDESC);
         P.hist = exp ? ctx->hist.as<uint32_t>() : nullptr;
-        P.binhist = exp ? nullptr : ctx->hist.as<uint32_t>();
+        P.binhist = exp ? nullptr : ctx->hist.as<unsigned long long>();
         P.stats = reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_CUT_STATS);
         P.overflow = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_OVERFLOW);
         P.xdesc = exp ? ctx->xdesc.as<uint64_t>() : nullptr;
@@ -788,6 +789,7 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
         P.sample_bin_base = cs.base;
         P.sample_bin_bits = cs.bits;
         P.n_samples = cs.n;
+        P.desc_sb = desc_start_bits(j->bin_bits);
         CK(cudaEventRecord(ctx->ev[2], ctx->st), "event");
         CK(launch_cut(P, ctx->tables.as<HashTables>(), exp, ctx->st), "k_cut");
         CK(cudaEventRecord(ctx->ev[3], ctx->st), "event");
@@ -836,7 +838,7 @@ static tg_status d2h_pageable(tg_ctx* ctx, void* dst, const void* src, size_t by
 // (0: chosen from the input size).
 struct P1Out {
     SampleBins B;
-    unsigned long long cstats[3] = {0, 0, 0};  // k-mers, records, runs
+    unsigned long long cstats[4] = {0, 0, 0, 0};  // k-mers, records, runs, extra packed records
     unsigned long long n_bases = 0;
     std::vector<uint32_t> nd;                   // descriptors per list
 };
@@ -872,10 +874,11 @@ static tg_status run_phase1(tg_job* j, int* launches_out, P1Out& r, uint32_t p1_
     if (!p1) p1 = std::max(j->n_shards, std::min<uint32_t>(1024, std::max<uint32_t>(16, next_pow2_u32(n / 32768))));
     uint32_t p1_bits = 0;
     while ((1u << p1_bits) < p1) ++p1_bits;
-    // the bins of the samples (2^20 in all, cut into p1 segments for one sample)
+    // the bins of the samples (cut into p1 segments for one sample)
     std::vector<unsigned long long> starts = j->sample_start;
     starts.push_back(n);
-    r.B = layout_bins(starts, (1u << BIN_BITS) >> p1_bits);
+    j->bin_bits = j->spill || j->n_shards > 1 ? BIN_BITS : job_bin_bits(n, (uint32_t)j->sample_start.size(), p1_bits);
+    r.B = layout_bins(starts, (1u << j->bin_bits) >> p1_bits, j->bin_bits);
     const SampleBins& B = r.B;
     const uint32_t ns = (uint32_t)B.base.size();
     if (j->n_shards > 1 && ns > 1) return ctx->fail(TG_ERR_UNSUPPORTED, "a job of several samples cannot be sharded");
@@ -898,7 +901,7 @@ static tg_status run_phase1(tg_job* j, int* launches_out, P1Out& r, uint32_t p1_
     if (s != TG_OK) return s;
     const uint32_t C = j->n_cta;
     r.nd.assign(C, 0);
-    CK(cudaMemcpyAsync(r.cstats, ctx->misc.as<uint8_t>() + MISC_CUT_STATS, 24, cudaMemcpyDeviceToHost, ctx->st),
+    CK(cudaMemcpyAsync(r.cstats, ctx->misc.as<uint8_t>() + MISC_CUT_STATS, 32, cudaMemcpyDeviceToHost, ctx->st),
        "d2h");
     CK(cudaMemcpyAsync(r.nd.data(), ctx->misc.as<uint8_t>() + MISC_NDESC, (size_t)C * 4, cudaMemcpyDeviceToHost,
                        ctx->st), "d2h");
@@ -934,26 +937,31 @@ static tg_status tg_job_run_impl(tg_job* j) {
     // (bins), each pass's pairs going to host memory before the next
     // the segments this run counts: all of them, or the job's shard of them
     std::vector<Segment> segs = B.segs;
-    std::vector<uint32_t> hist;  // k-mers per bin, downloaded when a shard or the passes need it
+    std::vector<uint64_t> hist;  // k-mers and packed records per bin, downloaded when a shard or the passes need it
     auto load_hist = [&]() -> cudaError_t {
         if (!hist.empty()) return cudaSuccess;
-        hist.resize((size_t)1 << BIN_BITS);
-        return cudaMemcpy(hist.data(), ctx->hist.p, hist.size() * 4, cudaMemcpyDeviceToHost);
+        hist.resize((size_t)1 << j->bin_bits);
+        return cudaMemcpy(hist.data(), ctx->hist.p, hist.size() * 8, cudaMemcpyDeviceToHost);
     };
-    uint64_t n_kmers = cstats[0];
+    uint64_t n_kmers = cstats[0], n_recs = cstats[1] + cstats[3];
     if (j->n_shards > 1) {  // one sample: 2^p1_bits >= n_shards segments of consecutive bins
         const size_t P = B.segs.size();
         segs.assign(B.segs.begin() + P * j->shard / j->n_shards, B.segs.begin() + P * (j->shard + 1) / j->n_shards);
         CK(load_hist(), "d2h");
-        n_kmers = 0;
+        n_kmers = n_recs = 0;
         for (const Segment& g : segs)
-            for (uint32_t b = g.bin_lo; b < g.bin_hi; ++b) n_kmers += hist[b];
+            for (uint32_t b = g.bin_lo; b < g.bin_hi; ++b) {
+                n_kmers += hist[b] & 0xFFFFFFFFull;
+                n_recs += hist[b] >> 32;
+            }
     }
     P2Input in{};
     in.W = W;
     in.k = k;
     in.segs = segs.data();
     in.n_segs = (uint32_t)segs.size();
+    in.all_bins = in.bin_hi = 1u << j->bin_bits;
+    in.desc_sb = desc_start_bits(j->bin_bits);
     if (j->n_shards > 1) {
         in.bin_lo = segs.front().bin_lo;
         in.bin_hi = segs.back().bin_hi;
@@ -963,14 +971,16 @@ static tg_status tg_job_run_impl(tg_job* j) {
     in.desc = ctx->desc.as<uint64_t>();
     in.desc_cap = j->desc_cap;
     in.n_lists = C;
-    in.n_desc = nd.data();
-    in.binhist = ctx->hist.as<uint32_t>();
+    in.n_desc = reinterpret_cast<const uint32_t*>(ctx->misc.as<uint8_t>() + MISC_NDESC);
+    in.max_desc = (uint32_t)std::min<uint64_t>(*std::max_element(nd.begin(), nd.end()), j->desc_cap);
+    in.binhist = ctx->hist.as<unsigned long long>();
     in.n_kmers = n_kmers;
+    in.n_recs = n_recs;
     in.ci = j->o.ci;
     in.cx = j->o.cx;
     in.n_samples = ns;
     std::vector<std::pair<uint32_t, uint32_t>> passes;  // segment ranges
-    std::vector<uint64_t> seg_keys;
+    std::vector<uint64_t> seg_keys, seg_recs;
     {
         const uint64_t per_key = 2 * key_bytes(W) + 4 + 24;  // key, pair, groups and slack
         size_t free_b = 0, total_b = 0;
@@ -984,9 +994,13 @@ static tg_status tg_job_run_impl(tg_job* j) {
             uint32_t s0 = 0;
             uint64_t acc = 0;
             for (uint32_t sg = 0; sg < segs.size(); ++sg) {
-                uint64_t kk = 0;
-                for (uint32_t b = segs[sg].bin_lo; b < segs[sg].bin_hi; ++b) kk += hist[b];
+                uint64_t kk = 0, rr = 0;
+                for (uint32_t b = segs[sg].bin_lo; b < segs[sg].bin_hi; ++b) {
+                    kk += hist[b] & 0xFFFFFFFFull;
+                    rr += hist[b] >> 32;
+                }
                 seg_keys.push_back(kk);
+                seg_recs.push_back(rr);
                 if (sg > s0 && acc + kk > max_keys) {
                     passes.emplace_back(s0, sg);
                     s0 = sg;
@@ -1083,8 +1097,11 @@ static tg_status tg_job_run_impl(tg_job* j) {
             ip.n_segs = s1 - s0;
             ip.bin_lo = segs[s0].bin_lo;
             ip.bin_hi = segs[s1 - 1].bin_hi;
-            ip.n_kmers = 0;
-            for (uint32_t sg = s0; sg < s1; ++sg) ip.n_kmers += seg_keys[sg];
+            ip.n_kmers = ip.n_recs = 0;
+            for (uint32_t sg = s0; sg < s1; ++sg) {
+                ip.n_kmers += seg_keys[sg];
+                ip.n_recs += seg_recs[sg];
+            }
             max_keys = std::max(max_keys, ip.n_kmers);
             p2_bytes = std::max(p2_bytes, phase2_scratch_bytes(ip));
         }
@@ -1198,6 +1215,7 @@ tg_status tg_job_set_spill(tg_job* j, uint64_t chunk_bytes, const char* dir) {
         st->n_bytes.assign(st->nb, 0);
         st->n_desc.assign(st->nb, 0);
         st->hist.assign((size_t)1 << BIN_BITS, 0);
+        st->rec_hist.assign((size_t)1 << BIN_BITS, 0);
         if (dir) {  // fresh, empty bucket files
             for (uint32_t b = 0; b < st->nb; ++b)
                 for (const char* what : {"bytes", "desc"}) {
@@ -1243,9 +1261,12 @@ static tg_status spill_flush(tg_job* j) {
     const uint32_t nb = S.nb, C = j->n_cta;
     const uint32_t* d_nd = reinterpret_cast<const uint32_t*>(ctx->misc.as<uint8_t>() + MISC_NDESC);
     {  // k-mers per bin
-        std::vector<uint32_t> h((size_t)1 << BIN_BITS);
-        CK(cudaMemcpy(h.data(), ctx->hist.p, h.size() * 4, cudaMemcpyDeviceToHost), "d2h");
-        for (size_t b = 0; b < h.size(); ++b) S.hist[b] += h[b];
+        std::vector<uint64_t> h((size_t)1 << BIN_BITS);
+        CK(cudaMemcpy(h.data(), ctx->hist.p, h.size() * 8, cudaMemcpyDeviceToHost), "d2h");
+        for (size_t b = 0; b < h.size(); ++b) {
+            S.hist[b] += h[b] & 0xFFFFFFFFull;
+            S.rec_hist[b] += h[b] >> 32;
+        }
     }
     // per-bucket records and bytes, then the staging layout
     // sp_aux: totals [2 nb], cursors [2 nb], host shifts [nb] (u64 / i64 each)
@@ -1326,16 +1347,17 @@ static tg_status run_spill(tg_job* j) {
     const uint32_t nb = S.nb;
     const uint32_t seg_bins = (1u << BIN_BITS) / nb;
     int launches = 0;
-    // k-mers per bin of all chunks, for the scan of each pass
-    std::vector<uint32_t> h32(S.hist.size());
-    std::vector<uint64_t> bk(nb, 0);
+    // k-mers and packed records per bin of all chunks, for the scan of each pass
+    std::vector<uint64_t> hu(S.hist.size());
+    std::vector<uint64_t> bk(nb, 0), br(nb, 0);
     for (size_t b = 0; b < S.hist.size(); ++b) {
         if (S.hist[b] > 0xFFFFFFFFull) return ctx->fail(TG_ERR_UNSUPPORTED, "a bin holds more than 2^32 k-mers");
-        h32[b] = (uint32_t)S.hist[b];
+        hu[b] = S.hist[b] | (S.rec_hist[b] << 32);
         bk[b / seg_bins] += S.hist[b];
+        br[b / seg_bins] += S.rec_hist[b];
     }
-    CK(ctx->ensure(ctx->hist, (size_t)4 << BIN_BITS), "alloc bin histogram");
-    CK(cudaMemcpy(ctx->hist.p, h32.data(), h32.size() * 4, cudaMemcpyHostToDevice), "h2d");
+    CK(ctx->ensure(ctx->hist, (size_t)8 << BIN_BITS), "alloc bin histogram");
+    CK(cudaMemcpy(ctx->hist.p, hu.data(), hu.size() * 8, cudaMemcpyHostToDevice), "h2d");
     const SampleBins B = layout_bins({0ull, 1ull}, seg_bins);
     uint64_t budget = 0;
     s = phase2_budget(ctx, &budget);
@@ -1369,8 +1391,13 @@ static tg_status run_spill(tg_job* j) {
     float ms = 0;
     const double t0 = now_ms();
     for (const auto& pr : passes) {
-        uint64_t nbytes = 0, ndesc = 0, nk = 0;
-        for (uint32_t b = pr.first; b < pr.second; ++b) { nbytes += S.n_bytes[b]; ndesc += S.n_desc[b]; nk += bk[b]; }
+        uint64_t nbytes = 0, ndesc = 0, nk = 0, nr = 0;
+        for (uint32_t b = pr.first; b < pr.second; ++b) {
+            nbytes += S.n_bytes[b];
+            ndesc += S.n_desc[b];
+            nk += bk[b];
+            nr += br[b];
+        }
         if (ndesc > 0xFFFFFFFFull) return ctx->fail(TG_ERR_UNSUPPORTED, "a spill pass holds more than 2^32 records");
         // the pass stream: 8 bytes (TG_PAD bases) of padding, the buckets, slack
         const uint64_t words = packed_words_for(4 * nbytes);
@@ -1399,7 +1426,6 @@ static tg_status run_spill(tg_job* j) {
             bo += S.n_bytes[b];
             dof += S.n_desc[b];
         }
-        const uint32_t nlist = (uint32_t)ndesc;
         P2Input in{};
         in.W = W;
         in.k = k;
@@ -1412,9 +1438,11 @@ static tg_status run_spill(tg_job* j) {
         in.desc = ctx->desc.as<uint64_t>();
         in.desc_cap = std::max<uint64_t>(ndesc, 1);
         in.n_lists = 1;
-        in.n_desc = &nlist;
-        in.binhist = ctx->hist.as<uint32_t>();
+        in.n_desc = nullptr;
+        in.max_desc = (uint32_t)ndesc;
+        in.binhist = ctx->hist.as<unsigned long long>();
         in.n_kmers = nk;
+        in.n_recs = nr;
         in.ci = j->o.ci;
         in.cx = j->o.cx;
         in.n_samples = 1;

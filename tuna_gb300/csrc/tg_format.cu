@@ -233,7 +233,7 @@ cudaError_t launch_digest(int k, const uint64_t* keys, const uint32_t* counts, u
 
 size_t fmt_scratch_bytes(uint64_t n_pairs) {
     const uint64_t n_tiles = (n_pairs + FMT_T - 1) / FMT_T;
-    return 512 + n_tiles * 4 + (n_tiles + 1) * 8 + 64 * 8 + 3 * 256;
+    return 512 + n_tiles * 4 + (n_tiles + 1) * 8 + scan_scratch(n_tiles) * 8 + 3 * 256;
 }
 
 uint64_t fmt_max_bytes(int fmt, int k, uint64_t n_pairs) {
@@ -256,13 +256,13 @@ cudaError_t launch_format(int fmt, int k, const uint64_t* keys, const uint32_t* 
     };
     uint32_t* tile_len = reinterpret_cast<uint32_t*>(take(n_tiles * 4 + 4));
     unsigned long long* tile_off = reinterpret_cast<unsigned long long*>(take((n_tiles + 1) * 8));
-    unsigned long long* sums = reinterpret_cast<unsigned long long*>(take(64 * 8));
+    unsigned long long* sums = reinterpret_cast<unsigned long long*>(take(scan_scratch(n_tiles) * 8));
     cudaError_t e = cudaSuccess;
     if (n == 0) return cudaSuccess;
     if (fmt == TG_FMT_TSV) {
         k_fmt_tile_len<<<grid, FMT_T, 0, st>>>(counts, n, k, tile_len);
         ++*launches;
-        e = launch_scan(tile_len, n_tiles, tile_off, sums, d_total, st, launches);
+        e = launch_scan(tile_len, n_tiles, tile_off, sums, st, launches, d_total);
         if (e != cudaSuccess) return e;
         e = launch_fmt_w<TG_FMT_TSV>(W, keys, counts, n, k, tile_off, out, grid, st);
     } else {  // fixed record size: the caller knows the total (fmt_max_bytes)

@@ -8,12 +8,12 @@
 //                            index g + TG_PAD, the TG_PAD leading bases are 0
 //   valid   u32[]            1 bit per base, LSB-first, same TG_PAD offset
 //   desc    u64[C][cap]      per Phase-1 CTA: one descriptor per superkmer record
-//                            (start position, k-mer count, low 20 bits of its
-//                            minimizer hash; see desc_pack)
-//   binhist u32[2^20]        k-mer instances per bin (each sample owns a range of bins,
-//                            one picked by minimizer hash); scanned into kofs
-//   keys    u64 x W [K]      every canonical k-mer instance, grouped by bin
-//                            (W = 1 for k <= 31)
+//                            (start position, k-mer count, bin; see desc_pack)
+//   binhist u64[bins]        k-mer instances (low half) and packed records (high half) per
+//                            bin (each sample owns a range of bins, one picked by
+//                            minimizer hash); scanned into kofs and rofs
+//   recs    16 x W B [R]     every record with its bases, grouped by runs of bins (W = 1
+//                            for k <= 31; see REC_MAX)
 //   out     keys + u32 counts of the distinct k-mers that pass ci/cx
 //
 // Reference counterparts (paths relative to the reference project root):
@@ -50,20 +50,33 @@ struct HashTables {
 
 // Superkmer record descriptor (u64): the record covers the k-mers starting at
 // positions [start, start + nk) of the stream; its bases are read from
-// `packed` when it is counted. bin (20 bits) places the record's k-mers in the
-// key array: the 2^20 bins are shared out among the samples of a job, sample s
+// `packed` when it is counted. bin places the record's k-mers in the
+// group order: the bins are shared out among the samples of a job, sample s
 // owning [base_s, base_s + 2^bits_s), and a record of sample s goes to bin
 // base_s + (minimizer hash mod 2^bits_s). All instances of a canonical k-mer
 // of one sample share its minimizer, hence its bin. (The export cut stores
 // the low 20 bits of the minimizer hash there instead.)
+// A job has 2^bits bins, bits chosen from its length (job_bin_bits): the fields
+// are start (sb bits), k-mers (8), bin (56 - sb), with sb = 36 for up to 2^20
+// bins and 34 for more.
 constexpr int DESC_START_BITS = 36;
-constexpr int BIN_BITS = 20;
-__host__ __device__ __forceinline__ uint64_t desc_pack(uint64_t start, uint32_t nk, uint32_t bin) {
-    return start | ((uint64_t)nk << DESC_START_BITS) | ((uint64_t)(bin & 0xFFFFFu) << 44);
+constexpr int BIN_BITS = 20;       // bins of a sharded or spilled job, whose bins several runs share
+constexpr int MAX_BIN_BITS = 22;
+__host__ __device__ __forceinline__ int desc_start_bits(int bin_bits) { return bin_bits > BIN_BITS ? 34 : DESC_START_BITS; }
+__host__ __device__ __forceinline__ uint64_t desc_pack(uint64_t start, uint32_t nk, uint32_t bin,
+                                                       int sb = DESC_START_BITS) {
+    // sb >= 32: k-mers and bin lie in the high word
+    return start | ((uint64_t)(((bin << 8) | nk) << (sb - 32)) << 32);
 }
-__host__ __device__ __forceinline__ uint64_t desc_start(uint64_t d) { return d & ((1ull << DESC_START_BITS) - 1); }
-__host__ __device__ __forceinline__ uint32_t desc_nk(uint64_t d) { return (uint32_t)(d >> DESC_START_BITS) & 0xFFu; }
-__host__ __device__ __forceinline__ uint32_t desc_bin(uint64_t d) { return (uint32_t)(d >> 44); }
+__host__ __device__ __forceinline__ uint64_t desc_start(uint64_t d, int sb = DESC_START_BITS) {
+    return d & ((1ull << sb) - 1);
+}
+__host__ __device__ __forceinline__ uint32_t desc_nk(uint64_t d, int sb = DESC_START_BITS) {
+    return ((uint32_t)(d >> 32) >> (sb - 32)) & 0xFFu;
+}
+__host__ __device__ __forceinline__ uint32_t desc_bin(uint64_t d, int sb = DESC_START_BITS) {
+    return (uint32_t)(d >> 32) >> (sb - 24);
+}
 
 // Offset (in u32 units) of the u64 per-bucket k-mer counters that follow the
 // u32 [P][C] record histogram: rounded up so the u64 array is 8-byte aligned
@@ -85,29 +98,34 @@ struct CutParams {
     uint64_t desc_cap;
     uint32_t* n_desc;        // [n_cta]
     uint32_t* hist;          // export cut: u32 [P][n_cta] records, then u64 [P] k-mers per bucket
-    uint32_t* binhist;       // counting cut: [2^20] k-mers per bin
+    unsigned long long* binhist;  // counting cut: [bins] k-mers + 2^32 x packed records per bin
+    int desc_sb;             // counting cut: start bits of a descriptor (desc_start_bits)
     // samples of the job (counting cut): sample i is positions [start[i], start[i+1])
     const unsigned long long* sample_start;  // [n_samples + 1]
     const uint32_t* sample_bin_base;         // [n_samples] first bin of each sample
     const uint8_t* sample_bin_bits;          // [n_samples] log2 bins of each sample
     uint32_t n_samples;
-    unsigned long long* stats;  // [0] kmers, [1] records, [2] runs
+    unsigned long long* stats;  // [0] kmers, [1] records, [2] runs, [3] packed records beyond one per record
     uint32_t* overflow;      // set when a CTA's descriptor list is full
     // export mode: full descriptors (start, minimizer hash, min_pos, nk)
     uint64_t* xdesc;         // [n_cta][desc_cap][3] or null
 };
 
-// Phase 2 works on slices of the phase-1 descriptor lists and on groups: runs
-// of whole bins of one segment, whose keys are contiguous in the key array
-// (the keys are laid out bin-major).
-struct Slice {
-    uint64_t r_lo, r_hi;  // descriptor range in the phase-1 lists
-};
+// Packed record: the bases of up to REC_MAX consecutive k-mers, 16 x W bytes.
+// Base j at bits 62 - 2 (j mod 32) of u64 word j / 32; the number of k-mers in the
+// low 6 bits of the last word, so 61 (W = 1) or 125 (W = 2) bases fit: room for
+// the REC_MAX + k - 1 of any k. A record of more k-mers is packed as several,
+// of equal lengths but for the last. A warp that unpacks 32 records takes as many
+// steps as the longest has k-mers: most have at most k - m + 1.
+constexpr uint32_t REC_MAX = 16;
+__host__ __device__ __forceinline__ uint32_t rec_pieces(uint32_t nk) { return (nk + REC_MAX - 1) / REC_MAX; }
 
+// Phase 2 works on groups: runs of whole bins of one segment, whose packed
+// records are contiguous.
 struct Group {
-    unsigned long long lo, hi;  // key range [lo, hi)
+    unsigned long long lo, hi;  // range of packed records [lo, hi)
     uint32_t parts, part;       // count only the keys whose hash part is `part` of `parts`
-    uint32_t sample, pad;       // the sample whose keys these are
+    uint32_t sample, keys;      // the sample whose records these are; their k-mers
 };
 
 // A run of consecutive bins of one sample that k_plan cuts into groups.
@@ -118,8 +136,8 @@ struct Segment {
 // Counters of one Phase-2 run (device, u64 each).
 enum P2Counter : int {
     P2C_NORMAL = 0,   // groups of at most `target` k-mers
-    P2C_HEAVY,        // groups larger than `target`
-    P2C_RETRY,        // groups pushed back for another pass with more parts
+    P2C_HEAVY,        // larger groups
+    P2C_BIG,          // the largest, which many CTAs share
     P2C_FALLBACK,     // key ranges left to the global-memory table
     P2C_OUT,          // output cursor
     P2C_DISTINCT,     // distinct keys seen
@@ -128,27 +146,32 @@ enum P2Counter : int {
 
 struct KeysParams {
     const uint32_t* packed;
-    const uint64_t* desc;              // phase-1 descriptor lists
-    const Slice* slices;
-    unsigned long long* kofs;          // [2^20 + 1] first key of each bin; a group's first bin's entry
-                                       // is the group's cursor, advanced by k_keys
-    uint32_t* gfirst;                  // [2^20] first bin of each bin's group (written by k_plan)
+    const uint64_t* desc;              // phase-1 descriptor lists, desc_cap entries apart
+    uint64_t desc_cap;
+    const uint32_t* n_desc;            // descriptors per list (device), or null: one list of n_one
+    uint32_t n_one;
+    const unsigned long long* kofs;    // [bins + 1] k-mers before each bin
+    unsigned long long* rofs;          // [bins + 1] packed records before each bin; a group's first bin's
+                                       // entry is the group's cursor, advanced by k_recs
+    uint32_t* gfirst;                  // [bins] first bin of each bin's group (written by k_plan)
     const Segment* segs;               // k_plan: one warp per segment
     uint32_t n_segs;
     uint32_t target;                   // k-mer instances per group
     int k;
-    void* keys;                        // u64 x W per k-mer instance
-    Group* groups[2];                  // [0] normal, [1] heavy
+    void* recs;                        // packed records
+    Group* groups[3];                  // [0] normal, [1] heavy, [2] big
     uint64_t groups_cap;
     unsigned long long* ctr;           // P2Counter
-    uint32_t bin_lo, bin_hi;           // k_keys: only records of bins in [bin_lo, bin_hi)
+    uint32_t bin_lo, bin_hi;           // k_recs: only records of bins in [bin_lo, bin_hi)
+    int desc_sb;                       // start bits of a descriptor
+    uint32_t plan_split;               // k_plan: warps per segment
 };
 
 struct CountParams {
-    const void* keys;
-    const Group* list[2];              // processed in order: list[1] first, then list[0]
-    const unsigned long long* n_list;  // [0] entries of list[0], [1] of list[1]
-    Group* retry;                      // failed groups, split in two
+    const void* recs;                  // packed records
+    int k;
+    const Group* list;
+    Group* retry;                      // failed groups, split
     unsigned long long* n_retry;
     uint64_t retry_cap;
     Group* fallback;
@@ -159,16 +182,16 @@ struct CountParams {
     uint32_t* out_sample;              // sample of each pair (jobs of several samples), or null
     uint64_t out_cap;
     unsigned long long* ctr;           // P2Counter
-    uint32_t smem_slots;               // table capacity in shared memory
-    unsigned long long g_begin, g_end; // this launch counts groups [g_begin, g_end) of the sequence
+    unsigned long long g_begin, g_end; // this launch counts groups [g_begin, g_end) of the list
     unsigned long long* work;          // this launch's group counter (starts at 0)
 };
 
-// A key range that did not fit in shared memory, counted in a global table.
+// Key ranges counted in a global table.
 struct FallbackParams {
-    const void* keys;
-    unsigned long long lo, hi;
-    uint32_t parts, part, sample;
+    const void* recs;
+    int k;
+    unsigned long long lo, hi;  // packed records
+    uint32_t parts, part;
     void* tkeys;          // S slots
     uint32_t* tcnt;
     uint32_t mask;

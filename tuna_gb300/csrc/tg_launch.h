@@ -21,8 +21,13 @@ uint64_t packed_words_for(uint64_t n);
 cudaError_t launch_pack(const uint8_t* seq, uint64_t n, uint32_t* packed, uint32_t* valid, uint64_t n_words,
                         unsigned long long* n_bases, cudaStream_t st);
 cudaError_t launch_cut(const CutParams& P, const HashTables* gT, bool exp, cudaStream_t st);
-cudaError_t launch_scan(const uint32_t* in, uint64_t n, unsigned long long* out, unsigned long long* sums,
-                        unsigned long long* total, cudaStream_t st, int* launches);
+// Exclusive scans of n >= 1 counts into n + 1 entries (the last: the total, which
+// goes to *total too if given); scratch holds scan_scratch(n) u64, 16-byte aligned.
+uint64_t scan_scratch(uint64_t n);
+cudaError_t launch_scan(const uint32_t* in, uint64_t n, unsigned long long* out, unsigned long long* scratch,
+                        cudaStream_t st, int* launches, unsigned long long* total = nullptr);
+cudaError_t launch_bin_scan(const unsigned long long* hist, uint64_t n, unsigned long long* kofs,
+                            unsigned long long* rofs, unsigned long long* scratch, cudaStream_t st, int* launches);
 // FASTA/FASTQ lexing on the device (tg_lex.cu). raw must be 16-byte aligned;
 // out receives at most len bytes. Totals are written to device memory (*dtot,
 // inside scratch) and are valid once the stream reaches them.
@@ -84,10 +89,14 @@ struct SampleBins {
     std::vector<uint8_t> bits;              // [n] log2 bins
     std::vector<Segment> segs;
 };
-// Shares the 2^20 bins out among samples in proportion to their length (a
+// Shares 2^bin_bits bins out among samples in proportion to their length (a
 // power of two each) and cuts each sample's bins into segments of at most
 // seg_bins bins.
-SampleBins layout_bins(const std::vector<unsigned long long>& sample_start, uint32_t seg_bins);
+SampleBins layout_bins(const std::vector<unsigned long long>& sample_start, uint32_t seg_bins,
+                       int bin_bits = BIN_BITS);
+// log2 of the bins of a job of n stream bytes, n_samples samples and 2^seg_bits
+// segments that shares its bins with no other run.
+int job_bin_bits(uint64_t n, uint32_t n_samples, uint32_t seg_bits);
 struct P2Input {
     int W, k;                          // key words, k
     const Segment* segs;               // [n_segs] (host): runs of bins of one sample, cut into groups
@@ -97,14 +106,18 @@ struct P2Input {
     const uint64_t* desc;              // [n_lists][desc_cap] phase-1 descriptors
     uint64_t desc_cap;
     uint32_t n_lists;
-    const uint32_t* n_desc;            // [n_lists] descriptors per list (host)
-    const uint32_t* binhist;           // [2^20] k-mers per bin (device)
+    const uint32_t* n_desc;            // [n_lists] descriptors per list (device); null: one list of max_desc
+    uint32_t max_desc;                 // descriptors of the longest list
+    const unsigned long long* binhist; // [all_bins] k-mers and packed records per bin (device)
     uint64_t n_kmers;                  // k-mer instances in all
+    uint64_t n_recs;                   // packed records in all
     uint64_t ci, cx;
     uint32_t n_samples = 1;
-    // the bins counted by this run (all by default); segs must lie inside and
-    // n_kmers count only their keys
+    // the bins counted by this run (all by default); segs must lie inside, and
+    // n_kmers and n_recs count only theirs
     uint32_t bin_lo = 0, bin_hi = 1u << BIN_BITS;
+    uint32_t all_bins = 1u << BIN_BITS;  // bins of the job
+    int desc_sb = DESC_START_BITS;       // start bits of a descriptor
     uint32_t group_pct = 50;  // keys per group, % of the table's slots
 };
 struct P2Output {
@@ -140,11 +153,11 @@ struct P2Overlap {
 // not by cudaMemcpyAsync: a copy-engine read would queue behind the result
 // copies already issued on the copy stream.
 constexpr uint32_t OVERLAP_WORDS = 64;
-// Device scratch one run needs (key array included).
+// Device scratch one run needs (packed records included).
 size_t phase2_scratch_bytes(const P2Input& in);
 // Runs phase 2 on `st` and waits for it. fallback_table(bytes) returns device
 // memory for a global table (or null); ev_keys (optional) is recorded once the
-// keys are written.
+// packed records are written.
 tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Output& out,
                      const std::function<void*(size_t)>& fallback_table, cudaStream_t st, cudaEvent_t ev_keys,
                      int* launches, std::string& err, const P2Overlap& ov = P2Overlap());

@@ -156,25 +156,26 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     const uint64_t desc_cap = chunk + 2ull * tile + L + 64;
     uint64_t* desc = cv.take<uint64_t>((size_t)C * desc_cap);
     uint32_t* n_desc = cv.take<uint32_t>(C);
-    uint32_t* binhist = cv.take<uint32_t>((size_t)1 << BIN_BITS);
-    // one sample: all 2^20 bins, cut into p1 segments
-    const SampleBins B = layout_bins({0ull, (unsigned long long)n}, (1u << BIN_BITS) >> p1_bits);
+    const int bin_bits = job_bin_bits(n, 1, p1_bits);
+    unsigned long long* binhist = cv.take<unsigned long long>((size_t)1 << bin_bits);
+    // one sample: all bins, cut into p1 segments
+    const SampleBins B = layout_bins({0ull, (unsigned long long)n}, (1u << bin_bits) >> p1_bits, bin_bits);
     unsigned long long* s_start = cv.take<unsigned long long>(2);
     uint32_t* s_base = cv.take<uint32_t>(1);
     uint8_t* s_bits = cv.take<uint8_t>(1);
     if (!cv.ok) { set_err(errbuf, errlen, "input too large for the no-allocation scratch"); return TG_ERR_ARG; }
-    // counters in misc (u64 indices): [0..2] k-mers/records/runs, [3] bases, [4] overflow (u32)
-    uint32_t* overflow = reinterpret_cast<uint32_t*>(misc + 4);
+    // counters in misc (u64 indices): [0..3] k-mers, records, runs, extra packed records, [4] bases, [5] overflow (u32)
+    uint32_t* overflow = reinterpret_cast<uint32_t*>(misc + 5);
 
     const HashTables T = make_hash_tables(m);
     NA_CK(cudaMemcpyAsync(tables, &T, sizeof T, cudaMemcpyHostToDevice, st), "upload tables");
     NA_CK(cudaMemsetAsync(misc, 0, 32 * 8, st), "memset");
-    NA_CK(cudaMemsetAsync(binhist, 0, (size_t)4 << BIN_BITS, st), "memset");
+    NA_CK(cudaMemsetAsync(binhist, 0, (size_t)8 << bin_bits, st), "memset");
     NA_CK(cudaMemcpyAsync(s_start, B.start.data(), 16, cudaMemcpyHostToDevice, st), "h2d");
     NA_CK(cudaMemcpyAsync(s_base, B.base.data(), 4, cudaMemcpyHostToDevice, st), "h2d");
     NA_CK(cudaMemcpyAsync(s_bits, B.bits.data(), 1, cudaMemcpyHostToDevice, st), "h2d");
     // ---- phase 1
-    NA_CK(launch_pack(d_seq, n, packed, valid, pw, misc + 3, st), "k_pack");
+    NA_CK(launch_pack(d_seq, n, packed, valid, pw, misc + 4, st), "k_pack");
     CutParams P{};
     P.packed = packed; P.valid = valid; P.n = n;
     P.k = k; P.m = m; P.w = w; P.L = L;
@@ -182,22 +183,26 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     P.desc = desc; P.desc_cap = desc_cap; P.n_desc = n_desc;
     P.hist = nullptr; P.binhist = binhist; P.stats = misc; P.overflow = overflow; P.xdesc = nullptr;
     P.sample_start = s_start; P.sample_bin_base = s_base; P.sample_bin_bits = s_bits; P.n_samples = 1;
+    P.desc_sb = desc_start_bits(bin_bits);
     NA_CK(launch_cut(P, tables, false, st), "k_cut");
     int launches = 0;
     std::vector<uint32_t> nd(C);
-    unsigned long long cstats[3] = {0, 0, 0};
+    unsigned long long cstats[4] = {0, 0, 0, 0};
     uint32_t ovf = 0;
     NA_CK(cudaMemcpyAsync(nd.data(), n_desc, (size_t)C * 4, cudaMemcpyDeviceToHost, st), "d2h");
-    NA_CK(cudaMemcpyAsync(cstats, misc, 24, cudaMemcpyDeviceToHost, st), "d2h");
+    NA_CK(cudaMemcpyAsync(cstats, misc, 32, cudaMemcpyDeviceToHost, st), "d2h");
     NA_CK(cudaMemcpyAsync(&ovf, overflow, 4, cudaMemcpyDeviceToHost, st), "d2h");
     NA_CK(cudaStreamSynchronize(st), "phase 1");
     if (ovf) { set_err(errbuf, errlen, "descriptor capacity exceeded"); return TG_ERR_DEVICE; }
     // ---- phase 2 in what is left
     P2Input in{};
     in.W = W; in.k = k; in.segs = B.segs.data(); in.n_segs = (uint32_t)B.segs.size(); in.n_sm = (uint32_t)n_sm;
-    in.packed = packed; in.desc = desc; in.desc_cap = desc_cap; in.n_lists = C; in.n_desc = nd.data();
-    in.binhist = binhist; in.n_kmers = cstats[0];
+    in.packed = packed; in.desc = desc; in.desc_cap = desc_cap; in.n_lists = C; in.n_desc = n_desc;
+    in.max_desc = (uint32_t)std::min<uint64_t>(*std::max_element(nd.begin(), nd.end()), desc_cap);
+    in.binhist = binhist; in.n_kmers = cstats[0]; in.n_recs = cstats[1] + cstats[3];
     in.ci = o.ci; in.cx = o.cx;
+    in.bin_hi = in.all_bins = 1u << bin_bits;
+    in.desc_sb = desc_start_bits(bin_bits);
     const size_t p2_bytes = phase2_scratch_bytes(in);
     uint8_t* p2_scratch = cv.take<uint8_t>(p2_bytes);
     if (!cv.ok) { set_err(errbuf, errlen, "input too large for the no-allocation scratch"); return TG_ERR_ARG; }

@@ -423,7 +423,7 @@ k_cut(CutParams P, const HashTables* __restrict__ gT) {
             if (emit) {
                 const uint32_t idx = s_ndesc + di;
                 if (idx < P.desc_cap) {
-                    P.desc[(uint64_t)c * P.desc_cap + idx] = desc_pack(st, nk, mlo);
+                    P.desc[(uint64_t)c * P.desc_cap + idx] = desc_pack(st, nk, mlo & 0xFFFFFu);
                     if (EXPORT) {
                         uint64_t* x = P.xdesc + ((uint64_t)c * P.desc_cap + idx) * 3;
                         x[0] = st;
@@ -633,6 +633,7 @@ k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
     const uint64_t kmask = (1ull << k) - 1;  // k <= 63
     const int64_t Lr = P.L;
     unsigned long long loc_kmers = 0, loc_recs = 0, loc_runs = 0;
+    uint32_t loc_extra = 0;  // packed records beyond one per record
     bool overflowed = false;
     uint64_t* dlist = P.desc + (uint64_t)c * P.desc_cap;
     auto owned = [&](int64_t cs) { return cs >= cstart && cs < cend; };
@@ -652,9 +653,11 @@ k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
     auto put = [&](uint32_t idx, int64_t st, uint32_t nk, uint32_t mh) {
         const uint32_t smp = (seg_s != ~0u && st >= seg_lo && st < seg_lo + SEG) ? seg_s : sample_of(st);
         const uint32_t bin = P.sample_bin_base[smp] + (mh & ((1u << P.sample_bin_bits[smp]) - 1));
-        if (idx < P.desc_cap) dlist[idx] = desc_pack((uint64_t)st, nk, bin);
+        if (idx < P.desc_cap) dlist[idx] = desc_pack((uint64_t)st, nk, bin, P.desc_sb);
         else overflowed = true;
-        atomicAdd(&P.binhist[bin], nk);  // the key array's layout
+        const uint32_t pieces = rec_pieces(nk);
+        atomicAdd(&P.binhist[bin], ((unsigned long long)pieces << 32) | nk);
+        loc_extra += pieces - 1;
         loc_kmers += nk;
         loc_recs += 1;
     };
@@ -742,7 +745,7 @@ k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
                         last_ev = kp;
                         last_is_cs = cs;
                         open = cs;
-                        if (cs) { rs = kp; rm = (uint32_t)(M & 0xFFFFFu); last_cs = kp; last_cs_m = rm; }
+                        if (cs) { rs = kp; rm = (uint32_t)M; last_cs = kp; last_cs_m = rm; }
                     }
                 }
                 mprev = M;
@@ -809,11 +812,13 @@ k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
         loc_kmers += __shfl_down_sync(0xffffffffu, loc_kmers, o);
         loc_recs += __shfl_down_sync(0xffffffffu, loc_recs, o);
         loc_runs += __shfl_down_sync(0xffffffffu, loc_runs, o);
+        loc_extra += __shfl_down_sync(0xffffffffu, loc_extra, o);
     }
     if (lane == 0) {
         if (loc_kmers) atomicAdd(&P.stats[0], loc_kmers);
         if (loc_recs) atomicAdd(&P.stats[1], loc_recs);
         if (loc_runs) atomicAdd(&P.stats[2], loc_runs);
+        if (loc_extra) atomicAdd(&P.stats[3], (unsigned long long)loc_extra);
     }
 }
 
@@ -959,6 +964,7 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
     const int64_t cend = min(cstart + (int64_t)P.chunk, (int64_t)P.n);
     const int64_t Lr = P.L;
     unsigned long long loc_kmers = 0, loc_recs = 0, loc_runs = 0;
+    uint32_t loc_extra = 0;  // packed records beyond one per record
     bool overflowed = false;
     uint64_t* dlist = P.desc + (uint64_t)c * P.desc_cap;
     auto owned = [&](int64_t cs) { return cs >= cstart && cs < cend; };
@@ -982,9 +988,11 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
             const uint32_t smp = sample_of(st);
             bin = P.sample_bin_base[smp] + (mh & ((1u << P.sample_bin_bits[smp]) - 1));
         }
-        if (idx < P.desc_cap) dlist[idx] = desc_pack((uint64_t)st, nk, bin);
+        if (idx < P.desc_cap) dlist[idx] = desc_pack((uint64_t)st, nk, bin, P.desc_sb);
         else overflowed = true;
-        atomicAdd(&P.binhist[bin], nk);
+        const uint32_t pieces = rec_pieces(nk);
+        atomicAdd(&P.binhist[bin], ((unsigned long long)pieces << 32) | nk);
+        loc_extra += pieces - 1;
         loc_kmers += nk;
         loc_recs += 1;
     };
@@ -1119,7 +1127,7 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
                         cl &= cl - 1;
                         const uint32_t after = cut & (uint32_t)(~0ull << (cb + 1));
                         const int e = __ffs(after) - 1;
-                        put(idx++, pb + kp0 + cb, (uint32_t)(e - cb), s_mlo[cb * NT + tid] & 0xFFFFFu);
+                        put(idx++, pb + kp0 + cb, (uint32_t)(e - cb), s_mlo[cb * NT + tid]);
                     }
                 }
             }
@@ -1130,7 +1138,7 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
                 if (cs) {
                     const int lc = 31 - __clz(cs);
                     last_cs = kp0 + lc;
-                    last_cs_m = s_mlo[lc * NT + tid] & 0xFFFFFu;
+                    last_cs_m = s_mlo[lc * NT + tid];
                 }
                 open = last_is_cs;
                 if (open) { rs = last_cs; rm = last_cs_m; }
@@ -1179,64 +1187,96 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
         loc_kmers += __shfl_down_sync(0xffffffffu, loc_kmers, o);
         loc_recs += __shfl_down_sync(0xffffffffu, loc_recs, o);
         loc_runs += __shfl_down_sync(0xffffffffu, loc_runs, o);
+        loc_extra += __shfl_down_sync(0xffffffffu, loc_extra, o);
     }
     if (lane == 0) {
         if (loc_kmers) atomicAdd(&P.stats[0], loc_kmers);
         if (loc_recs) atomicAdd(&P.stats[1], loc_recs);
         if (loc_runs) atomicAdd(&P.stats[2], loc_runs);
+        if (loc_extra) atomicAdd(&P.stats[3], (unsigned long long)loc_extra);
     }
 }
 
 // ---------------------------------------------------------------- offsets
-// Exclusive scan of two u32 arrays of length n into u64 outputs, one CTA per
-// SCAN_ITEMS items, then a fix-up with the scanned block sums.
-constexpr int SCAN_T = 1024, SCAN_ITEMS = 8192;
+// Exclusive scan of n counts in two launches: the sums of blocks of SCAN_ITEMS
+// counts, then every block again, from the sum of the blocks before it (added up
+// by the block itself). A bin count holds k-mers and packed records (see
+// CutParams::binhist), scanned side by side.
+constexpr int SCAN_T = 512, SCAN_ITEMS = 4096;
 
-__global__ void k_scan_blocks(const uint32_t* __restrict__ in, uint64_t n, unsigned long long* __restrict__ out,
-                              unsigned long long* __restrict__ block_sums) {
-    __shared__ unsigned long long s[SCAN_T];
-    const uint64_t b0 = (uint64_t)blockIdx.x * SCAN_ITEMS;
-    constexpr int PER = SCAN_ITEMS / SCAN_T;
-    unsigned long long v[PER], acc = 0;
+struct ScanPair {
+    unsigned long long a, b;
+};
+__device__ __forceinline__ ScanPair scan_item(unsigned long long x) { return ScanPair{x & 0xFFFFFFFFull, x >> 32}; }
+__device__ __forceinline__ ScanPair scan_item(uint32_t x) { return ScanPair{x, 0}; }
+
+// sum of v over the block (the same in every thread)
+__device__ __forceinline__ ScanPair scan_block_sum(ScanPair v, ScanPair* s_w) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const uint64_t idx = b0 + (uint64_t)threadIdx.x * PER + i;
-        v[i] = idx < n ? in[idx] : 0;
-        acc += v[i];
+    for (int o = 16; o > 0; o >>= 1) {
+        v.a += __shfl_xor_sync(0xffffffffu, v.a, o);
+        v.b += __shfl_xor_sync(0xffffffffu, v.b, o);
     }
-    s[threadIdx.x] = acc;
     __syncthreads();
-    for (int o = 1; o < SCAN_T; o <<= 1) {
-        const unsigned long long y = threadIdx.x >= o ? s[threadIdx.x - o] : 0;
-        __syncthreads();
-        s[threadIdx.x] += y;
-        __syncthreads();
-    }
-    unsigned long long run = s[threadIdx.x] - acc;
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const uint64_t idx = b0 + (uint64_t)threadIdx.x * PER + i;
-        if (idx < n) out[idx] = run;
-        run += v[i];
-    }
-    if (threadIdx.x == SCAN_T - 1) block_sums[blockIdx.x] = s[SCAN_T - 1];
+    if (lane == 0) s_w[wid] = v;
+    __syncthreads();
+    ScanPair r{0, 0};
+    for (int i = 0; i < SCAN_T / 32; ++i) { r.a += s_w[i].a; r.b += s_w[i].b; }
+    return r;
 }
 
-__global__ void k_scan_sums(unsigned long long* __restrict__ sums, uint32_t nb, unsigned long long* __restrict__ total) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        unsigned long long acc = 0;
-        for (uint32_t i = 0; i < nb; ++i) {
-            const unsigned long long v = sums[i];
-            sums[i] = acc;
-            acc += v;
+template <typename T>
+__global__ void __launch_bounds__(SCAN_T) k_scan_sums(const T* __restrict__ in, uint64_t n, ScanPair* __restrict__ sums) {
+    __shared__ ScanPair s_w[SCAN_T / 32];
+    const uint64_t b0 = (uint64_t)blockIdx.x * SCAN_ITEMS;
+    ScanPair acc{0, 0};
+    for (uint32_t i = threadIdx.x; i < SCAN_ITEMS; i += SCAN_T)
+        if (b0 + i < n) {
+            const ScanPair x = scan_item(in[b0 + i]);
+            acc.a += x.a;
+            acc.b += x.b;
         }
-        *total = acc;
-    }
+    const ScanPair t = scan_block_sum(acc, s_w);
+    if (threadIdx.x == 0) sums[blockIdx.x] = t;
 }
 
-__global__ void k_scan_add(unsigned long long* __restrict__ out, uint64_t n, const unsigned long long* __restrict__ sums) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] += sums[i / SCAN_ITEMS];
+template <typename T>
+__global__ void __launch_bounds__(SCAN_T) k_scan(const T* __restrict__ in, uint64_t n, const ScanPair* __restrict__ sums,
+                                                 unsigned long long* __restrict__ oa, unsigned long long* __restrict__ ob,
+                                                 unsigned long long* __restrict__ total) {
+    __shared__ ScanPair s_w[SCAN_T / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    ScanPair run{0, 0};
+    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += SCAN_T) { run.a += sums[i].a; run.b += sums[i].b; }
+    run = scan_block_sum(run, s_w);
+    const uint64_t b0 = (uint64_t)blockIdx.x * SCAN_ITEMS;
+    for (uint32_t i0 = 0; i0 < SCAN_ITEMS && b0 + i0 < n; i0 += SCAN_T) {
+        const uint64_t i = b0 + i0 + threadIdx.x;
+        const ScanPair v = i < n ? scan_item(in[i]) : ScanPair{0, 0};
+        ScanPair x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long ya = __shfl_up_sync(0xffffffffu, x.a, o), yb = __shfl_up_sync(0xffffffffu, x.b, o);
+            if (lane >= o) { x.a += ya; x.b += yb; }
+        }
+        __syncthreads();
+        if (lane == 31) s_w[wid] = x;
+        __syncthreads();
+        for (int w = 0; w < SCAN_T / 32; ++w) {
+            if (w < wid) { x.a += s_w[w].a; x.b += s_w[w].b; }
+        }
+        if (i < n) {
+            oa[i] = run.a + x.a - v.a;
+            if (ob) ob[i] = run.b + x.b - v.b;
+            if (i + 1 == n) {
+                oa[n] = run.a + x.a;
+                if (total) *total = run.a + x.a;
+                if (ob) ob[n] = run.b + x.b;
+            }
+        }
+        for (int w = 0; w < SCAN_T / 32; ++w) { run.a += s_w[w].a; run.b += s_w[w].b; }
+    }
 }
 
 // ---------------------------------------------------------------- launchers
@@ -1333,15 +1373,30 @@ cudaError_t launch_cut(const CutParams& P, const HashTables* gT, bool exp, cudaS
     }
 }
 
-cudaError_t launch_scan(const uint32_t* in, uint64_t n, unsigned long long* out, unsigned long long* sums,
-                        unsigned long long* total, cudaStream_t st, int* launches) {
-    const uint32_t nb = (uint32_t)((n + SCAN_ITEMS - 1) / SCAN_ITEMS);
-    k_scan_blocks<<<nb, SCAN_T, 0, st>>>(in, n, out, sums);
-    k_scan_sums<<<1, 32, 0, st>>>(sums, nb, total);
-    k_scan_add<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, n, sums);
-    *launches += 3;
+uint64_t scan_scratch(uint64_t n) { return 2 * ((n + SCAN_ITEMS - 1) / SCAN_ITEMS + 1); }
+
+template <typename T>
+static cudaError_t scan_any(const T* in, uint64_t n, unsigned long long* oa, unsigned long long* ob,
+                            unsigned long long* total, unsigned long long* scratch, cudaStream_t st, int* launches) {
+    const uint32_t nb = (uint32_t)std::max<uint64_t>(1, (n + SCAN_ITEMS - 1) / SCAN_ITEMS);
+    ScanPair* sums = reinterpret_cast<ScanPair*>(scratch);
+    if (nb > 1) {
+        k_scan_sums<T><<<nb, SCAN_T, 0, st>>>(in, n, sums);
+        ++*launches;
+    }
+    k_scan<T><<<nb, SCAN_T, 0, st>>>(in, n, sums, oa, ob, total);
+    ++*launches;
     return cudaGetLastError();
 }
 
+cudaError_t launch_scan(const uint32_t* in, uint64_t n, unsigned long long* out, unsigned long long* scratch,
+                        cudaStream_t st, int* launches, unsigned long long* total) {
+    return scan_any(in, n, out, nullptr, total, scratch, st, launches);
+}
+
+cudaError_t launch_bin_scan(const unsigned long long* hist, uint64_t n, unsigned long long* kofs,
+                            unsigned long long* rofs, unsigned long long* scratch, cudaStream_t st, int* launches) {
+    return scan_any(hist, n, kofs, rofs, nullptr, scratch, st, launches);
+}
 
 }  // namespace tg

@@ -2,9 +2,8 @@
 // every bucket record, ci/cx filter and compaction of the surviving pairs.
 //
 // Reference behaviour (paths relative to the reference project root):
-//   every k-mer of a record       src/count.hpp:71-175 (the reference rolls through
-//                                 the record's packed bases; here each k-mer is read
-//                                 straight from the packed stream)
+//   every k-mer of a record       src/count.hpp:71-175 (rolled through the record's
+//                                 packed bases, one record per thread)
 //   canonical form                include/kache-hash/Kmer.hpp:446-456, :629-646
 //                                 (min of k-mer and reverse complement, word order)
 //   count += 1 per instance       src/count.hpp:81, Streaming_Kmer_Hash_Table::upsert
@@ -13,15 +12,14 @@
 // Pipeline (all instances of a canonical k-mer share its minimizer, hence its
 // bin: the sample's first bin + minimizer hash bits; phase 1 counted the k-mer
 // instances of every bin):
-//   k_scan_*    bin counts -> key offsets
+//   k_scan*     bin counts -> k-mer and record offsets
 //   k_plan      per segment (a run of bins of one sample): groups of whole bins
 //               of at most `target` k-mers
-//   k_keys      every k-mer's canonical key, written at its group's cursor, so
-//               the keys of a group are one contiguous range of the key array
-//   k_count     persistent, one CTA per SM: each group's keys are read with
-//               coalesced loads (the next round's already in flight while one
-//               is counted) into a shared-memory open-addressing table, then
-//               filtered and compacted.
+//   k_recs      every record with its bases at its group's cursor, so the records
+//               of a group are one contiguous range
+//   k_count     persistent: each group's records are read with coalesced loads
+//               and unpacked into canonical keys in shared memory, counted in an
+//               open-addressing table there, then filtered and compacted.
 //               A group with more distinct keys than the table holds comes back
 //               as key-hash parts in the next launch (as many as its distinct
 //               keys need, estimated); past MAX_PARTS parts it goes to the
@@ -33,14 +31,12 @@
 
 namespace tg {
 
-constexpr int P2_THREADS = 1024;         // threads of the phase-2 CTAs
-constexpr int COUNT_THREADS = 1024;      // threads of a k_count CTA
-constexpr int COUNT_PER_SM = 1;          // one CTA per SM: the largest table, the largest groups
-constexpr uint32_t PROBE_LIMIT = 128;    // linear-probe steps before a group is split
-constexpr uint32_t MAX_PARTS = 64;       // key-hash parts of one range before the global table
-constexpr uint32_t SLICE_DESC = 65536;   // descriptors per slice
-constexpr int KEYS_UNROLL = 4;           // k-mers per lane in flight in k_keys
+constexpr int COUNT_THREADS = 512;       // threads of a k_count CTA
+constexpr int COUNT_PER_SM = 2;          // CTAs per SM: one counts while the other waits at a barrier
+constexpr uint32_t MAX_PARTS = 128;      // key-hash parts of one range before the global table
 constexpr uint64_t FALLBACK_CAP = 4096;
+constexpr uint32_t BIG_KEYS = 1u << 16;  // k-mers above which many CTAs share a group (k_big)
+constexpr uint32_t BIG_CHUNK = 4096;     // packed records of such a group that a CTA takes at a time
 
 struct __align__(16) U128 {
     unsigned long long lo, hi;
@@ -88,89 +84,160 @@ __device__ __forceinline__ uint32_t key_part(const typename KeyOps<W>::Key& key,
     return (uint32_t)(KeyOps<W>::hash(key) >> 8) & (parts - 1);
 }
 
-// Insert one k-mer instance: count += 1. False if `limit` slots were taken.
+// Insert n instances of one k-mer: count += n. False if `limit` slots were taken.
 // 64-bit keys are probed with a plain load and claimed with a CAS. A 128-bit
 // key cannot be read in one single-copy-atomic load, and a read torn against a
 // concurrent claim could skip the slot that holds the same k-mer, so 128-bit
 // slots are probed with the CAS itself: it returns the whole current key.
 template <int W>
 __device__ __forceinline__ bool tbl_add(typename KeyOps<W>::Key* keys, uint32_t* cnt, uint32_t mask,
-                                        const typename KeyOps<W>::Key& key, uint32_t limit) {
+                                        const typename KeyOps<W>::Key& key, uint32_t n, uint32_t limit) {
     using O = KeyOps<W>;
     uint32_t h = (uint32_t)(O::hash(key) >> 32) & mask;
     for (uint32_t p = 0; p < limit; ++p) {
         if constexpr (W == 1) {
             const typename O::Key cur = O::load(&keys[h]);
-            if (O::eq(cur, key)) { atomicAdd(&cnt[h], 1u); return true; }
+            if (O::eq(cur, key)) { atomicAdd(&cnt[h], n); return true; }
             if (O::is_empty(cur)) {
                 const typename O::Key prev = O::cas(&keys[h], O::empty(), key);
-                if (O::is_empty(prev) || O::eq(prev, key)) { atomicAdd(&cnt[h], 1u); return true; }
+                if (O::is_empty(prev) || O::eq(prev, key)) { atomicAdd(&cnt[h], n); return true; }
             }
         } else {
             const typename O::Key prev = O::cas(&keys[h], O::empty(), key);
-            if (O::is_empty(prev) || O::eq(prev, key)) { atomicAdd(&cnt[h], 1u); return true; }
+            if (O::is_empty(prev) || O::eq(prev, key)) { atomicAdd(&cnt[h], n); return true; }
         }
         h = (h + 1) & mask;
     }
     return false;
 }
 
-// Canonical key of the k-mer starting at stream position s (bases read from
-// the packed array; array index = s + TG_PAD).
+// ---------------------------------------------------------------- packed records
 template <int W>
-__device__ __forceinline__ typename KeyOps<W>::Key kmer_key(const uint32_t* __restrict__ pk, uint64_t s, int k);
-
-template <>
-__device__ __forceinline__ unsigned long long kmer_key<1>(const uint32_t* __restrict__ pk, uint64_t s, int k) {
-    const uint64_t a = s + TG_PAD;
-    const uint64_t w = a >> 4;
-    const uint32_t o = (uint32_t)(a & 15);
-    const uint64_t hi = ((uint64_t)__ldg(pk + w) << 32) | __ldg(pk + w + 1);
-    const uint64_t win = o ? (hi << (2 * o)) | (__ldg(pk + w + 2) >> (32 - 2 * o)) : hi;
-    const uint64_t f = win >> (64 - 2 * k);
-    const uint64_t r = revcomp64(f, k);
-    return f < r ? f : r;
+struct Rec {
+    unsigned long long w[2 * W];
+    __device__ __forceinline__ uint32_t n() const { return (uint32_t)w[2 * W - 1] & 63u; }
+};
+template <int W>
+__device__ __forceinline__ Rec<W> load_rec(const void* recs, unsigned long long i) {
+    const ulonglong2* p = static_cast<const ulonglong2*>(recs) + i * W;
+    Rec<W> r;
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+        const ulonglong2 v = __ldg(p + j);
+        r.w[2 * j] = v.x;
+        r.w[2 * j + 1] = v.y;
+    }
+    return r;
 }
 
+// The k-mers of a packed record one after the other: the k-mer, its reverse
+// complement and the bases still to come (at most REC_MAX - 1), shifted by one
+// base per step.
+template <int W>
+struct Roll;
+
 template <>
-__device__ __forceinline__ U128 kmer_key<2>(const uint32_t* __restrict__ pk, uint64_t s, int k) {
-    const uint64_t a = s + TG_PAD;
-    const uint64_t w = a >> 4;
-    const uint32_t o = (uint32_t)(a & 15);
-    const uint32_t x0 = __ldg(pk + w), x1 = __ldg(pk + w + 1), x2 = __ldg(pk + w + 2), x3 = __ldg(pk + w + 3),
-                   x4 = __ldg(pk + w + 4);
-    uint64_t w01 = ((uint64_t)x0 << 32) | x1, w23 = ((uint64_t)x2 << 32) | x3;
-    if (o) {
-        w01 = (w01 << (2 * o)) | (x2 >> (32 - 2 * o));
-        w23 = (w23 << (2 * o)) | (x4 >> (32 - 2 * o));
+struct Roll<1> {
+    uint32_t f0, f1;  // the k-mer, low word first
+    uint32_t r0, r1;  // its reverse complement, left-aligned
+    uint32_t x;       // the bases to come, left-aligned
+    __device__ __forceinline__ void start(const Rec<1>& c, int k) {
+        const unsigned long long f = c.w[0] >> (64 - 2 * k), r = revcomp64(f, k) << (64 - 2 * k);
+        f0 = (uint32_t)f;
+        f1 = (uint32_t)(f >> 32);
+        r0 = (uint32_t)r;
+        r1 = (uint32_t)(r >> 32);
+        x = (uint32_t)(((c.w[0] << (2 * k)) | (c.w[1] >> (64 - 2 * k))) >> 32);
     }
-    const int sh = 128 - 2 * k;  // 2..64
-    K2 f;
-    if (sh >= 64) { f.lo = w01 >> (sh - 64); f.hi = 0; }
-    else { f.lo = (w23 >> sh) | (w01 << (64 - sh)); f.hi = w01 >> sh; }
-    const K2 r = revcomp128(f, k);
-    const K2& c = k2_less(f, r) ? f : r;
-    U128 key;
-    key.lo = c.lo;
-    key.hi = c.hi;
-    return key;
+    __device__ __forceinline__ unsigned long long key(int k) const {
+        const unsigned long long f = ((unsigned long long)f1 << 32) | f0;
+        const unsigned long long r = (((unsigned long long)r1 << 32) | r0) >> (64 - 2 * k);
+        return f < r ? f : r;
+    }
+    __device__ __forceinline__ void step(int k) {
+        const unsigned long long mask = ~0ull >> (64 - 2 * k);
+        f1 = __funnelshift_l(f0, f1, 2) & (uint32_t)(mask >> 32);
+        f0 = __funnelshift_l(x, f0, 2) & (uint32_t)mask;
+        r0 = __funnelshift_r(r0, r1, 2);
+        r1 = (r1 >> 2) | (~x & 0xC0000000u);
+        x <<= 2;
+    }
+};
+
+template <>
+struct Roll<2> {
+    K2 f, r;
+    uint32_t x;
+    __device__ __forceinline__ void start(const Rec<2>& c, int k) {
+        const int sh = 128 - 2 * k;  // 2..64
+        if (sh >= 64) { f.lo = c.w[0]; f.hi = 0; }
+        else { f.lo = (c.w[1] >> sh) | (c.w[0] << (64 - sh)); f.hi = c.w[0] >> sh; }
+        r = revcomp128(f, k);
+        const int s = 2 * k - 64;    // 0..62
+        x = (uint32_t)((s ? (c.w[1] << s) | (c.w[2] >> (64 - s)) : c.w[1]) >> 32);
+    }
+    __device__ __forceinline__ U128 key(int) const {
+        const bool l = k2_less(f, r);
+        U128 q;
+        q.lo = l ? f.lo : r.lo;
+        q.hi = l ? f.hi : r.hi;
+        return q;
+    }
+    __device__ __forceinline__ void step(int k) {
+        const uint32_t b = x >> 30;
+        x <<= 2;
+        f.hi = (f.hi << 2) | (f.lo >> 62);
+        if (2 * k > 64) f.hi &= ~0ull >> (128 - 2 * k);
+        else f.hi = 0;
+        f.lo = (f.lo << 2) | b;
+        r.lo = (r.lo >> 2) | (r.hi << 62);
+        r.hi >>= 2;
+        if (k == 32) r.lo |= (unsigned long long)(3u - b) << 62;
+        else r.hi |= (unsigned long long)(3u - b) << (2 * k - 66);
+    }
+};
+
+__device__ __forceinline__ uint32_t rec_hash(const Rec<1>& r) {
+    return (uint32_t)r.w[0] * 0x9E3779B1u + (uint32_t)(r.w[0] >> 32) * 0x85EBCA77u +
+           ((uint32_t)r.w[1] + (uint32_t)(r.w[1] >> 32)) * 0xC2B2AE3Du;
+}
+__device__ __forceinline__ uint32_t rec_hash(const Rec<2>& r) {
+    return (uint32_t)r.w[0] * 0x9E3779B1u + (uint32_t)(r.w[0] >> 32) * 0x85EBCA77u + (uint32_t)r.w[1] * 0xC2B2AE3Du +
+           (uint32_t)(r.w[1] >> 32) * 0x27D4EB2Fu + ((uint32_t)r.w[2] ^ (uint32_t)r.w[3]) * 0x165667B1u +
+           (uint32_t)(r.w[2] >> 32) * 0x9E3779B1u;
+}
+template <int W>
+__device__ __forceinline__ bool rec_equal(const Rec<W>& a, const Rec<W>& b) {
+    bool e = true;
+#pragma unroll
+    for (int j = 0; j < 2 * W; ++j) e = e && a.w[j] == b.w[j];
+    return e;
 }
 
 // ---------------------------------------------------------------- k_plan
-// One warp per segment (a run of consecutive bins of one sample): its groups,
-// from the scanned key offsets ko[bin]. Greedy, in bin order: a group starting
-// at bin s takes the most bins e - s with at most `target` keys (one bin if that
+// plan_split warps per segment (a run of consecutive bins of one sample), each
+// with an equal share of its bins: the share's groups,
+// from the scanned k-mer offsets ko[bin]. Greedy, in bin order: a group starting
+// at bin s takes the most bins e - s with at most `target` k-mers (one bin if that
 // bin alone is larger; such a group is listed as heavy). Each step is one
 // upper-bound search over ko, done by the warp as a 32-way search. Every bin of
-// the group gets the group's first bin in gfirst: k_keys appends all of the
-// group's keys at that bin's cursor.
+// the group gets the group's first bin in gfirst: k_recs appends all of the
+// group's records at that bin's cursor.
 constexpr int PLAN_THREADS = 256;
 
 __global__ void __launch_bounds__(PLAN_THREADS) k_plan(KeysParams P) {
     const int lane = threadIdx.x & 31;
-    const uint32_t sg = blockIdx.x * (PLAN_THREADS / 32) + (threadIdx.x >> 5);
+    const uint32_t wi = blockIdx.x * (PLAN_THREADS / 32) + (threadIdx.x >> 5);
+    const uint32_t sg = wi / P.plan_split, part = wi % P.plan_split;
     if (sg >= P.n_segs) return;  // warp-uniform
-    const Segment seg = P.segs[sg];
+    Segment seg = P.segs[sg];
+    {
+        const uint32_t per = (seg.bin_hi - seg.bin_lo + P.plan_split - 1) / P.plan_split;
+        const uint32_t hi = seg.bin_hi;
+        seg.bin_lo = min(hi, seg.bin_lo + part * per);
+        seg.bin_hi = min(hi, seg.bin_lo + per);
+        if (seg.bin_lo == seg.bin_hi) return;
+    }
     const uint32_t nb = seg.bin_hi - seg.bin_lo;
     const unsigned long long* ko = P.kofs + seg.bin_lo;
     const unsigned long long end = ko[nb];
@@ -195,17 +262,17 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(KeysParams P) {
         const uint32_t e = lo;
         const unsigned long long ke = ko[e];
         for (uint32_t b = s + (uint32_t)lane; b < e; b += 32) P.gfirst[seg.bin_lo + b] = seg.bin_lo + s;
-        if (lane == 0) {
-            const int heavy = ke - ks > T ? 1 : 0;
-            const unsigned long long q = atomicAdd(&P.ctr[heavy ? P2C_HEAVY : P2C_NORMAL], 1ull);
+        if (lane == 0 && ke > ks) {  // not the empty bins before a bin larger than the target
+            const int heavy = ke - ks > T ? (ke - ks > BIG_KEYS ? 2 : 1) : 0;
+            const unsigned long long q = atomicAdd(&P.ctr[heavy == 2 ? P2C_BIG : heavy ? P2C_HEAVY : P2C_NORMAL], 1ull);
             if (q < P.groups_cap) {
                 Group g;
-                g.lo = ks;
-                g.hi = ke;
+                g.lo = P.rofs[seg.bin_lo + s];
+                g.hi = P.rofs[seg.bin_lo + e];
                 g.parts = 1;
                 g.part = 0;
                 g.sample = seg.sample;
-                g.pad = 0;
+                g.keys = (uint32_t)(ke - ks);
                 P.groups[heavy][q] = g;
             }
         }
@@ -214,127 +281,81 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(KeysParams P) {
     }
 }
 
-// ---------------------------------------------------------------- k_keys
-// Every k-mer of a slice of the phase-1 descriptor lists (in stream order, so
-// the packed bases are read front to back): canonical key written at its
-// group's cursor (the cursor of the group's first bin, gfirst). A warp takes 32
-// descriptors at a time; each reserves its k-mers' places with one global
-// atomic on that cursor, then the warp's lanes take the batch's k-mers in order
-// (consecutive lanes, consecutive keys). Keys appended per group rather than
-// per bin: a group's keys are the same contiguous range, in another order
-// inside it, with about a third as many places being written at once (groups
-// of ~3 bins), so more of the partly written sectors are completed in L2.
-// The descriptors are loaded two batches ahead and the next batch's gfirst
-// entries one batch ahead, and each batch's atomic is issued before the
-// previous batch's keys are made (k_keys 19.8 -> 19.1 ms at 3.1 G keys).
-//
-// A run restricted to a range of bins (the passes of a job larger than the
-// memory budget) keeps only the records of those bins, moved to the front of
-// the warp's batch so that every active lane still holds one record.
+// ---------------------------------------------------------------- k_recs
+// Every record of the phase-1 descriptor lists (in stream order, so the packed
+// bases are read front to back) as packed records at its group's cursor (the
+// cursor of the group's first bin, gfirst), one thread per descriptor: the place
+// from one global atomic, the bases from an unaligned window of the packed
+// words. Four descriptors per thread in flight; the loads of a descriptor, its
+// group, its place and its bases depend on one another and nothing else bounds
+// the kernel but the scattered 16-byte writes.
+constexpr int RECS_THREADS = 256, RECS_UNROLL = 4, RECS_PER_CTA = 2 * RECS_UNROLL * RECS_THREADS;
+
+// The packed record of the nk k-mers from stream position s on.
 template <int W>
-__global__ void __launch_bounds__(P2_THREADS) k_keys(KeysParams P) {
-    using O = KeyOps<W>;
-    __shared__ uint64_t s_keep[P2_THREADS];
-    __shared__ uint32_t s_keepg[P2_THREADS];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const Slice sl = P.slices[blockIdx.x];
-    const uint64_t* d = P.desc + sl.r_lo;
-    const uint32_t n = (uint32_t)(sl.r_hi - sl.r_lo);
-    const int k = P.k;
-    const bool filt = P.bin_lo != 0 || P.bin_hi != (1u << BIN_BITS);
-    auto load_desc = [&](uint32_t i) -> uint64_t { return i < n ? d[i] : 0; };
-    // gfirst of a descriptor's bin (any bin of a descriptor is below 2^20;
-    // bins outside this run's range are read but not used)
-    auto group_of = [&](uint64_t dv) -> uint32_t { return desc_nk(dv) ? P.gfirst[desc_bin(dv)] : 0u; };
-    const uint32_t b0 = (uint32_t)wid * 32 + lane;
-    uint64_t dnext = load_desc(b0);                 // batch i + 1 (loaded)
-    uint32_t gnext = group_of(dnext);
-    uint64_t dnext2 = load_desc(b0 + P2_THREADS);   // batch i + 2 (in flight)
-    // A batch is prepared (restricted to this run's bins, moved to the front of
-    // the warp; its places reserved by the atomic) one batch ahead: the atomic's
-    // round trip overlaps the previous batch's keys.
-    auto prepare = [&](uint64_t& dv, uint32_t gv, unsigned long long& koff) {
-        koff = 0;
-        if (filt) {
-            const uint32_t b = desc_bin(dv);
-            const bool keep = desc_nk(dv) && b >= P.bin_lo && b < P.bin_hi;
-            const unsigned m = __ballot_sync(0xffffffffu, keep);
-            if (keep) {
-                const uint32_t j = wid * 32 + __popc(m & ((1u << lane) - 1u));
-                s_keep[j] = dv;
-                s_keepg[j] = gv;
-            }
-            __syncwarp();
-            dv = lane < __popc(m) ? s_keep[wid * 32 + lane] : 0;
-            gv = lane < __popc(m) ? s_keepg[wid * 32 + lane] : 0;
-            __syncwarp();
-        }
-        const uint32_t nk = desc_nk(dv);  // 0 past the slice; at least 1 otherwise
-        if (nk) koff = atomicAdd(&P.kofs[gv], (unsigned long long)nk);
-    };
-    uint64_t cdv = dnext;
-    unsigned long long ckoff;
-    {
-        const uint32_t cg = gnext;
-        dnext = dnext2;
-        gnext = group_of(dnext);
-        dnext2 = load_desc(b0 + 2 * P2_THREADS);
-        prepare(cdv, cg, ckoff);
+__device__ __forceinline__ void store_rec(const KeysParams& P, unsigned long long at, uint64_t s, uint32_t nk) {
+    const int bits = 2 * (P.k + (int)nk - 1);
+    const uint64_t a = s + TG_PAD;
+    const uint32_t* p = P.packed + (a >> 4);
+    const uint32_t sh = 2 * (uint32_t)(a & 15);
+    uint32_t x[4 * W + 1], y[4 * W];
+#pragma unroll
+    for (int i = 0; i <= 4 * W; ++i) x[i] = __ldg(p + i);
+#pragma unroll
+    for (int i = 0; i < 4 * W; ++i) {  // the record's bases alone: equal records are equal words
+        y[i] = __funnelshift_l(x[i + 1], x[i], sh);
+        const int v = bits - 32 * i;
+        if (v < 32) y[i] &= v > 0 ? ~(0xFFFFFFFFu >> v) : 0u;
     }
-    for (uint32_t base = (uint32_t)wid * 32; base < n; base += P2_THREADS) {
-        uint64_t ndv = dnext;
-        unsigned long long nkoff;
-        {
-            const uint32_t ng = gnext;
-            dnext = dnext2;
-            gnext = group_of(dnext);
-            dnext2 = load_desc(base + 3 * P2_THREADS + lane);
-            prepare(ndv, ng, nkoff);
-        }
-        const uint64_t dv = cdv;
-        const unsigned long long koff = ckoff;
-        cdv = ndv;
-        ckoff = nkoff;
-        const uint32_t nk = desc_nk(dv);
-        uint32_t incl = nk;
+    y[4 * W - 1] |= nk;
+    ulonglong2* d = static_cast<ulonglong2*>(P.recs) + at * W;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const uint32_t excl = incl - nk;
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        // k-mer t of the batch belongs to lane o: stream position srcb_o + t,
-        // key index dstb_o + t
-        const uint64_t srcb = desc_start(dv) - excl;
-        const uint64_t dstb = koff - excl;
-        for (uint32_t t0 = 0; t0 < total; t0 += 32 * KEYS_UNROLL) {
-            typename O::Key kv[KEYS_UNROLL];
-            uint64_t dst[KEYS_UNROLL];
-            bool act[KEYS_UNROLL];
+    for (int j = 0; j < W; ++j)
+        d[j] = make_ulonglong2(((unsigned long long)y[4 * j] << 32) | y[4 * j + 1],
+                               ((unsigned long long)y[4 * j + 2] << 32) | y[4 * j + 3]);
+}
+
+template <int W>
+__global__ void __launch_bounds__(RECS_THREADS) k_recs(KeysParams P) {
+    const uint32_t n = P.n_desc ? (uint32_t)min((uint64_t)P.n_desc[blockIdx.y], P.desc_cap) : P.n_one;
+    const uint64_t* d = P.desc + (uint64_t)blockIdx.y * P.desc_cap;
+    const int sb = P.desc_sb;
+    const uint64_t i0 = (uint64_t)blockIdx.x * RECS_PER_CTA;
 #pragma unroll
-            for (int u = 0; u < KEYS_UNROLL; ++u) {
-                const uint32_t r0 = t0 + 32 * u;  // warp-uniform
-                act[u] = false;
-                if (r0 >= total) continue;
-                // owner of k-mer r0 + l = (lanes starting before r0) + (starts in
-                // [r0, r0 + l]) - 1; starts are distinct since every nk >= 1
-                const uint32_t rel = excl - r0;
-                const unsigned starts = __reduce_or_sync(0xffffffffu, (nk && rel < 32) ? 1u << rel : 0u);
-                const unsigned before = __popc(__ballot_sync(0xffffffffu, excl < r0));
-                const uint32_t own = (before + __popc(starts & ((2u << lane) - 1u)) - 1u) & 31u;
-                const uint64_t sb = __shfl_sync(0xffffffffu, srcb, own);
-                const uint64_t db = __shfl_sync(0xffffffffu, dstb, own);
-                const uint32_t t = r0 + lane;
-                act[u] = t < total;
-                if (act[u]) {
-                    kv[u] = kmer_key<W>(P.packed, sb + t, k);
-                    dst[u] = db + t;
-                }
+    for (int b = 0; b < RECS_PER_CTA; b += RECS_UNROLL * RECS_THREADS) {
+        if (i0 + b >= n) return;
+        uint64_t dv[RECS_UNROLL];
+        uint32_t g[RECS_UNROLL];
+        unsigned long long at[RECS_UNROLL];
+#pragma unroll
+        for (int u = 0; u < RECS_UNROLL; ++u) {
+            const uint64_t i = i0 + b + u * RECS_THREADS + threadIdx.x;
+            dv[u] = i < n ? __ldcs(d + i) : 0;
+            const uint32_t bin = desc_bin(dv[u], sb);
+            if (bin < P.bin_lo || bin >= P.bin_hi) dv[u] = 0;  // not this run's: no k-mers
+        }
+#pragma unroll
+        for (int u = 0; u < RECS_UNROLL; ++u)
+            if (desc_nk(dv[u], sb)) g[u] = P.gfirst[desc_bin(dv[u], sb)];
+#pragma unroll
+        for (int u = 0; u < RECS_UNROLL; ++u) {
+            const uint32_t nk = desc_nk(dv[u], sb);
+            if (nk) at[u] = atomicAdd(&P.rofs[g[u]], (unsigned long long)rec_pieces(nk));
+        }
+#pragma unroll
+        for (int u = 0; u < RECS_UNROLL; ++u) {
+            const uint32_t nk = desc_nk(dv[u], sb);
+            const uint64_t s = desc_start(dv[u], sb);
+            if (!nk) continue;
+            if (nk <= REC_MAX) {
+                store_rec<W>(P, at[u], s, nk);
+                continue;
             }
-#pragma unroll
-            for (int u = 0; u < KEYS_UNROLL; ++u)
-                if (act[u]) O::store(P.keys, dst[u], kv[u]);
+            const uint32_t pieces = rec_pieces(nk), per = (nk + pieces - 1) / pieces;
+            for (uint32_t q = 0; q < pieces; ++q) {
+                const uint32_t o = min(q * per, nk);
+                store_rec<W>(P, at[u] + q, s + o, min(per, nk - o));
+            }
         }
     }
 }
@@ -344,94 +365,14 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// A slot's count in shared memory is its key's occurrences after the first:
-// the thread that claims a slot adds nothing (its key counts through the claim),
-// later occurrences add 1, and the output count is the stored value + 1. Most
-// keys of a group occur once, so most keys take one shared atomic (the CAS),
-// not two.
-//
-// 128-bit keys: slots probed in order from the home slot h with the CAS itself
-// (a 128-bit key cannot be read in one single-copy-atomic load, and a torn
-// read could skip the slot that holds the same k-mer). Returns 1 for a new key,
-// 0 for a known one, -1 after PROBE_LIMIT slots.
-__device__ __forceinline__ int claim_cas(U128* keys, uint32_t* cnt, uint32_t mask, const U128& key, uint32_t h,
-                                         uint32_t& slot) {
-    using O = KeyOps<2>;
-    for (uint32_t p = 0; p < PROBE_LIMIT; ++p) {
-        const U128 prev = O::cas(&keys[h], O::empty(), key);
-        if (O::is_empty(prev)) { slot = h; return 1; }
-        if (O::eq(prev, key)) { atomicAdd(&cnt[h], 1u); return 0; }
-        h = (h + 1) & mask;
-    }
-    return -1;
-}
-
-// The 64-bit table as buckets of 4 slots (32 bytes). A key's probe order is
-// fixed: its home slot, then the slots of its home bucket (which holds the home
-// slot) in order, then the next bucket's, and so on; a key takes the first slot
-// of that order that is empty when it comes, and slots are never emptied during
-// a group, so two inserts of one key meet in the same slot. After the home slot
-// one probe reads a whole bucket (two 16-byte loads; each 8-byte slot is read
-// atomically). If the key
-// is in the bucket, it is counted there (a slot once taken keeps its key);
-// otherwise the first empty slot is claimed by CAS, and a CAS lost to another
-// key re-reads the bucket. Returns 1 for a new key, 0 for a known one, -1 after
-// PROBE_BUCKETS buckets.
-constexpr uint32_t BUCKET = 4;
-constexpr uint32_t PROBE_BUCKETS = 32;
-
-__device__ __forceinline__ void lds_bucket(const unsigned long long* p, unsigned long long (&v)[BUCKET]) {
-    const uint32_t a = smem_addr(p);
-    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "r"(a));
-    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2+16];" : "=l"(v[2]), "=l"(v[3]) : "r"(a));
-}
-
-__device__ __forceinline__ int claim_bucket(unsigned long long* keys, uint32_t* cnt, uint32_t bmask,
-                                            unsigned long long key, uint32_t hs, uint32_t& slot) {
-    // the home slot first (one 8-byte load): in a table at most half full it is
-    // usually empty or holds the key (20 % less k_count time than reading the
-    // whole bucket first); the probe order goes on with the home bucket's slots
-    {
-        unsigned long long v0;
-        asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v0) : "r"(smem_addr(keys + hs)));
-        if (v0 == key) { atomicAdd(&cnt[hs], 1u); return 0; }
-        if (v0 == ~0ull) {
-            const unsigned long long prev = atomicCAS(&keys[hs], ~0ull, key);
-            if (prev == ~0ull) { slot = hs; return 1; }
-            if (prev == key) { atomicAdd(&cnt[hs], 1u); return 0; }
-        }
-    }
-    uint32_t b = hs / BUCKET;
-    for (uint32_t p = 0; p < PROBE_BUCKETS;) {
-        unsigned long long v[BUCKET];
-        lds_bucket(keys + b * BUCKET, v);
-        int hit = -1, emp = -1;
-#pragma unroll
-        for (int j = BUCKET - 1; j >= 0; --j) {
-            if (v[j] == key) hit = j;
-            if (v[j] == ~0ull) emp = j;
-        }
-        if (hit >= 0) { atomicAdd(&cnt[b * BUCKET + hit], 1u); return 0; }
-        if (emp < 0) { b = (b + 1) & bmask; ++p; continue; }
-        const unsigned long long prev = atomicCAS(&keys[b * BUCKET + emp], ~0ull, key);
-        if (prev == ~0ull) { slot = b * BUCKET + emp; return 1; }
-        if (prev == key) { atomicAdd(&cnt[b * BUCKET + emp], 1u); return 0; }
-        // the slot went to another key: read the bucket again
-    }
-    return -1;
-}
-
-// Asynchronous copy (cp.async, two 16-byte pieces) of group `gi` of the
-// launch's sequence (list 1 first, then list 0) into shared memory; an index
-// past the end gives an empty group.
-__device__ __forceinline__ void copy_group(Group* dst, const CountParams& P, unsigned long long gi,
-                                           unsigned long long n1, unsigned long long ntot) {
-    if (gi >= ntot) {
+// Asynchronous copy (cp.async, two 16-byte pieces) of group `gi` of the launch's
+// list into shared memory; an index past the end gives an empty group.
+__device__ __forceinline__ void copy_group(Group* dst, const CountParams& P, unsigned long long gi) {
+    if (gi >= P.g_end) {
         dst->lo = dst->hi = 0;
-        dst->parts = 0;
         return;
     }
-    const Group* src = gi < n1 ? P.list[1] + gi : P.list[0] + (gi - n1);
+    const Group* src = P.list + gi;
     const uint32_t d = smem_addr(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16),
@@ -440,278 +381,539 @@ __device__ __forceinline__ void copy_group(Group* dst, const CountParams& P, uns
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
+// Shape of the counting kernel for key width W. The table holds 32-bit entries,
+// not keys: an entry is the key's place in the CTA's key store (IDX_BITS) and a
+// fingerprint of the key (the rest); the store holds each key once, at that
+// place, with its count in a second array. So an insert is one 4-byte shared
+// CAS at a random slot, a full key is read at random only where the fingerprint
+// says that it is the same key, and the output walk reads keys and counts in
+// order. CAP keys fit in the store, COUNT_PER_SM CTAs in an SM's shared memory;
+// the table is at most a quarter (W = 1) or three eighths full, so that a warp's
+// longest probe stays short.
+template <int W>
+struct CountShape;
+template <>
+struct CountShape<1> {
+    static constexpr uint32_t SLOT_BITS = 14, CAP = 4096;
+};
+template <>
+struct CountShape<2> {
+    static constexpr uint32_t SLOT_BITS = 13, CAP = 3072;
+};
+constexpr int IDX_BITS = 13;                          // place in the key store
+constexpr uint32_t IDX_MASK = (1u << IDX_BITS) - 1;
+constexpr uint32_t DEDUP_MAX = 3;                     // records per thread among which equal ones are looked for
+constexpr uint32_t NO_ENTRY = 0xFFFFFFFFu;            // an empty slot; no entry has all bits set (CAP <= IDX_MASK)
+
 template <int W>
 struct CountSmem {
-    size_t keys, cnt, list, total;
-    __host__ __device__ void layout(uint32_t slots) {
-        size_t o = 0;
-        keys = o; o += KeyOps<W>::BYTES * (size_t)slots;
-        cnt = o; o += 4 * (size_t)slots;
-        list = o; o += 2 * (size_t)slots;  // slots claimed by the group, in claim order
-        total = (o + 15) & ~size_t(15);
-    }
+    using Key = typename KeyOps<W>::Key;
+    static constexpr uint32_t SLOTS = 1u << CountShape<W>::SLOT_BITS, CAP = CountShape<W>::CAP;
+    Key keys[CAP];
+    uint32_t table[SLOTS];
+    uint32_t cnt[CAP];          // occurrences after the first
+    Group grp[3];               // groups g, g + 1, g + 2
+    unsigned long long pending;
+    uint32_t staged;
+    uint32_t dedup, firsts;     // groups until equal records are looked for again; first ones found
+    static_assert(CAP <= IDX_MASK && CAP < SLOTS, "places and free slots");
 };
 
-// Persistent: COUNT_PER_SM CTAs per SM take groups in order (list 1, then list 0) from a
-// global counter. A group's keys are one contiguous range; they are inserted
-// in rounds of RK keys, thread t taking keys t, t + COUNT_THREADS, ... of a round,
-// and each thread's keys of the next round (or of the next group's first round)
-// are loaded into registers while it inserts the current ones, so there is no
-// barrier inside a group. Every slot a key claims goes onto a list in shared
-// memory (each round's new slots placed with one shared atomic per warp), so
-// after the group the threads walk the list, not the table: pair i of the group
-// is written to out[base + i] (coalesced) and its slot cleared. With ci/cx
-// limits the table is scanned instead and the kept pairs compacted by ballots.
-// A group with more distinct keys than 7/8 of the table (or a probe run past
-// the limit) comes back as F key-hash parts, F the power of two that gives
-// half-full tables for its distinct keys: known when the group ran to its end,
-// else estimated from the keys seen before the table filled. Halving at every
-// level instead re-read a heavy bin's keys once per level (all of k_count at
-// 3.1 G keys: 47.4 -> 41.9 ms). Group entries are fetched
-// two groups ahead (cp.async) into a ring of three. Groups are planned at half
-// the table (`target`): with the list the table's size no longer costs a scan,
-// and a half-full table has fewer collisions (measured: 0.7 -> 0.5 of the
-// table, 16.1 -> 14.0 ms for 0.93 G keys).
+// Home slot and entry of a key at place i: both the top bits of a multiply-add
+// hash. They share bits, so one in 32 keys that meet at a home slot are compared in
+// full without being equal; a second mixing step costs more than that.
+__device__ __forceinline__ uint32_t slot_hash(unsigned long long k) {
+    return (uint32_t)k * 0x9E3779B1u + (uint32_t)(k >> 32) * 0x85EBCA77u;
+}
+__device__ __forceinline__ uint32_t slot_hash(const U128& k) {
+    return slot_hash(k.lo) + (uint32_t)k.hi * 0xC2B2AE3Du + (uint32_t)(k.hi >> 32) * 0x27D4EB2Fu;
+}
 template <int W>
+__device__ __forceinline__ void place_of(uint32_t x, uint32_t i, uint32_t& h, uint32_t& entry) {
+    h = x >> (32 - CountShape<W>::SLOT_BITS);
+    entry = (x & ~IDX_MASK) | i;
+}
+
+// The slot probed after h for the key of `entry`: the stride is odd, so the
+// probe comes past every slot, and there are more slots than places, so it finds
+// a free one.
+template <int W>
+__device__ __forceinline__ uint32_t next_slot(uint32_t h, uint32_t entry) {
+    return (h + ((entry >> IDX_BITS) | 1u)) & (CountSmem<W>::SLOTS - 1);
+}
+
+template <int W>
+__device__ __forceinline__ void clear_table(CountSmem<W>& S) {
+    uint4* t4 = reinterpret_cast<uint4*>(S.table);
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < CountSmem<W>::SLOTS / 4; i += COUNT_THREADS)
+        t4[i] = make_uint4(NO_ENTRY, NO_ENTRY, NO_ENTRY, NO_ENTRY);
+}
+
+template <int W>
+__device__ __forceinline__ void start_store(CountSmem<W>& S) {
+    clear_table<W>(S);
+    for (uint32_t i = threadIdx.x; i < CountShape<W>::CAP; i += COUNT_THREADS) S.cnt[i] = 0;
+    if (threadIdx.x == 0) S.staged = S.dedup = S.firsts = 0;
+}
+
+// Writes the new keys of the first n places (bit u of newm: this thread's place
+// u * COUNT_THREADS + threadIdx.x holds one) that pass ci/cx to out, each warp's
+// next to each other, and empties the table and the counts. All threads call it
+// with the inserts done but for a barrier; after it, one barrier more and the
+// store may be filled again. Every warp reserves its own place in out, before the
+// barrier where it can, so that the atomic's round trip overlaps the wait there
+// (one atomic per CTA, between two barriers more, cost 0.2 of 1.3 ms for 0.15 G
+// distinct keys). behind() runs on every thread behind the barrier.
+template <int W, typename F>
+__device__ __forceinline__ void write_out(const CountParams& P, CountSmem<W>& S, uint32_t n, uint32_t newm,
+                                          uint32_t sample, uint32_t& distinct, F&& behind) {
+    using Key = typename KeyOps<W>::Key;
+    constexpr uint32_t UMAX = CountShape<W>::CAP / COUNT_THREADS;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    const bool filtered = P.ci > 1 || P.cx < 0xFFFFFFFFull;  // counts are at least 1 and fit in 32 bits
+    uint32_t wn = __reduce_add_sync(0xffffffffu, __popc(newm));
+    unsigned long long wb = 0;
+    distinct += wn;
+    if (!filtered && lane == 0 && wn) wb = atomicAdd(&P.ctr[P2C_OUT], (unsigned long long)wn);
+    __syncthreads();  // inserts done
+    behind();
+    clear_table<W>(S);
+    if (filtered) {
+        uint32_t keep = 0;
+        for (uint32_t u = 0; u < UMAX; ++u)
+            if ((newm >> u) & 1u) {
+                const uint32_t i = u * COUNT_THREADS + tid;
+                const uint64_t c = (uint64_t)S.cnt[i] + 1;
+                if (c >= P.ci && c <= P.cx) keep |= 1u << u;
+                else S.cnt[i] = 0;
+            }
+        newm = keep;
+        wn = __reduce_add_sync(0xffffffffu, __popc(newm));
+        if (lane == 0 && wn) wb = atomicAdd(&P.ctr[P2C_OUT], (unsigned long long)wn);
+    }
+    if (wn == 0) return;  // the whole warp
+    wb = __shfl_sync(0xffffffffu, wb, 0);
+    // every pair of the warp has room (the same for its lanes), or each is checked
+    const uint32_t room = wb + wn <= P.out_cap ? ~0u : (uint32_t)(wb < P.out_cap ? P.out_cap - wb : 0);
+    Key* okeys = static_cast<Key*>(P.out_keys) + wb;
+    uint32_t* ocnt = P.out_counts + wb;
+    uint32_t* osmp = P.out_sample ? P.out_sample + wb : nullptr;
+    uint32_t before = 0;
+    for (uint32_t u = 0; u * COUNT_THREADS < n; ++u) {
+        const uint32_t i = u * COUNT_THREADS + tid;
+        const bool kept = (newm >> u) & 1u;
+        const unsigned bal = __ballot_sync(0xffffffffu, kept);
+        const uint32_t o = before + __popc(bal & ((1u << lane) - 1));
+        before += __popc(bal);
+        if (kept) {
+            const uint32_t c = S.cnt[i];
+            if (o < room) {
+                okeys[o] = S.keys[i];
+                ocnt[o] = c + 1;
+                if (osmp) osmp[o] = sample;
+            }
+            if (c) S.cnt[i] = 0;
+        }
+    }
+}
+
+// Persistent: COUNT_PER_SM CTAs per SM take groups of at most CAP k-mers from a global
+// counter. A group's packed records are unpacked into the key store, a barrier, every
+// thread inserts the keys at places t, t + COUNT_THREADS, ... and notes which of them
+// are new, a barrier, and the new ones are written to out. The barrier between
+// unpacking and inserting makes every stored key readable, so a fingerprint match can
+// be checked against the store at once. Group entries are fetched two groups ahead
+// (cp.async) into a ring of three, a group's first records while the one before is
+// inserted.
 //
-// At most 56 registers per thread (no spills; 64 without the cap): 1,024 x 56
-// leaves 8,192 of the SM's registers, room for one CTA of the host-link copy
-// (tg_link.cu: 256 threads x 32 registers) beside each counting CTA, so the
-// copy of a wave's pairs to host memory runs while the next wave counts.
-__global__ void __maxnreg__(56) k_count(CountParams P) {
+// At most 56 registers per thread: 1,024 threads x 56 leave 8,192 of the SM's
+// registers, room for one CTA of the host-link copy (tg_link.cu: 256 threads x 32
+// registers) beside the counting CTAs, so the copy of a wave's pairs to host memory
+// runs while the next wave counts.
+template <int W>
+__global__ void __maxnreg__(56) k_count(const __grid_constant__ CountParams P) {
     using O = KeyOps<W>;
     using Key = typename O::Key;
-    constexpr int U = W == 1 ? 4 : 2;                 // keys per thread per round
-    constexpr uint32_t RK = U * COUNT_THREADS;           // keys per round
-    constexpr uint32_t SPT = W == 1 ? 16 : 8;         // table slots per thread
+    constexpr uint32_t CAP = CountShape<W>::CAP, SLOTS = CountSmem<W>::SLOTS;
+    constexpr uint32_t UMAX = CAP / COUNT_THREADS;           // places per thread
+    constexpr int U = 2;                                     // of them in flight
+    static_assert(CAP % (U * COUNT_THREADS) == 0 && UMAX <= 32, "one bit per place of a thread");
     extern __shared__ __align__(128) uint8_t smem[];
-    CountSmem<W> L;
-    L.layout(P.smem_slots);
-    Key* keys = reinterpret_cast<Key*>(smem + L.keys);
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem + L.cnt);
-    uint16_t* list = reinterpret_cast<uint16_t*>(smem + L.list);
-    __shared__ uint32_t s_nlist;                      // entries of list
-    __shared__ __align__(16) Group s_grp[3];          // groups g, g + 1, g + 2
-    __shared__ uint32_t s_fail;
-    __shared__ uint32_t s_bad;  // round in which a probe first gave up (the table was full); ~0: none
-    __shared__ uint32_t s_wnew[COUNT_THREADS / 32];      // new keys of the group, per warp
-    __shared__ uint32_t s_wout[COUNT_THREADS / 32];      // output keys per warp, then their offsets
-    __shared__ unsigned long long s_obase;
+    CountSmem<W>& S = *reinterpret_cast<CountSmem<W>*>(smem);
+    const int k = P.k;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    uint32_t distinct = 0;                                   // per warp
 
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const uint32_t S = P.smem_slots, mask = S - 1;    // S == SPT * COUNT_THREADS
-    const uint32_t fill_cap = S - S / 8;
-    // counts are at least 1 and fit in 32 bits: without ci/cx limits every key is kept
-    const bool filtered = P.ci > 1 || P.cx < 0xFFFFFFFFull;
-    const unsigned long long n1 = P.n_list[1];
-    const unsigned long long ntot = min(P.n_list[0] + n1, P.g_end);
-    const unsigned long long g0 = P.g_begin;
-    const Key* src = static_cast<const Key*>(P.keys);
-    unsigned long long distinct = 0;                  // per warp, in lane 0
-
-    for (uint32_t i = tid; i < S; i += COUNT_THREADS) { keys[i] = O::empty(); cnt[i] = 0; }
-    if (tid < COUNT_THREADS / 32) s_wnew[tid] = 0;
-    unsigned long long gi_pend = ~0ull;               // thread 0: index of group g + 3
+    start_store<W>(S);
     if (tid == 0) {
-        s_fail = 0;
-        s_bad = ~0u;
-        s_nlist = 0;
-        for (int q = 0; q < 3; ++q) copy_group(&s_grp[q], P, g0 + atomicAdd(P.work, 1ull), n1, ntot);
-        gi_pend = g0 + atomicAdd(P.work, 1ull);
+        for (int q = 0; q < 3; ++q) copy_group(&S.grp[q], P, P.g_begin + atomicAdd(P.work, 1ull));
+        S.pending = P.g_begin + atomicAdd(P.work, 1ull);     // index of group g + 3
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
     __syncthreads();
 
-    // keys of round r of group g into K (EMPTY past the group's end)
-    auto load_round = [&](const Group& g, uint32_t r, Key (&K)[U]) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const unsigned long long i = g.lo + (unsigned long long)r * RK + (uint32_t)u * COUNT_THREADS + tid;
-            K[u] = i < g.hi ? src[i] : O::empty();
-        }
+    // this thread's first packed record of a group (no k-mers past the group's end)
+    auto load_at = [&](const Group& g, uint32_t i) {
+        Rec<W> c;
+        c.w[2 * W - 1] = 0;
+        if (i < (uint32_t)(g.hi - g.lo)) c = load_rec<W>(P.recs, g.lo + i);
+        return c;
     };
-
-    Key K[U];
-    {
-        const Group g0 = s_grp[0];
-        load_round(g0, 0, K);
-    }
+    Rec<W> ahead = load_at(S.grp[0], tid);
     for (uint32_t q = 0;; q = q == 2 ? 0 : q + 1) {
-        const Group g = s_grp[q];
-        if (g.hi <= g.lo) break;  // no more groups
-        const uint32_t nr = (uint32_t)((g.hi - g.lo + RK - 1) / RK);
-        bool bad = false;
-        for (uint32_t r = 0; r < nr; ++r) {
-            Key N[U];
-            if (r + 1 < nr) load_round(g, r + 1, N);
-            else load_round(s_grp[q == 2 ? 0 : q + 1], 0, N);
-            uint32_t newm = 0, nsl[U];
-            if (!bad) {
+        const Group& g = S.grp[q];
+        if (g.hi == g.lo) break;  // no more groups
+        const uint32_t sample = g.sample, nrec = (uint32_t)(g.hi - g.lo);
+        // Equal records first, where the last groups had enough of them (read sets: a
+        // record inside several reads): one of them is unpacked, with their number as the
+        // weight of its keys. The table holds record numbers meanwhile, cnt their
+        // occurrences after the first; both are empty again before the keys come.
+        constexpr uint32_t DM = W == 1 ? DEDUP_MAX : 1;
+        Rec<W> mine[DM];
+        uint32_t weight[DM];
+        const bool dedup = W == 1 && S.dedup == 0 && nrec <= DM * COUNT_THREADS;
+        if (W == 1 && dedup) {
+            Rec<W>* recs = reinterpret_cast<Rec<W>*>(S.keys);
+            uint32_t first = 0;  // bit j: this thread's j-th record is the first of its kind
+            mine[0] = ahead;
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    nsl[u] = 0;
-                    if (bad || O::is_empty(K[u])) continue;
-                    const uint64_t h = O::hash(K[u]);
-                    if (g.parts > 1 && ((uint32_t)(h >> 8) & (g.parts - 1)) != g.part) continue;
-                    int res;
-                    if constexpr (W == 1)
-                        res = claim_bucket(reinterpret_cast<unsigned long long*>(keys), cnt, mask / BUCKET, K[u],
-                                           (uint32_t)(h >> 32) & mask, nsl[u]);
-                    else
-                        res = claim_cas(reinterpret_cast<U128*>(keys), cnt, mask, K[u], (uint32_t)(h >> 32) & mask,
-                                        nsl[u]);
-                    if (res < 0) { if (!bad) atomicMin(&s_bad, r); bad = true; }
-                    else newm |= (uint32_t)res << u;
+            for (uint32_t j = 1; j < DM; ++j) mine[j] = load_at(g, j * COUNT_THREADS + tid);
+#pragma unroll
+            for (uint32_t j = 0; j < DM; ++j)
+                if (j * COUNT_THREADS + tid < nrec) recs[j * COUNT_THREADS + tid] = mine[j];
+            __syncthreads();
+#pragma unroll
+            for (uint32_t j = 0; j < DM; ++j) {
+                const uint32_t i = j * COUNT_THREADS + tid;
+                weight[j] = 0;
+                if (i >= nrec) continue;
+                uint32_t h, en;
+                place_of<W>(rec_hash(mine[j]), i, h, en);
+                for (uint32_t p = 0; p < SLOTS; ++p) {
+                    const uint32_t e = atomicCAS(&S.table[h], NO_ENTRY, en);
+                    if (e == NO_ENTRY) {
+                        weight[j] = 1;
+                        ++first;
+                        break;
+                    }
+                    if (((e ^ en) >> IDX_BITS) == 0 && rec_equal(recs[e & IDX_MASK], mine[j])) {
+                        atomicAdd(&S.cnt[e & IDX_MASK], 1u);
+                        break;
+                    }
+                    h = next_slot<W>(h, en);
                 }
             }
-            {  // this round's new slots onto the list: one shared atomic per warp
-                const uint32_t nn = __popc(newm);
-                uint32_t x = nn;
+            __syncwarp();
+            first = __reduce_add_sync(0xffffffffu, first);
+            if (lane == 0) atomicAdd(&S.firsts, first);
+            __syncthreads();
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= o) x += y;
+            for (uint32_t j = 0; j < DM; ++j)
+                if (weight[j]) {
+                    weight[j] += S.cnt[j * COUNT_THREADS + tid];
+                    S.cnt[j * COUNT_THREADS + tid] = 0;
                 }
-                uint32_t lb = 0;
-                if (lane == 31 && x) lb = atomicAdd(&s_nlist, x);
-                lb = __shfl_sync(0xffffffffu, lb, 31) + x - nn;
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if ((newm >> u) & 1u) list[min(lb + __popc(newm & ((1u << u) - 1u)), S - 1)] = (uint16_t)nsl[u];
+            clear_table<W>(S);
+            if (tid == 0) {  // too few were equal: the next 15 groups without
+                if (S.firsts > nrec - nrec / 4) S.dedup = 15;
+                S.firsts = 0;
             }
+            __syncthreads();
+        }
+        // A warp unpacks 32 records, each lane its own: the keys of a record one after
+        // the other in the store, the warp's records next to each other.
+        auto unpack = [&](const Rec<W>& rec, uint32_t nk, uint32_t w) {
+            uint32_t x = nk;
 #pragma unroll
-            for (int u = 0; u < U; ++u) K[u] = N[u];
-        }
-        if (bad) s_fail = 1;
-        __syncthreads();  // inserts done; every thread has read slot q
-        if (tid == 0) {
-            // group g + 3's entry into slot q (landed before the group's last
-            // barrier), the index after it claimed
-            copy_group(&s_grp[q], P, gi_pend, n1, ntot);
-            gi_pend = g0 + atomicAdd(P.work, 1ull);
-        }
-        if (tid == 32) {
-            const uint32_t t = s_nlist;
-            if (t > fill_cap) s_fail = 1;  // more than 7/8 full: split the group
-            if (!filtered && !s_fail) s_obase = t ? atomicAdd(&P.ctr[P2C_OUT], (unsigned long long)t) : 0;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            uint32_t at = 0;
+            if (lane == 31) at = atomicAdd(&S.staged, x);
+            at = __shfl_sync(0xffffffffu, at, 31) + x - nk;
+            if (at + nk <= CAP) {
+                Key* d = S.keys + at;
+                Roll<W> roll;
+                roll.start(rec, k);
+                for (uint32_t t = 0; t < nk; ++t) {
+                    *d++ = roll.key(k);
+                    roll.step(k);
+                }
+                if (w > 1)
+                    for (uint32_t t = 0; t < nk; ++t) S.cnt[at + t] = w - 1;
+            }
+            __syncwarp();
+        };
+        if (W == 1 && dedup) {
+#pragma unroll
+            for (uint32_t j = 0; j < DM; ++j)
+                if (j * COUNT_THREADS + (tid & ~31u) < nrec) unpack(mine[j], weight[j] ? mine[j].n() : 0, weight[j]);
+        } else {
+            for (uint32_t i = tid; (i & ~31u) < nrec; i += COUNT_THREADS) {
+                const Rec<W> rec = ahead;
+                if ((i & ~31u) + COUNT_THREADS < nrec) ahead = load_at(g, i + COUNT_THREADS);
+                unpack(rec, rec.n(), 1);
+            }
         }
         __syncthreads();
-        if (s_fail) {
-            // clear the table; the group comes back as two halves
-            const uint32_t nl = min(s_nlist, S);
-            for (uint32_t i = tid; i < nl; i += COUNT_THREADS) { keys[list[i]] = O::empty(); cnt[list[i]] = 0; }
+        const uint32_t n = min(S.staged, CAP);
+        ahead = load_at(S.grp[q == 2 ? 0 : q + 1], tid);
+        uint32_t newm = 0, pend = 0;
+        // A CAS per key at its home slot, and one at the next slot of its probe if the
+        // home slot holds another key; the few keys (1.5 % in a table a quarter full)
+        // that both find taken stay pending (bit u of pend).
+#pragma unroll 1
+        for (uint32_t u0 = 0; u0 * COUNT_THREADS < n; u0 += U) {
+            Key K[U];
+            uint32_t en[U], h[U], e[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint32_t i = (u0 + u) * COUNT_THREADS + tid;
+                K[u] = S.keys[i];
+                place_of<W>(slot_hash(K[u]), i, h[u], en[u]);
+                e[u] = IDX_MASK;  // no key: nothing below happens
+                if (i < n) e[u] = atomicCAS(&S.table[h[u]], NO_ENTRY, en[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint32_t bit = 1u << (u0 + u);
+                uint32_t f = e[u];
+                if (f == NO_ENTRY) newm |= bit;
+                if (f < NO_ENTRY && f != IDX_MASK) {
+                    if (((f ^ en[u]) >> IDX_BITS) != 0 || !O::eq(S.keys[f & IDX_MASK], K[u])) {
+                        f = atomicCAS(&S.table[next_slot<W>(h[u], en[u])], NO_ENTRY, en[u]);
+                        if (f == NO_ENTRY) newm |= bit;
+                        else if (((f ^ en[u]) >> IDX_BITS) != 0 || !O::eq(S.keys[f & IDX_MASK], K[u])) { pend |= bit; f = NO_ENTRY; }
+                    }
+                    if (f != NO_ENTRY) {  // known: its weight to the place that came first
+                        const uint32_t i = (u0 + u) * COUNT_THREADS + tid, w = S.cnt[i];
+                        atomicAdd(&S.cnt[f & IDX_MASK], w + 1);
+                        if (w) S.cnt[i] = 0;
+                    }
+                }
+            }
+        }
+        while (pend) {
+            const uint32_t bit = pend & (0u - pend), i = (31 - __clz(bit)) * COUNT_THREADS + tid;
+            pend ^= bit;
+            const Key key = S.keys[i];
+            uint32_t h, en;
+            place_of<W>(slot_hash(key), i, h, en);
+            h = next_slot<W>(h, en);
+            for (uint32_t p = 0; p < SLOTS; ++p) {
+                h = next_slot<W>(h, en);
+                const uint32_t e = atomicCAS(&S.table[h], NO_ENTRY, en);
+                if (e == NO_ENTRY) { newm |= bit; break; }
+                if (((e ^ en) >> IDX_BITS) == 0 && O::eq(S.keys[e & IDX_MASK], key)) {
+                    const uint32_t w = S.cnt[i];
+                    atomicAdd(&S.cnt[e & IDX_MASK], w + 1);
+                    if (w) S.cnt[i] = 0;
+                    break;
+                }
+            }
+        }
+        __syncwarp();
+        write_out<W>(P, S, n, newm, sample, distinct, [&] {
+            if (tid == 0) {  // group g + 3's entry into slot q, the index after it claimed
+                S.staged = 0;
+                if (!dedup && S.dedup) --S.dedup;
+                copy_group(&S.grp[q], P, S.pending);
+                S.pending = P.g_begin + atomicAdd(P.work, 1ull);
+            }
+        });
+        if (tid == 0) asm volatile("cp.async.wait_all;" ::: "memory");  // group g + 3's entry has landed
+        __syncthreads();  // the store may be filled again
+    }
+    if (lane == 0 && distinct) atomicAdd(&P.ctr[P2C_DISTINCT], (unsigned long long)distinct);
+}
+
+// ---------------------------------------------------------------- larger groups
+// The next records of a range in rounds. A round looks its keys up first: the
+// ones that the store holds are counted (equal records of a warp, a repeat's, as
+// one of their number), only the others are staged behind the store's keys and
+// inserted; those that another of the round came before stay as holes. The first
+// round is short, since all of its keys are staged. Takes records [r, nrec) until
+// they are all counted or the store is 7/8 full and returns how far it came; n:
+// places in use, newm: bit u set if this thread's place u * COUNT_THREADS + threadIdx.x
+// holds a new key. Every thread of the CTA calls it; ends with a barrier.
+template <int W>
+__device__ __forceinline__ unsigned long long count_rounds(const CountParams& P, CountSmem<W>& S,
+                                                           unsigned long long lo, unsigned long long r,
+                                                           unsigned long long nrec, uint32_t parts, uint32_t part,
+                                                           uint32_t& n, uint32_t& newm) {
+    using O = KeyOps<W>;
+    using Key = typename O::Key;
+    constexpr uint32_t CAP = CountShape<W>::CAP, SLOTS = CountSmem<W>::SLOTS;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    const int k = P.k;
+    while (r < nrec && CAP - n >= CAP / 8) {
+        // as many records as fit if all of their keys are new; the warps share them evenly
+        const uint32_t take = (uint32_t)min((unsigned long long)((n ? CAP - n : 512u) / REC_MAX), nrec - r);
+        const uint32_t per = (take + COUNT_THREADS / 32 - 1) / (COUNT_THREADS / 32), w0 = (tid >> 5) * per;
+        const uint32_t w1 = min(w0 + per, take);
+        for (uint32_t i0 = w0; i0 < w1; i0 += 32) {
+            Rec<W> c;
+            uint32_t nk = 0;
+            if (i0 + lane < w1) {
+                c = load_rec<W>(P.recs, lo + r + i0 + lane);
+                nk = c.n();
+            }
+            unsigned same = __match_any_sync(0xffffffffu, nk ? c.w[0] : (unsigned long long)lane);
+            same &= __match_any_sync(0xffffffffu, nk ? c.w[1] : ~(unsigned long long)lane);
+            if constexpr (W == 2) {
+                same &= __match_any_sync(0xffffffffu, nk ? c.w[2] : (unsigned long long)lane);
+                same &= __match_any_sync(0xffffffffu, nk ? c.w[3] : ~(unsigned long long)lane);
+            }
+            const uint32_t weight = __popc(same);
+            if (lane != (uint32_t)__ffs(same) - 1) nk = 0;
+            const uint32_t steps = __reduce_max_sync(0xffffffffu, nk);
+            Roll<W> roll;
+            if (nk) roll.start(c, k);
+            for (uint32_t t = 0; t < steps; ++t) {
+                bool a = t < nk;
+                Key key;
+                if (a) {
+                    key = roll.key(k);
+                    roll.step(k);
+                    a = parts == 1 || key_part<W>(key, parts) == part;
+                }
+                if (a) {
+                    uint32_t h, en;
+                    place_of<W>(slot_hash(key), 0, h, en);
+                    for (uint32_t p = 0; p < SLOTS; ++p) {
+                        const uint32_t e = *(const volatile uint32_t*)&S.table[h];
+                        if (e == NO_ENTRY) break;
+                        if (((e ^ en) >> IDX_BITS) == 0 && O::eq(S.keys[e & IDX_MASK], key)) {
+                            atomicAdd(&S.cnt[e & IDX_MASK], weight);
+                            a = false;
+                            break;
+                        }
+                        h = next_slot<W>(h, en);
+                    }
+                }
+                const unsigned bal = __ballot_sync(0xffffffffu, a);
+                uint32_t base = 0;
+                if (lane == 0 && bal) base = atomicAdd(&S.staged, (uint32_t)__popc(bal));
+                base = n + __shfl_sync(0xffffffffu, base, 0) + __popc(bal & ((1u << lane) - 1));
+                if (a && base < CAP) {
+                    S.keys[base] = key;
+                    S.cnt[base] = weight - 1;
+                }
+            }
+        }
+        __syncthreads();
+        const uint32_t m = min(n + S.staged, CAP);
+        for (uint32_t u = n / COUNT_THREADS; u * COUNT_THREADS < m; ++u) {
+            const uint32_t i = u * COUNT_THREADS + tid;
+            if (i < n || i >= m) continue;
+            const Key key = S.keys[i];
+            uint32_t h, en;
+            place_of<W>(slot_hash(key), i, h, en);
+            for (uint32_t p = 0; p < SLOTS; ++p) {
+                const uint32_t e = atomicCAS(&S.table[h], NO_ENTRY, en);
+                if (e == NO_ENTRY) { newm |= 1u << u; break; }
+                if (((e ^ en) >> IDX_BITS) == 0 && O::eq(S.keys[e & IDX_MASK], key)) {
+                    // only this thread reads or clears the count of a place that is in no entry
+                    atomicAdd(&S.cnt[e & IDX_MASK], S.cnt[i] + 1);
+                    S.cnt[i] = 0;
+                    break;
+                }
+                h = next_slot<W>(h, en);
+            }
+        }
+        __syncthreads();  // the round is in the table; every thread has its size
+        if (tid == 0) S.staged = 0;
+        n = m;
+        r += take;
+        __syncthreads();
+    }
+    return r;
+}
+
+// Groups of more than CAP and at most BIG_KEYS k-mers (one bin each), and key-hash parts
+// of such groups, one CTA each. A group whose distinct keys do not fit comes back as F
+// key-hash parts, F the power of two that gives half-full stores for the places
+// estimated from the share of the group seen; past MAX_PARTS parts it goes to the
+// global-memory table.
+template <int W>
+__global__ void __launch_bounds__(COUNT_THREADS, COUNT_PER_SM) k_rounds(const __grid_constant__ CountParams P) {
+    constexpr uint32_t CAP = CountShape<W>::CAP;
+    extern __shared__ __align__(128) uint8_t smem[];
+    CountSmem<W>& S = *reinterpret_cast<CountSmem<W>*>(smem);
+    const uint32_t tid = threadIdx.x;
+    uint32_t distinct = 0;
+    start_store<W>(S);
+    __syncthreads();
+    for (unsigned long long gi = P.g_begin + blockIdx.x; gi < P.g_end; gi += gridDim.x) {
+        const Group g = P.list[gi];
+        const unsigned long long nrec = g.hi - g.lo;
+        uint32_t n = 0, newm = 0;
+        const unsigned long long r = count_rounds<W>(P, S, g.lo, 0, nrec, g.parts, g.part, n, newm);
+        if (r < nrec) {  // too many distinct keys
             if (tid == 0) {
                 Group f = g;
                 if (g.parts < MAX_PARTS) {
-                    // split into F key-hash parts: enough for half-full tables when the
-                    // group ran to its end (its distinct keys are known), else 4
-                    // distinct keys of the group: known when it ran to its end; else
-                    // estimated from the keys seen before the table filled
-                    uint64_t est = s_nlist;
-                    if (s_bad != ~0u) {
-                        const uint64_t hk = g.hi - g.lo;
-                        uint64_t seen = (uint64_t)(s_bad + 1) * RK;
-                        if (seen > hk) seen = hk;
-                        est = (uint64_t)s_nlist * hk / (seen ? seen : 1);
-                    }
-                    const uint64_t need = (est + S / 2 - 1) / (S / 2);
+                    const uint64_t need = ((uint64_t)n * nrec / r + CAP / 2 - 1) / (CAP / 2);
                     uint32_t F = 2;
                     while (F < need) F <<= 1;
                     while (g.parts * F > MAX_PARTS) F >>= 1;
                     const unsigned long long i = atomicAdd(P.n_retry, (unsigned long long)F);
                     f.parts = F * g.parts;
-                    if (i + F - 1 < P.retry_cap) {
-                        for (uint32_t jf = 0; jf < F; ++jf) {
-                            f.part = g.part + jf * g.parts;
-                            P.retry[i + jf] = f;
+                    if (i + F - 1 < P.retry_cap)
+                        for (uint32_t j = 0; j < F; ++j) {
+                            f.part = g.part + j * g.parts;
+                            P.retry[i + j] = f;
                         }
-                    }
                 } else {
                     const unsigned long long i = atomicAdd(&P.ctr[P2C_FALLBACK], 1ull);
                     if (i < P.fallback_cap) P.fallback[i] = f;
                 }
             }
-        } else if (!filtered) {
-            // ---- output: the listed slots in list order, pair i of the group to out[base + i]
-            const uint32_t nl = s_nlist;
-            const unsigned long long ob = s_obase;
-            for (uint32_t i = tid; i < nl; i += COUNT_THREADS) {
-                const uint32_t sl = list[i];
-                const unsigned long long oi = ob + i;
-                const uint32_t c = cnt[sl];
-                if (oi < P.out_cap) {
-                    O::store(P.out_keys, oi, keys[sl]);
-                    P.out_counts[oi] = c + 1;
-                    if (P.out_sample) P.out_sample[oi] = g.sample;
-                }
-                keys[sl] = O::empty();
-                if (c) cnt[sl] = 0;
-            }
-            if (tid == 0) distinct += nl;
+            for (uint32_t i = tid; i < n; i += COUNT_THREADS) S.cnt[i] = 0;
+            clear_table<W>(S);
         } else {
-            // ---- output: thread t owns slots t + j * COUNT_THREADS (a warp's accesses
-            // are consecutive); per warp and round j one ballot places the kept
-            // keys contiguously
-            uint32_t keepm = 0, nocc = 0;
-#pragma unroll
-            for (uint32_t j = 0; j < SPT; ++j) {
-                const uint32_t sl = tid + j * COUNT_THREADS;
-                const bool occ = !O::is_empty(keys[sl]);
-                nocc += occ ? 1u : 0u;
-                bool keep = occ;
-                if (filtered && occ) {
-                    const uint32_t c = cnt[sl] + 1;
-                    keep = (uint64_t)c >= P.ci && (uint64_t)c <= P.cx;
-                }
-                keepm |= (keep ? 1u : 0u) << j;
-            }
-            uint32_t wtot = 0;
-#pragma unroll
-            for (uint32_t j = 0; j < SPT; ++j) wtot += __popc(__ballot_sync(0xffffffffu, (keepm >> j) & 1u));
-            nocc = __reduce_add_sync(0xffffffffu, nocc);
-            if (lane == 0) { s_wout[wid] = wtot; distinct += nocc; }
-            __syncthreads();
-            if (wid == 0) {
-                const uint32_t v = lane < COUNT_THREADS / 32 ? s_wout[lane] : 0u;
-                uint32_t x = v;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= o) x += y;
-                }
-                if (lane < COUNT_THREADS / 32) s_wout[lane] = x - v;
-                if (lane == 31) s_obase = x ? atomicAdd(&P.ctr[P2C_OUT], (unsigned long long)x) : 0;
-            }
-            __syncthreads();
-            unsigned long long o = s_obase + s_wout[wid];
-#pragma unroll
-            for (uint32_t j = 0; j < SPT; ++j) {
-                const uint32_t sl = tid + j * COUNT_THREADS;
-                const bool keep = (keepm >> j) & 1u;
-                const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                if (keep) {
-                    const unsigned long long i = o + __popc(bal & ((1u << lane) - 1));
-                    if (i < P.out_cap) {
-                        O::store(P.out_keys, i, keys[sl]);
-                        P.out_counts[i] = cnt[sl] + 1;
-                        if (P.out_sample) P.out_sample[i] = g.sample;
-                    }
-                }
-                keys[sl] = O::empty();
-                cnt[sl] = 0;
-                o += __popc(bal);
-            }
-        }
-        __syncthreads();  // every thread is done with the list
-        if (tid == 0) {
-            s_fail = 0;
-            s_bad = ~0u;
-            s_nlist = 0;
-            asm volatile("cp.async.wait_all;" ::: "memory");  // group g + 3's entry has landed
+            write_out<W>(P, S, n, newm, g.sample, distinct, [] {});
         }
         __syncthreads();
     }
-    if (lane == 0 && distinct) atomicAdd(&P.ctr[P2C_DISTINCT], distinct);
+    if ((tid & 31) == 0 && distinct) atomicAdd(&P.ctr[P2C_DISTINCT], (unsigned long long)distinct);
+}
+
+// Groups of more than BIG_KEYS k-mers (one bin: a repeat's, or one conserved
+// minimizer's), each shared by many CTAs: blockIdx.y picks the group, the CTAs of a row
+// its chunks of BIG_CHUNK records. A chunk's keys are counted in the CTA's own store as
+// above, and the store's (key, count) pairs added to a table in global memory whenever it
+// fills up and at the end, so a k-mer that the group repeats costs a global atomic per
+// store, not per instance.
+template <int W>
+__global__ void __launch_bounds__(COUNT_THREADS, COUNT_PER_SM)
+    k_big(const __grid_constant__ CountParams P, const __grid_constant__ FallbackParams F) {
+    using Key = typename KeyOps<W>::Key;
+    extern __shared__ __align__(128) uint8_t smem[];
+    CountSmem<W>& S = *reinterpret_cast<CountSmem<W>*>(smem);
+    const uint32_t tid = threadIdx.x;
+    start_store<W>(S);
+    __syncthreads();
+    const Group g = P.list[P.g_begin + blockIdx.y];
+    const unsigned long long nrec = g.hi - g.lo;
+    for (unsigned long long c = (unsigned long long)blockIdx.x * BIG_CHUNK; c < nrec; c += (unsigned long long)gridDim.x * BIG_CHUNK) {
+        const unsigned long long end = min(nrec, c + BIG_CHUNK);
+        for (unsigned long long r = c; r < end;) {
+            uint32_t n = 0, newm = 0;
+            r = count_rounds<W>(P, S, g.lo, r, end, 1, 0, n, newm);
+            for (uint32_t u = 0; u * COUNT_THREADS < n; ++u) {
+                const uint32_t i = u * COUNT_THREADS + tid;
+                if ((newm >> u) & 1u)
+                    if (!tbl_add<W>(static_cast<Key*>(F.tkeys), F.tcnt, F.mask, S.keys[i], S.cnt[i] + 1, F.mask + 1))
+                        atomicExch(F.fail, 1u);
+                if (i < n) S.cnt[i] = 0;
+            }
+            clear_table<W>(S);
+            __syncthreads();
+        }
+    }
 }
 
 // ---------------------------------------------------------------- fallback
@@ -721,12 +923,17 @@ template <int W>
 __global__ void k_fb_insert(FallbackParams F) {
     using O = KeyOps<W>;
     auto* tk = reinterpret_cast<typename O::Key*>(F.tkeys);
-    const auto* src = reinterpret_cast<const typename O::Key*>(F.keys);
     for (unsigned long long i = F.lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < F.hi;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        const typename O::Key key = src[i];
-        if (key_part<W>(key, F.parts) != F.part) continue;
-        if (!tbl_add<W>(tk, F.tcnt, F.mask, key, F.mask + 1)) atomicExch(F.fail, 1u);
+        const Rec<W> c = load_rec<W>(F.recs, i);
+        const uint32_t n = c.n();
+        Roll<W> roll;
+        roll.start(c, F.k);
+        for (uint32_t t = 0; t < n; ++t, roll.step(F.k)) {
+            const typename O::Key key = roll.key(F.k);
+            if (key_part<W>(key, F.parts) != F.part) continue;
+            if (!tbl_add<W>(tk, F.tcnt, F.mask, key, 1, F.mask + 1)) atomicExch(F.fail, 1u);
+        }
     }
 }
 
@@ -820,16 +1027,13 @@ __global__ void k_samp_scatter(const void* __restrict__ keys, const uint32_t* __
 // ---------------------------------------------------------------- host side
 size_t key_bytes(int W) { return W == 1 ? 8 : 16; }
 
-// Table slots of a k_count CTA: the largest power of two whose keys and counts
-// fit in one SM's shared memory (large tables mean large groups, and fewer of
-// them to set up and drain).
-uint32_t count_slots(int W) { return W == 1 ? 16384 : 8192; }
+// The unit of a group's planned size (group_pct).
+uint32_t count_slots(int) { return 8192; }
 
-static size_t count_smem_bytes(int W, uint32_t slots) {
-    if (W == 1) { CountSmem<1> L; L.layout(slots); return L.total; }
-    CountSmem<2> L;
-    L.layout(slots);
-    return L.total;
+// Keys that k_plan puts in a group: group_pct of the unit, at most a store full.
+static uint32_t group_target(const P2Input& in) {
+    const uint32_t cap = in.W == 1 ? CountShape<1>::CAP : CountShape<2>::CAP;
+    return std::max<uint32_t>(1, std::min(count_slots(in.W) * in.group_pct / 100, cap));
 }
 
 namespace {
@@ -847,75 +1051,87 @@ struct Carve {
     }
 };
 
-constexpr uint32_t NBIN_ALL = 1u << BIN_BITS;
-
 struct P2Plan {
-    uint64_t n_slices = 0, groups_cap = 0, retry_cap = 0, n_keys_alloc = 0, nsum = 0;
-    std::vector<Slice> slices;
+    uint64_t groups_cap = 0, retry_cap = 0, nsum = 0;
 };
+
+// Warps of k_plan per segment. Its steps are serial within a warp (one group
+// each, about a microsecond of dependent reads), so long segments are shared out
+// until a share has about 32 groups; fewer would leave more of the last groups of
+// the shares half filled.
+uint32_t plan_split(const P2Input& in) {
+    uint32_t s = 1;
+    while (s < 64 && in.n_kmers / ((uint64_t)in.n_segs * 2 * s + 1) > 32ull * group_target(in)) s *= 2;
+    return s;
+}
 
 P2Plan make_plan(const P2Input& in) {
     P2Plan L;
-    for (uint32_t c = 0; c < in.n_lists; ++c) {
-        const uint64_t nd = std::min<uint64_t>(in.n_desc[c], in.desc_cap);
-        for (uint64_t s = 0; s < nd; s += SLICE_DESC) {
-            Slice sl;
-            sl.r_lo = (uint64_t)c * in.desc_cap + s;
-            sl.r_hi = (uint64_t)c * in.desc_cap + std::min<uint64_t>(nd, s + SLICE_DESC);
-            L.slices.push_back(sl);
-        }
-    }
-    L.n_slices = L.slices.size();
     // a segment of K keys has fewer than 2 K / target + 1 groups (two neighbouring
     // groups of k_plan hold more than `target` keys together)
-    const uint64_t target = std::max<uint64_t>(1, (uint64_t)count_slots(in.W) * in.group_pct / 100);
-    L.groups_cap = 2 * in.n_kmers / target + in.n_segs + 1;
+    const uint64_t target = group_target(in);
+    L.groups_cap = 2 * in.n_kmers / target + (uint64_t)in.n_segs * plan_split(in) + 1;
     L.retry_cap = std::max<uint64_t>(4096, 2 * L.groups_cap);
-    L.n_keys_alloc = in.n_kmers + 1;
-    L.nsum = (NBIN_ALL + 8191) / 8192 + 2;
+    L.nsum = scan_scratch(std::max<uint64_t>(in.all_bins, in.n_samples));
     return L;
 }
 
 // The scratch regions of one run, in order (the same walk sizes and places them).
 struct P2Regions {
     unsigned long long* ctr;
-    unsigned long long* aux;  // [0..1] retry counters, [2..3] list sizes of a retry pass
-    unsigned long long* work; // [0..15] group counters of the first pass's launches, [16] of a retry pass
+    unsigned long long* aux;  // [0..1] retry counters
+    unsigned long long* work; // [0..15] group counters of k_count's launches
     unsigned long long* kofs;
+    unsigned long long* rofs;
     uint32_t* gfirst;
     unsigned long long* sums;
     Segment* segs;
-    Slice* slices;
     Group* normal;
     Group* heavy;
+    Group* big;
     Group* retry[2];
     Group* fb;
     unsigned long long* scur;  // [n_samples] cursors of the sample-major copy
-    uint8_t* keys;
+    uint8_t* recs;
 };
 
 P2Regions carve(Carve& c, const P2Input& in, const P2Plan& L) {
     P2Regions R;
     R.ctr = c.take<unsigned long long>(P2C_COUNT);
-    R.aux = c.take<unsigned long long>(4);
-    R.work = c.take<unsigned long long>(17);
-    R.kofs = c.take<unsigned long long>(NBIN_ALL + 1);
-    R.gfirst = c.take<uint32_t>(NBIN_ALL);
+    R.aux = c.take<unsigned long long>(2);
+    R.work = c.take<unsigned long long>(16);
+    R.kofs = c.take<unsigned long long>((size_t)in.all_bins + 1);
+    R.rofs = c.take<unsigned long long>((size_t)in.all_bins + 1);
+    R.gfirst = c.take<uint32_t>(in.all_bins);
     R.sums = c.take<unsigned long long>(L.nsum);
     R.segs = c.take<Segment>(in.n_segs + 1);
-    R.slices = c.take<Slice>(L.n_slices + 1);
     R.normal = c.take<Group>(L.groups_cap);
     R.heavy = c.take<Group>(L.groups_cap);
+    R.big = c.take<Group>(in.n_kmers / BIG_KEYS + 1);
     R.retry[0] = c.take<Group>(L.retry_cap);
     R.retry[1] = c.take<Group>(L.retry_cap);
     R.fb = c.take<Group>(FALLBACK_CAP);
     R.scur = c.take<unsigned long long>(in.n_samples + 1);
-    R.keys = c.take<uint8_t>(L.n_keys_alloc * key_bytes(in.W));
+    R.recs = c.take<uint8_t>((in.n_recs + 1) * 16 * (size_t)in.W);
     return R;
 }
 }  // namespace
 
-SampleBins layout_bins(const std::vector<unsigned long long>& sample_start, uint32_t seg_bins) {
+// The work that goes with every bin (histogram, scan, plan) is small next to the
+// keys', and bins of a few hundred keys pack into groups with little left over:
+// about 512 stream bytes per bin, up to 2^22 bins. (3.1 Gbp in 2^20 bins of 2,950
+// k-mers filled groups of 4,096 to 72 %; small calls spent most of their time on
+// 2^20 empty bins.)
+int job_bin_bits(uint64_t n, uint32_t n_samples, uint32_t seg_bits) {
+    const int most = n < (1ull << 34) ? MAX_BIN_BITS : BIN_BITS;
+    int b = std::max<int>(8, (int)seg_bits);
+    while ((2ull << b) <= n / 256 && b < most) ++b;
+    while (b < BIN_BITS && (1ull << b) < 4ull * n_samples) ++b;
+    return b;
+}
+
+SampleBins layout_bins(const std::vector<unsigned long long>& sample_start, uint32_t seg_bins, int bin_bits) {
+    const uint32_t all = 1u << bin_bits;
     SampleBins B;
     B.start = sample_start;
     const size_t n = sample_start.size() - 1;
@@ -928,14 +1144,14 @@ SampleBins layout_bins(const std::vector<unsigned long long>& sample_start, uint
         for (size_t i = 0; i < n; ++i) {
             const double share = budget * (double)(sample_start[i + 1] - sample_start[i]) / total;
             uint32_t b = 0;
-            while (b < BIN_BITS && (double)(2ull << b) <= share) ++b;
+            while (b < (uint32_t)bin_bits && (double)(2ull << b) <= share) ++b;
             B.bits[i] = (uint8_t)b;
             B.base[i] = (uint32_t)used;
             used += 1ull << b;
         }
         return used;
     };
-    if (assign((double)NBIN_ALL) > NBIN_ALL) assign((double)(NBIN_ALL - n));  // one bin set aside per sample
+    if (assign((double)all) > all) assign((double)(all - n));  // one bin set aside per sample
     seg_bins = std::max<uint32_t>(1, seg_bins);
     for (size_t i = 0; i < n; ++i) {
         const uint32_t hi = B.base[i] + (1u << B.bits[i]);
@@ -1005,68 +1221,68 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     Carve c{static_cast<uint8_t*>(scratch), 0, scratch_cap, true};
     const P2Regions R = carve(c, in, L);
     if (!c.ok) { err = "phase-2 scratch too small"; return TG_ERR_OOM; }
-    const uint32_t slots = count_slots(W);
 
     P2_CK(cudaMemsetAsync(R.ctr, 0, P2C_COUNT * 8, st), "memset");
-    if (L.n_slices)
-        P2_CK(cudaMemcpyAsync(R.slices, L.slices.data(), L.n_slices * sizeof(Slice), cudaMemcpyHostToDevice, st),
-              "h2d");
     P2_CK(cudaMemcpyAsync(R.segs, in.segs, (size_t)in.n_segs * sizeof(Segment), cudaMemcpyHostToDevice, st), "h2d");
-    // k-mer counts per bin -> first key of each bin (of this run's bins)
-    P2_CK(launch_scan(in.binhist + in.bin_lo, in.bin_hi - in.bin_lo, R.kofs + in.bin_lo, R.sums, R.kofs + in.bin_hi,
-                      st, launches),
+    // counts per bin -> k-mers and packed records before each bin (of this run's bins)
+    P2_CK(launch_bin_scan(in.binhist + in.bin_lo, in.bin_hi - in.bin_lo, R.kofs + in.bin_lo, R.rofs + in.bin_lo,
+                          R.sums, st, launches),
           "scan");
 
     KeysParams K{};
     K.packed = in.packed;
     K.desc = in.desc;
-    K.slices = R.slices;
+    K.desc_cap = in.desc_cap;
+    K.n_desc = in.n_desc;
+    K.n_one = in.max_desc;
     K.kofs = R.kofs;
+    K.rofs = R.rofs;
     K.gfirst = R.gfirst;
     K.segs = R.segs;
     K.n_segs = in.n_segs;
-    K.target = std::max<uint32_t>(1, slots * in.group_pct / 100);  // as in make_plan
+    K.target = group_target(in);
     K.k = in.k;
-    K.keys = R.keys;
+    K.recs = R.recs;
     K.groups[0] = R.normal;
     K.groups[1] = R.heavy;
+    K.groups[2] = R.big;
     K.groups_cap = L.groups_cap;
     K.ctr = R.ctr;
     K.bin_lo = in.bin_lo;
     K.bin_hi = in.bin_hi;
+    K.desc_sb = in.desc_sb;
+    K.plan_split = plan_split(in);
     {
-        const uint32_t warps = PLAN_THREADS / 32;
-        k_plan<<<(in.n_segs + warps - 1) / warps, PLAN_THREADS, 0, st>>>(K);  // before k_keys moves the cursors
+        const uint32_t warps = PLAN_THREADS / 32, n = in.n_segs * K.plan_split;
+        k_plan<<<(n + warps - 1) / warps, PLAN_THREADS, 0, st>>>(K);  // before k_recs moves the cursors
     }
     P2_CK(cudaGetLastError(), "k_plan");
     ++*launches;
-    if (L.n_slices) {
-        // Large jobs: two launches, each writing the keys of half of the bins.
-        // A record's keys land at its group's cursor; with every group open at
-        // once fewer of the partly written sectors stay in L2 until their
-        // neighbours fill them; with half of them open more do (3.1 G keys, bin
-        // cursors: 28.0 -> 23.4 ms, four launches 25.1, eight 39.4; group
-        // cursors: one launch 22.9, two 19.8), though every launch reads all
-        // descriptors.
-        const uint32_t KP = in.n_kmers > (1ull << 28) ? 2 : 1;
+    if (in.n_lists && in.max_desc) {
+        // A group's records land one 16 x W byte piece at a time at its cursor. With too
+        // many groups open at once their partly written lines no longer stay in L2
+        // until they are full, so jobs of many groups take several launches, each for
+        // a share of the bins, although every launch reads all descriptors (603 M
+        // records into 0.8 M groups: 1 launch 23.8 ms, 2 17.6, 4 16.7; 180 M records
+        // into 0.23 M groups: 4.37, 4.53, 4.54).
+        const uint32_t KP = 1 + (uint32_t)std::min<uint64_t>(7, in.n_kmers / group_target(in) >> 18);
         const uint32_t span = in.bin_hi - in.bin_lo;
+        const dim3 grid((in.max_desc + RECS_PER_CTA - 1) / RECS_PER_CTA, in.n_lists);
         for (uint32_t kp = 0; kp < KP; ++kp) {
             KeysParams Kp = K;
             Kp.bin_lo = in.bin_lo + (uint32_t)((uint64_t)span * kp / KP);
             Kp.bin_hi = in.bin_lo + (uint32_t)((uint64_t)span * (kp + 1) / KP);
-            if (W == 1) k_keys<1><<<(unsigned)L.n_slices, P2_THREADS, 0, st>>>(Kp);
-            else k_keys<2><<<(unsigned)L.n_slices, P2_THREADS, 0, st>>>(Kp);
-            P2_CK(cudaGetLastError(), "k_keys");
+            if (W == 1) k_recs<1><<<grid, RECS_THREADS, 0, st>>>(Kp);
+            else k_recs<2><<<grid, RECS_THREADS, 0, st>>>(Kp);
+            P2_CK(cudaGetLastError(), "k_recs");
             ++*launches;
         }
     }
     if (ev_keys) P2_CK(cudaEventRecord(ev_keys, st), "event");
 
     CountParams Q{};
-    Q.keys = R.keys;
-    Q.list[0] = R.normal;
-    Q.list[1] = R.heavy;
-    Q.n_list = R.ctr + P2C_NORMAL;  // [0] normal, [1] heavy: the heavy groups go first
+    Q.recs = R.recs;
+    Q.k = in.k;
     Q.fallback = R.fb;
     Q.fallback_cap = FALLBACK_CAP;
     Q.ci = in.ci;
@@ -1077,70 +1293,150 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     Q.out_cap = out.cap;
     Q.ctr = R.ctr;
     Q.retry_cap = L.retry_cap;
-    Q.smem_slots = slots;
-    const size_t sm = count_smem_bytes(W, slots);
-    if (W == 1)
-        P2_CK(set_smem_cap(k_count<1>, sm), "smem");
-    else
-        P2_CK(set_smem_cap(k_count<2>, sm), "smem");
+    const size_t sm = W == 1 ? sizeof(CountSmem<1>) : sizeof(CountSmem<2>);
+    P2_CK(W == 1 ? set_smem_cap(k_count<1>, sm) : set_smem_cap(k_count<2>, sm), "smem");
     unsigned long long h[P2C_COUNT];
-    // the groups of the first pass: their number is known once k_plan has run
+    // the groups: their number is known once k_plan has run
     P2_CK(cudaMemcpyAsync(h, R.ctr, sizeof h, cudaMemcpyDeviceToHost, st), "d2h");
     P2_CK(cudaStreamSynchronize(st), "phase 2");
-    if (h[P2C_NORMAL] > L.groups_cap || h[P2C_HEAVY] > L.groups_cap) {
+    if (h[P2C_NORMAL] > L.groups_cap || h[P2C_HEAVY] > L.groups_cap || h[P2C_BIG] > L.groups_cap) {
         err = "group list overflow";
         return TG_ERR_TABLE;
     }
-    const unsigned long long ngroups = h[P2C_NORMAL] + h[P2C_HEAVY];
+    const unsigned long long ngroups = h[P2C_NORMAL];
+    const unsigned cgrid = in.n_sm * COUNT_PER_SM;
+    auto rounds = [&](const Group* list, unsigned long long n) -> cudaError_t {
+        Q.list = list;
+        Q.g_begin = 0;
+        Q.g_end = n;
+        const unsigned grid = (unsigned)std::min<unsigned long long>(n, cgrid);
+        cudaError_t e = W == 1 ? set_smem_cap(k_rounds<1>, sm) : set_smem_cap(k_rounds<2>, sm);
+        if (e != cudaSuccess) return e;
+        if (W == 1) k_rounds<1><<<grid, COUNT_THREADS, sm, st>>>(Q);
+        else k_rounds<2><<<grid, COUNT_THREADS, sm, st>>>(Q);
+        ++*launches;
+        return cudaGetLastError();
+    };
+    // a global table with room for n keys: count() launches what fills it, then its pairs are written
+    auto in_table = [&](uint64_t n, uint32_t sample, const std::function<cudaError_t(const FallbackParams&)>& count,
+                        bool may_lack_room) -> tg_status {
+        uint64_t S = 1024;
+        while (S < 2 * n + 2) S <<= 1;
+        if (S > (1ull << 32)) {
+            if (!may_lack_room) err = "fallback table too large";
+            return TG_ERR_TABLE;
+        }
+        const size_t kbytes = (size_t)S * key_bytes(W);
+        uint8_t* tab = static_cast<uint8_t*>(fallback_table(kbytes + (size_t)S * 4 + 16));
+        if (!tab) {
+            if (!may_lack_room) err = "no room for the fallback table";
+            return TG_ERR_OOM;
+        }
+        FallbackParams F{};
+        F.recs = R.recs;
+        F.k = in.k;
+        F.tkeys = tab;
+        F.tcnt = reinterpret_cast<uint32_t*>(tab + kbytes);
+        F.mask = (uint32_t)(S - 1);
+        F.fail = reinterpret_cast<uint32_t*>(tab + kbytes + (size_t)S * 4);
+        P2_CK(cudaMemsetAsync(F.fail, 0, 4, st), "memset");
+        const unsigned grid = (unsigned)std::min<uint64_t>((S + 255) / 256, (uint64_t)in.n_sm * 8);
+        if (W == 1) k_fb_init<1><<<grid, 256, 0, st>>>(F.tkeys, F.tcnt, S);
+        else k_fb_init<2><<<grid, 256, 0, st>>>(F.tkeys, F.tcnt, S);
+        P2_CK(count(F), "fallback");
+        if (W == 1) k_fb_extract<1><<<grid, 256, 0, st>>>(F.tkeys, F.tcnt, S, Q, sample);
+        else k_fb_extract<2><<<grid, 256, 0, st>>>(F.tkeys, F.tcnt, S, Q, sample);
+        P2_CK(cudaGetLastError(), "fallback");
+        *launches += 3;
+        uint32_t failed = 0;
+        P2_CK(cudaMemcpyAsync(&failed, F.fail, 4, cudaMemcpyDeviceToHost, st), "d2h");
+        P2_CK(cudaStreamSynchronize(st), "fallback");
+        if (failed) { err = "fallback table overflow"; return TG_ERR_TABLE; }
+        return TG_OK;
+    };
+    Q.retry = R.retry[0];
+    Q.n_retry = R.aux;
+    P2_CK(cudaMemsetAsync(R.aux, 0, 16, st), "memset");
+    // ---- the largest groups, one table for those of a sample (of few MB for a group of a
+    // million k-mers; without room for it, they are counted like the other large ones)
+    uint64_t n_big = 0;
+    if (h[P2C_BIG]) {
+        std::vector<Group> big(h[P2C_BIG]);
+        P2_CK(cudaMemcpyAsync(big.data(), R.big, big.size() * sizeof(Group), cudaMemcpyDeviceToHost, st), "d2h");
+        P2_CK(cudaStreamSynchronize(st), "d2h");
+        std::sort(big.begin(), big.end(), [](const Group& a, const Group& b) { return a.sample < b.sample; });
+        P2_CK(cudaMemcpyAsync(R.big, big.data(), big.size() * sizeof(Group), cudaMemcpyHostToDevice, st), "h2d");
+        P2_CK(W == 1 ? set_smem_cap(k_big<1>, sm) : set_smem_cap(k_big<2>, sm), "smem");
+        for (size_t a = 0; a < big.size();) {
+            size_t b = a;
+            uint64_t nk = 0, most = 0;
+            while (b < big.size() && big[b].sample == big[a].sample && b - a < 32768) {
+                nk += big[b].keys;
+                most = std::max<uint64_t>(most, big[b].hi - big[b].lo);
+                ++b;
+            }
+            const dim3 grid((unsigned)std::min<uint64_t>((most + BIG_CHUNK - 1) / BIG_CHUNK, cgrid), (unsigned)(b - a));
+            const tg_status s = in_table(nk, big[a].sample, [&](const FallbackParams& F) {
+                Q.list = R.big;
+                Q.g_begin = a;
+                if (W == 1) k_big<1><<<grid, COUNT_THREADS, sm, st>>>(Q, F);
+                else k_big<2><<<grid, COUNT_THREADS, sm, st>>>(Q, F);
+                return cudaGetLastError();
+            }, true);
+            if (s == TG_OK) n_big += b - a;
+            else if (s != TG_ERR_OOM && !(s == TG_ERR_TABLE && err.empty())) return s;
+            else P2_CK(rounds(R.big + a, b - a), "k_rounds");
+            a = b;
+        }
+    }
+    if (h[P2C_HEAVY]) P2_CK(rounds(R.heavy, h[P2C_HEAVY]), "k_rounds");
+    // ---- the others, in `waves` launches over slices of their list; each slice's output
+    // range goes to on_range as soon as it is final
     const uint32_t waves = ov.on_range && ov.wave_out && ov.wave_ev ? std::max<uint32_t>(1, std::min(ov.waves, 16u)) : 1;
-    P2_CK(cudaMemsetAsync(R.work, 0, 8 * 17, st), "memset");
+    P2_CK(cudaMemsetAsync(R.work, 0, 8 * 16, st), "memset");
     uint64_t done = 0;  // output keys already handed to on_range
-    for (int pass = 0;; ++pass) {
-        // pass p writes its split groups to retry[p & 1]; pass p + 1 counts them
-        Q.retry = R.retry[pass & 1];
-        Q.n_retry = R.aux + (pass & 1);
-        P2_CK(cudaMemsetAsync(Q.n_retry, 0, 8, st), "memset");
-        // the first pass in `waves` launches over slices of the group sequence;
-        // each slice's output range goes to on_range as soon as it is final
-        const uint32_t nw = pass == 0 ? waves : 1;
-        for (uint32_t wv = 0; wv < nw; ++wv) {
-            Q.g_begin = pass == 0 ? ngroups * wv / nw : 0;
-            Q.g_end = pass == 0 ? ngroups * (wv + 1) / nw : ~0ull;
-            Q.work = R.work + (pass == 0 ? wv : 16);
-            if (pass > 0) P2_CK(cudaMemsetAsync(Q.work, 0, 8, st), "memset");
-            if (W == 1) k_count<1><<<in.n_sm * COUNT_PER_SM, COUNT_THREADS, sm, st>>>(Q);
-            else k_count<2><<<in.n_sm * COUNT_PER_SM, COUNT_THREADS, sm, st>>>(Q);
+    for (uint32_t wv = 0; wv < waves; ++wv) {
+        Q.list = R.normal;
+        Q.g_begin = ngroups * wv / waves;
+        Q.g_end = ngroups * (wv + 1) / waves;
+        Q.work = R.work + wv;
+        if (Q.g_end > Q.g_begin) {
+            if (W == 1) k_count<1><<<cgrid, COUNT_THREADS, sm, st>>>(Q);
+            else k_count<2><<<cgrid, COUNT_THREADS, sm, st>>>(Q);
             P2_CK(cudaGetLastError(), "k_count");
             ++*launches;
-            if (nw > 1) {
-                if (ov.wave_out_dev) k_peek<<<1, 32, 0, st>>>(R.ctr + P2C_OUT, 1, nullptr, 0, ov.wave_out_dev + wv);
-                else P2_CK(cudaMemcpyAsync(ov.wave_out + wv, R.ctr + P2C_OUT, 8, cudaMemcpyDeviceToHost, st), "d2h");
-                P2_CK(cudaEventRecord(ov.wave_ev[wv], st), "event");
+        }
+        if (waves > 1) {
+            if (ov.wave_out_dev) k_peek<<<1, 32, 0, st>>>(R.ctr + P2C_OUT, 1, nullptr, 0, ov.wave_out_dev + wv);
+            else P2_CK(cudaMemcpyAsync(ov.wave_out + wv, R.ctr + P2C_OUT, 8, cudaMemcpyDeviceToHost, st), "d2h");
+            P2_CK(cudaEventRecord(ov.wave_ev[wv], st), "event");
+        }
+    }
+    if (waves > 1) {
+        for (uint32_t wv = 0; wv < waves; ++wv) {
+            P2_CK(cudaEventSynchronize(ov.wave_ev[wv]), "wave");
+            const uint64_t hi = std::min<uint64_t>(*(const volatile unsigned long long*)(ov.wave_out + wv), out.cap);
+            if (hi > done) {
+                const tg_status rs = ov.on_range(done, hi);
+                if (rs != TG_OK) { err = "result copy failed"; return rs; }
+                done = hi;
             }
         }
-        if (nw > 1) {
-            for (uint32_t wv = 0; wv < nw; ++wv) {
-                P2_CK(cudaEventSynchronize(ov.wave_ev[wv]), "wave");
-                const uint64_t hi = std::min<uint64_t>(*(const volatile unsigned long long*)(ov.wave_out + wv), out.cap);
-                if (hi > done) {
-                    const tg_status rs = ov.on_range(done, hi);
-                    if (rs != TG_OK) { err = "result copy failed"; return rs; }
-                    done = hi;
-                }
-            }
-        }
+    }
+    // ---- groups that came back as key-hash parts: pass p reads retry[p & 1], writes the other
+    for (int pass = 0;; ++pass) {
         unsigned long long hr[P2C_COUNT + 1];
-        P2_CK(read_counters(ov, Q.n_retry, 1, R.ctr, P2C_COUNT, hr, st), "phase 2");
+        P2_CK(read_counters(ov, R.aux + (pass & 1), 1, R.ctr, P2C_COUNT, hr, st), "phase 2");
         const unsigned long long nret = hr[0];
         for (int c = 0; c < P2C_COUNT; ++c) h[c] = hr[c + 1];
         if (nret > L.retry_cap) { err = "too many groups to split"; return TG_ERR_TABLE; }
         if (nret == 0) break;
-        const unsigned long long nl[2] = {0, nret};
-        P2_CK(cudaMemcpyAsync(R.aux + 2, nl, 16, cudaMemcpyHostToDevice, st), "h2d");
-        Q.list[0] = Q.list[1] = R.retry[pass & 1];
-        Q.n_list = R.aux + 2;
+        Q.retry = R.retry[(pass + 1) & 1];
+        Q.n_retry = R.aux + ((pass + 1) & 1);
+        P2_CK(cudaMemsetAsync(Q.n_retry, 0, 8, st), "memset");
+        P2_CK(rounds(R.retry[pass & 1], nret), "k_rounds");
     }
-    out.fallback_groups = h[P2C_FALLBACK];
+    out.fallback_groups = h[P2C_FALLBACK] + n_big;
     // ---- key ranges that did not fit in shared memory
     if (h[P2C_FALLBACK] > 0) {
         if (h[P2C_FALLBACK] > FALLBACK_CAP) { err = "too many overflowing groups"; return TG_ERR_TABLE; }
@@ -1148,40 +1444,17 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
         P2_CK(cudaMemcpyAsync(fl.data(), R.fb, fl.size() * sizeof(Group), cudaMemcpyDeviceToHost, st), "d2h");
         P2_CK(cudaStreamSynchronize(st), "d2h");
         for (const Group& g : fl) {
-            uint64_t S = 1024;
-            while (S < 2 * (g.hi - g.lo) + 2) S <<= 1;
-            if (S > (1ull << 32)) { err = "fallback table too large"; return TG_ERR_TABLE; }
-            const size_t kbytes = (size_t)S * key_bytes(W);
-            uint8_t* tab = static_cast<uint8_t*>(fallback_table(kbytes + (size_t)S * 4 + 16));
-            if (!tab) { err = "no room for the fallback table"; return TG_ERR_OOM; }
-            FallbackParams F{};
-            F.keys = R.keys;
-            F.lo = g.lo;
-            F.hi = g.hi;
-            F.parts = g.parts;
-            F.part = g.part;
-            F.sample = g.sample;
-            F.tkeys = tab;
-            F.tcnt = reinterpret_cast<uint32_t*>(tab + kbytes);
-            F.mask = (uint32_t)(S - 1);
-            F.fail = reinterpret_cast<uint32_t*>(tab + kbytes + (size_t)S * 4);
-            P2_CK(cudaMemsetAsync(F.fail, 0, 4, st), "memset");
-            const unsigned grid = (unsigned)in.n_sm * 4;
-            if (W == 1) {
-                k_fb_init<1><<<grid, 256, 0, st>>>(F.tkeys, F.tcnt, S);
-                k_fb_insert<1><<<grid, 256, 0, st>>>(F);
-                k_fb_extract<1><<<grid, 256, 0, st>>>(F.tkeys, F.tcnt, S, Q, g.sample);
-            } else {
-                k_fb_init<2><<<grid, 256, 0, st>>>(F.tkeys, F.tcnt, S);
-                k_fb_insert<2><<<grid, 256, 0, st>>>(F);
-                k_fb_extract<2><<<grid, 256, 0, st>>>(F.tkeys, F.tcnt, S, Q, g.sample);
-            }
-            P2_CK(cudaGetLastError(), "fallback");
-            *launches += 3;
-            uint32_t failed = 0;
-            P2_CK(cudaMemcpyAsync(&failed, F.fail, 4, cudaMemcpyDeviceToHost, st), "d2h");
-            P2_CK(cudaStreamSynchronize(st), "fallback");
-            if (failed) { err = "fallback table overflow"; return TG_ERR_TABLE; }
+            const tg_status s = in_table(g.keys, g.sample, [&](FallbackParams F) {
+                F.lo = g.lo;
+                F.hi = g.hi;
+                F.parts = g.parts;
+                F.part = g.part;
+                const unsigned grid = (unsigned)in.n_sm * 4;
+                if (W == 1) k_fb_insert<1><<<grid, 256, 0, st>>>(F);
+                else k_fb_insert<2><<<grid, 256, 0, st>>>(F);
+                return cudaGetLastError();
+            }, false);
+            if (s != TG_OK) return s;
         }
         P2_CK(read_counters(ov, R.ctr, P2C_COUNT, nullptr, 0, h, st), "fallback");
     }
@@ -1199,8 +1472,7 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
         const unsigned grid = (unsigned)in.n_sm * 8;
         k_samp_hist<<<grid, 256, 0, st>>>(out.samples, n, hist);
         P2_CK(cudaGetLastError(), "k_samp_hist");
-        P2_CK(launch_scan(hist, out.n_samples, out.sample_off, R.sums, out.sample_off + out.n_samples, st, launches),
-              "scan");
+        P2_CK(launch_scan(hist, out.n_samples, out.sample_off, R.sums, st, launches), "scan");
         unsigned long long* cur = R.scur;  // the offsets, copied, as cursors
         P2_CK(cudaMemcpyAsync(cur, out.sample_off, 8 * (size_t)out.n_samples, cudaMemcpyDeviceToDevice, st), "copy");
         if (out.reorder_after) P2_CK(cudaStreamWaitEvent(st, out.reorder_after, 0), "wait");
@@ -1210,8 +1482,8 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
         *launches += 2;
         P2_CK(cudaStreamSynchronize(st), "sample order");
     }
-    out.groups = h[P2C_NORMAL] + h[P2C_HEAVY];
-    out.heavy_groups = h[P2C_HEAVY];
+    out.groups = h[P2C_NORMAL] + h[P2C_HEAVY] + h[P2C_BIG];
+    out.heavy_groups = h[P2C_HEAVY] + h[P2C_BIG];
     if (out.n_out > out.cap) { err = "output capacity exceeded"; return TG_ERR_TABLE; }
     return TG_OK;
 }
