@@ -950,6 +950,7 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
     __shared__ uint32_t s_ndesc;
 
     const int tid = threadIdx.x, lane = tid & 31;
+    const unsigned below = (1u << lane) - 1;
     const uint32_t c = blockIdx.x;
     {
         const uint64_t* src = reinterpret_cast<const uint64_t*>(gT);
@@ -1107,28 +1108,26 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
                 cl = cs & own & ~(1u << top);
                 nrec = __popc(cl) + ((open && rs >= ownlo && rs < ownhi) ? 1u : 0u);
             }
-            uint32_t incl = nrec;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += y;
-            }
-            const uint32_t wtot = __shfl_sync(0xffffffffu, incl, 31);
+            const uint32_t wtot = __reduce_add_sync(0xffffffffu, nrec);
             if (wtot) {
                 uint32_t base = 0;
-                if (lane == 31) base = atomicAdd(&s_ndesc, wtot);
-                base = __shfl_sync(0xffffffffu, base, 31);
-                uint32_t idx = base + incl - nrec;
-                if (cut) {
-                    const int f0 = __ffs(cut) - 1;
-                    if (open && rs >= ownlo && rs < ownhi) put(idx++, pb + rs, (uint32_t)(kp0 + f0 - rs), rm);
-                    while (cl) {
+                if (lane == 0) base = atomicAdd(&s_ndesc, wtot);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                // one record per lane and step, the lanes' next to each other
+                const bool closes = cut && open && rs >= ownlo && rs < ownhi;
+                unsigned bal = __ballot_sync(0xffffffffu, closes);
+                if (closes)
+                    put(base + __popc(bal & below), pb + rs, (uint32_t)(kp0 + __ffs(cut) - 1 - rs), rm);
+                base += __popc(bal);
+                while ((bal = __ballot_sync(0xffffffffu, cl != 0)) != 0) {
+                    if (cl) {
                         const int cb = __ffs(cl) - 1;
                         cl &= cl - 1;
                         const uint32_t after = cut & (uint32_t)(~0ull << (cb + 1));
                         const int e = __ffs(after) - 1;
-                        put(idx++, pb + kp0 + cb, (uint32_t)(e - cb), s_mlo[cb * NT + tid]);
+                        put(base + __popc(bal & below), pb + kp0 + cb, (uint32_t)(e - cb), s_mlo[cb * NT + tid]);
                     }
+                    base += __popc(bal);
                 }
             }
             if (cut) {
