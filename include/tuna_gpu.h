@@ -361,8 +361,8 @@ tg_status tg_host_free(void* p);
  *     caller's own allocator takes the device's memory and before any stream
  *     capture; or set CUDA_MODULE_LOADING=EAGER to reserve it when the library
  *     is loaded. Later calls allocate nothing.
- *   - The call blocks the calling host thread twice while it runs: once after
- *     Phase 1, to size Phase 2 from the record counts, and at the end.
+ *   - The call blocks the calling host thread at the end (and in between for an
+ *     input with more than 65,536 k-mers of one minimizer bin).
  *   - gpu_parts: 0 or a power of two up to 4096, as tg_job_begin.
  *   - All calls share the one scratch array, so calls whose work overlaps on the
  *     GPU (two host threads, or two streams without ordering) race; serialise

@@ -48,41 +48,6 @@ using namespace tg;
 
 namespace {
 
-constexpr uint64_t FWD_SEED[4] = {0x3c8bfbb395c60474ULL, 0x3193c18562a02b4cULL, 0x295549f54be24456ULL,
-                                  0x20323ed082572324ULL};  // A C T G (nt codes), include/nt_hash.hpp:26-31
-
-inline uint64_t hrol(uint64_t x, int s) { s &= 63; return s ? (x << s) | (x >> (64 - s)) : x; }
-inline uint64_t hror(uint64_t x, int s) { s &= 63; return s ? (x >> s) | (x << (64 - s)) : x; }
-
-}  // namespace
-
-HashTables tg::make_hash_tables(int m) {
-    HashTables T;
-    for (int b = 0; b < 4; ++b) {
-        const int nt = b ^ (b >> 1);  // kache A0 C1 G2 T3 -> nt A0 C1 T2 G3
-        T.FW[b] = FWD_SEED[nt];
-        T.RV[b] = FWD_SEED[nt ^ 2];   // REV[b] = FWD[complement(b)], complement = b ^ 2
-    }
-    for (int o = 0; o < 4; ++o)
-        for (int i = 0; i < 4; ++i) {
-            T.CTF[o * 4 + i] = hrol(T.FW[o], m) ^ T.FW[i];
-            T.CTR[o * 4 + i] = hror(T.RV[o], 1) ^ hrol(T.RV[i], m - 1);
-        }
-    for (int v = 0; v < 256; ++v) {
-        uint64_t f = 0, r = 0;
-        for (int j = 0; j < 4; ++j) {
-            const int b = (v >> (6 - 2 * j)) & 3;
-            f ^= hrol(T.FW[b], 3 - j);
-            r ^= hrol(T.RV[b], j);
-        }
-        T.GF[v] = f;
-        T.GR[v] = r;
-    }
-    return T;
-}
-
-namespace {
-
 struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
@@ -99,6 +64,8 @@ uint32_t next_pow2_u32(uint64_t v) {
 constexpr size_t MISC_CUT_STATS = 0;    // u64[4]: k-mers, records, runs, extra packed records (k_cut)
 constexpr size_t MISC_BASES = 32;       // u64: ACGT bases (k_pack)
 constexpr size_t MISC_OVERFLOW = 40;    // u32: descriptor list overflow (k_cut)
+constexpr size_t MISC_MAX_DESC = 48;    // u32: descriptors of the longest list (k_cut)
+constexpr uint32_t MISC_READ = 7;       // u64 words read back after phase 1
 constexpr size_t MISC_DIGEST = 64;      // u64[4]: result digest (tg_job_result_digest)
 constexpr size_t MISC_NDESC = 256;      // u32[C]: descriptors per Phase-1 CTA
 constexpr size_t MISC_BYTES = MISC_NDESC + 4 * 65536;
@@ -738,14 +705,35 @@ struct CutSamples {
     uint32_t n = 0;
 };
 
-static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, const CutSamples& cs = CutSamples()) {
+// What phase 1 leaves in the first MISC_READ words of ctx->misc.
+struct P1Counts {
+    unsigned long long kmers = 0, records = 0, runs = 0, extra_recs = 0, bases = 0;
+    uint32_t overflow = 0, max_desc = 0;
+    P1Counts() = default;
+    explicit P1Counts(const volatile unsigned long long* w)
+        : kmers(w[0]), records(w[1]), runs(w[2]), extra_recs(w[3]), bases(w[4]), overflow((uint32_t)w[5]),
+          max_desc((uint32_t)w[6]) {}
+};
+
+static tg_status read_misc(tg_ctx* ctx, P1Counts& r) {
+    CK(launch_peek(ctx->misc.as<unsigned long long>(), MISC_READ, ctx->wave_out_dev + 16, ctx->st), "k_peek");
+    CK(cudaStreamSynchronize(ctx->st), "phase 1");
+    r = P1Counts(ctx->wave_out + 16);
+    return TG_OK;
+}
+
+// deferred: the cut is launched and not waited for; its descriptor lists have
+// room for a record at every position.
+static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, const CutSamples& cs = CutSamples(),
+                         P1Counts* counts = nullptr, bool deferred = false) {
     tg_ctx* ctx = j->ctx;
     const uint64_t n = j->n;
     const uint32_t p1 = 1u << p1_bits;
-    const size_t smem = cut_smem_bytes(j->w, j->o.k, p1, exp);
+    const int seg = cut_seg(j->w, j->o.k, n, (uint32_t)ctx->n_sm);
+    const size_t smem = cut_smem_bytes(j->w, j->o.k, p1, exp, seg);
     if (smem > ctx->smem_optin) return ctx->fail(TG_ERR_UNSUPPORTED, "phase-1 tile does not fit in shared memory");
-    const uint64_t tile = cut_tile(j->w, exp);
-    uint32_t C = (uint32_t)ctx->n_sm * cut_ctas_per_sm(j->w, j->o.k, p1, exp);
+    const uint64_t tile = cut_tile(j->w, exp, seg);
+    uint32_t C = (uint32_t)ctx->n_sm * cut_ctas_per_sm(j->w, j->o.k, p1, exp, seg);
     uint64_t chunk = (n + C - 1) / C;
     chunk = std::max<uint64_t>(tile, (chunk + tile - 1) / tile * tile);
     C = (uint32_t)std::max<uint64_t>(1, (n + chunk - 1) / chunk);
@@ -753,7 +741,7 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
     j->chunk = chunk;
     j->p1_bits = p1_bits;
     // descriptors: about 2/(w+2) records per k-mer for random minimizers; grow on overflow
-    double factor = std::min(1.0, 3.0 / (j->w + 2));
+    double factor = deferred ? 1.0 : std::min(1.0, 3.0 / (j->w + 2));
     for (int attempt = 0; attempt < 2; ++attempt) {
         const uint64_t cap = (uint64_t)(chunk * factor) + 2ull * tile + j->L + 64;
         j->desc_cap = cap;
@@ -763,12 +751,13 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
             const size_t kmers_off = 4 * (size_t)hist_kmers_offset(p1, C);
             CK(ctx->ensure(ctx->hist, kmers_off + (size_t)p1 * 8), "alloc histograms");
             CK(cudaMemsetAsync(ctx->hist.as<uint8_t>() + kmers_off, 0, (size_t)p1 * 8, ctx->st), "memset");
-        } else {
-            CK(ctx->ensure(ctx->hist, (size_t)8 << j->bin_bits), "alloc bin histogram");
+        } else if (attempt) {  // the first time they are zero (k_prepare)
             CK(cudaMemsetAsync(ctx->hist.p, 0, (size_t)8 << j->bin_bits, ctx->st), "memset");
         }
-        CK(cudaMemsetAsync(ctx->misc.as<uint8_t>() + MISC_CUT_STATS, 0, 32, ctx->st), "memset");
-        CK(cudaMemsetAsync(ctx->misc.as<uint8_t>() + MISC_OVERFLOW, 0, 4, ctx->st), "memset");
+        if (exp || attempt) {
+            CK(cudaMemsetAsync(ctx->misc.as<uint8_t>() + MISC_CUT_STATS, 0, 32, ctx->st), "memset");
+            CK(cudaMemsetAsync(ctx->misc.as<uint8_t>() + MISC_OVERFLOW, 0, 16, ctx->st), "memset");
+        }
         CutParams P{};
         P.packed = ctx->packed.as<uint32_t>();
         P.valid = ctx->valid.as<uint32_t>();
@@ -779,7 +768,9 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
         P.chunk = chunk;
         P.desc = ctx->desc.as<uint64_t>();
         P.desc_cap = cap;
+        P.seg = seg;
         P.n_desc = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_NDESC);
+        P.max_desc = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_MAX_DESC);
         P.hist = exp ? ctx->hist.as<uint32_t>() : nullptr;
         P.binhist = exp ? nullptr : ctx->hist.as<unsigned long long>();
         P.stats = reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_CUT_STATS);
@@ -794,10 +785,12 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
         CK(launch_cut(P, ctx->tables.as<HashTables>(), exp, ctx->st), "k_cut");
         CK(cudaEventRecord(ctx->ev[3], ctx->st), "event");
         ++*launches;
-        uint32_t ovf = 0;
-        CK(cudaMemcpyAsync(&ovf, ctx->misc.as<uint8_t>() + MISC_OVERFLOW, 4, cudaMemcpyDeviceToHost, ctx->st), "d2h");
-        CK(cudaStreamSynchronize(ctx->st), "k_cut");
-        if (!ovf) return TG_OK;
+        if (deferred) return TG_OK;
+        P1Counts r;
+        const tg_status s = read_misc(ctx, r);
+        if (s != TG_OK) return s;
+        if (counts) *counts = r;
+        if (!r.overflow) return TG_OK;
         factor = 1.0;  // every k-mer start can open a record at most once
     }
     return ctx->fail(TG_ERR_DEVICE, "descriptor capacity exceeded");
@@ -838,38 +831,20 @@ static tg_status d2h_pageable(tg_ctx* ctx, void* dst, const void* src, size_t by
 // (0: chosen from the input size).
 struct P1Out {
     SampleBins B;
-    unsigned long long cstats[4] = {0, 0, 0, 0};  // k-mers, records, runs, extra packed records
-    unsigned long long n_bases = 0;
-    std::vector<uint32_t> nd;                   // descriptors per list
+    P1Counts c;  // deferred: not yet read
 };
 
-static tg_status run_phase1(tg_job* j, int* launches_out, P1Out& r, uint32_t p1_force = 0) {
+static tg_status run_phase1(tg_job* j, int* launches_out, P1Out& r, uint32_t p1_force = 0, bool deferred = false) {
     tg_ctx* ctx = j->ctx;
     int launches = 0;
     const uint64_t n = j->n;
     if (n >= (1ull << DESC_START_BITS)) return ctx->fail(TG_ERR_ARG, "input stream longer than 2^36 bytes");
-    // hash tables for m
     CK(ctx->ensure(ctx->tables, sizeof(HashTables)), "alloc tables");
-    if (ctx->prepared_m != j->o.m) {
-        const HashTables T = make_hash_tables(j->o.m);
-        CK(cudaMemcpy(ctx->tables.p, &T, sizeof T, cudaMemcpyHostToDevice), "upload tables");
-        ctx->prepared_m = j->o.m;
-    }
     CK(ctx->ensure(ctx->misc, MISC_BYTES), "alloc misc");
-    // ---- pack
     const uint64_t pw = packed_words_for(n);
     j->packed_words = pw;
     CK(ctx->ensure(ctx->packed, pw * 4), "alloc packed");
     CK(ctx->ensure(ctx->valid, (pw / 2) * 4 + 64), "alloc valid");
-    CK(cudaMemsetAsync(ctx->misc.p, 0, MISC_NDESC, ctx->st), "memset");
-    CK(cudaEventRecord(ctx->ev[0], ctx->st), "event");
-    CK(launch_pack(j->seq_ptr(), n, ctx->packed.as<uint32_t>(), ctx->valid.as<uint32_t>(), pw,
-                   reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_BASES), ctx->st), "k_pack");
-    ++launches;
-    CK(cudaEventRecord(ctx->ev[1], ctx->st), "event");
-    CK(cudaMemcpyAsync(&r.n_bases, ctx->misc.as<uint8_t>() + MISC_BASES, 8, cudaMemcpyDeviceToHost, ctx->st), "d2h");
-    // ---- phase 1: cut
-    nvtxMarkA("tuna.phase1");
     uint32_t p1 = p1_force ? p1_force : j->o.gpu_parts;
     if (!p1) p1 = std::max(j->n_shards, std::min<uint32_t>(1024, std::max<uint32_t>(16, next_pow2_u32(n / 32768))));
     uint32_t p1_bits = 0;
@@ -882,31 +857,50 @@ static tg_status run_phase1(tg_job* j, int* launches_out, P1Out& r, uint32_t p1_
     const SampleBins& B = r.B;
     const uint32_t ns = (uint32_t)B.base.size();
     if (j->n_shards > 1 && ns > 1) return ctx->fail(TG_ERR_UNSUPPORTED, "a job of several samples cannot be sharded");
-    {
-        const size_t bytes = 8 * (size_t)(ns + 1) + 4 * (size_t)ns + ns + 64;
-        CK(ctx->ensure(ctx->samp, bytes), "alloc samples");
-        uint8_t* d = ctx->samp.as<uint8_t>();
-        CK(cudaMemcpyAsync(d, B.start.data(), 8 * (size_t)(ns + 1), cudaMemcpyHostToDevice, ctx->st), "h2d");
-        CK(cudaMemcpyAsync(d + 8 * (size_t)(ns + 1), B.base.data(), 4 * (size_t)ns, cudaMemcpyHostToDevice, ctx->st),
-           "h2d");
-        CK(cudaMemcpyAsync(d + 12 * (size_t)ns + 8, B.bits.data(), ns, cudaMemcpyHostToDevice, ctx->st), "h2d");
+    CK(ctx->ensure(ctx->hist, (size_t)8 << j->bin_bits), "alloc bin histogram");
+    CK(ctx->ensure(ctx->samp, 8 * (size_t)(ns + 1) + 4 * (size_t)ns + ns + 64), "alloc samples");
+    uint8_t* d_samp = ctx->samp.as<uint8_t>();
+    PrepareParams pp{};
+    pp.misc = ctx->misc.as<unsigned long long>();
+    pp.n_misc = MISC_NDESC / 8;
+    pp.hist = ctx->hist.as<unsigned long long>();
+    pp.n_bins = 1u << j->bin_bits;
+    if (ctx->prepared_m != j->o.m) {
+        pp.tables = ctx->tables.as<HashTables>();
+        pp.m = j->o.m;
     }
+    if (ns == 1) {
+        pp.sample_start = ctx->samp.as<unsigned long long>();
+        pp.sample_bin_base = reinterpret_cast<uint32_t*>(d_samp + 16);
+        pp.sample_bin_bits = d_samp + 20;
+        pp.n = n;
+        pp.bin_bits = j->bin_bits;
+    }
+    CK(launch_prepare(pp, ctx->st), "k_prepare");
+    ctx->prepared_m = j->o.m;
+    ++launches;
+    if (ns > 1) {
+        CK(cudaMemcpyAsync(d_samp, B.start.data(), 8 * (size_t)(ns + 1), cudaMemcpyHostToDevice, ctx->st), "h2d");
+        CK(cudaMemcpyAsync(d_samp + 8 * (size_t)(ns + 1), B.base.data(), 4 * (size_t)ns, cudaMemcpyHostToDevice, ctx->st),
+           "h2d");
+        CK(cudaMemcpyAsync(d_samp + 12 * (size_t)ns + 8, B.bits.data(), ns, cudaMemcpyHostToDevice, ctx->st), "h2d");
+    }
+    // ---- pack
+    CK(cudaEventRecord(ctx->ev[0], ctx->st), "event");
+    CK(launch_pack(j->seq_ptr(), n, ctx->packed.as<uint32_t>(), ctx->valid.as<uint32_t>(), pw,
+                   reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_BASES), ctx->st), "k_pack");
+    ++launches;
+    CK(cudaEventRecord(ctx->ev[1], ctx->st), "event");
+    // ---- phase 1: cut
+    nvtxMarkA("tuna.phase1");
     CutSamples cs;
     cs.start = ctx->samp.as<unsigned long long>();
     cs.base = reinterpret_cast<const uint32_t*>(ctx->samp.as<uint8_t>() + 8 * (size_t)(ns + 1));
     cs.bits = ctx->samp.as<uint8_t>() + 12 * (size_t)ns + 8;
     cs.n = ns;
-    tg_status s = run_cut(j, false, p1_bits, &launches, cs);
+    const tg_status s = run_cut(j, false, p1_bits, &launches, cs, &r.c, deferred);
     *launches_out += launches;
-    if (s != TG_OK) return s;
-    const uint32_t C = j->n_cta;
-    r.nd.assign(C, 0);
-    CK(cudaMemcpyAsync(r.cstats, ctx->misc.as<uint8_t>() + MISC_CUT_STATS, 32, cudaMemcpyDeviceToHost, ctx->st),
-       "d2h");
-    CK(cudaMemcpyAsync(r.nd.data(), ctx->misc.as<uint8_t>() + MISC_NDESC, (size_t)C * 4, cudaMemcpyDeviceToHost,
-                       ctx->st), "d2h");
-    CK(cudaStreamSynchronize(ctx->st), "phase 1");
-    return TG_OK;
+    return s;
 }
 
 static tg_status run_spill(tg_job* j);
@@ -922,15 +916,15 @@ static tg_status tg_job_run_impl(tg_job* j) {
     const int k = j->o.k;
     const int W = j->W;
     j->ran = true;
+    const uint64_t per_key = 2 * key_bytes(W) + 4 + 24;  // key, pair, groups and slack
+    const bool deferred = j->n <= DEFER_BYTES && j->n_shards == 1 &&
+                          (!ctx->hbm_budget || std::max<uint64_t>(j->n, 1) * per_key <= ctx->hbm_budget);
     P1Out r1;
-    const tg_status s1 = run_phase1(j, &launches, r1);
+    const tg_status s1 = run_phase1(j, &launches, r1, 0, deferred);
     if (s1 != TG_OK) return s1;
     const SampleBins& B = r1.B;
     const uint32_t ns = (uint32_t)B.base.size();
-    const unsigned long long* cstats = r1.cstats;
-    const unsigned long long n_bases = r1.n_bases;
     const uint32_t C = j->n_cta;
-    std::vector<uint32_t>& nd = r1.nd;
     nvtxMarkA("tuna.phase2");
     // ---- phase 2: one run over all bins or, when their keys and pairs do not
     // fit in the memory budget, passes over ranges of consecutive segments
@@ -943,7 +937,8 @@ static tg_status tg_job_run_impl(tg_job* j) {
         hist.resize((size_t)1 << j->bin_bits);
         return cudaMemcpy(hist.data(), ctx->hist.p, hist.size() * 8, cudaMemcpyDeviceToHost);
     };
-    uint64_t n_kmers = cstats[0], n_recs = cstats[1] + cstats[3];
+    // deferred: at most one k-mer, and one record, per position
+    uint64_t n_kmers = deferred ? j->n : r1.c.kmers, n_recs = deferred ? j->n : r1.c.records + r1.c.extra_recs;
     if (j->n_shards > 1) {  // one sample: 2^p1_bits >= n_shards segments of consecutive bins
         const size_t P = B.segs.size();
         segs.assign(B.segs.begin() + P * j->shard / j->n_shards, B.segs.begin() + P * (j->shard + 1) / j->n_shards);
@@ -972,7 +967,12 @@ static tg_status tg_job_run_impl(tg_job* j) {
     in.desc_cap = j->desc_cap;
     in.n_lists = C;
     in.n_desc = reinterpret_cast<const uint32_t*>(ctx->misc.as<uint8_t>() + MISC_NDESC);
-    in.max_desc = (uint32_t)std::min<uint64_t>(*std::max_element(nd.begin(), nd.end()), j->desc_cap);
+    in.max_desc = (uint32_t)(deferred ? j->desc_cap : std::min<uint64_t>(r1.c.max_desc, j->desc_cap));
+    in.deferred = deferred;
+    if (deferred) {
+        in.read_back = ctx->misc.as<unsigned long long>();
+        in.n_read = MISC_READ;
+    }
     in.binhist = ctx->hist.as<unsigned long long>();
     in.n_kmers = n_kmers;
     in.n_recs = n_recs;
@@ -981,14 +981,21 @@ static tg_status tg_job_run_impl(tg_job* j) {
     in.n_samples = ns;
     std::vector<std::pair<uint32_t, uint32_t>> passes;  // segment ranges
     std::vector<uint64_t> seg_keys, seg_recs;
-    {
-        const uint64_t per_key = 2 * key_bytes(W) + 4 + 24;  // key, pair, groups and slack
-        size_t free_b = 0, total_b = 0;
-        CK(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-        const uint64_t have = free_b + ctx->scratch.cap + ctx->okeys.cap + ctx->ocnt.cap;
-        const uint64_t reserve = (2ull << 30) + total_b / 50;
-        const uint64_t budget = ctx->hbm_budget ? ctx->hbm_budget : (have > reserve ? have - reserve : 0);
-        if (ns == 1 && segs.size() > 1 && n_kmers * per_key > budget) {
+    // whether they fit is asked of the device (tens of microseconds) only when a
+    // buffer has to grow; a small job's always fit
+    in.group_pct = ctx->tuned_pct[W - 1] ? ctx->tuned_pct[W - 1] : 50;
+    const bool held = !ctx->hbm_budget && ctx->okeys.cap >= n_kmers * key_bytes(W) && ctx->ocnt.cap >= n_kmers * 4 &&
+                      ctx->scratch.cap >= phase2_scratch_bytes(in);
+    if (!deferred && !held && ns == 1 && segs.size() > 1) {
+        uint64_t budget = ctx->hbm_budget;
+        if (!budget) {
+            size_t free_b = 0, total_b = 0;
+            CK(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+            const uint64_t have = free_b + ctx->scratch.cap + ctx->okeys.cap + ctx->ocnt.cap;
+            const uint64_t reserve = (2ull << 30) + total_b / 50;
+            budget = have > reserve ? have - reserve : 0;
+        }
+        if (n_kmers * per_key > budget) {
             CK(load_hist(), "d2h");
             const uint64_t max_keys = std::max<uint64_t>(1, budget / per_key);
             uint32_t s0 = 0;
@@ -1072,6 +1079,7 @@ static tg_status tg_job_run_impl(tg_job* j) {
         const tg_status ps = phase2_run(in, ctx->scratch.p, p2_bytes, out, fallback_table, ctx->st, ctx->ev[7],
                                         &launches, msg, j->overlap ? *j->overlap : P2Overlap());
         if (ps != TG_OK) return ctx->fail(ps, msg);
+        if (deferred) r1.c = P1Counts(out.read_back);
         CK(cudaEventRecord(ctx->ev[8], ctx->st), "event");
         CK(cudaEventSynchronize(ctx->ev[8]), "sync");
         j->n_out = out.n_out;
@@ -1161,13 +1169,13 @@ static tg_status tg_job_run_impl(tg_job* j) {
         j->n_out = acc;
     }
     // ---- stats
-    S.bases = n_bases;
-    S.runs = cstats[2];
-    S.kmers = cstats[0];
-    S.superkmers = cstats[1];
+    S.bases = r1.c.bases;
+    S.runs = r1.c.runs;
+    S.kmers = r1.c.kmers;
+    S.superkmers = r1.c.records;
     S.out = j->n_out;
     S.gpu_parts = (uint32_t)B.segs.size();
-    S.record_bytes = cstats[1] * 8;
+    S.record_bytes = r1.c.records * 8;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]); S.pack_ms = ms;
     cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]); S.phase1_cut_ms = ms;
     S.phase1_scatter_ms = 0;  // records stay in the cut's lists
@@ -1322,10 +1330,10 @@ static tg_status spill_flush(tg_job* j) {
         S.n_desc[b] += rn;
         S.n_bytes[b] += bn;
     }
-    S.kmers += r.cstats[0];
-    S.records += r.cstats[1];
-    S.runs += r.cstats[2];
-    S.bases += r.n_bases;
+    S.kmers += r.c.kmers;
+    S.records += r.c.records;
+    S.runs += r.c.runs;
+    S.bases += r.c.bases;
     S.spilled_bytes += recs * 8 + bytes;
     ++S.chunks;
     j->n = 0;
@@ -1821,12 +1829,13 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
     const int W = j->W;
     uint64_t* kdst = keys ? keys + base * W : nullptr;
     uint32_t* cdst = counts ? counts + base : nullptr;
-    // one buffer, separators everywhere, then every sample copied to its place
+    // one buffer, separators between samples, then every sample copied to its place
     uint64_t total = 0;
     for (uint32_t i = a; i < b; ++i) {
         if (!seqs[i] && lens[i]) s = TG_ERR_ARG;
-        total += lens[i] + 1;
+        total += lens[i] + (n > 1 ? 1 : 0);
     }
+    bool fed = false;
     if (s == TG_OK && fastx) {
         // each sample's FASTA/FASTQ bytes lexed on the device into its own sample
         // (an empty sample stays empty)
@@ -1835,10 +1844,11 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
             if (s == TG_OK && lens[i]) s = lex_append_host(j, seqs[i], lens[i]);
         }
     } else if (s == TG_OK && total) {
-        const double t0 = now_ms();
+        // not waited for: the call returns only after the counts, or waits when it fails
         cudaError_t e = cudaSetDevice(ctx->device);
         if (e == cudaSuccess) e = ctx->ensure(ctx->seq, total + 1);
-        if (e == cudaSuccess) e = cudaMemsetAsync(ctx->seq.p, '\n', total, ctx->st);
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->ev[9], ctx->st);
+        if (e == cudaSuccess && n > 1) e = cudaMemsetAsync(ctx->seq.p, '\n', total, ctx->st);
         uint64_t off = 0;
         for (uint32_t i = a; i < b && e == cudaSuccess; ++i) {
             if (i > a) j->sample_start.push_back(off);
@@ -1847,11 +1857,10 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
             off += lens[i] + 1;
             j->st.input_bytes += lens[i];
         }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
         if (e != cudaSuccess) s = ctx->cuda_fail(e, "copy input");
         j->n = total;
         j->used_ctx_seq = true;
-        j->st.h2d_ms += now_ms() - t0;
+        fed = true;
     }
     P2Overlap ov;
     ov.waves = 8;
@@ -1880,6 +1889,11 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
     j->sink_counts = cdst;
     j->sink_cap = room;
     if (s == TG_OK) s = tg_job_run(j);
+    if (fed) {
+        float ms = 0;
+        if (s != TG_OK) cudaStreamSynchronize(ctx->st);
+        else if (cudaEventElapsedTime(&ms, ctx->ev[9], ctx->ev[0]) == cudaSuccess) j->st.h2d_ms += ms;
+    }
     if (s == TG_OK && multi) {
         const uint64_t h = std::min<uint64_t>(j->n_out, room);
         const double t0 = now_ms();

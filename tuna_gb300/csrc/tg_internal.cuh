@@ -93,10 +93,12 @@ struct CutParams {
     uint32_t L;              // max k-mers per record (forced split period)
     uint32_t p1_bits;        // log2 internal bucket count
     uint32_t n_cta;
+    int seg;                 // counting cut: k-mer start positions per thread and tile (cut_seg)
     uint64_t chunk;          // k-mer start positions per CTA (multiple of CUT_TILE)
     uint64_t* desc;          // [n_cta][desc_cap] record descriptors
     uint64_t desc_cap;
     uint32_t* n_desc;        // [n_cta]
+    uint32_t* max_desc;      // counting cut: the most of them
     uint32_t* hist;          // export cut: u32 [P][n_cta] records, then u64 [P] k-mers per bucket
     unsigned long long* binhist;  // counting cut: [bins] k-mers + 2^32 x packed records per bin
     int desc_sb;             // counting cut: start bits of a descriptor (desc_start_bits)
@@ -109,6 +111,21 @@ struct CutParams {
     uint32_t* overflow;      // set when a CTA's descriptor list is full
     // export mode: full descriptors (start, minimizer hash, min_pos, nk)
     uint64_t* xdesc;         // [n_cta][desc_cap][3] or null
+};
+
+// Written before the cut (k_prepare). Null pointers: nothing of that kind.
+struct PrepareParams {
+    unsigned long long* misc;   // n_misc (at most 256) counters to zero
+    uint32_t n_misc;
+    unsigned long long* hist;   // n_bins bin counts to zero (n_bins even, 16-byte aligned)
+    uint32_t n_bins;
+    HashTables* tables;         // of m
+    int m;
+    unsigned long long* sample_start;  // a job of one sample of n bytes with 2^bin_bits bins
+    uint32_t* sample_bin_base;
+    uint8_t* sample_bin_bits;
+    uint64_t n;
+    int bin_bits;
 };
 
 // Packed record: the bases of up to REC_MAX consecutive k-mers, 16 x W bytes.
@@ -157,6 +174,7 @@ struct KeysParams {
     const Segment* segs;               // k_plan: one warp per segment
     uint32_t n_segs;
     uint32_t target;                   // k-mer instances per group
+    uint32_t store;                    // the most that k_count takes
     int k;
     void* recs;                        // packed records
     Group* groups[3];                  // [0] normal, [1] heavy, [2] big
@@ -171,6 +189,7 @@ struct CountParams {
     const void* recs;                  // packed records
     int k;
     const Group* list;
+    const unsigned long long* n_list;  // entries of list, or null: g_end is at most their number
     Group* retry;                      // failed groups, split
     unsigned long long* n_retry;
     uint64_t retry_cap;

@@ -13,9 +13,15 @@
 #include "tg_internal.cuh"
 
 namespace tg {
-size_t cut_smem_bytes(int w, int k, uint32_t p1, bool exp);
-uint64_t cut_tile(int w, bool exp);                 // k-mer start positions per tile of a cut CTA
-uint32_t cut_ctas_per_sm(int w, int k, uint32_t p1, bool exp);
+// A job of at most this many stream bytes runs in one go: buffers sized by bounds, the
+// counts read on the device, one wait at the end (P2Input::deferred).
+constexpr uint64_t DEFER_BYTES = 4u << 20;
+// Shapes of the cut; seg: k-mer start positions per thread and tile (cut_seg).
+size_t cut_smem_bytes(int w, int k, uint32_t p1, bool exp, int seg = 128);
+uint64_t cut_tile(int w, bool exp, int seg = 128);  // k-mer start positions per tile of a cut CTA
+uint32_t cut_ctas_per_sm(int w, int k, uint32_t p1, bool exp, int seg = 128);
+int cut_seg(int w, int k, uint64_t n, uint32_t n_sm);
+cudaError_t launch_prepare(const PrepareParams& P, cudaStream_t st);
 // Packed words (a multiple of 4) for a stream of n bytes, padding included.
 uint64_t packed_words_for(uint64_t n);
 cudaError_t launch_pack(const uint8_t* seq, uint64_t n, uint32_t* packed, uint32_t* valid, uint64_t n_words,
@@ -119,6 +125,12 @@ struct P2Input {
     uint32_t all_bins = 1u << BIN_BITS;  // bins of the job
     int desc_sb = DESC_START_BITS;       // start bits of a descriptor
     uint32_t group_pct = 50;  // keys per group, % of the table's slots
+    // Phase 1 may still run: n_kmers, n_recs and max_desc are upper bounds, the
+    // counts are read on the device, and the host waits once, at the end; read_back
+    // (n_read u64, device) then goes to P2Output::read_back.
+    bool deferred = false;
+    const unsigned long long* read_back = nullptr;
+    uint32_t n_read = 0;
 };
 struct P2Output {
     void* keys;                        // u64 x W per distinct k-mer
@@ -135,6 +147,7 @@ struct P2Output {
     // the sample-major scatter waits for this event first (an earlier job's
     // copy of keys2/counts2 to the host may still be running), or null
     cudaEvent_t reorder_after = nullptr;
+    unsigned long long read_back[8] = {};
 };
 // Results handed out while phase 2 still runs: the first counting pass runs in
 // `waves` launches, and after each one on_range(lo, hi) is called (on the host,
@@ -153,6 +166,8 @@ struct P2Overlap {
 // not by cudaMemcpyAsync: a copy-engine read would queue behind the result
 // copies already issued on the copy stream.
 constexpr uint32_t OVERLAP_WORDS = 64;
+// n u64 of device memory to mapped host memory (device address dst), by a kernel.
+cudaError_t launch_peek(const unsigned long long* src, uint32_t n, unsigned long long* dst, cudaStream_t st);
 // Device scratch one run needs (packed records included).
 size_t phase2_scratch_bytes(const P2Input& in);
 // Runs phase 2 on `st` and waits for it. fallback_table(bytes) returns device
@@ -161,8 +176,5 @@ size_t phase2_scratch_bytes(const P2Input& in);
 tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Output& out,
                      const std::function<void*(size_t)>& fallback_table, cudaStream_t st, cudaEvent_t ev_keys,
                      int* launches, std::string& err, const P2Overlap& ov = P2Overlap());
-
-// ntHash roll / init tables for minimizer length m (host side).
-HashTables make_hash_tables(int m);
 
 }  // namespace tg

@@ -47,6 +47,10 @@ namespace {
 std::mutex g_mu;
 constexpr int MAX_DEV = 64;
 uint8_t* g_scratch_addr[MAX_DEV] = {};
+// Page-locked, mapped host words per device for the counters read back, made with
+// the scratch array's address.
+unsigned long long* g_words[MAX_DEV] = {};
+unsigned long long* g_words_dev[MAX_DEV] = {};
 
 void set_err(char* buf, size_t len, const std::string& msg) {
     if (buf && len) {
@@ -64,6 +68,14 @@ cudaError_t scratch_address(int dev, uint8_t** out) {
         void* p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, tg_noalloc_scratch);
         if (e != cudaSuccess) return e;
+        void *w = nullptr, *wd = nullptr;
+        if (cudaHostAlloc(&w, OVERLAP_WORDS * 8, cudaHostAllocMapped) == cudaSuccess &&
+            cudaHostGetDevicePointer(&wd, w, 0) == cudaSuccess) {
+            g_words[dev] = static_cast<unsigned long long*>(w);
+            g_words_dev[dev] = static_cast<unsigned long long*>(wd);
+        } else {
+            (void)cudaGetLastError();  // without them the counters are copied
+        }
         g_scratch_addr[dev] = static_cast<uint8_t*>(p);
     }
     *out = g_scratch_addr[dev];
@@ -148,8 +160,9 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     uint32_t p1_bits = 0;
     while ((1u << p1_bits) < p1) ++p1_bits;
     p1 = 1u << p1_bits;
-    const uint64_t tile = cut_tile(w, false);
-    uint32_t C = (uint32_t)n_sm * cut_ctas_per_sm(w, k, p1, false);
+    const int seg = cut_seg(w, k, n, (uint32_t)n_sm);
+    const uint64_t tile = cut_tile(w, false, seg);
+    uint32_t C = (uint32_t)n_sm * cut_ctas_per_sm(w, k, p1, false, seg);
     uint64_t chunk = (n + C - 1) / C;
     chunk = std::max<uint64_t>(tile, (chunk + tile - 1) / tile * tile);
     C = (uint32_t)std::max<uint64_t>(1, (n + chunk - 1) / chunk);
@@ -164,16 +177,22 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     uint32_t* s_base = cv.take<uint32_t>(1);
     uint8_t* s_bits = cv.take<uint8_t>(1);
     if (!cv.ok) { set_err(errbuf, errlen, "input too large for the no-allocation scratch"); return TG_ERR_ARG; }
-    // counters in misc (u64 indices): [0..3] k-mers, records, runs, extra packed records, [4] bases, [5] overflow (u32)
-    uint32_t* overflow = reinterpret_cast<uint32_t*>(misc + 5);
-
-    const HashTables T = make_hash_tables(m);
-    NA_CK(cudaMemcpyAsync(tables, &T, sizeof T, cudaMemcpyHostToDevice, st), "upload tables");
-    NA_CK(cudaMemsetAsync(misc, 0, 32 * 8, st), "memset");
-    NA_CK(cudaMemsetAsync(binhist, 0, (size_t)8 << bin_bits, st), "memset");
-    NA_CK(cudaMemcpyAsync(s_start, B.start.data(), 16, cudaMemcpyHostToDevice, st), "h2d");
-    NA_CK(cudaMemcpyAsync(s_base, B.base.data(), 4, cudaMemcpyHostToDevice, st), "h2d");
-    NA_CK(cudaMemcpyAsync(s_bits, B.bits.data(), 1, cudaMemcpyHostToDevice, st), "h2d");
+    // counters in misc (u64 indices): [0..3] k-mers, records, runs, extra packed records, [4] bases,
+    // [5] overflow (u32), [6] descriptors of the longest list (u32)
+    constexpr uint32_t N_MISC = 7;
+    PrepareParams pp{};
+    pp.misc = misc;
+    pp.n_misc = N_MISC;
+    pp.hist = binhist;
+    pp.n_bins = 1u << bin_bits;
+    pp.tables = tables;
+    pp.m = m;
+    pp.sample_start = s_start;
+    pp.sample_bin_base = s_base;
+    pp.sample_bin_bits = s_bits;
+    pp.n = n;
+    pp.bin_bits = bin_bits;
+    NA_CK(launch_prepare(pp, st), "k_prepare");
     // ---- phase 1
     NA_CK(launch_pack(d_seq, n, packed, valid, pw, misc + 4, st), "k_pack");
     CutParams P{};
@@ -181,25 +200,19 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     P.k = k; P.m = m; P.w = w; P.L = L;
     P.p1_bits = p1_bits; P.n_cta = C; P.chunk = chunk;
     P.desc = desc; P.desc_cap = desc_cap; P.n_desc = n_desc;
-    P.hist = nullptr; P.binhist = binhist; P.stats = misc; P.overflow = overflow; P.xdesc = nullptr;
+    P.hist = nullptr; P.binhist = binhist; P.stats = misc; P.overflow = reinterpret_cast<uint32_t*>(misc + 5); P.xdesc = nullptr;
+    P.seg = seg; P.max_desc = reinterpret_cast<uint32_t*>(misc + 6);
     P.sample_start = s_start; P.sample_bin_base = s_base; P.sample_bin_bits = s_bits; P.n_samples = 1;
     P.desc_sb = desc_start_bits(bin_bits);
     NA_CK(launch_cut(P, tables, false, st), "k_cut");
     int launches = 0;
-    std::vector<uint32_t> nd(C);
-    unsigned long long cstats[4] = {0, 0, 0, 0};
-    uint32_t ovf = 0;
-    NA_CK(cudaMemcpyAsync(nd.data(), n_desc, (size_t)C * 4, cudaMemcpyDeviceToHost, st), "d2h");
-    NA_CK(cudaMemcpyAsync(cstats, misc, 32, cudaMemcpyDeviceToHost, st), "d2h");
-    NA_CK(cudaMemcpyAsync(&ovf, overflow, 4, cudaMemcpyDeviceToHost, st), "d2h");
-    NA_CK(cudaStreamSynchronize(st), "phase 1");
-    if (ovf) { set_err(errbuf, errlen, "descriptor capacity exceeded"); return TG_ERR_DEVICE; }
-    // ---- phase 2 in what is left
+    // ---- phase 2 in what is left, sized by bounds: at most a k-mer and a record per position
     P2Input in{};
     in.W = W; in.k = k; in.segs = B.segs.data(); in.n_segs = (uint32_t)B.segs.size(); in.n_sm = (uint32_t)n_sm;
     in.packed = packed; in.desc = desc; in.desc_cap = desc_cap; in.n_lists = C; in.n_desc = n_desc;
-    in.max_desc = (uint32_t)std::min<uint64_t>(*std::max_element(nd.begin(), nd.end()), desc_cap);
-    in.binhist = binhist; in.n_kmers = cstats[0]; in.n_recs = cstats[1] + cstats[3];
+    in.max_desc = (uint32_t)desc_cap;
+    in.deferred = true; in.read_back = misc; in.n_read = N_MISC;
+    in.binhist = binhist; in.n_kmers = n; in.n_recs = n;
     in.ci = o.ci; in.cx = o.cx;
     in.bin_hi = in.all_bins = 1u << bin_bits;
     in.desc_sb = desc_start_bits(bin_bits);
@@ -217,9 +230,13 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     P2Output out{};
     out.keys = d_keys; out.counts = d_counts; out.cap = cap;
     std::string msg;
+    P2Overlap ov;
+    ov.wave_out = g_words[dev];
+    ov.wave_out_dev = g_words_dev[dev];
     // straight into the caller's buffers
-    const tg_status ps = phase2_run(in, p2_scratch, p2_bytes, out, fallback_table, st, nullptr, &launches, msg);
+    const tg_status ps = phase2_run(in, p2_scratch, p2_bytes, out, fallback_table, st, nullptr, &launches, msg, ov);
     *n_out = out.n_out;
+    if (ps == TG_OK && (uint32_t)out.read_back[5]) { set_err(errbuf, errlen, "descriptor capacity exceeded"); return TG_ERR_DEVICE; }
     if (ps != TG_OK) {
         if (out.n_out > cap) {
             set_err(errbuf, errlen, "output capacity too small: " + std::to_string(out.n_out) + " k-mers");

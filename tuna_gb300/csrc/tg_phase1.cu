@@ -499,8 +499,11 @@ k_cut(CutParams P, const HashTables* __restrict__ gT) {
 // 7.12 ms for 0.93 Gbp; k=63 m=21 reads: 13.35 -> 11.86 ms against 64). The
 // forced split period L = 256 - k stays above SEG for every k <= 63, so a
 // segment holds at most one forced split.
-constexpr int SEG = 128;
-static_assert(SEG * 256 <= CUT_SPAN, "a cut tile must fit the packed arrays' slack");
+// Jobs too short to give every CTA a few tiles of such segments take 32 positions
+// per thread: more warm-up, but four times the CTAs and a quarter of the steps in
+// sequence (cut_seg).
+constexpr int LONG_SEG = 128, SHORT_SEG = 32;
+static_assert(LONG_SEG * 256 <= CUT_SPAN, "a cut tile must fit the packed arrays' slack");
 
 constexpr size_t SEQ_TABLE_BYTES = offsetof(HashTables, GF);
 
@@ -508,9 +511,9 @@ struct SeqSmem {
     size_t tables, pk, vb, vh, sum, total;
     uint32_t npk, nvb;
     __host__ __device__ static size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
-    __host__ __device__ void layout(int w, int nt, int k) {
-        // bases [t0 - 1, t0 + nt * SEG + k) from a 32-base boundary
-        const uint32_t span = (uint32_t)nt * SEG + (uint32_t)k + 96;
+    __host__ __device__ void layout(int w, int nt, int k, int seg) {
+        // bases [t0 - 1, t0 + nt * seg + k) from a 32-base boundary
+        const uint32_t span = (uint32_t)nt * seg + (uint32_t)k + 96;
         npk = span / 16 + 2;
         nvb = span / 32 + 2;
         size_t o = 0;
@@ -592,12 +595,12 @@ __device__ __forceinline__ int seq_excl_min_rev(int v, int* s_w, int& all) {
     return min(after, ex);
 }
 
-template <int NT>
+template <int NT, int SEG>
 __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 2)
 k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
     extern __shared__ __align__(16) uint8_t smem[];
     SeqSmem L;
-    L.layout(P.w, NT, P.k);
+    L.layout(P.w, NT, P.k, SEG);
     HashTables& T = *reinterpret_cast<HashTables*>(smem + L.tables);
     uint32_t* s_pk = reinterpret_cast<uint32_t*>(smem + L.pk);
     uint32_t* s_vb = reinterpret_cast<uint32_t*>(smem + L.vb);
@@ -806,7 +809,10 @@ k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
         __syncthreads();
     }
     // ---- counters
-    if (tid == 0) P.n_desc[c] = s_ndesc;
+    if (tid == 0) {
+        P.n_desc[c] = s_ndesc;
+        atomicMax(P.max_desc, s_ndesc);
+    }
     if (overflowed) atomicExch(P.overflow, 1u);
     for (int o = 16; o > 0; o >>= 1) {
         loc_kmers += __shfl_down_sync(0xffffffffu, loc_kmers, o);
@@ -853,7 +859,6 @@ struct FixedShape {
     static constexpr int W = K - MM, B = W + 1;
     static constexpr int R = 32 / B;            // blocks per batch
     static constexpr int SB = R * B;            // k-mers per batch (<= 32)
-    static constexpr int NBLK = (SEG + B - 1) / B;
     static constexpr int NT = 256;
     static_assert(B >= 2 && B <= 16, "fixed cut: window of 2..16 m-mers");
 };
@@ -863,10 +868,10 @@ struct FixedSmem {
     size_t tables, ct, pk, vb, mlo, sum, total;
     uint32_t npk, nvb;
     __host__ __device__ static size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
-    __host__ __device__ void layout(int nt, int k) {
-        // bases [t0 - 1, t0 + nt * SEG + 16 + k) from a 32-base boundary, with
+    __host__ __device__ void layout(int nt, int k, int seg) {
+        // bases [t0 - 1, t0 + nt * seg + 16 + k) from a 32-base boundary, with
         // room for the validity window of the last batch (128 bits)
-        const uint32_t span = (uint32_t)nt * SEG + (uint32_t)k + 288;
+        const uint32_t span = (uint32_t)nt * seg + (uint32_t)k + 288;
         npk = span / 16 + 2;
         nvb = span / 32 + 2;
         size_t o = 0;
@@ -925,14 +930,14 @@ __device__ __forceinline__ uint64_t run_and(uint64_t lo, uint64_t hi) {
 
 constexpr uint32_t FIXED_CUT_CTAS = 3;  // CTAs of 256 threads per SM
 
-template <int K, int MM>
+template <int K, int MM, int SEG>
 __global__ void __launch_bounds__(256, FIXED_CUT_CTAS)
 k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
     using S = FixedShape<K, MM>;
     constexpr int NT = S::NT, W = S::W, B = S::B, SB = S::SB, R = S::R;
     extern __shared__ __align__(16) uint8_t smem[];
     FixedSmem Ly;
-    Ly.layout(NT, K);
+    Ly.layout(NT, K, SEG);
     HashTables& T = *reinterpret_cast<HashTables*>(smem + Ly.tables);
     ulonglong2* s_ct = reinterpret_cast<ulonglong2*>(smem + Ly.ct);   // {CTF, CTR}[16]
     uint32_t* s_pk = reinterpret_cast<uint32_t*>(smem + Ly.pk);
@@ -1180,7 +1185,10 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
         if (tid == 0 && last_t >= 0) { s_carry_cs = s_cs[last_t]; s_carry_m = s_cm[last_t]; }
         __syncthreads();
     }
-    if (tid == 0) P.n_desc[c] = s_ndesc;
+    if (tid == 0) {
+        P.n_desc[c] = s_ndesc;
+        atomicMax(P.max_desc, s_ndesc);
+    }
     if (overflowed) atomicExch(P.overflow, 1u);
     for (int o = 16; o > 0; o >>= 1) {
         loc_kmers += __shfl_down_sync(0xffffffffu, loc_kmers, o);
@@ -1225,18 +1233,25 @@ __device__ __forceinline__ ScanPair scan_block_sum(ScanPair v, ScanPair* s_w) {
     return r;
 }
 
+// a thread's SCAN_PER consecutive counts (0 past the end) and their sum
+constexpr int SCAN_PER = SCAN_ITEMS / SCAN_T;
+template <typename T>
+__device__ __forceinline__ ScanPair scan_load(const T* in, uint64_t i0, uint64_t n, ScanPair (&v)[SCAN_PER]) {
+    ScanPair s{0, 0};
+#pragma unroll
+    for (int j = 0; j < SCAN_PER; ++j) {
+        v[j] = i0 + j < n ? scan_item(in[i0 + j]) : ScanPair{0, 0};
+        s.a += v[j].a;
+        s.b += v[j].b;
+    }
+    return s;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(SCAN_T) k_scan_sums(const T* __restrict__ in, uint64_t n, ScanPair* __restrict__ sums) {
     __shared__ ScanPair s_w[SCAN_T / 32];
-    const uint64_t b0 = (uint64_t)blockIdx.x * SCAN_ITEMS;
-    ScanPair acc{0, 0};
-    for (uint32_t i = threadIdx.x; i < SCAN_ITEMS; i += SCAN_T)
-        if (b0 + i < n) {
-            const ScanPair x = scan_item(in[b0 + i]);
-            acc.a += x.a;
-            acc.b += x.b;
-        }
-    const ScanPair t = scan_block_sum(acc, s_w);
+    ScanPair v[SCAN_PER];
+    const ScanPair t = scan_block_sum(scan_load(in, (uint64_t)blockIdx.x * SCAN_ITEMS + threadIdx.x * SCAN_PER, n, v), s_w);
     if (threadIdx.x == 0) sums[blockIdx.x] = t;
 }
 
@@ -1246,36 +1261,82 @@ __global__ void __launch_bounds__(SCAN_T) k_scan(const T* __restrict__ in, uint6
                                                  unsigned long long* __restrict__ total) {
     __shared__ ScanPair s_w[SCAN_T / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint64_t i0 = (uint64_t)blockIdx.x * SCAN_ITEMS + threadIdx.x * SCAN_PER;
+    ScanPair v[SCAN_PER];
+    const ScanPair mine = scan_load(in, i0, n, v);
     ScanPair run{0, 0};
     for (uint32_t i = threadIdx.x; i < blockIdx.x; i += SCAN_T) { run.a += sums[i].a; run.b += sums[i].b; }
-    run = scan_block_sum(run, s_w);
-    const uint64_t b0 = (uint64_t)blockIdx.x * SCAN_ITEMS;
-    for (uint32_t i0 = 0; i0 < SCAN_ITEMS && b0 + i0 < n; i0 += SCAN_T) {
-        const uint64_t i = b0 + i0 + threadIdx.x;
-        const ScanPair v = i < n ? scan_item(in[i]) : ScanPair{0, 0};
-        ScanPair x = v;
+    if (blockIdx.x) run = scan_block_sum(run, s_w);
+    ScanPair x = mine;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long ya = __shfl_up_sync(0xffffffffu, x.a, o), yb = __shfl_up_sync(0xffffffffu, x.b, o);
-            if (lane >= o) { x.a += ya; x.b += yb; }
-        }
-        __syncthreads();
-        if (lane == 31) s_w[wid] = x;
-        __syncthreads();
-        for (int w = 0; w < SCAN_T / 32; ++w) {
-            if (w < wid) { x.a += s_w[w].a; x.b += s_w[w].b; }
-        }
-        if (i < n) {
-            oa[i] = run.a + x.a - v.a;
-            if (ob) ob[i] = run.b + x.b - v.b;
-            if (i + 1 == n) {
-                oa[n] = run.a + x.a;
-                if (total) *total = run.a + x.a;
-                if (ob) ob[n] = run.b + x.b;
-            }
-        }
-        for (int w = 0; w < SCAN_T / 32; ++w) { run.a += s_w[w].a; run.b += s_w[w].b; }
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long ya = __shfl_up_sync(0xffffffffu, x.a, o), yb = __shfl_up_sync(0xffffffffu, x.b, o);
+        if (lane >= o) { x.a += ya; x.b += yb; }
     }
+    __syncthreads();
+    if (lane == 31) s_w[wid] = x;
+    __syncthreads();
+    for (int w = 0; w < wid; ++w) { run.a += s_w[w].a; run.b += s_w[w].b; }
+    run.a += x.a - mine.a;
+    run.b += x.b - mine.b;
+#pragma unroll
+    for (int j = 0; j < SCAN_PER; ++j) {
+        if (i0 + j < n) {
+            oa[i0 + j] = run.a;
+            if (ob) ob[i0 + j] = run.b;
+        }
+        run.a += v[j].a;
+        run.b += v[j].b;
+        if (i0 + j + 1 == n) {
+            oa[n] = run.a;
+            if (ob) ob[n] = run.b;
+            if (total) *total = run.a;
+        }
+    }
+}
+
+// ---------------------------------------------------------------- preparation
+// What has to be in place before the cut, in one launch instead of a memset or a
+// small copy each (a small call spent more time on those than on its kernels):
+// counters and the bin histogram at zero, the hash tables of m, the layout of a
+// job of one sample.
+__constant__ uint64_t c_fwd_seed[4] = {0x3c8bfbb395c60474ULL, 0x3193c18562a02b4cULL, 0x295549f54be24456ULL,
+                                       0x20323ed082572324ULL};  // A C T G (nt codes), include/nt_hash.hpp:26-31
+__device__ __forceinline__ uint64_t seed_fw(int b) { return c_fwd_seed[b ^ (b >> 1)]; }        // kache A0 C1 G2 T3
+__device__ __forceinline__ uint64_t seed_rv(int b) { return c_fwd_seed[(b ^ (b >> 1)) ^ 2]; }
+
+__global__ void __launch_bounds__(256) k_prepare(PrepareParams P) {
+    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    ulonglong2* h2 = reinterpret_cast<ulonglong2*>(P.hist);
+    for (uint32_t i = i0; i < P.n_bins / 2; i += stride) h2[i] = make_ulonglong2(0, 0);
+    if (blockIdx.x) return;
+    if (threadIdx.x < P.n_misc) P.misc[threadIdx.x] = 0;
+    if (P.sample_start && threadIdx.x == 0) {
+        P.sample_start[0] = 0;
+        P.sample_start[1] = P.n;
+        P.sample_bin_base[0] = 0;
+        P.sample_bin_bits[0] = (uint8_t)P.bin_bits;
+    }
+    if (!P.tables) return;
+    HashTables& T = *P.tables;
+    const int m = P.m;
+    if (threadIdx.x < 4) {
+        T.FW[threadIdx.x] = seed_fw(threadIdx.x);
+        T.RV[threadIdx.x] = seed_rv(threadIdx.x);
+    }
+    if (threadIdx.x < 16) {
+        const int o = threadIdx.x >> 2, i = threadIdx.x & 3;
+        T.CTF[threadIdx.x] = rol64(seed_fw(o), m) ^ seed_fw(i);
+        T.CTR[threadIdx.x] = ror64(seed_rv(o), 1) ^ rol64(seed_rv(i), m - 1);
+    }
+    uint64_t f = 0, r = 0;
+    for (int j = 0; j < 4; ++j) {
+        const int b = (threadIdx.x >> (6 - 2 * j)) & 3;
+        f ^= rol64(seed_fw(b), 3 - j);
+        r ^= rol64(seed_rv(b), j);
+    }
+    T.GF[threadIdx.x] = f;
+    T.GR[threadIdx.x] = r;
 }
 
 // ---------------------------------------------------------------- launchers
@@ -1286,7 +1347,7 @@ static bool fixed_cut(int k, int w) {
     return (k == 31 && (m == 21 || m == 23)) || (k == 21 && m == 17) || (k == 25 && m == 21);
 }
 
-size_t cut_smem_bytes(int w, int k, uint32_t p1, bool exp) {
+size_t cut_smem_bytes(int w, int k, uint32_t p1, bool exp, int seg) {
     if (exp) {
         CutSmem L;
         L.layout(w, p1, exp);
@@ -1294,18 +1355,18 @@ size_t cut_smem_bytes(int w, int k, uint32_t p1, bool exp) {
     }
     if (fixed_cut(k, w)) {
         FixedSmem F;
-        F.layout(256, k);
+        F.layout(256, k, seg);
         return F.total;
     }
     SeqSmem L;
-    L.layout(w, seq_threads(w), k);
+    L.layout(w, seq_threads(w), k, seg);
     return L.total;
 }
 
-uint64_t cut_tile(int w, bool exp) { return exp ? (uint64_t)CUT_TILE : (uint64_t)seq_threads(w) * SEG; }
+uint64_t cut_tile(int w, bool exp, int seg) { return exp ? (uint64_t)CUT_TILE : (uint64_t)seq_threads(w) * seg; }
 
-uint32_t cut_ctas_per_sm(int w, int k, uint32_t p1, bool exp) {
-    const size_t sm = cut_smem_bytes(w, k, p1, exp) + 1024;
+uint32_t cut_ctas_per_sm(int w, int k, uint32_t p1, bool exp, int seg) {
+    const size_t sm = cut_smem_bytes(w, k, p1, exp, seg) + 1024;
     const uint32_t by_smem = (uint32_t)(228u * 1024u / sm);
     if (!exp && fixed_cut(k, w)) return std::max<uint32_t>(1, std::min<uint32_t>(FIXED_CUT_CTAS, by_smem));
     // the sequential cut: up to 768 threads per SM (three CTAs of 256; for wide
@@ -1313,6 +1374,19 @@ uint32_t cut_ctas_per_sm(int w, int k, uint32_t p1, bool exp) {
     // 3 -> 4 CTAs, 11.9 -> 9.0 ms for 0.9 Gbp; one block buffer instead of two,
     // 4 -> 7 CTAs)
     return std::max<uint32_t>(1, std::min<uint32_t>(exp ? 2u : 768u / (uint32_t)seq_threads(w), by_smem));
+}
+
+// Long segments once every CTA that fits on the device gets two tiles of them
+// (k=31 m=21, 1.5 Mbp: 88 us with long segments).
+int cut_seg(int w, int k, uint64_t n, uint32_t n_sm) {
+    const uint64_t ctas = (uint64_t)n_sm * cut_ctas_per_sm(w, k, 1, false, LONG_SEG);
+    return n >= 2 * ctas * cut_tile(w, false, LONG_SEG) ? LONG_SEG : SHORT_SEG;
+}
+
+cudaError_t launch_prepare(const PrepareParams& P, cudaStream_t st) {
+    const uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>(P.n_bins / 2 / 256, 1024));
+    k_prepare<<<blocks, 256, 0, st>>>(P);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_pack(const uint8_t* seq, uint64_t n, uint32_t* packed, uint32_t* valid, uint64_t n_words,
@@ -1333,24 +1407,30 @@ uint64_t packed_words_for(uint64_t n) {
     return (pw + 3) & ~uint64_t(3);
 }
 
+template <typename Kernel>
+static cudaError_t launch_one(Kernel kernel, int threads, const CutParams& P, const HashTables* gT, size_t sm,
+                              cudaStream_t st) {
+    const cudaError_t e = set_smem_cap(kernel, sm);
+    if (e != cudaSuccess) return e;
+    kernel<<<P.n_cta, threads, sm, st>>>(P, gT);
+    return cudaGetLastError();
+}
+
 template <int NT>
 static cudaError_t launch_cut_seq(const CutParams& P, const HashTables* gT, size_t sm, cudaStream_t st) {
-    const cudaError_t e = set_smem_cap(k_cut_seq<NT>, sm);
-    if (e != cudaSuccess) return e;
-    k_cut_seq<NT><<<P.n_cta, NT, sm, st>>>(P, gT);
-    return cudaGetLastError();
+    return P.seg == LONG_SEG ? launch_one(k_cut_seq<NT, LONG_SEG>, NT, P, gT, sm, st)
+                             : launch_one(k_cut_seq<NT, SHORT_SEG>, NT, P, gT, sm, st);
 }
 
 template <int K, int MM>
 static cudaError_t launch_cut_fixed(const CutParams& P, const HashTables* gT, size_t sm, cudaStream_t st) {
-    const cudaError_t e = set_smem_cap(k_cut_fixed<K, MM>, sm);
-    if (e != cudaSuccess) return e;
-    k_cut_fixed<K, MM><<<P.n_cta, FixedShape<K, MM>::NT, sm, st>>>(P, gT);
-    return cudaGetLastError();
+    constexpr int NT = FixedShape<K, MM>::NT;
+    return P.seg == LONG_SEG ? launch_one(k_cut_fixed<K, MM, LONG_SEG>, NT, P, gT, sm, st)
+                             : launch_one(k_cut_fixed<K, MM, SHORT_SEG>, NT, P, gT, sm, st);
 }
 
 cudaError_t launch_cut(const CutParams& P, const HashTables* gT, bool exp, cudaStream_t st) {
-    const size_t sm = cut_smem_bytes(P.w, P.k, 1u << P.p1_bits, exp);
+    const size_t sm = cut_smem_bytes(P.w, P.k, 1u << P.p1_bits, exp, P.seg);
     if (!exp && fixed_cut(P.k, P.w)) {
         switch (P.k * 100 + P.m) {
             case 3121: return launch_cut_fixed<31, 21>(P, gT, sm, st);

@@ -36,6 +36,7 @@ constexpr int COUNT_PER_SM = 2;          // CTAs per SM: one counts while the ot
 constexpr uint32_t MAX_PARTS = 128;      // key-hash parts of one range before the global table
 constexpr uint64_t FALLBACK_CAP = 4096;
 constexpr uint32_t BIG_KEYS = 1u << 16;  // k-mers above which many CTAs share a group (k_big)
+constexpr uint64_t WAVE_KEYS = 1u << 22; // k-mers of a wave of the first counting pass (P2Overlap)
 constexpr uint32_t BIG_CHUNK = 4096;     // packed records of such a group that a CTA takes at a time
 
 struct __align__(16) U128 {
@@ -219,7 +220,7 @@ __device__ __forceinline__ bool rec_equal(const Rec<W>& a, const Rec<W>& b) {
 // with an equal share of its bins: the share's groups,
 // from the scanned k-mer offsets ko[bin]. Greedy, in bin order: a group starting
 // at bin s takes the most bins e - s with at most `target` k-mers (one bin if that
-// bin alone is larger; such a group is listed as heavy). Each step is one
+// bin alone is larger; a group that a CTA's store cannot hold is listed apart). Each step is one
 // upper-bound search over ko, done by the warp as a 32-way search. Every bin of
 // the group gets the group's first bin in gfirst: k_recs appends all of the
 // group's records at that bin's cursor.
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(KeysParams P) {
         const unsigned long long ke = ko[e];
         for (uint32_t b = s + (uint32_t)lane; b < e; b += 32) P.gfirst[seg.bin_lo + b] = seg.bin_lo + s;
         if (lane == 0 && ke > ks) {  // not the empty bins before a bin larger than the target
-            const int heavy = ke - ks > T ? (ke - ks > BIG_KEYS ? 2 : 1) : 0;
+            const int heavy = ke - ks > P.store ? (ke - ks > BIG_KEYS ? 2 : 1) : 0;
             const unsigned long long q = atomicAdd(&P.ctr[heavy == 2 ? P2C_BIG : heavy ? P2C_HEAVY : P2C_NORMAL], 1ull);
             if (q < P.groups_cap) {
                 Group g;
@@ -365,10 +366,16 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// End of the launch's slice of the list.
+__device__ __forceinline__ unsigned long long list_end(const CountParams& P) {
+    return P.n_list ? min(P.g_end, *P.n_list) : P.g_end;
+}
+
 // Asynchronous copy (cp.async, two 16-byte pieces) of group `gi` of the launch's
 // list into shared memory; an index past the end gives an empty group.
-__device__ __forceinline__ void copy_group(Group* dst, const CountParams& P, unsigned long long gi) {
-    if (gi >= P.g_end) {
+__device__ __forceinline__ void copy_group(Group* dst, const CountParams& P, unsigned long long gi,
+                                           unsigned long long g_end) {
+    if (gi >= g_end) {
         dst->lo = dst->hi = 0;
         return;
     }
@@ -545,9 +552,11 @@ __global__ void __maxnreg__(56) k_count(const __grid_constant__ CountParams P) {
     const uint32_t tid = threadIdx.x, lane = tid & 31;
     uint32_t distinct = 0;                                   // per warp
 
+    const unsigned long long g_end = list_end(P);
+    if (P.g_begin + blockIdx.x >= g_end) return;  // fewer groups than CTAs
     start_store<W>(S);
     if (tid == 0) {
-        for (int q = 0; q < 3; ++q) copy_group(&S.grp[q], P, P.g_begin + atomicAdd(P.work, 1ull));
+        for (int q = 0; q < 3; ++q) copy_group(&S.grp[q], P, P.g_begin + atomicAdd(P.work, 1ull), g_end);
         S.pending = P.g_begin + atomicAdd(P.work, 1ull);     // index of group g + 3
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
@@ -719,7 +728,7 @@ __global__ void __maxnreg__(56) k_count(const __grid_constant__ CountParams P) {
             if (tid == 0) {  // group g + 3's entry into slot q, the index after it claimed
                 S.staged = 0;
                 if (!dedup && S.dedup) --S.dedup;
-                copy_group(&S.grp[q], P, S.pending);
+                copy_group(&S.grp[q], P, S.pending, g_end);
                 S.pending = P.g_begin + atomicAdd(P.work, 1ull);
             }
         });
@@ -844,9 +853,11 @@ __global__ void __launch_bounds__(COUNT_THREADS, COUNT_PER_SM) k_rounds(const __
     CountSmem<W>& S = *reinterpret_cast<CountSmem<W>*>(smem);
     const uint32_t tid = threadIdx.x;
     uint32_t distinct = 0;
+    const unsigned long long g_end = list_end(P);
+    if (P.g_begin + blockIdx.x >= g_end) return;
     start_store<W>(S);
     __syncthreads();
-    for (unsigned long long gi = P.g_begin + blockIdx.x; gi < P.g_end; gi += gridDim.x) {
+    for (unsigned long long gi = P.g_begin + blockIdx.x; gi < g_end; gi += gridDim.x) {
         const Group g = P.list[gi];
         const unsigned long long nrec = g.hi - g.lo;
         uint32_t n = 0, newm = 0;
@@ -1033,7 +1044,10 @@ uint32_t count_slots(int) { return 8192; }
 // Keys that k_plan puts in a group: group_pct of the unit, at most a store full.
 static uint32_t group_target(const P2Input& in) {
     const uint32_t cap = in.W == 1 ? CountShape<1>::CAP : CountShape<2>::CAP;
-    return std::max<uint32_t>(1, std::min(count_slots(in.W) * in.group_pct / 100, cap));
+    const uint32_t t = std::max<uint32_t>(1, std::min(count_slots(in.W) * in.group_pct / 100, cap));
+    // jobs too small for a full group per CTA: smaller groups, so that more SMs count
+    const uint64_t share = in.n_kmers / (COUNT_PER_SM * (uint64_t)std::max<uint32_t>(1, in.n_sm));
+    return (uint32_t)std::min<uint64_t>(t, std::max<uint64_t>(COUNT_THREADS, share));
 }
 
 namespace {
@@ -1057,11 +1071,12 @@ struct P2Plan {
 
 // Warps of k_plan per segment. Its steps are serial within a warp (one group
 // each, about a microsecond of dependent reads), so long segments are shared out
-// until a share has about 32 groups; fewer would leave more of the last groups of
-// the shares half filled.
+// until a share has about 32 groups (8 in a small job, where the steps count most);
+// fewer would leave more of the last groups of the shares half filled.
 uint32_t plan_split(const P2Input& in) {
     uint32_t s = 1;
-    while (s < 64 && in.n_kmers / ((uint64_t)in.n_segs * 2 * s + 1) > 32ull * group_target(in)) s *= 2;
+    const uint64_t groups = in.deferred ? 8 : 32;
+    while (s < 64 && in.n_kmers / ((uint64_t)in.n_segs * 2 * s + 1) > groups * group_target(in)) s *= 2;
     return s;
 }
 
@@ -1183,34 +1198,72 @@ size_t phase2_scratch_bytes(const P2Input& in) {
         }                                                            \
     } while (0)
 
-// Small counter reads (see OVERLAP_WORDS): src[0, n) to the mapped host words
-// dst (device address), fenced for the host.
-__global__ void k_peek(const unsigned long long* __restrict__ a, uint32_t na, const unsigned long long* __restrict__ b,
-                       uint32_t nb, unsigned long long* dst) {
+// Small counter reads (see OVERLAP_WORDS): up to three ranges to the mapped host
+// words dst (device address), fenced for the host.
+struct PeekRange {
+    const unsigned long long* p;
+    uint32_t n;
+};
+__global__ void k_peek(PeekRange a, PeekRange b, PeekRange c, unsigned long long* dst) {
     const uint32_t i = threadIdx.x;
-    if (i < na) dst[i] = a[i];
-    else if (i < na + nb) dst[i] = b[i - na];
+    if (i < a.n) dst[i] = a.p[i];
+    else if (i < a.n + b.n) dst[i] = b.p[i - a.n];
+    else if (i < a.n + b.n + c.n) dst[i] = c.p[i - a.n - b.n];
     __threadfence_system();
 }
 
-// Reads na counters at a and nb at b into out (host), then waits for the
+cudaError_t launch_peek(const unsigned long long* src, uint32_t n, unsigned long long* dst, cudaStream_t st) {
+    k_peek<<<1, 32, 0, st>>>({src, n}, {}, {}, dst);
+    return cudaGetLastError();
+}
+
+// Reads the ranges into out (host), one after the other, then waits for the
 // stream. With mapped words (ov.wave_out_dev) a kernel stores them there;
 // otherwise cudaMemcpyAsync.
-static cudaError_t read_counters(const P2Overlap& ov, const unsigned long long* a, uint32_t na,
-                                 const unsigned long long* b, uint32_t nb, unsigned long long* out, cudaStream_t st) {
-    if (ov.wave_out && ov.wave_out_dev && na + nb <= OVERLAP_WORDS - 16) {
-        k_peek<<<1, 32, 0, st>>>(a, na, b, nb, ov.wave_out_dev + 16);
+static cudaError_t read_counters(const P2Overlap& ov, PeekRange a, PeekRange b, PeekRange c, unsigned long long* out,
+                                 cudaStream_t st) {
+    const uint32_t n = a.n + b.n + c.n;
+    if (ov.wave_out && ov.wave_out_dev && n <= 32) {
+        k_peek<<<1, 32, 0, st>>>(a, b, c, ov.wave_out_dev + 16);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return e;
         const volatile unsigned long long* w = ov.wave_out + 16;
-        for (uint32_t i = 0; i < na + nb; ++i) out[i] = w[i];
+        for (uint32_t i = 0; i < n; ++i) out[i] = w[i];
         return cudaSuccess;
     }
-    cudaError_t e = cudaMemcpyAsync(out, a, 8 * (size_t)na, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && nb) e = cudaMemcpyAsync(out + na, b, 8 * (size_t)nb, cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaSuccess;
+    for (const PeekRange& r : {a, b, c}) {
+        if (e == cudaSuccess && r.n) e = cudaMemcpyAsync(out, r.p, 8 * (size_t)r.n, cudaMemcpyDeviceToHost, st);
+        out += r.n;
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     return e;
+}
+
+// The segments of a job of one sample are equal runs of its bins: written by a
+// kernel (no copy from pageable memory, which the host waits for).
+__global__ void k_segments(Segment* segs, uint32_t n, uint32_t lo, uint32_t per, uint32_t sample) {
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        Segment s;
+        s.bin_lo = lo + i * per;
+        s.bin_hi = s.bin_lo + per;
+        s.sample = sample;
+        s.pad = 0;
+        segs[i] = s;
+    }
+}
+
+static cudaError_t put_segments(const P2Input& in, Segment* dst, cudaStream_t st) {
+    const Segment& f = in.segs[0];
+    const uint32_t per = f.bin_hi - f.bin_lo;
+    bool equal = true;
+    for (uint32_t i = 0; i < in.n_segs && equal; ++i)
+        equal = in.segs[i].sample == f.sample && in.segs[i].bin_lo == f.bin_lo + i * per &&
+                in.segs[i].bin_hi == f.bin_lo + (i + 1) * per;
+    if (!equal) return cudaMemcpyAsync(dst, in.segs, (size_t)in.n_segs * sizeof(Segment), cudaMemcpyHostToDevice, st);
+    k_segments<<<1, 256, 0, st>>>(dst, in.n_segs, f.bin_lo, per, f.sample);
+    return cudaGetLastError();
 }
 
 tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Output& out,
@@ -1222,8 +1275,10 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     const P2Regions R = carve(c, in, L);
     if (!c.ok) { err = "phase-2 scratch too small"; return TG_ERR_OOM; }
 
-    P2_CK(cudaMemsetAsync(R.ctr, 0, P2C_COUNT * 8, st), "memset");
-    P2_CK(cudaMemcpyAsync(R.segs, in.segs, (size_t)in.n_segs * sizeof(Segment), cudaMemcpyHostToDevice, st), "h2d");
+    // counters: ctr, aux and work lie one after the other
+    P2_CK(cudaMemsetAsync(R.ctr, 0, reinterpret_cast<uint8_t*>(R.work + 16) - reinterpret_cast<uint8_t*>(R.ctr), st),
+          "memset");
+    if (in.n_segs) P2_CK(put_segments(in, R.segs, st), "segments");
     // counts per bin -> k-mers and packed records before each bin (of this run's bins)
     P2_CK(launch_bin_scan(in.binhist + in.bin_lo, in.bin_hi - in.bin_lo, R.kofs + in.bin_lo, R.rofs + in.bin_lo,
                           R.sums, st, launches),
@@ -1241,6 +1296,7 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     K.segs = R.segs;
     K.n_segs = in.n_segs;
     K.target = group_target(in);
+    K.store = W == 1 ? CountShape<1>::CAP : CountShape<2>::CAP;
     K.k = in.k;
     K.recs = R.recs;
     K.groups[0] = R.normal;
@@ -1295,13 +1351,13 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     Q.retry_cap = L.retry_cap;
     const size_t sm = W == 1 ? sizeof(CountSmem<1>) : sizeof(CountSmem<2>);
     P2_CK(W == 1 ? set_smem_cap(k_count<1>, sm) : set_smem_cap(k_count<2>, sm), "smem");
-    unsigned long long h[P2C_COUNT];
-    // the groups: their number is known once k_plan has run
-    P2_CK(cudaMemcpyAsync(h, R.ctr, sizeof h, cudaMemcpyDeviceToHost, st), "d2h");
-    P2_CK(cudaStreamSynchronize(st), "phase 2");
-    if (h[P2C_NORMAL] > L.groups_cap || h[P2C_HEAVY] > L.groups_cap || h[P2C_BIG] > L.groups_cap) {
-        err = "group list overflow";
-        return TG_ERR_TABLE;
+    unsigned long long h[P2C_COUNT] = {};
+    auto lists_ok = [&] {
+        return h[P2C_NORMAL] <= L.groups_cap && h[P2C_HEAVY] <= L.groups_cap && h[P2C_BIG] <= L.groups_cap;
+    };
+    if (!in.deferred) {  // the groups: their number is known once k_plan has run
+        P2_CK(read_counters(ov, {R.ctr, P2C_COUNT}, {}, {}, h, st), "phase 2");
+        if (!lists_ok()) { err = "group list overflow"; return TG_ERR_TABLE; }
     }
     const unsigned long long ngroups = h[P2C_NORMAL];
     const unsigned cgrid = in.n_sm * COUNT_PER_SM;
@@ -1310,6 +1366,7 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
         Q.g_begin = 0;
         Q.g_end = n;
         const unsigned grid = (unsigned)std::min<unsigned long long>(n, cgrid);
+        if (!grid) return cudaSuccess;
         cudaError_t e = W == 1 ? set_smem_cap(k_rounds<1>, sm) : set_smem_cap(k_rounds<2>, sm);
         if (e != cudaSuccess) return e;
         if (W == 1) k_rounds<1><<<grid, COUNT_THREADS, sm, st>>>(Q);
@@ -1356,11 +1413,11 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     };
     Q.retry = R.retry[0];
     Q.n_retry = R.aux;
-    P2_CK(cudaMemsetAsync(R.aux, 0, 16, st), "memset");
     // ---- the largest groups, one table for those of a sample (of few MB for a group of a
     // million k-mers; without room for it, they are counted like the other large ones)
     uint64_t n_big = 0;
-    if (h[P2C_BIG]) {
+    auto count_big = [&]() -> tg_status {
+        if (!h[P2C_BIG]) return TG_OK;
         std::vector<Group> big(h[P2C_BIG]);
         P2_CK(cudaMemcpyAsync(big.data(), R.big, big.size() * sizeof(Group), cudaMemcpyDeviceToHost, st), "d2h");
         P2_CK(cudaStreamSynchronize(st), "d2h");
@@ -1388,26 +1445,37 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
             else P2_CK(rounds(R.big + a, b - a), "k_rounds");
             a = b;
         }
+        return TG_OK;
+    };
+    if (in.deferred) {
+        Q.n_list = R.ctr + P2C_HEAVY;
+        P2_CK(rounds(R.heavy, std::min<uint64_t>(L.groups_cap, in.n_kmers / group_target(in))), "k_rounds");
+    } else {
+        const tg_status s = count_big();
+        if (s != TG_OK) return s;
+        P2_CK(rounds(R.heavy, h[P2C_HEAVY]), "k_rounds");
     }
-    if (h[P2C_HEAVY]) P2_CK(rounds(R.heavy, h[P2C_HEAVY]), "k_rounds");
     // ---- the others, in `waves` launches over slices of their list; each slice's output
     // range goes to on_range as soon as it is final
-    const uint32_t waves = ov.on_range && ov.wave_out && ov.wave_ev ? std::max<uint32_t>(1, std::min(ov.waves, 16u)) : 1;
-    P2_CK(cudaMemsetAsync(R.work, 0, 8 * 16, st), "memset");
+    // (at least WAVE_KEYS k-mers each: a launch, and what it waits for, costs about 15 us)
+    const uint32_t waves = ov.on_range && ov.wave_out && ov.wave_ev && !in.deferred
+                               ? (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({ov.waves, 16u, in.n_kmers / WAVE_KEYS})) : 1;
     uint64_t done = 0;  // output keys already handed to on_range
     for (uint32_t wv = 0; wv < waves; ++wv) {
         Q.list = R.normal;
+        Q.n_list = in.deferred ? R.ctr + P2C_NORMAL : nullptr;
         Q.g_begin = ngroups * wv / waves;
-        Q.g_end = ngroups * (wv + 1) / waves;
+        Q.g_end = in.deferred ? L.groups_cap : ngroups * (wv + 1) / waves;
         Q.work = R.work + wv;
         if (Q.g_end > Q.g_begin) {
-            if (W == 1) k_count<1><<<cgrid, COUNT_THREADS, sm, st>>>(Q);
-            else k_count<2><<<cgrid, COUNT_THREADS, sm, st>>>(Q);
+            const unsigned grid = (unsigned)std::min<uint64_t>(cgrid, Q.g_end - Q.g_begin);
+            if (W == 1) k_count<1><<<grid, COUNT_THREADS, sm, st>>>(Q);
+            else k_count<2><<<grid, COUNT_THREADS, sm, st>>>(Q);
             P2_CK(cudaGetLastError(), "k_count");
             ++*launches;
         }
         if (waves > 1) {
-            if (ov.wave_out_dev) k_peek<<<1, 32, 0, st>>>(R.ctr + P2C_OUT, 1, nullptr, 0, ov.wave_out_dev + wv);
+            if (ov.wave_out_dev) k_peek<<<1, 32, 0, st>>>({R.ctr + P2C_OUT, 1}, {}, {}, ov.wave_out_dev + wv);
             else P2_CK(cudaMemcpyAsync(ov.wave_out + wv, R.ctr + P2C_OUT, 8, cudaMemcpyDeviceToHost, st), "d2h");
             P2_CK(cudaEventRecord(ov.wave_ev[wv], st), "event");
         }
@@ -1423,12 +1491,27 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
             }
         }
     }
+    Q.n_list = nullptr;
     // ---- groups that came back as key-hash parts: pass p reads retry[p & 1], writes the other
     for (int pass = 0;; ++pass) {
-        unsigned long long hr[P2C_COUNT + 1];
-        P2_CK(read_counters(ov, R.aux + (pass & 1), 1, R.ctr, P2C_COUNT, hr, st), "phase 2");
-        const unsigned long long nret = hr[0];
+        unsigned long long hr[1 + P2C_COUNT + 8];
+        P2_CK(read_counters(ov, {R.aux + (pass & 1), 1}, {R.ctr, P2C_COUNT},
+                            {in.read_back, pass == 0 ? std::min(in.n_read, 8u) : 0}, hr, st), "phase 2");
+        unsigned long long nret = hr[0];
         for (int c = 0; c < P2C_COUNT; ++c) h[c] = hr[c + 1];
+        if (pass == 0) {
+            for (uint32_t c = 0; c < std::min(in.n_read, 8u); ++c) out.read_back[c] = hr[1 + P2C_COUNT + c];
+            if (in.deferred) {
+                if (!lists_ok()) { err = "group list overflow"; return TG_ERR_TABLE; }
+                if (h[P2C_BIG]) {  // counted now; its groups may come back as parts too
+                    const tg_status s = count_big();
+                    if (s != TG_OK) return s;
+                    P2_CK(read_counters(ov, {R.aux, 1}, {R.ctr, P2C_COUNT}, {}, hr, st), "phase 2");
+                    nret = hr[0];
+                    for (int c = 0; c < P2C_COUNT; ++c) h[c] = hr[c + 1];
+                }
+            }
+        }
         if (nret > L.retry_cap) { err = "too many groups to split"; return TG_ERR_TABLE; }
         if (nret == 0) break;
         Q.retry = R.retry[(pass + 1) & 1];
@@ -1456,7 +1539,7 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
             }, false);
             if (s != TG_OK) return s;
         }
-        P2_CK(read_counters(ov, R.ctr, P2C_COUNT, nullptr, 0, h, st), "fallback");
+        P2_CK(read_counters(ov, {R.ctr, P2C_COUNT}, {}, {}, h, st), "fallback");
     }
     out.n_out = h[P2C_OUT];
     if (ov.on_range && std::min<uint64_t>(out.n_out, out.cap) > done) {
