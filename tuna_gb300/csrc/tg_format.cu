@@ -186,21 +186,38 @@ cudaError_t launch_fmt_w(int W, const uint64_t* keys, const uint32_t* counts, ui
 
 // Digest of pairs [0, n): each thread sums the terms of its pairs, a warp
 // reduces them, one atomic per warp and field. out[4] = pairs, count sum, h1,
-// h2 (zeroed by the caller).
-__global__ void __launch_bounds__(256) k_digest(const uint64_t* __restrict__ keys, int W, int nw,
-                                                const uint32_t* __restrict__ counts, uint64_t n,
+// h2 (zeroed by the caller). Bound by its arithmetic (four 64-bit finalisers, eight
+// 64-bit products per pair), so key width and words are compile-time and several
+// pairs per thread are in flight.
+constexpr int DIGEST_UNROLL = 4;
+template <int W, int NW>
+__global__ void __launch_bounds__(256) k_digest(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ counts, uint64_t n,
                                                 unsigned long long* __restrict__ out) {
     unsigned long long h1 = 0, h2 = 0, cs = 0, np = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t w0 = keys[i * W];
-        const uint64_t w1 = W > 1 ? keys[i * W + 1] : 0;
-        const uint32_t c = counts[i];
-        uint64_t a, b;
-        digest_terms(w0, w1, nw, c, a, b);
-        h1 += a;
-        h2 += b;
-        cs += c;
-        ++np;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += DIGEST_UNROLL * stride) {
+        uint64_t w0[DIGEST_UNROLL], w1[DIGEST_UNROLL];
+        uint32_t c[DIGEST_UNROLL];
+#pragma unroll
+        for (int u = 0; u < DIGEST_UNROLL; ++u) {
+            const uint64_t i = i0 + u * stride;
+            w1[u] = 0;
+            if (i < n) {
+                w0[u] = __ldcs(keys + i * W);
+                if (W > 1) w1[u] = __ldcs(keys + i * W + 1);
+                c[u] = __ldcs(counts + i);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < DIGEST_UNROLL; ++u) {
+            if (i0 + u * stride >= n) continue;
+            uint64_t a, b;
+            digest_terms(w0[u], w1[u], NW, c[u], a, b);
+            h1 += a;
+            h2 += b;
+            cs += c[u];
+            ++np;
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -226,7 +243,9 @@ cudaError_t launch_digest(int k, const uint64_t* keys, const uint32_t* counts, u
     cudaError_t e = cudaMemsetAsync(out, 0, 4 * sizeof(unsigned long long), st);
     if (e != cudaSuccess || n == 0) return e;
     const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, (uint64_t)std::max(n_sm, 1) * 8);
-    k_digest<<<(unsigned)blocks, 256, 0, st>>>(keys, W, nw, counts, n, out);
+    if (W == 1) k_digest<1, 1><<<(unsigned)blocks, 256, 0, st>>>(keys, counts, n, out);
+    else if (nw == 1) k_digest<2, 1><<<(unsigned)blocks, 256, 0, st>>>(keys, counts, n, out);
+    else k_digest<2, 2><<<(unsigned)blocks, 256, 0, st>>>(keys, counts, n, out);
     ++*launches;
     return cudaGetLastError();
 }
