@@ -112,7 +112,7 @@ struct tg_ctx {
     unsigned host_threads = 1;
     std::string err;
     DevBuf seq, packed, valid, desc, xdesc, hist, scratch, okeys, ocnt, osamp, samp, okeys2, ocnt2, osoff,
-        misc, fbtab, tables, raw, lexs, fbuf, fscr, sp_desc, sp_bytes, sp_aux;
+        misc, fbtab, tables, raw, lexs, fbuf, fscr, sp_desc, sp_bytes, sp_aux, pieces;
     uint8_t* fhost[2] = {nullptr, nullptr};  // pinned host buffers of the output drain
     size_t fhost_cap = 0;
     uint8_t* stage[2] = {nullptr, nullptr};  // pinned staging of copies to pageable host memory
@@ -330,7 +330,7 @@ tg_status tg_ctx_destroy(tg_ctx* ctx) {
     DevBuf* bufs[] = {&ctx->seq, &ctx->packed, &ctx->valid, &ctx->desc, &ctx->xdesc, &ctx->hist,
                       &ctx->scratch,
                       &ctx->okeys, &ctx->ocnt, &ctx->osamp, &ctx->samp, &ctx->okeys2, &ctx->ocnt2, &ctx->osoff, &ctx->misc, &ctx->fbtab, &ctx->tables,
-                      &ctx->raw, &ctx->lexs, &ctx->fbuf, &ctx->fscr, &ctx->sp_desc, &ctx->sp_bytes, &ctx->sp_aux};
+                      &ctx->raw, &ctx->lexs, &ctx->fbuf, &ctx->fscr, &ctx->sp_desc, &ctx->sp_bytes, &ctx->sp_aux, &ctx->pieces};
     for (DevBuf* b : bufs)
         if (b->p) cudaFree(b->p);
     for (auto& e : ctx->ev)
@@ -1846,16 +1846,58 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
     } else if (s == TG_OK && total) {
         // not waited for: the call returns only after the counts, or waits when it fails
         cudaError_t e = cudaSetDevice(ctx->device);
+        // samples in page-locked memory: all of them by one kernel, each at a place
+        // aligned like its source (up to 15 separators more before it)
+        std::vector<const uint8_t*> mapped;
+        if (n > 1) {
+            mapped.reserve(n);
+            for (uint32_t i = a; i < b; ++i) {
+                const uint8_t* m = lens[i] ? static_cast<const uint8_t*>(mapped_address(seqs[i])) : seqs[i];
+                if (lens[i] && !m) { mapped.clear(); break; }
+                mapped.push_back(m);
+            }
+        }
+        const bool gather = mapped.size() == n && n > 1;
+        if (gather) total += 16 * (uint64_t)n;
         if (e == cudaSuccess) e = ctx->ensure(ctx->seq, total + 1);
         if (e == cudaSuccess) e = cudaEventRecord(ctx->ev[9], ctx->st);
-        if (e == cudaSuccess && n > 1) e = cudaMemsetAsync(ctx->seq.p, '\n', total, ctx->st);
         uint64_t off = 0;
-        for (uint32_t i = a; i < b && e == cudaSuccess; ++i) {
-            if (i > a) j->sample_start.push_back(off);
-            if (lens[i])
-                e = link_copy(ctx->seq.as<uint8_t>() + off, seqs[i], lens[i], cudaMemcpyHostToDevice, ctx->st, ctx->n_sm);
-            off += lens[i] + 1;
-            j->st.input_bytes += lens[i];
+        if (gather && e == cudaSuccess) {
+            std::vector<LinkPiece> ps;
+            uint8_t* const d = ctx->seq.as<uint8_t>();
+            uint64_t end = 0;  // of the sample before, past its separators
+            for (uint32_t i = a; i < b; ++i) {
+                const uint8_t* m = mapped[i - a];
+                off = end;
+                if (lens[i]) {
+                    off += (reinterpret_cast<uintptr_t>(m) - reinterpret_cast<uintptr_t>(d + end)) & 15;
+                    if (ps.empty()) ps.push_back({d, d, 0, (uint32_t)(off - end)});
+                    else ps.back().fill += (uint32_t)(off - end);
+                    for (uint64_t o = 0; o < lens[i]; o += LINK_PIECE)
+                        ps.push_back({m + o, d + off + o, (uint32_t)std::min<uint64_t>(LINK_PIECE, lens[i] - o), 0});
+                    ps.back().fill = 1;
+                    end = off + lens[i] + 1;
+                }
+                if (i > a) j->sample_start.push_back(off);
+                j->st.input_bytes += lens[i];
+            }
+            total = end;
+            if (!ps.empty()) {
+                e = ctx->ensure(ctx->pieces, ps.size() * sizeof(LinkPiece));
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(ctx->pieces.p, ps.data(), ps.size() * sizeof(LinkPiece), cudaMemcpyHostToDevice, ctx->st);
+                if (e == cudaSuccess)
+                    e = link_gather(ctx->pieces.as<LinkPiece>(), (uint32_t)ps.size(), ctx->st, ctx->n_sm);
+            }
+        } else {
+            if (e == cudaSuccess && n > 1) e = cudaMemsetAsync(ctx->seq.p, '\n', total, ctx->st);
+            for (uint32_t i = a; i < b && e == cudaSuccess; ++i) {
+                if (i > a) j->sample_start.push_back(off);
+                if (lens[i])
+                    e = link_copy(ctx->seq.as<uint8_t>() + off, seqs[i], lens[i], cudaMemcpyHostToDevice, ctx->st, ctx->n_sm);
+                off += lens[i] + 1;
+                j->st.input_bytes += lens[i];
+            }
         }
         if (e != cudaSuccess) s = ctx->cuda_fail(e, "copy input");
         j->n = total;

@@ -199,6 +199,7 @@ struct CountParams {
     void* out_keys;                    // u64 x W per distinct k-mer
     uint32_t* out_counts;
     uint32_t* out_sample;              // sample of each pair (jobs of several samples), or null
+    uint32_t* sample_tot;              // pairs of each sample (jobs of several samples), or null
     uint64_t out_cap;
     unsigned long long* ctr;           // P2Counter
     unsigned long long g_begin, g_end; // this launch counts groups [g_begin, g_end) of the list

@@ -65,6 +65,16 @@ cudaError_t launch_digest(int k, const uint64_t* keys, const uint32_t* counts, u
 // cudaMemcpyAsync; ordered on st like cudaMemcpyAsync.
 cudaError_t link_copy(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t st, int n_sm,
                       int* launches = nullptr);
+// Many copies from mapped host memory in one launch (a copy of its own for each of
+// 400 samples of half a megabyte ran at 120 GB/s of the link's 200): piece q is len
+// bytes from src to dst, equally aligned mod 16, then `fill` (at most 32) line feeds.
+struct LinkPiece {
+    const uint8_t* src;
+    uint8_t* dst;
+    uint32_t len, fill;
+};
+constexpr uint32_t LINK_PIECE = 128u << 10;  // bytes per piece, a multiple of 16
+cudaError_t link_gather(const LinkPiece* pieces, uint32_t n, cudaStream_t st, int n_sm, int* launches = nullptr);
 // The device address of host memory that is page-locked and mapped for the
 // current device, else null (pageable memory, device memory, bad pointers).
 const void* mapped_address(const void* host);

@@ -46,7 +46,39 @@ __global__ void k_link_edges(const uint8_t* __restrict__ src, uint8_t* __restric
     for (size_t b = tail0 + threadIdx.x; b < n; b += blockDim.x) dst[b] = src[b];
 }
 
+// A CTA per piece: head bytes to dst's 16-byte boundary, 16-byte words, tail, and
+// the separators after it.
+__global__ void __launch_bounds__(LINK_THREADS, 8) k_link_gather(const LinkPiece* __restrict__ pieces, uint32_t n) {
+    for (uint32_t q = blockIdx.x; q < n; q += gridDim.x) {
+        const LinkPiece p = pieces[q];
+        const uint32_t mis = (16 - ((uint32_t)reinterpret_cast<uintptr_t>(p.dst) & 15u)) & 15u;
+        const uint32_t head = min(mis, p.len), nv = (p.len - head) / 16;
+        const uint4* s = reinterpret_cast<const uint4*>(p.src + head);
+        uint4* d = reinterpret_cast<uint4*>(p.dst + head);
+        uint32_t i = threadIdx.x;
+        for (; i + 3 * LINK_THREADS < nv; i += 4 * LINK_THREADS) {
+            const uint4 a = s[i], b = s[i + LINK_THREADS], c = s[i + 2 * LINK_THREADS], e = s[i + 3 * LINK_THREADS];
+            d[i] = a;
+            d[i + LINK_THREADS] = b;
+            d[i + 2 * LINK_THREADS] = c;
+            d[i + 3 * LINK_THREADS] = e;
+        }
+        for (; i < nv; i += LINK_THREADS) d[i] = s[i];
+        const uint32_t tail = head + nv * 16;
+        if (threadIdx.x < head) p.dst[threadIdx.x] = p.src[threadIdx.x];
+        if (tail + threadIdx.x < p.len) p.dst[tail + threadIdx.x] = p.src[tail + threadIdx.x];
+        if (threadIdx.x < p.fill) p.dst[p.len + threadIdx.x] = '\n';
+    }
+}
+
 }  // namespace
+
+cudaError_t link_gather(const LinkPiece* pieces, uint32_t n, cudaStream_t st, int n_sm, int* launches) {
+    if (!n) return cudaSuccess;
+    k_link_gather<<<std::min<uint32_t>(n, (uint32_t)std::max(n_sm, 1) * 4), LINK_THREADS, 0, st>>>(pieces, n);
+    if (launches) ++*launches;
+    return cudaGetLastError();
+}
 
 // The device address of a host pointer when it lies in page-locked memory
 // mapped for the current device, else null.

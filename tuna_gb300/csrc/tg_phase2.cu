@@ -500,6 +500,7 @@ __device__ __forceinline__ void write_out(const CountParams& P, CountSmem<W>& S,
         if (lane == 0 && wn) wb = atomicAdd(&P.ctr[P2C_OUT], (unsigned long long)wn);
     }
     if (wn == 0) return;  // the whole warp
+    if (P.sample_tot && lane == 0) atomicAdd(&P.sample_tot[sample], wn);
     wb = __shfl_sync(0xffffffffu, wb, 0);
     // every pair of the warp has room (the same for its lanes), or each is checked
     const uint32_t room = wb + wn <= P.out_cap ? ~0u : (uint32_t)(wb < P.out_cap ? P.out_cap - wb : 0);
@@ -983,7 +984,10 @@ __global__ void __launch_bounds__(256) k_fb_extract(const void* keys, const uint
         const unsigned bal = __ballot_sync(0xffffffffu, keep);
         if (!bal) continue;
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&P.ctr[P2C_OUT], (unsigned long long)__popc(bal));
+        if (lane == 0) {
+            base = atomicAdd(&P.ctr[P2C_OUT], (unsigned long long)__popc(bal));
+            if (P.sample_tot) atomicAdd(&P.sample_tot[sample], (uint32_t)__popc(bal));
+        }
         base = __shfl_sync(0xffffffffu, base, 0);
         if (keep) {
             const uint64_t o = base + __popc(bal & ((1u << lane) - 1));
@@ -1000,37 +1004,56 @@ __global__ void __launch_bounds__(256) k_fb_extract(const void* keys, const uint
 
 // ---------------------------------------------------------------- sample-major output
 // Jobs of several samples: the pairs, in group order, go sample-major so that
-// each sample's pairs are one range. The pairs of one group are contiguous and
-// of one sample, so the lanes of a warp nearly always share a sample: one
-// atomic per distinct sample in the warp (match_any).
-__global__ void k_samp_hist(const uint32_t* __restrict__ samp, uint64_t n, uint32_t* __restrict__ hist) {
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t i = i0 + threadIdx.x;
-        const uint32_t s = i < n ? samp[i] : 0xFFFFFFFFu;
-        const unsigned peers = __match_any_sync(0xffffffffu, s);
-        if (s != 0xFFFFFFFFu && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&hist[s], (uint32_t)__popc(peers));
-    }
-}
-
+// each sample's pairs are one range (the counting kernels add up the samples'
+// totals). The pairs that a counting warp wrote are contiguous and of one sample,
+// so the 128 pairs that a warp takes here at a time nearly always share it: one
+// atomic for them, else one per sample in each 32 (match_any).
+constexpr int SAMP_UNROLL = 4;
 template <int W>
-__global__ void k_samp_scatter(const void* __restrict__ keys, const uint32_t* __restrict__ cnt,
-                               const uint32_t* __restrict__ samp, uint64_t n, unsigned long long* __restrict__ cur,
-                               void* __restrict__ keys2, uint32_t* __restrict__ cnt2) {
+__global__ void __launch_bounds__(256) k_samp_scatter(const void* __restrict__ keys, const uint32_t* __restrict__ cnt,
+                                                      const uint32_t* __restrict__ samp, uint64_t n,
+                                                      unsigned long long* __restrict__ cur, void* __restrict__ keys2,
+                                                      uint32_t* __restrict__ cnt2) {
     using O = KeyOps<W>;
-    const int lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31;
     const auto* kk = static_cast<const typename O::Key*>(keys);
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t i = i0 + threadIdx.x;
-        const uint32_t s = i < n ? samp[i] : 0xFFFFFFFFu;
-        const unsigned peers = __match_any_sync(0xffffffffu, s);
-        const int leader = __ffs(peers) - 1;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (uint64_t)gridDim.x * blockDim.x >> 5;
+    for (uint64_t i0 = warp * 32 * SAMP_UNROLL; i0 < n; i0 += warps * 32 * SAMP_UNROLL) {
+        uint32_t s[SAMP_UNROLL], c[SAMP_UNROLL];
+        typename O::Key k[SAMP_UNROLL];
+        const uint32_t m = (uint32_t)min((uint64_t)(32 * SAMP_UNROLL), n - i0);
+        bool one = true;
+#pragma unroll
+        for (int u = 0; u < SAMP_UNROLL; ++u) {
+            const uint32_t j = 32 * u + lane;
+            s[u] = 0xFFFFFFFFu;
+            if (j < m) {
+                s[u] = samp[i0 + j];
+                k[u] = kk[i0 + j];
+                c[u] = cnt[i0 + j];
+            }
+        }
+        const uint32_t first = __shfl_sync(0xffffffffu, s[0], 0);
+#pragma unroll
+        for (int u = 0; u < SAMP_UNROLL; ++u) one = one && (s[u] == first || 32 * u + lane >= m);
+        one = __all_sync(0xffffffffu, one);
         unsigned long long base = 0;
-        if (s != 0xFFFFFFFFu && lane == leader) base = atomicAdd(&cur[s], (unsigned long long)__popc(peers));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (s != 0xFFFFFFFFu) {
-            const uint64_t o = base + __popc(peers & ((1u << lane) - 1));
-            O::store(keys2, o, kk[i]);
-            cnt2[o] = cnt[i];
+        if (one && lane == 0) base = atomicAdd(&cur[first], (unsigned long long)m);
+        base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+        for (int u = 0; u < SAMP_UNROLL; ++u) {
+            uint64_t o = base + 32 * u + lane;
+            if (!one) {
+                const unsigned peers = __match_any_sync(0xffffffffu, s[u]);
+                const uint32_t leader = __ffs(peers) - 1;
+                unsigned long long b = 0;
+                if (s[u] != 0xFFFFFFFFu && lane == leader) b = atomicAdd(&cur[s[u]], (unsigned long long)__popc(peers));
+                o = __shfl_sync(0xffffffffu, b, leader) + __popc(peers & ((1u << lane) - 1));
+            }
+            if (32 * u + lane < m) {
+                O::store(keys2, o, k[u]);
+                cnt2[o] = c[u];
+            }
         }
     }
 }
@@ -1107,6 +1130,7 @@ struct P2Regions {
     Group* retry[2];
     Group* fb;
     unsigned long long* scur;  // [n_samples] cursors of the sample-major copy
+    uint32_t* stot;            // [n_samples] pairs of each sample
     uint8_t* recs;
 };
 
@@ -1127,6 +1151,7 @@ P2Regions carve(Carve& c, const P2Input& in, const P2Plan& L) {
     R.retry[1] = c.take<Group>(L.retry_cap);
     R.fb = c.take<Group>(FALLBACK_CAP);
     R.scur = c.take<unsigned long long>(in.n_samples + 1);
+    R.stot = c.take<uint32_t>(in.n_samples + 1);
     R.recs = c.take<uint8_t>((in.n_recs + 1) * 16 * (size_t)in.W);
     return R;
 }
@@ -1346,6 +1371,8 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     Q.out_keys = out.keys;
     Q.out_counts = out.counts;
     Q.out_sample = out.samples;
+    Q.sample_tot = out.samples ? R.stot : nullptr;
+    if (out.samples) P2_CK(cudaMemsetAsync(R.stot, 0, 4 * (size_t)in.n_samples, st), "memset");
     Q.out_cap = out.cap;
     Q.ctr = R.ctr;
     Q.retry_cap = L.retry_cap;
@@ -1461,11 +1488,17 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     const uint32_t waves = ov.on_range && ov.wave_out && ov.wave_ev && !in.deferred
                                ? (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({ov.waves, 16u, in.n_kmers / WAVE_KEYS})) : 1;
     uint64_t done = 0;  // output keys already handed to on_range
+    // the first and the last wave are half as long as the others: nothing is copied
+    // before the first, and nothing counted while the last one's pairs are
+    auto wave_at = [&](uint32_t w) -> unsigned long long {
+        if (w == 0 || w >= waves) return w ? ngroups : 0;
+        return ngroups * (2 * w - 1) / (2 * (waves - 1));
+    };
     for (uint32_t wv = 0; wv < waves; ++wv) {
         Q.list = R.normal;
         Q.n_list = in.deferred ? R.ctr + P2C_NORMAL : nullptr;
-        Q.g_begin = ngroups * wv / waves;
-        Q.g_end = in.deferred ? L.groups_cap : ngroups * (wv + 1) / waves;
+        Q.g_begin = wave_at(wv);
+        Q.g_end = in.deferred ? L.groups_cap : wave_at(wv + 1);
         Q.work = R.work + wv;
         if (Q.g_end > Q.g_begin) {
             const unsigned grid = (unsigned)std::min<uint64_t>(cgrid, Q.g_end - Q.g_begin);
@@ -1548,21 +1581,17 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     }
     out.distinct = h[P2C_DISTINCT];
     if (out.samples && out.n_samples > 1 && out.n_samples <= in.n_samples && out.keys2 && out.counts2 && out.sample_off) {
-        // sample-major copy: per-sample totals, their scan, the scatter
+        // sample-major copy: the scan of the samples' totals, the scatter
         const uint64_t n = std::min<uint64_t>(out.n_out, out.cap);
-        uint32_t* hist = reinterpret_cast<uint32_t*>(R.kofs);  // the bin offsets are no longer needed
-        P2_CK(cudaMemsetAsync(hist, 0, 4 * (size_t)out.n_samples, st), "memset");
         const unsigned grid = (unsigned)in.n_sm * 8;
-        k_samp_hist<<<grid, 256, 0, st>>>(out.samples, n, hist);
-        P2_CK(cudaGetLastError(), "k_samp_hist");
-        P2_CK(launch_scan(hist, out.n_samples, out.sample_off, R.sums, st, launches), "scan");
+        P2_CK(launch_scan(R.stot, out.n_samples, out.sample_off, R.sums, st, launches), "scan");
         unsigned long long* cur = R.scur;  // the offsets, copied, as cursors
         P2_CK(cudaMemcpyAsync(cur, out.sample_off, 8 * (size_t)out.n_samples, cudaMemcpyDeviceToDevice, st), "copy");
         if (out.reorder_after) P2_CK(cudaStreamWaitEvent(st, out.reorder_after, 0), "wait");
         if (W == 1) k_samp_scatter<1><<<grid, 256, 0, st>>>(out.keys, out.counts, out.samples, n, cur, out.keys2, out.counts2);
         else k_samp_scatter<2><<<grid, 256, 0, st>>>(out.keys, out.counts, out.samples, n, cur, out.keys2, out.counts2);
         P2_CK(cudaGetLastError(), "k_samp_scatter");
-        *launches += 2;
+        *launches += 1;
         P2_CK(cudaStreamSynchronize(st), "sample order");
     }
     out.groups = h[P2C_NORMAL] + h[P2C_HEAVY] + h[P2C_BIG];
