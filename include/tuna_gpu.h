@@ -131,7 +131,7 @@ typedef struct {
     double phase2_count_ms;   /* part of phase2_ms: the shared-memory counting kernel(s) */
     double phase2_keys_ms;    /* part of phase2_ms: bin offsets, group plan, packed records */
     uint64_t groups;          /* phase-2 groups (runs of minimizer bins counted in one table) */
-    double lex_ms;            /* device time: FASTA/FASTQ lexing of the feeds */
+    double lex_ms;            /* device time: FASTA/FASTQ lexing of the feeds, past the end of their copies */
     uint64_t fastx_bytes;     /* FASTA/FASTQ bytes fed (before lexing) */
     uint64_t host_parsed_bytes; /* of those, bytes parsed on the host (see tg_job_feed_fastx) */
     uint64_t phase2_passes;   /* phase-2 passes over ranges of bins (more than 1 when the keys and

@@ -428,9 +428,13 @@ static tg_status append_stream(tg_job* j, const uint8_t* src, size_t len, cudaMe
     return TG_OK;
 }
 
+// Bytes of a piece: 80 us of copying, several times what its launches cost.
+constexpr uint64_t LEX_PIECE = 16u << 20;
+
 // FASTA/FASTQ bytes in device memory (16-byte aligned) lexed on the device
 // onto the end of the stream. host_raw, when given, is the same bytes in host
-// memory. A FASTQ file the device lexer flags (an empty header line at file
+// memory, copied to draw (ctx->raw) here: a long file in pieces, each lexed while
+// the next is copied. A FASTQ file the device lexer flags (an empty header line at file
 // offset 63 mod 64, where the reference's block walk departs from line
 // counting) is parsed by the host parser instead.
 static tg_status lex_append(tg_job* j, const uint8_t* draw, size_t len, const uint8_t* host_raw) {
@@ -452,15 +456,39 @@ static tg_status lex_append(tg_job* j, const uint8_t* draw, size_t len, const ui
     CK(ctx->ensure(ctx->lexs, lex_scratch_bytes(len)), "alloc lexer scratch");
     LexTotals* dt = nullptr;
     int launches = 0;
-    CK(cudaEventRecord(ctx->ev[10], ctx->st), "event");
-    CK(launch_lex(draw, len, fastq, at, ctx->lexs.p, ctx->n_sm, ctx->st, &dt, &launches), "k_lex");
+    const uint64_t np = host_raw && !ctx->copy_pending ? std::max<uint64_t>(1, std::min<uint64_t>(16, len / LEX_PIECE)) : 1;
+    // more than one piece: the copies on the copy stream, in order (not behind a result copy)
+    cudaStream_t cst = np > 1 ? ctx->st_copy : ctx->st;
+    const size_t per = (size_t)((len + np - 1) / np + LEX_PIECE_UNIT - 1) / LEX_PIECE_UNIT * LEX_PIECE_UNIT;
+    if (host_raw) CK(cudaEventRecord(ctx->ev[4], cst), "event");
+    for (uint64_t lo = 0, q = 0; lo < len; lo += per, ++q) {
+        const uint64_t hi = std::min<uint64_t>(len, lo + per);
+        if (host_raw) {
+            cudaError_t e = link_copy(const_cast<uint8_t*>(draw) + lo, host_raw + lo, hi - lo, cudaMemcpyHostToDevice, cst, ctx->n_sm);
+            if (e == cudaSuccess && hi == len) e = cudaEventRecord(ctx->ev[10], cst);
+            if (e == cudaSuccess && np > 1) e = cudaEventRecord(ctx->wave_ev[q], cst);
+            if (e == cudaSuccess && np > 1) e = cudaStreamWaitEvent(ctx->st, ctx->wave_ev[q], 0);
+            if (e != cudaSuccess) {
+                cudaStreamSynchronize(cst);  // the caller's bytes are read no more
+                return ctx->cuda_fail(e, "copy input");
+            }
+        } else {
+            CK(cudaEventRecord(ctx->ev[10], ctx->st), "event");
+        }
+        const cudaError_t e = launch_lex(draw, len, fastq, at, ctx->lexs.p, ctx->n_sm, ctx->st, &dt, &launches, lo, hi);
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(cst);
+            return ctx->cuda_fail(e, "k_lex");
+        }
+    }
     CK(cudaEventRecord(ctx->ev[11], ctx->st), "event");
     LexTotals t{};
     CK(cudaMemcpyAsync(&t, dt, sizeof t, cudaMemcpyDeviceToHost, ctx->st), "d2h");
     CK(cudaStreamSynchronize(ctx->st), "k_lex");
     float ms = 0;
-    cudaEventElapsedTime(&ms, ctx->ev[10], ctx->ev[11]);
+    cudaEventElapsedTime(&ms, ctx->ev[10], ctx->ev[11]);  // from the last copy's end on
     j->st.lex_ms += ms;
+    if (host_raw && cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[10]) == cudaSuccess) j->st.h2d_ms += ms;
     j->st.fastx_bytes += len;
     j->lex_launches += launches;
     if (t.irregular & 2u) return ctx->fail(TG_ERR_DEVICE, "FASTA/FASTQ lexer: a staging copy did not complete");
@@ -490,10 +518,6 @@ static tg_status lex_append_host(tg_job* j, const uint8_t* data, size_t len) {
     if (len == 0) return ctx->fail(TG_ERR_PARSE, "Empty file");
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     CK(ctx->ensure(ctx->raw, len + 16), "alloc raw input");
-    const double t0 = now_ms();
-    CK(link_copy(ctx->raw.p, data, len, cudaMemcpyHostToDevice, ctx->st, ctx->n_sm), "copy input");
-    CK(cudaStreamSynchronize(ctx->st), "copy input");
-    j->st.h2d_ms += now_ms() - t0;
     return lex_append(j, ctx->raw.as<uint8_t>(), len, data);
 }
 
@@ -888,7 +912,7 @@ static tg_status run_phase1(tg_job* j, int* launches_out, P1Out& r, uint32_t p1_
     // ---- pack
     CK(cudaEventRecord(ctx->ev[0], ctx->st), "event");
     CK(launch_pack(j->seq_ptr(), n, ctx->packed.as<uint32_t>(), ctx->valid.as<uint32_t>(), pw,
-                   reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_BASES), ctx->st), "k_pack");
+                   reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_BASES), ctx->n_sm, ctx->st), "k_pack");
     ++launches;
     CK(cudaEventRecord(ctx->ev[1], ctx->st), "event");
     // ---- phase 1: cut

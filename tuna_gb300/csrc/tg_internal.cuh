@@ -24,6 +24,7 @@
 // include/kache-hash/Kmer.hpp:38-48.
 #pragma once
 #include <cstdint>
+#include <mutex>
 #include <cuda_runtime.h>
 
 namespace tg {
@@ -221,18 +222,42 @@ struct FallbackParams {
 // Dynamic shared-memory cap of a kernel: the device's opt-in shared memory per
 // block minus the kernel's static shared memory. It is a cap, not a
 // reservation; every launch, from every host thread, sets this same value, so
-// one thread's launch never finds the cap lowered by another's.
+// one thread's launch never finds the cap lowered by another's. The value is a
+// property of kernel and device, asked for once each (4 us of a small call's launch).
 template <typename Kernel>
 inline cudaError_t set_smem_cap(Kernel kernel, size_t need) {
-    int dev = 0, optin = 0;
+    constexpr int MAX_DEV = 64;
+    struct Known {
+        const void* kernel;
+        int cap[MAX_DEV];
+    };
+    static Known known[16] = {};  // of the kernels of this type (an instance per template argument list)
+    static std::mutex mu;
+    int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncAttributes a{};
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
     if (e != cudaSuccess) return e;
-    const size_t cap = (size_t)optin > a.sharedSizeBytes ? (size_t)optin - a.sharedSizeBytes : 0;
-    if (need > cap) return cudaErrorInvalidValue;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
+    const void* id = reinterpret_cast<const void*>(kernel);
+    int cap = -1;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        Known* k = nullptr;
+        for (Known& x : known) {
+            if (x.kernel == id) { k = &x; break; }
+            if (!x.kernel) { x.kernel = id; for (auto& c : x.cap) c = -1; k = &x; break; }
+        }
+        if (k && dev < MAX_DEV) cap = k->cap[dev];
+        if (cap < 0) {
+            int optin = 0;
+            cudaFuncAttributes a{};
+            e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+            if (e != cudaSuccess) return e;
+            cap = (size_t)optin > a.sharedSizeBytes ? optin - (int)a.sharedSizeBytes : 0;
+            if (k && dev < MAX_DEV) k->cap[dev] = cap;
+        }
+    }
+    if (need > (size_t)cap) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
 }
 
 // ---------------------------------------------------------------- bit helpers

@@ -25,7 +25,7 @@ cudaError_t launch_prepare(const PrepareParams& P, cudaStream_t st);
 // Packed words (a multiple of 4) for a stream of n bytes, padding included.
 uint64_t packed_words_for(uint64_t n);
 cudaError_t launch_pack(const uint8_t* seq, uint64_t n, uint32_t* packed, uint32_t* valid, uint64_t n_words,
-                        unsigned long long* n_bases, cudaStream_t st);
+                        unsigned long long* n_bases, int n_sm, cudaStream_t st);
 cudaError_t launch_cut(const CutParams& P, const HashTables* gT, bool exp, cudaStream_t st);
 // Exclusive scans of n >= 1 counts into n + 1 entries (the last: the total, which
 // goes to *total too if given); scratch holds scan_scratch(n) u64, 16-byte aligned.
@@ -41,12 +41,16 @@ struct LexTotals {
     unsigned long long out;        // stream bytes written
     unsigned long long drop_from;  // FASTQ: bytes from here on were not emitted (end-of-file rule)
     uint32_t final_state;          // automaton state at the end of the file
+    long long last_na;             // FASTQ: 1 + offset of the last non-ACGT byte so far, 0: none
     uint32_t irregular;            // bit 0: FASTQ with an empty header line at offset 63 mod 64 (parse
                                    // on the host); bit 1: a staging wait timed out (device error)
 };
 size_t lex_scratch_bytes(uint64_t len);
+// A file may be lexed in pieces, in order, while the rest of it is still copied:
+// bytes [lo, hi) of it, lo a multiple of LEX_PIECE_UNIT and hi too or len.
+constexpr uint64_t LEX_PIECE_UNIT = 16384;
 cudaError_t launch_lex(const uint8_t* raw, uint64_t len, bool fastq, uint8_t* out, void* scratch, int n_sm,
-                       cudaStream_t st, LexTotals** dtot, int* launches);
+                       cudaStream_t st, LexTotals** dtot, int* launches, uint64_t lo, uint64_t hi);
 // Output formatting on the device (tg_format.cu): n pairs to the bytes of
 // format fmt (tg_format). TSV writes its byte count to d_total (device-
 // writable, e.g. mapped host memory); KFF and RAW records have a fixed size,

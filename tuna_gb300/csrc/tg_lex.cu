@@ -298,7 +298,7 @@ typedef unsigned long long ull;
 // Pass 1: the summary of each CTA's range of chunks.
 template <int FASTQ>
 __global__ void __launch_bounds__(LEX_THREADS, LEX_CTAS_PER_SM)
-    k_lex_sum(const uint8_t* __restrict__ raw, uint64_t len, uint64_t n_chunks, uint64_t per_cta,
+    k_lex_sum(const uint8_t* __restrict__ raw, uint64_t len, uint64_t c_begin, uint64_t c_end, uint64_t per_cta,
               LexFn<ull>* __restrict__ fn, long long* __restrict__ last_na, LexTotals* tot) {
     __shared__ __align__(128) uint8_t s_in[2][LEX_CHUNK + 32];
     __shared__ __align__(8) uint64_t s_bar[2];
@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(LEX_THREADS, LEX_CTAS_PER_SM)
     __shared__ long long s_na;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     LexStage S{s_in, s_bar, raw, len, 0, 0, len / LEX_CHUNK};
-    S.c_lo = min(n_chunks, (uint64_t)blockIdx.x * per_cta);
-    S.c_hi = min(n_chunks, S.c_lo + per_cta);
+    S.c_lo = min(c_end, c_begin + (uint64_t)blockIdx.x * per_cta);
+    S.c_hi = min(c_end, S.c_lo + per_cta);
     if (threadIdx.x == 0) {
         mbar_init(&s_bar[0]);
         mbar_init(&s_bar[1]);
@@ -365,10 +365,12 @@ __device__ __forceinline__ LexFn<C> lex_bcast(const LexFn<C>& f, int src) {
                     __shfl_sync(~0u, f.c2, src), __shfl_sync(~0u, f.c3, src)};
 }
 
-// Pass 2, one CTA: the state and output offset at the start of each range.
+// Pass 2, one CTA: the state and output offset at the start of each range, from
+// where the file's piece before this one ended (tot).
 // Warp w reads a contiguous run of the range summaries 32 at a time.
 __global__ void __launch_bounds__(SCAN_THREADS) k_lex_scan(const LexFn<ull>* __restrict__ fn, uint64_t n_items,
-                                                           int fastq, uint64_t len, const long long* __restrict__ last_na,
+                                                           int fastq, int last, uint64_t len,
+                                                           const long long* __restrict__ last_na,
                                                            uint8_t* __restrict__ cstate, ull* __restrict__ coff,
                                                            LexTotals* tot) {
     constexpr int NW = SCAN_THREADS / 32;
@@ -402,8 +404,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_lex_scan(const LexFn<ull>* __r
     if (lane == 0) s_w[warp] = agg;
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t s = 0;
-        ull off = 0;
+        uint32_t s = tot->final_state;
+        ull off = tot->out;
         for (int i = 0; i < NW; ++i) {
             s_st[i] = s;
             s_off[i] = off;
@@ -413,8 +415,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_lex_scan(const LexFn<ull>* __r
         ull drop = len;
         // FASTQ, length a multiple of 64, file ending on an ACGT byte of a
         // sequence line: the run reaching the end is dropped
-        const long long lna = s_na;
-        if (fastq && s == 1 && len && (len & 63) == 0 && lna < (long long)len - 1) {
+        const long long lna = max(s_na, tot->last_na - 1);
+        tot->last_na = lna + 1;
+        if (fastq && last && s == 1 && len && (len & 63) == 0 && lna < (long long)len - 1) {
             drop = (ull)(lna + 1);
             off -= len - drop;
         }
@@ -448,7 +451,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_lex_scan(const LexFn<ull>* __r
 // with 16-byte stores.
 template <int FASTQ>
 __global__ void __launch_bounds__(LEX_THREADS, LEX_CTAS_PER_SM)
-    k_lex_emit(const uint8_t* __restrict__ raw, uint64_t len, uint64_t n_chunks, uint64_t per_cta,
+    k_lex_emit(const uint8_t* __restrict__ raw, uint64_t len, uint64_t c_begin, uint64_t c_end, uint64_t per_cta,
                const uint8_t* __restrict__ cstate, const ull* __restrict__ coff, LexTotals* tot,
                uint8_t* __restrict__ out) {
     __shared__ __align__(128) uint8_t s_in[2][LEX_CHUNK + 32];
@@ -459,8 +462,8 @@ __global__ void __launch_bounds__(LEX_THREADS, LEX_CTAS_PER_SM)
     __shared__ ull s_off;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     LexStage S{s_in, s_bar, raw, len, 0, 0, len / LEX_CHUNK};
-    S.c_lo = min(n_chunks, (uint64_t)blockIdx.x * per_cta);
-    S.c_hi = min(n_chunks, S.c_lo + per_cta);
+    S.c_lo = min(c_end, c_begin + (uint64_t)blockIdx.x * per_cta);
+    S.c_hi = min(c_end, S.c_lo + per_cta);
     const ull total = tot->out, drop = tot->drop_from;
     if (threadIdx.x == 0) {
         mbar_init(&s_bar[0]);
@@ -559,10 +562,11 @@ size_t lex_scratch_bytes(uint64_t len) {
 }
 
 cudaError_t launch_lex(const uint8_t* raw, uint64_t len, bool fastq, uint8_t* out, void* scratch, int n_sm,
-                       cudaStream_t st, LexTotals** dtot, int* launches) {
-    const uint64_t nc = (len + LEX_CHUNK - 1) / LEX_CHUNK;
+                       cudaStream_t st, LexTotals** dtot, int* launches, uint64_t lo, uint64_t hi) {
+    static_assert(LEX_PIECE_UNIT == LEX_CHUNK, "pieces of whole chunks");
+    const uint64_t c0 = lo / LEX_CHUNK, c1 = (hi + LEX_CHUNK - 1) / LEX_CHUNK, nc = c1 - c0;
     const uint64_t G = std::max<uint64_t>(1, std::min<uint64_t>({nc, (uint64_t)n_sm * LEX_CTAS_PER_SM, LEX_MAX_CTAS}));
-    const uint64_t per = (nc + G - 1) / std::max<uint64_t>(G, 1);
+    const uint64_t per = (nc + G - 1) / G;
     uint8_t* p = static_cast<uint8_t*>(scratch);
     auto take = [&](size_t bytes) {
         uint8_t* r = p;
@@ -575,13 +579,14 @@ cudaError_t launch_lex(const uint8_t* raw, uint64_t len, bool fastq, uint8_t* ou
     ull* coff = reinterpret_cast<ull*>(take(G * 8));
     uint8_t* cstate = take(G);
     *dtot = tot;
-    cudaError_t e = cudaMemsetAsync(tot, 0, sizeof(LexTotals), st);
+    const cudaError_t e = lo == 0 ? cudaMemsetAsync(tot, 0, sizeof(LexTotals), st) : cudaSuccess;
     if (e != cudaSuccess || nc == 0) return e;
-    if (fastq) k_lex_sum<1><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, nc, per, fn, last_na, tot);
-    else k_lex_sum<0><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, nc, per, fn, last_na, tot);
-    k_lex_scan<<<1, SCAN_THREADS, 0, st>>>(fn, G, fastq ? 1 : 0, len, last_na, cstate, coff, tot);
-    if (fastq) k_lex_emit<1><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, nc, per, cstate, coff, tot, out);
-    else k_lex_emit<0><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, nc, per, cstate, coff, tot, out);
+    const int last = hi == len;
+    if (fastq) k_lex_sum<1><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, c0, c1, per, fn, last_na, tot);
+    else k_lex_sum<0><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, c0, c1, per, fn, last_na, tot);
+    k_lex_scan<<<1, SCAN_THREADS, 0, st>>>(fn, G, fastq ? 1 : 0, last, len, last_na, cstate, coff, tot);
+    if (fastq) k_lex_emit<1><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, c0, c1, per, cstate, coff, tot, out);
+    else k_lex_emit<0><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, c0, c1, per, cstate, coff, tot, out);
     if (launches) *launches += 3;
     return cudaGetLastError();
 }

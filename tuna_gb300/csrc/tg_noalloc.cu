@@ -194,7 +194,7 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     pp.bin_bits = bin_bits;
     NA_CK(launch_prepare(pp, st), "k_prepare");
     // ---- phase 1
-    NA_CK(launch_pack(d_seq, n, packed, valid, pw, misc + 4, st), "k_pack");
+    NA_CK(launch_pack(d_seq, n, packed, valid, pw, misc + 4, n_sm, st), "k_pack");
     CutParams P{};
     P.packed = packed; P.valid = valid; P.n = n;
     P.k = k; P.m = m; P.w = w; P.L = L;

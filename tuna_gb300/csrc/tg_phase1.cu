@@ -1390,12 +1390,9 @@ cudaError_t launch_prepare(const PrepareParams& P, cudaStream_t st) {
 }
 
 cudaError_t launch_pack(const uint8_t* seq, uint64_t n, uint32_t* packed, uint32_t* valid, uint64_t n_words,
-                        unsigned long long* n_bases, cudaStream_t st) {
+                        unsigned long long* n_bases, int n_sm, cudaStream_t st) {
     // n_words is a multiple of 4 (packed_words_for): groups of 4 words
     const uint64_t groups = n_words / 4;
-    int dev = 0, n_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     const uint32_t threads = 256;
     const uint64_t blocks = std::min<uint64_t>((groups + threads - 1) / threads, (uint64_t)std::max(n_sm, 1) * 8);
     k_pack<<<(unsigned)std::max<uint64_t>(blocks, 1), threads, 0, st>>>(seq, n, packed, valid, groups, n_bases);

@@ -1266,10 +1266,14 @@ static cudaError_t read_counters(const P2Overlap& ov, PeekRange a, PeekRange b, 
     return e;
 }
 
-// The segments of a job of one sample are equal runs of its bins: written by a
-// kernel (no copy from pageable memory, which the host waits for).
-__global__ void k_segments(Segment* segs, uint32_t n, uint32_t lo, uint32_t per, uint32_t sample) {
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+// Before phase 2, in one launch: its counters at zero and, for a job of one sample,
+// whose segments are equal runs of its bins, the segments (no copy from pageable
+// memory, which the host waits for).
+__global__ void __launch_bounds__(256) k_setup(unsigned long long* ctr, uint32_t n_ctr, Segment* segs, uint32_t n,
+                                               uint32_t lo, uint32_t per, uint32_t sample) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (uint32_t i = t; i < n_ctr; i += stride) ctr[i] = 0;
+    for (uint32_t i = t; i < n; i += stride) {
         Segment s;
         s.bin_lo = lo + i * per;
         s.bin_hi = s.bin_lo + per;
@@ -1279,16 +1283,19 @@ __global__ void k_segments(Segment* segs, uint32_t n, uint32_t lo, uint32_t per,
     }
 }
 
-static cudaError_t put_segments(const P2Input& in, Segment* dst, cudaStream_t st) {
-    const Segment& f = in.segs[0];
+static cudaError_t setup(const P2Input& in, const P2Regions& R, cudaStream_t st) {
+    const Segment f = in.n_segs ? in.segs[0] : Segment{};
     const uint32_t per = f.bin_hi - f.bin_lo;
     bool equal = true;
     for (uint32_t i = 0; i < in.n_segs && equal; ++i)
         equal = in.segs[i].sample == f.sample && in.segs[i].bin_lo == f.bin_lo + i * per &&
                 in.segs[i].bin_hi == f.bin_lo + (i + 1) * per;
-    if (!equal) return cudaMemcpyAsync(dst, in.segs, (size_t)in.n_segs * sizeof(Segment), cudaMemcpyHostToDevice, st);
-    k_segments<<<1, 256, 0, st>>>(dst, in.n_segs, f.bin_lo, per, f.sample);
-    return cudaGetLastError();
+    // ctr, aux and work lie one after the other
+    k_setup<<<2, 256, 0, st>>>(R.ctr, (uint32_t)(R.work + 16 - R.ctr), R.segs, equal ? in.n_segs : 0, f.bin_lo, per, f.sample);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && !equal)
+        e = cudaMemcpyAsync(R.segs, in.segs, (size_t)in.n_segs * sizeof(Segment), cudaMemcpyHostToDevice, st);
+    return e;
 }
 
 tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Output& out,
@@ -1300,10 +1307,8 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     const P2Regions R = carve(c, in, L);
     if (!c.ok) { err = "phase-2 scratch too small"; return TG_ERR_OOM; }
 
-    // counters: ctr, aux and work lie one after the other
-    P2_CK(cudaMemsetAsync(R.ctr, 0, reinterpret_cast<uint8_t*>(R.work + 16) - reinterpret_cast<uint8_t*>(R.ctr), st),
-          "memset");
-    if (in.n_segs) P2_CK(put_segments(in, R.segs, st), "segments");
+    P2_CK(setup(in, R, st), "k_setup");
+    ++*launches;
     // counts per bin -> k-mers and packed records before each bin (of this run's bins)
     P2_CK(launch_bin_scan(in.binhist + in.bin_lo, in.bin_hi - in.bin_lo, R.kofs + in.bin_lo, R.rofs + in.bin_lo,
                           R.sums, st, launches),
@@ -1474,10 +1479,7 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
         }
         return TG_OK;
     };
-    if (in.deferred) {
-        Q.n_list = R.ctr + P2C_HEAVY;
-        P2_CK(rounds(R.heavy, std::min<uint64_t>(L.groups_cap, in.n_kmers / group_target(in))), "k_rounds");
-    } else {
+    if (!in.deferred) {
         const tg_status s = count_big();
         if (s != TG_OK) return s;
         P2_CK(rounds(R.heavy, h[P2C_HEAVY]), "k_rounds");
@@ -1536,9 +1538,10 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
             for (uint32_t c = 0; c < std::min(in.n_read, 8u); ++c) out.read_back[c] = hr[1 + P2C_COUNT + c];
             if (in.deferred) {
                 if (!lists_ok()) { err = "group list overflow"; return TG_ERR_TABLE; }
-                if (h[P2C_BIG]) {  // counted now; its groups may come back as parts too
+                if (h[P2C_BIG] || h[P2C_HEAVY]) {  // larger groups, rare in a small job, counted now
                     const tg_status s = count_big();
                     if (s != TG_OK) return s;
+                    P2_CK(rounds(R.heavy, h[P2C_HEAVY]), "k_rounds");
                     P2_CK(read_counters(ov, {R.aux, 1}, {R.ctr, P2C_COUNT}, {}, hr, st), "phase 2");
                     nret = hr[0];
                     for (int c = 0; c < P2C_COUNT; ++c) h[c] = hr[c + 1];
