@@ -1479,12 +1479,7 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
         }
         return TG_OK;
     };
-    if (!in.deferred) {
-        const tg_status s = count_big();
-        if (s != TG_OK) return s;
-        P2_CK(rounds(R.heavy, h[P2C_HEAVY]), "k_rounds");
-    }
-    // ---- the others, in `waves` launches over slices of their list; each slice's output
+    // ---- the others first, in `waves` launches over slices of their list; each slice's output
     // range goes to on_range as soon as it is final
     // (at least WAVE_KEYS k-mers each: a launch, and what it waits for, costs about 15 us)
     const uint32_t waves = ov.on_range && ov.wave_out && ov.wave_ev && !in.deferred
@@ -1515,6 +1510,9 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
             P2_CK(cudaEventRecord(ov.wave_ev[wv], st), "event");
         }
     }
+    Q.n_list = nullptr;
+    // the large groups behind them, counted while the waves' pairs are copied
+    if (!in.deferred) P2_CK(rounds(R.heavy, h[P2C_HEAVY]), "k_rounds");
     if (waves > 1) {
         for (uint32_t wv = 0; wv < waves; ++wv) {
             P2_CK(cudaEventSynchronize(ov.wave_ev[wv]), "wave");
@@ -1526,7 +1524,10 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
             }
         }
     }
-    Q.n_list = nullptr;
+    if (!in.deferred) {
+        const tg_status s = count_big();
+        if (s != TG_OK) return s;
+    }
     // ---- groups that came back as key-hash parts: pass p reads retry[p & 1], writes the other
     for (int pass = 0;; ++pass) {
         unsigned long long hr[1 + P2C_COUNT + 8];
