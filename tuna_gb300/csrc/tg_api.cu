@@ -67,6 +67,7 @@ constexpr size_t MISC_OVERFLOW = 40;    // u32: descriptor list overflow (k_cut)
 constexpr size_t MISC_MAX_DESC = 48;    // u32: descriptors of the longest list (k_cut)
 constexpr uint32_t MISC_READ = 7;       // u64 words read back after phase 1
 constexpr size_t MISC_DIGEST = 64;      // u64[4]: result digest (tg_job_result_digest)
+constexpr size_t MISC_AVAIL = 128;      // u64[MAX_PIECES]: stream length after each piece of a lexed file
 constexpr size_t MISC_NDESC = 256;      // u32[C]: descriptors per Phase-1 CTA
 constexpr size_t MISC_BYTES = MISC_NDESC + 4 * 65536;
 
@@ -112,7 +113,7 @@ struct tg_ctx {
     unsigned host_threads = 1;
     std::string err;
     DevBuf seq, packed, valid, desc, xdesc, hist, scratch, okeys, ocnt, osamp, samp, okeys2, ocnt2, osoff,
-        misc, fbtab, tables, raw, lexs, fbuf, fscr, sp_desc, sp_bytes, sp_aux, pieces;
+        misc, fbtab, tables, raw, lexs, fbuf, fscr, sp_desc, sp_bytes, sp_aux, pieces, cstate;
     uint8_t* fhost[2] = {nullptr, nullptr};  // pinned host buffers of the output drain
     size_t fhost_cap = 0;
     uint8_t* stage[2] = {nullptr, nullptr};  // pinned staging of copies to pageable host memory
@@ -225,6 +226,8 @@ struct tg_job {
     bool spill = false;
     uint64_t spill_chunk = 0;
     std::unique_ptr<SpillStore> store;
+    // phase 1 done while the input came in (count_run), or null
+    struct P1Out* done = nullptr;
     const uint8_t* seq_ptr() const { return ext ? ext : ctx->seq.as<uint8_t>(); }
 };
 
@@ -330,7 +333,7 @@ tg_status tg_ctx_destroy(tg_ctx* ctx) {
     DevBuf* bufs[] = {&ctx->seq, &ctx->packed, &ctx->valid, &ctx->desc, &ctx->xdesc, &ctx->hist,
                       &ctx->scratch,
                       &ctx->okeys, &ctx->ocnt, &ctx->osamp, &ctx->samp, &ctx->okeys2, &ctx->ocnt2, &ctx->osoff, &ctx->misc, &ctx->fbtab, &ctx->tables,
-                      &ctx->raw, &ctx->lexs, &ctx->fbuf, &ctx->fscr, &ctx->sp_desc, &ctx->sp_bytes, &ctx->sp_aux, &ctx->pieces};
+                      &ctx->raw, &ctx->lexs, &ctx->fbuf, &ctx->fscr, &ctx->sp_desc, &ctx->sp_bytes, &ctx->sp_aux, &ctx->pieces, &ctx->cstate};
     for (DevBuf* b : bufs)
         if (b->p) cudaFree(b->p);
     for (auto& e : ctx->ev)
@@ -428,97 +431,17 @@ static tg_status append_stream(tg_job* j, const uint8_t* src, size_t len, cudaMe
     return TG_OK;
 }
 
-// Bytes of a piece: 80 us of copying, several times what its launches cost.
-constexpr uint64_t LEX_PIECE = 16u << 20;
-
-// FASTA/FASTQ bytes in device memory (16-byte aligned) lexed on the device
-// onto the end of the stream. host_raw, when given, is the same bytes in host
-// memory, copied to draw (ctx->raw) here: a long file in pieces, each lexed while
-// the next is copied. A FASTQ file the device lexer flags (an empty header line at file
-// offset 63 mod 64, where the reference's block walk departs from line
-// counting) is parsed by the host parser instead.
-static tg_status lex_append(tg_job* j, const uint8_t* draw, size_t len, const uint8_t* host_raw) {
-    const TraceRange tr("tuna.lex");
-    tg_ctx* ctx = j->ctx;
-    if (j->ran) return ctx->fail(TG_ERR_STATE, "feed after run");
-    if (len == 0) return ctx->fail(TG_ERR_PARSE, "Empty file");
-    uint8_t* at = nullptr;
-    tg_status s = stream_reserve(j, len + 1, &at);
-    if (s != TG_OK) return s;
-    uint8_t first = 0;
-    if (host_raw) {
-        first = host_raw[0];
-    } else {
-        CK(cudaMemcpyAsync(&first, draw, 1, cudaMemcpyDeviceToHost, ctx->st), "d2h");
-        CK(cudaStreamSynchronize(ctx->st), "d2h");
-    }
-    const bool fastq = first == '@';
-    CK(ctx->ensure(ctx->lexs, lex_scratch_bytes(len)), "alloc lexer scratch");
-    LexTotals* dt = nullptr;
-    int launches = 0;
-    const uint64_t np = host_raw && !ctx->copy_pending ? std::max<uint64_t>(1, std::min<uint64_t>(16, len / LEX_PIECE)) : 1;
-    // more than one piece: the copies on the copy stream, in order (not behind a result copy)
-    cudaStream_t cst = np > 1 ? ctx->st_copy : ctx->st;
-    const size_t per = (size_t)((len + np - 1) / np + LEX_PIECE_UNIT - 1) / LEX_PIECE_UNIT * LEX_PIECE_UNIT;
-    if (host_raw) CK(cudaEventRecord(ctx->ev[4], cst), "event");
-    for (uint64_t lo = 0, q = 0; lo < len; lo += per, ++q) {
-        const uint64_t hi = std::min<uint64_t>(len, lo + per);
-        if (host_raw) {
-            cudaError_t e = link_copy(const_cast<uint8_t*>(draw) + lo, host_raw + lo, hi - lo, cudaMemcpyHostToDevice, cst, ctx->n_sm);
-            if (e == cudaSuccess && hi == len) e = cudaEventRecord(ctx->ev[10], cst);
-            if (e == cudaSuccess && np > 1) e = cudaEventRecord(ctx->wave_ev[q], cst);
-            if (e == cudaSuccess && np > 1) e = cudaStreamWaitEvent(ctx->st, ctx->wave_ev[q], 0);
-            if (e != cudaSuccess) {
-                cudaStreamSynchronize(cst);  // the caller's bytes are read no more
-                return ctx->cuda_fail(e, "copy input");
-            }
-        } else {
-            CK(cudaEventRecord(ctx->ev[10], ctx->st), "event");
-        }
-        const cudaError_t e = launch_lex(draw, len, fastq, at, ctx->lexs.p, ctx->n_sm, ctx->st, &dt, &launches, lo, hi);
-        if (e != cudaSuccess) {
-            cudaStreamSynchronize(cst);
-            return ctx->cuda_fail(e, "k_lex");
-        }
-    }
-    CK(cudaEventRecord(ctx->ev[11], ctx->st), "event");
-    LexTotals t{};
-    CK(cudaMemcpyAsync(&t, dt, sizeof t, cudaMemcpyDeviceToHost, ctx->st), "d2h");
-    CK(cudaStreamSynchronize(ctx->st), "k_lex");
-    float ms = 0;
-    cudaEventElapsedTime(&ms, ctx->ev[10], ctx->ev[11]);  // from the last copy's end on
-    j->st.lex_ms += ms;
-    if (host_raw && cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[10]) == cudaSuccess) j->st.h2d_ms += ms;
-    j->st.fastx_bytes += len;
-    j->lex_launches += launches;
-    if (t.irregular & 2u) return ctx->fail(TG_ERR_DEVICE, "FASTA/FASTQ lexer: a staging copy did not complete");
-    if (t.irregular) {
-        std::vector<uint8_t> hraw;
-        if (!host_raw) {
-            hraw.resize(len);
-            CK(cudaMemcpy(hraw.data(), draw, len, cudaMemcpyDeviceToHost), "d2h");
-            host_raw = hraw.data();
-        }
-        std::vector<uint8_t> st;
-        tgh::fastx_to_stream(host_raw, len, st);
-        j->st.host_parsed_bytes += len;
-        return append_stream(j, st.data(), st.size(), cudaMemcpyHostToDevice);
-    }
-    CK(cudaMemsetAsync(at + t.out, '\n', 1, ctx->st), "separator");
-    j->n += t.out + 1;
-    j->used_ctx_seq = true;
-    j->st.input_bytes += t.out;
-    return TG_OK;
-}
+struct P1Pipe;
+static tg_status lex_append(tg_job* j, const uint8_t* draw, size_t len, const uint8_t* host_raw, P1Pipe* pipe = nullptr);
 
 // Host FASTA/FASTQ bytes: copied to the device, lexed there.
-static tg_status lex_append_host(tg_job* j, const uint8_t* data, size_t len) {
+static tg_status lex_append_host(tg_job* j, const uint8_t* data, size_t len, P1Pipe* pipe = nullptr) {
     tg_ctx* ctx = j->ctx;
     if (j->ran) return ctx->fail(TG_ERR_STATE, "feed after run");
     if (len == 0) return ctx->fail(TG_ERR_PARSE, "Empty file");
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     CK(ctx->ensure(ctx->raw, len + 16), "alloc raw input");
-    return lex_append(j, ctx->raw.as<uint8_t>(), len, data);
+    return lex_append(j, ctx->raw.as<uint8_t>(), len, data, pipe);
 }
 
 static inline bool is_acgt_byte(uint8_t c) {
@@ -746,6 +669,33 @@ static tg_status read_misc(tg_ctx* ctx, P1Counts& r) {
     return TG_OK;
 }
 
+// The counting cut of the job's layout (n_cta, chunk, desc_cap, bin_bits), the stream
+// left open.
+static CutParams cut_params(tg_job* j, int seg, const CutSamples& cs) {
+    tg_ctx* ctx = j->ctx;
+    CutParams P{};
+    P.packed = ctx->packed.as<uint32_t>();
+    P.valid = ctx->valid.as<uint32_t>();
+    P.k = j->o.k; P.m = j->o.m; P.w = j->w; P.L = j->L;
+    P.p1_bits = j->p1_bits;
+    P.n_cta = j->n_cta;
+    P.chunk = j->chunk;
+    P.desc = ctx->desc.as<uint64_t>();
+    P.desc_cap = j->desc_cap;
+    P.seg = seg;
+    P.n_desc = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_NDESC);
+    P.max_desc = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_MAX_DESC);
+    P.binhist = ctx->hist.as<unsigned long long>();
+    P.stats = reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_CUT_STATS);
+    P.overflow = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_OVERFLOW);
+    P.sample_start = cs.start;
+    P.sample_bin_base = cs.base;
+    P.sample_bin_bits = cs.bits;
+    P.n_samples = cs.n;
+    P.desc_sb = desc_start_bits(j->bin_bits);
+    return P;
+}
+
 // deferred: the cut is launched and not waited for; its descriptor lists have
 // room for a record at every position.
 static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, const CutSamples& cs = CutSamples(),
@@ -753,21 +703,19 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
     tg_ctx* ctx = j->ctx;
     const uint64_t n = j->n;
     const uint32_t p1 = 1u << p1_bits;
-    const int seg = cut_seg(j->w, j->o.k, n, (uint32_t)ctx->n_sm);
+    const CutLayout lay = cut_layout(j->w, j->o.k, p1, exp, n, (uint32_t)ctx->n_sm);
+    const int seg = lay.seg;
     const size_t smem = cut_smem_bytes(j->w, j->o.k, p1, exp, seg);
     if (smem > ctx->smem_optin) return ctx->fail(TG_ERR_UNSUPPORTED, "phase-1 tile does not fit in shared memory");
-    const uint64_t tile = cut_tile(j->w, exp, seg);
-    uint32_t C = (uint32_t)ctx->n_sm * cut_ctas_per_sm(j->w, j->o.k, p1, exp, seg);
-    uint64_t chunk = (n + C - 1) / C;
-    chunk = std::max<uint64_t>(tile, (chunk + tile - 1) / tile * tile);
-    C = (uint32_t)std::max<uint64_t>(1, (n + chunk - 1) / chunk);
+    const uint64_t tile = lay.tile, chunk = lay.chunk;
+    const uint32_t C = lay.n_cta;
     j->n_cta = C;
     j->chunk = chunk;
     j->p1_bits = p1_bits;
     // descriptors: about 2/(w+2) records per k-mer for random minimizers; grow on overflow
     double factor = deferred ? 1.0 : std::min(1.0, 3.0 / (j->w + 2));
     for (int attempt = 0; attempt < 2; ++attempt) {
-        const uint64_t cap = (uint64_t)(chunk * factor) + 2ull * tile + j->L + 64;
+        const uint64_t cap = (uint64_t)(lay.tiles * tile * factor) + 2ull * tile + j->L + 64;
         j->desc_cap = cap;
         CK(ctx->ensure(ctx->desc, (size_t)C * cap * 8), "alloc descriptors");
         if (exp) CK(ctx->ensure(ctx->xdesc, (size_t)C * cap * 24), "alloc export descriptors");
@@ -782,29 +730,14 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
             CK(cudaMemsetAsync(ctx->misc.as<uint8_t>() + MISC_CUT_STATS, 0, 32, ctx->st), "memset");
             CK(cudaMemsetAsync(ctx->misc.as<uint8_t>() + MISC_OVERFLOW, 0, 16, ctx->st), "memset");
         }
-        CutParams P{};
-        P.packed = ctx->packed.as<uint32_t>();
-        P.valid = ctx->valid.as<uint32_t>();
+        CutParams P = cut_params(j, seg, cs);
         P.n = n;
-        P.k = j->o.k; P.m = j->o.m; P.w = j->w; P.L = j->L;
-        P.p1_bits = p1_bits;
-        P.n_cta = C;
-        P.chunk = chunk;
-        P.desc = ctx->desc.as<uint64_t>();
-        P.desc_cap = cap;
-        P.seg = seg;
-        P.n_desc = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_NDESC);
-        P.max_desc = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_MAX_DESC);
-        P.hist = exp ? ctx->hist.as<uint32_t>() : nullptr;
-        P.binhist = exp ? nullptr : ctx->hist.as<unsigned long long>();
-        P.stats = reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_CUT_STATS);
-        P.overflow = reinterpret_cast<uint32_t*>(ctx->misc.as<uint8_t>() + MISC_OVERFLOW);
-        P.xdesc = exp ? ctx->xdesc.as<uint64_t>() : nullptr;
-        P.sample_start = cs.start;
-        P.sample_bin_base = cs.base;
-        P.sample_bin_bits = cs.bits;
-        P.n_samples = cs.n;
-        P.desc_sb = desc_start_bits(j->bin_bits);
+        P.avail = Avail{nullptr, nullptr, 0, n, 1};
+        if (exp) {
+            P.hist = ctx->hist.as<uint32_t>();
+            P.binhist = nullptr;
+            P.xdesc = ctx->xdesc.as<uint64_t>();
+        }
         CK(cudaEventRecord(ctx->ev[2], ctx->st), "event");
         CK(launch_cut(P, ctx->tables.as<HashTables>(), exp, ctx->st), "k_cut");
         CK(cudaEventRecord(ctx->ev[3], ctx->st), "event");
@@ -858,10 +791,10 @@ struct P1Out {
     P1Counts c;  // deferred: not yet read
 };
 
-static tg_status run_phase1(tg_job* j, int* launches_out, P1Out& r, uint32_t p1_force = 0, bool deferred = false) {
+// Buffers and layout for a stream of at most n bytes, and what is written before
+// the cut (k_prepare).
+static tg_status setup_phase1(tg_job* j, uint64_t n, uint32_t p1_force, P1Out& r, CutSamples& cs, int* launches) {
     tg_ctx* ctx = j->ctx;
-    int launches = 0;
-    const uint64_t n = j->n;
     if (n >= (1ull << DESC_START_BITS)) return ctx->fail(TG_ERR_ARG, "input stream longer than 2^36 bytes");
     CK(ctx->ensure(ctx->tables, sizeof(HashTables)), "alloc tables");
     CK(ctx->ensure(ctx->misc, MISC_BYTES), "alloc misc");
@@ -902,29 +835,222 @@ static tg_status run_phase1(tg_job* j, int* launches_out, P1Out& r, uint32_t p1_
     }
     CK(launch_prepare(pp, ctx->st), "k_prepare");
     ctx->prepared_m = j->o.m;
-    ++launches;
+    j->p1_bits = p1_bits;
+    ++*launches;
     if (ns > 1) {
         CK(cudaMemcpyAsync(d_samp, B.start.data(), 8 * (size_t)(ns + 1), cudaMemcpyHostToDevice, ctx->st), "h2d");
         CK(cudaMemcpyAsync(d_samp + 8 * (size_t)(ns + 1), B.base.data(), 4 * (size_t)ns, cudaMemcpyHostToDevice, ctx->st),
            "h2d");
         CK(cudaMemcpyAsync(d_samp + 12 * (size_t)ns + 8, B.bits.data(), ns, cudaMemcpyHostToDevice, ctx->st), "h2d");
     }
-    // ---- pack
-    CK(cudaEventRecord(ctx->ev[0], ctx->st), "event");
-    CK(launch_pack(j->seq_ptr(), n, ctx->packed.as<uint32_t>(), ctx->valid.as<uint32_t>(), pw,
-                   reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_BASES), ctx->n_sm, ctx->st), "k_pack");
-    ++launches;
-    CK(cudaEventRecord(ctx->ev[1], ctx->st), "event");
-    // ---- phase 1: cut
-    nvtxMarkA("tuna.phase1");
-    CutSamples cs;
     cs.start = ctx->samp.as<unsigned long long>();
     cs.base = reinterpret_cast<const uint32_t*>(ctx->samp.as<uint8_t>() + 8 * (size_t)(ns + 1));
     cs.bits = ctx->samp.as<uint8_t>() + 12 * (size_t)ns + 8;
     cs.n = ns;
-    const tg_status s = run_cut(j, false, p1_bits, &launches, cs, &r.c, deferred);
-    *launches_out += launches;
-    return s;
+    return TG_OK;
+}
+
+static tg_status pack_avail(tg_job* j, const Avail& av, uint64_t most, int* launches) {
+    tg_ctx* ctx = j->ctx;
+    CK(launch_pack(j->seq_ptr(), av, most, ctx->packed.as<uint32_t>(), ctx->valid.as<uint32_t>(),
+                   reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_BASES), ctx->n_sm, ctx->st),
+       "k_pack");
+    ++*launches;
+    return TG_OK;
+}
+
+static tg_status run_phase1(tg_job* j, int* launches_out, P1Out& r, uint32_t p1_force = 0, bool deferred = false) {
+    tg_ctx* ctx = j->ctx;
+    CutSamples cs;
+    tg_status s = setup_phase1(j, j->n, p1_force, r, cs, launches_out);
+    if (s != TG_OK) return s;
+    CK(cudaEventRecord(ctx->ev[0], ctx->st), "event");
+    s = pack_avail(j, Avail{nullptr, nullptr, 0, j->n, 1}, j->n, launches_out);
+    if (s != TG_OK) return s;
+    CK(cudaEventRecord(ctx->ev[1], ctx->st), "event");
+    nvtxMarkA("tuna.phase1");
+    return run_cut(j, false, j->p1_bits, launches_out, cs, &r.c, deferred);
+}
+
+// Bytes of a piece: 80 us of copying, several times what its launches cost.
+constexpr uint64_t LEX_PIECE = 16u << 20;
+constexpr uint64_t MAX_PIECES = 16;
+// Input bytes from which phase 1 runs along with the copy.
+constexpr uint64_t PIPE_MIN = 32u << 20;
+
+// Phase 1 of a one-sample job while its input is still being copied (and lexed): a
+// launch of pack and cut per piece, over what is there (Avail); a cut CTA that runs
+// into the end of that stops and goes on in the next launch (CutState). Its lists
+// are those of many short chunks, so that every piece has work for every SM.
+struct P1Pipe {
+    P1Out r;
+    CutSamples cs;
+    int seg = 0, launches = 0;
+    uint64_t most = 0;
+    Avail last{};
+    bool begun = false;
+
+    // The chunks for an input of len bytes. A piece's are as many as the device holds
+    // CTAs beside the copy's (a CTA on every fourth SM), or a few would run alone after
+    // the others (150 M bases, k=21: 85 us a piece against 62); of at most MAX_PIECES.
+    static CutLayout piece_layout(const tg_job* j, uint64_t len) {
+        const uint32_t n_sm = (uint32_t)j->ctx->n_sm;
+        const CutLayout one = cut_layout(j->w, j->o.k, 1, false, LEX_PIECE, n_sm);
+        const uint64_t wave = (one.slots - n_sm / 4) * one.tile;
+        const uint64_t tiles = std::max((LEX_PIECE - (LEX_PIECE >> 2) + wave - 1) / wave,
+                                        (len + (MAX_PIECES - 1) * wave - 1) / ((MAX_PIECES - 1) * wave));
+        CutLayout l = cut_layout(j->w, j->o.k, 1, false, one.slots * (one.tile * tiles - one.tile / 32), n_sm);
+        l.slots -= n_sm / 4;
+        return l;
+    }
+    static uint64_t piece_bytes(const tg_job* j, uint64_t len) {
+        const CutLayout l = piece_layout(j, len);
+        return l.slots * l.chunk / LEX_PIECE_UNIT * LEX_PIECE_UNIT;
+    }
+    // most: an upper bound of the stream's length.
+    // False: not begun, phase 1 is left to run over the whole.
+    bool begin(tg_job* j, uint64_t most_) {
+        most = most_;
+        begun = most < (1ull << 33) && most <= MAX_PIECES * piece_bytes(j, most) && start(j) == TG_OK;
+        return begun;
+    }
+    tg_status start(tg_job* j) {
+        tg_ctx* ctx = j->ctx;
+        const tg_status s = setup_phase1(j, most, 0, r, cs, &launches);
+        if (s != TG_OK) return s;
+        const CutLayout l = piece_layout(j, most);
+        seg = l.seg;
+        j->chunk = l.chunk;
+        if (cut_smem_bytes(j->w, j->o.k, 1u << j->p1_bits, false, seg) > ctx->smem_optin) return TG_ERR_UNSUPPORTED;
+        j->n_cta = (uint32_t)std::max<uint64_t>(1, (most + j->chunk - 1) / j->chunk);
+        j->desc_cap = (uint64_t)(j->chunk * std::min(1.0, 3.0 / (j->w + 2))) + l.tile / 8 + j->L + 64;
+        CK(ctx->ensure(ctx->desc, (size_t)j->n_cta * j->desc_cap * 8), "alloc descriptors");
+        CK(ctx->ensure(ctx->cstate, (size_t)j->n_cta * sizeof(CutState)), "alloc cut states");
+        CK(cudaMemsetAsync(ctx->cstate.p, 0, (size_t)j->n_cta * sizeof(CutState), ctx->st), "memset");
+        return TG_OK;
+    }
+    // av.prev as the call before left it; hi: an upper bound of av's length
+    tg_status piece(tg_job* j, Avail av, uint64_t hi) {
+        tg_ctx* ctx = j->ctx;
+        av.prev_p = last.cur_p;
+        av.prev = last.cur;
+        if (av.last) CK(cudaEventRecord(ctx->ev[0], ctx->st), "event");
+        const tg_status s = pack_avail(j, av, av.last ? most : hi, &launches);
+        if (s != TG_OK) return s;
+        CutParams P = cut_params(j, seg, cs);
+        P.avail = av;
+        P.state = ctx->cstate.as<CutState>();
+        if (!av.last) P.n_cta = (uint32_t)std::min<uint64_t>(P.n_cta, (hi + P.chunk - 1) / P.chunk);
+        if (av.last) CK(cudaEventRecord(ctx->ev[1], ctx->st), "event");
+        if (av.last) CK(cudaEventRecord(ctx->ev[2], ctx->st), "event");
+        CK(launch_cut(P, ctx->tables.as<HashTables>(), false, ctx->st), "k_cut");
+        if (av.last) CK(cudaEventRecord(ctx->ev[3], ctx->st), "event");
+        ++launches;
+        last = av;
+        return TG_OK;
+    }
+    // waits; true in `ok` when the job may go on from here (else phase 1 runs as usual)
+    tg_status finish(tg_job* j, bool& ok) {
+        const tg_status s = read_misc(j->ctx, r.c);
+        ok = s == TG_OK && !r.c.overflow;
+        return s;
+    }
+};
+
+// FASTA/FASTQ bytes in device memory (16-byte aligned) lexed on the device
+// onto the end of the stream. host_raw, when given, is the same bytes in host
+// memory, copied to draw (ctx->raw) here: a long file in pieces, each lexed while
+// the next is copied. A FASTQ file the device lexer flags (an empty header line at file
+// offset 63 mod 64, where the reference's block walk departs from line
+// counting) is parsed by the host parser instead.
+static tg_status lex_append(tg_job* j, const uint8_t* draw, size_t len, const uint8_t* host_raw, P1Pipe* pipe) {
+    const TraceRange tr("tuna.lex");
+    tg_ctx* ctx = j->ctx;
+    if (j->ran) return ctx->fail(TG_ERR_STATE, "feed after run");
+    if (len == 0) return ctx->fail(TG_ERR_PARSE, "Empty file");
+    uint8_t* at = nullptr;
+    tg_status s = stream_reserve(j, len + 1, &at);
+    if (s != TG_OK) return s;
+    uint8_t first = 0;
+    if (host_raw) {
+        first = host_raw[0];
+    } else {
+        CK(cudaMemcpyAsync(&first, draw, 1, cudaMemcpyDeviceToHost, ctx->st), "d2h");
+        CK(cudaStreamSynchronize(ctx->st), "d2h");
+    }
+    const bool fastq = first == '@';
+    CK(ctx->ensure(ctx->lexs, lex_scratch_bytes(len)), "alloc lexer scratch");
+    LexTotals* dt = nullptr;
+    int launches = 0;
+    uint64_t np = host_raw && !ctx->copy_pending ? std::max<uint64_t>(1, std::min<uint64_t>(MAX_PIECES, len / LEX_PIECE)) : 1;
+    // more than one piece: the copies on the copy stream, in order (not behind a result copy)
+    cudaStream_t cst = np > 1 ? ctx->st_copy : ctx->st;
+    size_t per = (size_t)((len + np - 1) / np + LEX_PIECE_UNIT - 1) / LEX_PIECE_UNIT * LEX_PIECE_UNIT;
+    // one FASTA file: phase 1 runs along. Not for FASTQ: its lexer takes as long as the
+    // copy, and behind it the cut in pieces gains 3 % (138 M bases, k=31) or loses 2 %
+    // (300 M, k=63). Nor beside a run's result copy.
+    if (pipe && (fastq || np < 2 || j->n || !pipe->begin(j, len))) pipe = nullptr;
+    if (pipe) per = P1Pipe::piece_bytes(j, len);
+    if (host_raw) CK(cudaEventRecord(ctx->ev[4], cst), "event");
+    unsigned long long* avail =
+        pipe ? reinterpret_cast<unsigned long long*>(ctx->misc.as<uint8_t>() + MISC_AVAIL) : nullptr;
+    for (uint64_t lo = 0, q = 0; lo < len; lo += per, ++q) {
+        const uint64_t hi = std::min<uint64_t>(len, lo + per);
+        if (host_raw) {
+            cudaError_t e = link_copy(const_cast<uint8_t*>(draw) + lo, host_raw + lo, hi - lo, cudaMemcpyHostToDevice, cst, ctx->n_sm);
+            if (e == cudaSuccess && hi == len) e = cudaEventRecord(ctx->ev[10], cst);
+            if (e == cudaSuccess && np > 1) e = cudaEventRecord(ctx->wave_ev[q], cst);
+            if (e == cudaSuccess && np > 1) e = cudaStreamWaitEvent(ctx->st, ctx->wave_ev[q], 0);
+            if (e != cudaSuccess) {
+                cudaStreamSynchronize(cst);  // the caller's bytes are read no more
+                return ctx->cuda_fail(e, "copy input");
+            }
+        } else {
+            CK(cudaEventRecord(ctx->ev[10], ctx->st), "event");
+        }
+        const cudaError_t e = launch_lex(draw, len, fastq, at, ctx->lexs.p, ctx->n_sm, ctx->st, &dt, &launches, lo, hi,
+                                         pipe ? avail + q : nullptr);
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(cst);
+            return ctx->cuda_fail(e, "k_lex");
+        }
+        if (hi == len) CK(cudaEventRecord(ctx->ev[11], ctx->st), "event");
+        if (pipe) {
+            s = pipe->piece(j, Avail{nullptr, avail + q, 0, 0, hi == len}, hi);
+            if (s != TG_OK) {
+                cudaStreamSynchronize(cst);
+                return s;
+            }
+        }
+    }
+    LexTotals t{};
+    CK(cudaMemcpyAsync(&t, dt, sizeof t, cudaMemcpyDeviceToHost, ctx->st), "d2h");
+    CK(cudaStreamSynchronize(ctx->st), "k_lex");
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ctx->ev[10], ctx->ev[11]);  // from the last copy's end on
+    j->st.lex_ms += ms;
+    if (host_raw && cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[10]) == cudaSuccess) j->st.h2d_ms += ms;
+    j->st.fastx_bytes += len;
+    j->lex_launches += launches;
+    if (pipe && t.irregular) pipe->begun = false;  // phase 1 again, over the stream as it is
+    if (t.irregular & 2u) return ctx->fail(TG_ERR_DEVICE, "FASTA/FASTQ lexer: a staging copy did not complete");
+    if (t.irregular) {
+        std::vector<uint8_t> hraw;
+        if (!host_raw) {
+            hraw.resize(len);
+            CK(cudaMemcpy(hraw.data(), draw, len, cudaMemcpyDeviceToHost), "d2h");
+            host_raw = hraw.data();
+        }
+        std::vector<uint8_t> st;
+        tgh::fastx_to_stream(host_raw, len, st);
+        j->st.host_parsed_bytes += len;
+        return append_stream(j, st.data(), st.size(), cudaMemcpyHostToDevice);
+    }
+    CK(cudaMemsetAsync(at + t.out, '\n', 1, ctx->st), "separator");
+    j->n += t.out + 1;
+    j->used_ctx_seq = true;
+    j->st.input_bytes += t.out;
+    return TG_OK;
 }
 
 static tg_status run_spill(tg_job* j);
@@ -941,11 +1067,15 @@ static tg_status tg_job_run_impl(tg_job* j) {
     const int W = j->W;
     j->ran = true;
     const uint64_t per_key = 2 * key_bytes(W) + 4 + 24;  // key, pair, groups and slack
-    const bool deferred = j->n <= DEFER_BYTES && j->n_shards == 1 &&
+    const bool deferred = !j->done && j->n <= DEFER_BYTES && j->n_shards == 1 &&
                           (!ctx->hbm_budget || std::max<uint64_t>(j->n, 1) * per_key <= ctx->hbm_budget);
     P1Out r1;
-    const tg_status s1 = run_phase1(j, &launches, r1, 0, deferred);
-    if (s1 != TG_OK) return s1;
+    if (j->done) {
+        r1 = std::move(*j->done);
+    } else {
+        const tg_status s1 = run_phase1(j, &launches, r1, 0, deferred);
+        if (s1 != TG_OK) return s1;
+    }
     const SampleBins& B = r1.B;
     const uint32_t ns = (uint32_t)B.base.size();
     const uint32_t C = j->n_cta;
@@ -1860,12 +1990,13 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
         total += lens[i] + (n > 1 ? 1 : 0);
     }
     bool fed = false;
+    P1Pipe pipe;
     if (s == TG_OK && fastx) {
         // each sample's FASTA/FASTQ bytes lexed on the device into its own sample
         // (an empty sample stays empty)
         for (uint32_t i = a; i < b && s == TG_OK; ++i) {
             if (i > a) s = tg_job_next_sample(j);
-            if (s == TG_OK && lens[i]) s = lex_append_host(j, seqs[i], lens[i]);
+            if (s == TG_OK && lens[i]) s = lex_append_host(j, seqs[i], lens[i], n == 1 ? &pipe : nullptr);
         }
     } else if (s == TG_OK && total) {
         // not waited for: the call returns only after the counts, or waits when it fails
@@ -1886,7 +2017,23 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
         if (e == cudaSuccess) e = ctx->ensure(ctx->seq, total + 1);
         if (e == cudaSuccess) e = cudaEventRecord(ctx->ev[9], ctx->st);
         uint64_t off = 0;
-        if (gather && e == cudaSuccess) {
+        if (n == 1 && lens[a] >= PIPE_MIN && !ctx->copy_pending && mapped_address(seqs[a]) && e == cudaSuccess) {
+            j->used_ctx_seq = true;
+            pipe.begin(j, lens[a]);
+        }
+        if (pipe.begun) {
+            // one long stream: phase 1 runs along with the copy
+            const uint64_t len = lens[a], per = P1Pipe::piece_bytes(j, len);
+            j->st.input_bytes += len;
+            for (uint64_t lo = 0, q = 0; lo < len && e == cudaSuccess && s == TG_OK; lo += per, ++q) {
+                const uint64_t hi = std::min(len, lo + per);
+                e = link_copy(ctx->seq.as<uint8_t>() + lo, seqs[a] + lo, hi - lo, cudaMemcpyHostToDevice, ctx->st_copy, ctx->n_sm);
+                if (e == cudaSuccess) e = cudaEventRecord(ctx->wave_ev[q], ctx->st_copy);
+                if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->st, ctx->wave_ev[q], 0);
+                if (e == cudaSuccess) s = pipe.piece(j, Avail{nullptr, nullptr, 0, hi, hi == len}, hi);
+            }
+            if (e != cudaSuccess || s != TG_OK) cudaStreamSynchronize(ctx->st_copy);
+        } else if (gather && e == cudaSuccess) {
             std::vector<LinkPiece> ps;
             uint8_t* const d = ctx->seq.as<uint8_t>();
             uint64_t end = 0;  // of the sample before, past its separators
@@ -1954,6 +2101,12 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
     j->sink_keys = kdst;
     j->sink_counts = cdst;
     j->sink_cap = room;
+    if (s == TG_OK && pipe.begun) {
+        bool ok = false;
+        s = pipe.finish(j, ok);
+        if (ok) j->done = &pipe.r;
+        j->lex_launches += pipe.launches;
+    }
     if (s == TG_OK) s = tg_job_run(j);
     if (fed) {
         float ms = 0;

@@ -86,15 +86,48 @@ __host__ __device__ __forceinline__ uint64_t hist_kmers_offset(uint64_t p1, uint
     return (p1 * n_cta + 1) & ~uint64_t(1);
 }
 
+// How much of a stream is there: all of it (last), or its first bytes while the rest
+// is still copied or lexed. The lengths are values, or in device memory where a
+// kernel before this one wrote them.
+struct Avail {
+    const unsigned long long* prev_p;  // length at the launch before (0 at the first)
+    const unsigned long long* cur_p;   // length now
+    unsigned long long prev, cur;      // the same, where the pointers are null
+    int last;
+};
+__device__ __forceinline__ uint64_t avail_prev(const Avail& a) { return a.prev_p ? *a.prev_p : a.prev; }
+__device__ __forceinline__ uint64_t avail_now(const Avail& a) { return a.cur_p ? *a.cur_p : a.cur; }
+
+// How a stream of n bytes is cut: positions per thread and tile, and per tile; CTAs the
+// device holds; tiles per chunk; positions per chunk (one CTA's, one descriptor list's); chunks.
+struct CutLayout {
+    int seg;
+    uint64_t tile;
+    uint32_t slots;
+    uint64_t tiles, chunk;
+    uint32_t n_cta;
+};
+
+// Where a cut CTA stopped for want of input, to go on from in a later launch.
+struct CutState {
+    int64_t t0, carry_cs, open;
+    uint32_t carry_m, open_m, n_desc;
+    int open_own;
+    uint32_t phase;  // 0: not begun, 1: stopped before tile t0, 2: done
+    uint32_t pad[3];
+};
+
 struct CutParams {
     const uint32_t* packed;
     const uint32_t* valid;
-    uint64_t n;              // sequence stream length (positions)
+    uint64_t n;              // export cut: sequence stream length (positions)
+    Avail avail;             // counting cut: the stream
+    CutState* state;         // counting cut in several launches: [n_cta], zero before the first; else null
     int k, m, w;
     uint32_t L;              // max k-mers per record (forced split period)
     uint32_t p1_bits;        // log2 internal bucket count
     uint32_t n_cta;
-    int seg;                 // counting cut: k-mer start positions per thread and tile (cut_seg)
+    int seg;                 // counting cut: k-mer start positions per thread and tile (cut_layout)
     uint64_t chunk;          // k-mer start positions per CTA (multiple of CUT_TILE)
     uint64_t* desc;          // [n_cta][desc_cap] record descriptors
     uint64_t desc_cap;

@@ -16,15 +16,17 @@ namespace tg {
 // A job of at most this many stream bytes runs in one go: buffers sized by bounds, the
 // counts read on the device, one wait at the end (P2Input::deferred).
 constexpr uint64_t DEFER_BYTES = 4u << 20;
-// Shapes of the cut; seg: k-mer start positions per thread and tile (cut_seg).
+// Shapes of the cut; seg: k-mer start positions per thread and tile (cut_layout).
 size_t cut_smem_bytes(int w, int k, uint32_t p1, bool exp, int seg = 128);
 uint64_t cut_tile(int w, bool exp, int seg = 128);  // k-mer start positions per tile of a cut CTA
 uint32_t cut_ctas_per_sm(int w, int k, uint32_t p1, bool exp, int seg = 128);
-int cut_seg(int w, int k, uint64_t n, uint32_t n_sm);
+CutLayout cut_layout(int w, int k, uint32_t p1, bool exp, uint64_t n, uint32_t n_sm);
 cudaError_t launch_prepare(const PrepareParams& P, cudaStream_t st);
 // Packed words (a multiple of 4) for a stream of n bytes, padding included.
 uint64_t packed_words_for(uint64_t n);
-cudaError_t launch_pack(const uint8_t* seq, uint64_t n, uint32_t* packed, uint32_t* valid, uint64_t n_words,
+// Packs what of the stream is there and was not at the launch before; most: an
+// upper bound of its length.
+cudaError_t launch_pack(const uint8_t* seq, const Avail& av, uint64_t most, uint32_t* packed, uint32_t* valid,
                         unsigned long long* n_bases, int n_sm, cudaStream_t st);
 cudaError_t launch_cut(const CutParams& P, const HashTables* gT, bool exp, cudaStream_t st);
 // Exclusive scans of n >= 1 counts into n + 1 entries (the last: the total, which
@@ -50,7 +52,8 @@ size_t lex_scratch_bytes(uint64_t len);
 // bytes [lo, hi) of it, lo a multiple of LEX_PIECE_UNIT and hi too or len.
 constexpr uint64_t LEX_PIECE_UNIT = 16384;
 cudaError_t launch_lex(const uint8_t* raw, uint64_t len, bool fastq, uint8_t* out, void* scratch, int n_sm,
-                       cudaStream_t st, LexTotals** dtot, int* launches, uint64_t lo, uint64_t hi);
+                       cudaStream_t st, LexTotals** dtot, int* launches, uint64_t lo, uint64_t hi,
+                       unsigned long long* piece_out = nullptr);  // receives the stream's length so far
 // Output formatting on the device (tg_format.cu): n pairs to the bytes of
 // format fmt (tg_format). TSV writes its byte count to d_total (device-
 // writable, e.g. mapped host memory); KFF and RAW records have a fixed size,

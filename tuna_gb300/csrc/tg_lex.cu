@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_lex_scan(const LexFn<ull>* __r
                                                            int fastq, int last, uint64_t len,
                                                            const long long* __restrict__ last_na,
                                                            uint8_t* __restrict__ cstate, ull* __restrict__ coff,
-                                                           LexTotals* tot) {
+                                                           LexTotals* tot, ull* __restrict__ piece_out) {
     constexpr int NW = SCAN_THREADS / 32;
     __shared__ LexFn<ull> s_w[NW];
     __shared__ ull s_off[NW];
@@ -422,6 +422,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_lex_scan(const LexFn<ull>* __r
             off -= len - drop;
         }
         tot->out = off;
+        if (piece_out) *piece_out = off;
         tot->drop_from = drop;
         tot->final_state = s;
     }
@@ -562,7 +563,8 @@ size_t lex_scratch_bytes(uint64_t len) {
 }
 
 cudaError_t launch_lex(const uint8_t* raw, uint64_t len, bool fastq, uint8_t* out, void* scratch, int n_sm,
-                       cudaStream_t st, LexTotals** dtot, int* launches, uint64_t lo, uint64_t hi) {
+                       cudaStream_t st, LexTotals** dtot, int* launches, uint64_t lo, uint64_t hi,
+                       unsigned long long* piece_out) {
     static_assert(LEX_PIECE_UNIT == LEX_CHUNK, "pieces of whole chunks");
     const uint64_t c0 = lo / LEX_CHUNK, c1 = (hi + LEX_CHUNK - 1) / LEX_CHUNK, nc = c1 - c0;
     const uint64_t G = std::max<uint64_t>(1, std::min<uint64_t>({nc, (uint64_t)n_sm * LEX_CTAS_PER_SM, LEX_MAX_CTAS}));
@@ -584,7 +586,7 @@ cudaError_t launch_lex(const uint8_t* raw, uint64_t len, bool fastq, uint8_t* ou
     const int last = hi == len;
     if (fastq) k_lex_sum<1><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, c0, c1, per, fn, last_na, tot);
     else k_lex_sum<0><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, c0, c1, per, fn, last_na, tot);
-    k_lex_scan<<<1, SCAN_THREADS, 0, st>>>(fn, G, fastq ? 1 : 0, last, len, last_na, cstate, coff, tot);
+    k_lex_scan<<<1, SCAN_THREADS, 0, st>>>(fn, G, fastq ? 1 : 0, last, len, last_na, cstate, coff, tot, piece_out);
     if (fastq) k_lex_emit<1><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, c0, c1, per, cstate, coff, tot, out);
     else k_lex_emit<0><<<(unsigned)G, LEX_THREADS, 0, st>>>(raw, len, c0, c1, per, cstate, coff, tot, out);
     if (launches) *launches += 3;

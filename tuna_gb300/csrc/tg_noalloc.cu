@@ -160,13 +160,10 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     uint32_t p1_bits = 0;
     while ((1u << p1_bits) < p1) ++p1_bits;
     p1 = 1u << p1_bits;
-    const int seg = cut_seg(w, k, n, (uint32_t)n_sm);
-    const uint64_t tile = cut_tile(w, false, seg);
-    uint32_t C = (uint32_t)n_sm * cut_ctas_per_sm(w, k, p1, false, seg);
-    uint64_t chunk = (n + C - 1) / C;
-    chunk = std::max<uint64_t>(tile, (chunk + tile - 1) / tile * tile);
-    C = (uint32_t)std::max<uint64_t>(1, (n + chunk - 1) / chunk);
-    const uint64_t desc_cap = chunk + 2ull * tile + L + 64;
+    const CutLayout lay = cut_layout(w, k, p1, false, n, (uint32_t)n_sm);
+    const uint32_t C = lay.n_cta;
+    const uint64_t chunk = lay.chunk;
+    const uint64_t desc_cap = lay.tiles * lay.tile + 2ull * lay.tile + L + 64;
     uint64_t* desc = cv.take<uint64_t>((size_t)C * desc_cap);
     uint32_t* n_desc = cv.take<uint32_t>(C);
     const int bin_bits = job_bin_bits(n, 1, p1_bits);
@@ -194,14 +191,15 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     pp.bin_bits = bin_bits;
     NA_CK(launch_prepare(pp, st), "k_prepare");
     // ---- phase 1
-    NA_CK(launch_pack(d_seq, n, packed, valid, pw, misc + 4, n_sm, st), "k_pack");
+    const Avail all{nullptr, nullptr, 0, n, 1};
+    NA_CK(launch_pack(d_seq, all, n, packed, valid, misc + 4, n_sm, st), "k_pack");
     CutParams P{};
-    P.packed = packed; P.valid = valid; P.n = n;
+    P.packed = packed; P.valid = valid; P.n = n; P.avail = all;
     P.k = k; P.m = m; P.w = w; P.L = L;
     P.p1_bits = p1_bits; P.n_cta = C; P.chunk = chunk;
     P.desc = desc; P.desc_cap = desc_cap; P.n_desc = n_desc;
     P.hist = nullptr; P.binhist = binhist; P.stats = misc; P.overflow = reinterpret_cast<uint32_t*>(misc + 5); P.xdesc = nullptr;
-    P.seg = seg; P.max_desc = reinterpret_cast<uint32_t*>(misc + 6);
+    P.seg = lay.seg; P.max_desc = reinterpret_cast<uint32_t*>(misc + 6);
     P.sample_start = s_start; P.sample_bin_base = s_base; P.sample_bin_bits = s_bits; P.n_samples = 1;
     P.desc_sb = desc_start_bits(bin_bits);
     NA_CK(launch_cut(P, tables, false, st), "k_cut");

@@ -40,15 +40,26 @@ __device__ __forceinline__ void pack_word4(uint32_t x, uint32_t& code8, uint32_t
     ok4 = ((ok & 0x01010101u) * 0x01020408u) >> 24;
 }
 
-__global__ void __launch_bounds__(256) k_pack(const uint8_t* __restrict__ seq, uint64_t n,
+// A stream that arrives in pieces is packed in as many launches, each the groups
+// that lie wholly in what is there and were not before; the last launch adds the
+// ragged end and the padding behind it.
+__host__ __device__ __forceinline__ uint64_t pack_words(uint64_t n) {
+    const uint64_t pw = (TG_PAD + n + CUT_SPAN + 2 * MAX_W + 640) / 16 + 16;
+    return (pw + 3) & ~uint64_t(3);
+}
+__host__ __device__ __forceinline__ uint64_t whole_groups(uint64_t n) { return (n + TG_PAD) / 64; }
+
+__global__ void __launch_bounds__(256) k_pack(const uint8_t* __restrict__ seq, Avail av,
                                               uint32_t* __restrict__ packed, uint32_t* __restrict__ valid,
-                                              uint64_t n_groups, unsigned long long* __restrict__ n_bases) {
+                                              unsigned long long* __restrict__ n_bases) {
+    const uint64_t n = avail_now(av), n_groups = av.last ? pack_words(n) / 4 : whole_groups(n);
+    const uint64_t first = av.prev_p || av.prev ? whole_groups(avail_prev(av)) : 0;  // 0: the first launch, padding and all
     __shared__ unsigned s_cnt;
     if (threadIdx.x == 0) s_cnt = 0;
     __syncthreads();
     unsigned cnt = 0;
     const bool aligned = (reinterpret_cast<uintptr_t>(seq) & 15u) == 0;
-    for (uint64_t gi = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gi < n_groups;
+    for (uint64_t gi = first + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gi < n_groups;
          gi += (uint64_t)gridDim.x * blockDim.x) {
         const int64_t g0 = (int64_t)(gi * 64) - TG_PAD;
         uint32_t x[16];
@@ -501,8 +512,9 @@ k_cut(CutParams P, const HashTables* __restrict__ gT) {
 // segment holds at most one forced split.
 // Jobs too short to give every CTA a few tiles of such segments take 32 positions
 // per thread: more warm-up, but four times the CTAs and a quarter of the steps in
-// sequence (cut_seg).
+// sequence (cut_layout).
 constexpr int LONG_SEG = 128, SHORT_SEG = 32;
+constexpr int CUT_AHEAD = 512;  // bases past a tile's end that it may read (k, the last batch's windows)
 static_assert(LONG_SEG * 256 <= CUT_SPAN, "a cut tile must fit the packed arrays' slack");
 
 constexpr size_t SEQ_TABLE_BYTES = offsetof(HashTables, GF);
@@ -623,16 +635,35 @@ k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
     const int tid = threadIdx.x, lane = tid & 31;
     const int k = P.k, m = P.m, w = P.w, B = w + 1;
     const uint32_t c = blockIdx.x;
+    const int64_t cstart = (int64_t)c * (int64_t)P.chunk;
+    // a launch before the last: the stream's end is not known, and a tile waits until
+    // all that it reads is packed
+    const uint64_t here = avail_now(P.avail);
+    const int64_t n = P.avail.last ? (int64_t)here : INT64_MAX;
+    const int64_t ready = P.avail.last ? INT64_MAX
+                                       : (int64_t)(64 * whole_groups(here)) - TG_PAD - (NT * SEG + CUT_AHEAD);
+    CutState was{};
+    if (P.state) {
+        was = P.state[c];
+        if (was.phase == 2 || (was.phase == 0 && cstart > ready)) return;
+    }
+    const int64_t t_begin = was.phase ? was.t0 : cstart;
     {
         const uint64_t* src = reinterpret_cast<const uint64_t*>(gT);
         uint64_t* dst = reinterpret_cast<uint64_t*>(&T);  // T.GF and T.GR are not staged
         for (int i = tid; i < (int)(SEQ_TABLE_BYTES / 8); i += NT) dst[i] = src[i];
-        if (tid == 0) { s_carry_cs = -1; s_carry_m = 0; s_open = -1; s_open_m = 0; s_open_own = 0; s_ndesc = 0; }
+        if (tid == 0) {
+            s_carry_cs = was.phase ? was.carry_cs : -1;
+            s_carry_m = was.carry_m;
+            s_open = was.phase ? was.open : -1;
+            s_open_m = was.open_m;
+            s_open_own = was.open_own;
+            s_ndesc = was.n_desc;
+        }
     }
     __syncthreads();
 
-    const int64_t cstart = (int64_t)c * (int64_t)P.chunk;
-    const int64_t cend = min(cstart + (int64_t)P.chunk, (int64_t)P.n);
+    const int64_t cend = min(cstart + (int64_t)P.chunk, n);
     const uint64_t kmask = (1ull << k) - 1;  // k <= 63
     const int64_t Lr = P.L;
     unsigned long long loc_kmers = 0, loc_recs = 0, loc_runs = 0;
@@ -674,8 +705,11 @@ k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
         if (e) put(base + __popc(bal & ((1u << lane) - 1)), st, nk, mlo);
     };
 
-    for (int64_t t0 = cstart; t0 < (int64_t)P.n; t0 += (int64_t)NT * SEG) {
+    int64_t t0 = t_begin;
+    bool stopped = false;
+    for (; t0 < n; t0 += (int64_t)NT * SEG) {
         if (t0 >= cend && !(s_open >= 0 && s_open_own)) break;  // nothing of ours is still open
+        if (t0 > ready) { stopped = true; break; }
         // ---- stage packed and validity words: array bases [A0, A0 + 16 npk)
         const uint64_t A0 = (uint64_t)(t0 + TG_PAD - 1) & ~uint64_t(31);
         for (uint32_t i = tid; i < L.npk; i += NT) s_pk[i] = P.packed[(A0 >> 4) + i];
@@ -809,6 +843,17 @@ k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
         __syncthreads();
     }
     // ---- counters
+    if (tid == 0 && P.state) {
+        CutState& s = P.state[c];
+        s.t0 = t0;
+        s.carry_cs = s_carry_cs;
+        s.carry_m = s_carry_m;
+        s.open = s_open;
+        s.open_m = s_open_m;
+        s.open_own = s_open_own;
+        s.n_desc = s_ndesc;
+        s.phase = stopped ? 1 : 2;
+    }
     if (tid == 0) {
         P.n_desc[c] = s_ndesc;
         atomicMax(P.max_desc, s_ndesc);
@@ -957,17 +1002,36 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
     const int tid = threadIdx.x, lane = tid & 31;
     const unsigned below = (1u << lane) - 1;
     const uint32_t c = blockIdx.x;
+    const int64_t cstart = (int64_t)c * (int64_t)P.chunk;
+    // a launch before the last: the stream's end is not known, and a tile waits until
+    // all that it reads is packed
+    const uint64_t here = avail_now(P.avail);
+    const int64_t n = P.avail.last ? (int64_t)here : INT64_MAX;
+    const int64_t ready = P.avail.last ? INT64_MAX
+                                       : (int64_t)(64 * whole_groups(here)) - TG_PAD - (NT * SEG + CUT_AHEAD);
+    CutState was{};
+    if (P.state) {
+        was = P.state[c];
+        if (was.phase == 2 || (was.phase == 0 && cstart > ready)) return;
+    }
+    const int64_t t_begin = was.phase ? was.t0 : cstart;
     {
         const uint64_t* src = reinterpret_cast<const uint64_t*>(gT);
         uint64_t* dst = reinterpret_cast<uint64_t*>(&T);
         for (int i = tid; i < (int)(sizeof(HashTables) / 8); i += NT) dst[i] = src[i];
         if (tid < 16) s_ct[tid] = make_ulonglong2(gT->CTF[tid], gT->CTR[tid]);
-        if (tid == 0) { s_carry_cs = -1; s_carry_m = 0; s_open = -1; s_open_m = 0; s_open_own = 0; s_ndesc = 0; }
+        if (tid == 0) {
+            s_carry_cs = was.phase ? was.carry_cs : -1;
+            s_carry_m = was.carry_m;
+            s_open = was.phase ? was.open : -1;
+            s_open_m = was.open_m;
+            s_open_own = was.open_own;
+            s_ndesc = was.n_desc;
+        }
     }
     __syncthreads();
 
-    const int64_t cstart = (int64_t)c * (int64_t)P.chunk;
-    const int64_t cend = min(cstart + (int64_t)P.chunk, (int64_t)P.n);
+    const int64_t cend = min(cstart + (int64_t)P.chunk, n);
     const int64_t Lr = P.L;
     unsigned long long loc_kmers = 0, loc_recs = 0, loc_runs = 0;
     uint32_t loc_extra = 0;  // packed records beyond one per record
@@ -1011,8 +1075,11 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
         if (e) put(base + __popc(bal & ((1u << lane) - 1)), st, nk, mlo);
     };
 
-    for (int64_t t0 = cstart; t0 < (int64_t)P.n; t0 += (int64_t)NT * SEG) {
+    int64_t t0 = t_begin;
+    bool stopped = false;
+    for (; t0 < n; t0 += (int64_t)NT * SEG) {
         if (t0 >= cend && !(s_open >= 0 && s_open_own)) break;
+        if (t0 > ready) { stopped = true; break; }
         const uint64_t A0 = (uint64_t)(t0 + TG_PAD - 1) & ~uint64_t(31);
         for (uint32_t i = tid; i < Ly.npk; i += NT) s_pk[i] = P.packed[(A0 >> 4) + i];
         for (uint32_t i = tid; i < Ly.nvb; i += NT) s_vb[i] = P.valid[(A0 >> 5) + i];
@@ -1184,6 +1251,17 @@ k_cut_fixed(CutParams P, const HashTables* __restrict__ gT) {
         if (oo && nxt == NT) { s_open = os; s_open_m = om; s_open_own = oown ? 1 : 0; }
         if (tid == 0 && last_t >= 0) { s_carry_cs = s_cs[last_t]; s_carry_m = s_cm[last_t]; }
         __syncthreads();
+    }
+    if (tid == 0 && P.state) {
+        CutState& s = P.state[c];
+        s.t0 = t0;
+        s.carry_cs = s_carry_cs;
+        s.carry_m = s_carry_m;
+        s.open = s_open;
+        s.open_m = s_open_m;
+        s.open_own = s_open_own;
+        s.n_desc = s_ndesc;
+        s.phase = stopped ? 1 : 2;
     }
     if (tid == 0) {
         P.n_desc[c] = s_ndesc;
@@ -1376,11 +1454,30 @@ uint32_t cut_ctas_per_sm(int w, int k, uint32_t p1, bool exp, int seg) {
     return std::max<uint32_t>(1, std::min<uint32_t>(exp ? 2u : 768u / (uint32_t)seq_threads(w), by_smem));
 }
 
-// Long segments once every CTA that fits on the device gets two tiles of them
-// (k=31 m=21, 1.5 Mbp: 88 us with long segments).
-int cut_seg(int w, int k, uint64_t n, uint32_t n_sm) {
-    const uint64_t ctas = (uint64_t)n_sm * cut_ctas_per_sm(w, k, 1, false, LONG_SEG);
-    return n >= 2 * ctas * cut_tile(w, false, LONG_SEG) ? LONG_SEG : SHORT_SEG;
+// A chunk ends CUT_TAIL positions before its CTA's last tile does, so that a record
+// open at the chunk's end nearly always closes in that tile (a chain without a
+// repeated minimizer is at most w + 1 k-mers long): with chunks of whole tiles every
+// CTA walks one tile more to close it.
+constexpr uint64_t CUT_TAIL = 64;
+
+// Of the two segment lengths the one whose tiles take less: a CTA with all its
+// neighbours busy takes about 19 us for a tile of short segments and 48 us for one of
+// long segments, of four times the positions (k=31 m=21 and k=21 m=17).
+CutLayout cut_layout(int w, int k, uint32_t p1, bool exp, uint64_t n, uint32_t n_sm) {
+    CutLayout best{};
+    for (const int seg : {LONG_SEG, SHORT_SEG}) {
+        CutLayout l{};
+        l.seg = seg;
+        l.tile = cut_tile(w, exp, seg);
+        l.slots = n_sm * cut_ctas_per_sm(w, k, p1, exp, seg);
+        const uint64_t tail = exp ? 0 : CUT_TAIL, each = (n + l.slots - 1) / l.slots;
+        l.tiles = std::max<uint64_t>(1, (each + tail + l.tile - 1) / l.tile);
+        l.chunk = l.tiles * l.tile - tail;
+        l.n_cta = (uint32_t)std::max<uint64_t>(1, (n + l.chunk - 1) / l.chunk);
+        if (seg == LONG_SEG || (!exp && 2 * l.tiles < 5 * best.tiles)) best = l;
+        if (exp) break;
+    }
+    return best;
 }
 
 cudaError_t launch_prepare(const PrepareParams& P, cudaStream_t st) {
@@ -1389,20 +1486,16 @@ cudaError_t launch_prepare(const PrepareParams& P, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_pack(const uint8_t* seq, uint64_t n, uint32_t* packed, uint32_t* valid, uint64_t n_words,
+cudaError_t launch_pack(const uint8_t* seq, const Avail& av, uint64_t most, uint32_t* packed, uint32_t* valid,
                         unsigned long long* n_bases, int n_sm, cudaStream_t st) {
-    // n_words is a multiple of 4 (packed_words_for): groups of 4 words
-    const uint64_t groups = n_words / 4;
+    const uint64_t groups = pack_words(most) / 4;
     const uint32_t threads = 256;
     const uint64_t blocks = std::min<uint64_t>((groups + threads - 1) / threads, (uint64_t)std::max(n_sm, 1) * 8);
-    k_pack<<<(unsigned)std::max<uint64_t>(blocks, 1), threads, 0, st>>>(seq, n, packed, valid, groups, n_bases);
+    k_pack<<<(unsigned)std::max<uint64_t>(blocks, 1), threads, 0, st>>>(seq, av, packed, valid, n_bases);
     return cudaGetLastError();
 }
 
-uint64_t packed_words_for(uint64_t n) {
-    const uint64_t pw = (TG_PAD + n + CUT_SPAN + 2 * MAX_W + 640) / 16 + 16;
-    return (pw + 3) & ~uint64_t(3);
-}
+uint64_t packed_words_for(uint64_t n) { return pack_words(n); }
 
 template <typename Kernel>
 static cudaError_t launch_one(Kernel kernel, int threads, const CutParams& P, const HashTables* gT, size_t sm,
