@@ -62,3 +62,38 @@ def test_overlapped_phase1(kind, k, m, size):
                 assert np.array_equal(got.keys, want.keys)
                 assert np.array_equal(got.counts, want.counts)
                 assert st.kmers == want.stats["kmers"] and st.superkmers == want.stats["superkmers"]
+
+
+@pytest.mark.parametrize("k,m", [(31, 23), (63, 21)])
+def test_overlapped_batch(k, m):
+    """Samples of page-locked memory at odd addresses, an empty one and one of a base among them."""
+    import tuna_gb300 as T
+    L = T.library()
+    W = 1 if k <= 31 else 2
+    lens = [11 * MIB + 5, 0, 1, 20 * MIB + 17, 33, 9 * MIB]
+    with T.Context(0) as ctx, T.HostBuffer(sum(lens) + 64 * len(lens)) as h_in:
+        buf, at, smp = h_in.array(), 0, []
+        for i, ln in enumerate(lens):
+            at = (at + 15) // 16 * 16 + 3 * i
+            buf[at:at + ln] = _bases(ln, i) if ln > 10 * MIB else _bases(11 * MIB, i)[:ln]
+            smp.append(buf[at:at + ln])
+            at += ln
+        want, _ = ctx.run(k, m, samples=[s.copy() for s in smp])
+        n = len(want)
+        with T.HostBuffer(8 * W * n) as h_keys, T.HostBuffer(4 * n) as h_cnt:
+            o = T._JobOpts(k, m, 16, 1, (1 << 64) - 1, 0, 0)
+            n_out = ctypes.c_uint64()
+            off = np.zeros(len(lens) + 1, dtype=np.uint64)
+            ptrs = (ctypes.c_void_p * len(lens))(*[s.ctypes.data for s in smp])
+            szs = (ctypes.c_size_t * len(lens))(*lens)
+            rc = L.tg_count_batch(ctx.h, ctypes.byref(o), len(lens), ptrs, szs, ctypes.c_void_p(h_keys.ptr),
+                                  ctypes.c_void_p(h_cnt.ptr), ctypes.c_void_p(off.ctypes.data), n, ctypes.byref(n_out),
+                                  ctypes.byref(T._Stats()))
+            assert rc == 0, L.tg_last_error(ctx.h)
+            assert n_out.value == n and off[-1] == n
+            keys, cnt = h_keys.array(np.uint64).reshape(n, W), h_cnt.array(np.uint32)
+            for i in range(len(lens)):
+                a, b = int(off[i]), int(off[i + 1])
+                got = T.Result(keys[a:b].copy(), cnt[a:b].copy(), {}, k).sorted()
+                w = want.sample(i).sorted()
+                assert np.array_equal(got.keys, w.keys) and np.array_equal(got.counts, w.counts)

@@ -2017,23 +2017,26 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
         if (e == cudaSuccess) e = ctx->ensure(ctx->seq, total + 1);
         if (e == cudaSuccess) e = cudaEventRecord(ctx->ev[9], ctx->st);
         uint64_t off = 0;
-        if (n == 1 && lens[a] >= PIPE_MIN && !ctx->copy_pending && mapped_address(seqs[a]) && e == cudaSuccess) {
+        // a long stream in page-locked memory: phase 1 runs along with the copy (P1Pipe),
+        // copy(hi) of whose next piece, up to about hi, says what has arrived
+        uint64_t arrived = 0;
+        auto along = [&](uint64_t len) {
             j->used_ctx_seq = true;
-            pipe.begin(j, lens[a]);
-        }
-        if (pipe.begun) {
-            // one long stream: phase 1 runs along with the copy
-            const uint64_t len = lens[a], per = P1Pipe::piece_bytes(j, len);
-            j->st.input_bytes += len;
-            for (uint64_t lo = 0, q = 0; lo < len && e == cudaSuccess && s == TG_OK; lo += per, ++q) {
-                const uint64_t hi = std::min(len, lo + per);
-                e = link_copy(ctx->seq.as<uint8_t>() + lo, seqs[a] + lo, hi - lo, cudaMemcpyHostToDevice, ctx->st_copy, ctx->n_sm);
+            return len >= PIPE_MIN && !ctx->copy_pending && pipe.begin(j, len);
+        };
+        auto copy_along = [&](auto&& copy) {
+            const uint64_t len = pipe.most, per = P1Pipe::piece_bytes(j, len);
+            e = cudaEventRecord(ctx->ev[9], ctx->st);  // behind what the stream does before
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->st_copy, ctx->ev[9], 0);
+            for (uint64_t q = 0; arrived < len && e == cudaSuccess && s == TG_OK; ++q) {
+                e = copy((q + 1) * per);
                 if (e == cudaSuccess) e = cudaEventRecord(ctx->wave_ev[q], ctx->st_copy);
                 if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->st, ctx->wave_ev[q], 0);
-                if (e == cudaSuccess) s = pipe.piece(j, Avail{nullptr, nullptr, 0, hi, hi == len}, hi);
+                if (e == cudaSuccess) s = pipe.piece(j, Avail{nullptr, nullptr, 0, arrived, arrived == len}, arrived);
             }
             if (e != cudaSuccess || s != TG_OK) cudaStreamSynchronize(ctx->st_copy);
-        } else if (gather && e == cudaSuccess) {
+        };
+        if (gather && e == cudaSuccess) {
             std::vector<LinkPiece> ps;
             uint8_t* const d = ctx->seq.as<uint8_t>();
             uint64_t end = 0;  // of the sample before, past its separators
@@ -2057,9 +2060,28 @@ static tg_status count_run(tg_ctx* ctx, const tg_job_opts* opts, uint32_t a, uin
                 e = ctx->ensure(ctx->pieces, ps.size() * sizeof(LinkPiece));
                 if (e == cudaSuccess)
                     e = cudaMemcpyAsync(ctx->pieces.p, ps.data(), ps.size() * sizeof(LinkPiece), cudaMemcpyHostToDevice, ctx->st);
-                if (e == cudaSuccess)
-                    e = link_gather(ctx->pieces.as<LinkPiece>(), (uint32_t)ps.size(), ctx->st, ctx->n_sm);
             }
+            if (!ps.empty() && e == cudaSuccess && along(total)) {
+                auto at = [&](size_t i) { return (uint64_t)(ps[i].dst - d); };
+                size_t i = 0;
+                copy_along([&](uint64_t hi) -> cudaError_t {  // the pieces that begin before hi
+                    const size_t i0 = i;
+                    while (i < ps.size() && at(i) < hi) ++i;
+                    arrived = i < ps.size() ? at(i) : total;
+                    return link_gather(ctx->pieces.as<LinkPiece>() + i0, (uint32_t)(i - i0), ctx->st_copy, ctx->n_sm / 4);
+                });
+            } else if (!ps.empty() && e == cudaSuccess) {
+                e = link_gather(ctx->pieces.as<LinkPiece>(), (uint32_t)ps.size(), ctx->st, ctx->n_sm * 4);
+            }
+        } else if (n == 1 && e == cudaSuccess && mapped_address(seqs[a]) && along(lens[a])) {
+            const uint64_t len = lens[a];
+            j->st.input_bytes += len;
+            copy_along([&](uint64_t hi) -> cudaError_t {
+                const uint64_t lo = arrived;
+                arrived = std::min(hi, len);
+                return link_copy(ctx->seq.as<uint8_t>() + lo, seqs[a] + lo, arrived - lo, cudaMemcpyHostToDevice,
+                                 ctx->st_copy, ctx->n_sm);
+            });
         } else {
             if (e == cudaSuccess && n > 1) e = cudaMemsetAsync(ctx->seq.p, '\n', total, ctx->st);
             for (uint32_t i = a; i < b && e == cudaSuccess; ++i) {

@@ -80,8 +80,8 @@ struct LinkPiece {
     uint8_t* dst;
     uint32_t len, fill;
 };
-constexpr uint32_t LINK_PIECE = 128u << 10;  // bytes per piece, a multiple of 16
-cudaError_t link_gather(const LinkPiece* pieces, uint32_t n, cudaStream_t st, int n_sm, int* launches = nullptr);
+constexpr uint32_t LINK_PIECE = 32u << 10;  // bytes per piece, a multiple of 16; small: 38 CTAs share 13 MB evenly
+cudaError_t link_gather(const LinkPiece* pieces, uint32_t n, cudaStream_t st, int ctas, int* launches = nullptr);
 // The device address of host memory that is page-locked and mapped for the
 // current device, else null (pageable memory, device memory, bad pointers).
 const void* mapped_address(const void* host);

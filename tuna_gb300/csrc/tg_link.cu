@@ -73,9 +73,9 @@ __global__ void __launch_bounds__(LINK_THREADS, 8) k_link_gather(const LinkPiece
 
 }  // namespace
 
-cudaError_t link_gather(const LinkPiece* pieces, uint32_t n, cudaStream_t st, int n_sm, int* launches) {
+cudaError_t link_gather(const LinkPiece* pieces, uint32_t n, cudaStream_t st, int ctas, int* launches) {
     if (!n) return cudaSuccess;
-    k_link_gather<<<std::min<uint32_t>(n, (uint32_t)std::max(n_sm, 1) * 4), LINK_THREADS, 0, st>>>(pieces, n);
+    k_link_gather<<<std::min<uint32_t>(n, (uint32_t)std::max(ctas, 1)), LINK_THREADS, 0, st>>>(pieces, n);
     if (launches) ++*launches;
     return cudaGetLastError();
 }
