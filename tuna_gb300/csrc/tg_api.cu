@@ -1130,6 +1130,7 @@ static tg_status tg_job_run_impl(tg_job* j) {
     in.binhist = ctx->hist.as<unsigned long long>();
     in.n_kmers = n_kmers;
     in.n_recs = n_recs;
+    in.roomy = !ctx->hbm_budget;
     in.ci = j->o.ci;
     in.cx = j->o.cx;
     in.n_samples = ns;

@@ -220,6 +220,7 @@ struct KeysParams {
 };
 
 struct CountParams {
+    void* split;             // k_rounds: room for BIG_KEYS keys of each CTA, or null
     const void* recs;                  // packed records
     int k;
     const Group* list;

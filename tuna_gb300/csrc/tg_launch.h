@@ -135,6 +135,7 @@ struct P2Input {
     uint64_t n_kmers;                  // k-mer instances in all
     uint64_t n_recs;                   // packed records in all
     uint64_t ci, cx;
+    bool roomy = false;                // scratch for splitting large groups may be taken
     uint32_t n_samples = 1;
     // the bins counted by this run (all by default); segs must lie inside, and
     // n_kmers and n_recs count only theirs

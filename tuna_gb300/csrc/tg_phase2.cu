@@ -37,7 +37,12 @@ constexpr uint32_t MAX_PARTS = 128;      // key-hash parts of one range before t
 constexpr uint64_t FALLBACK_CAP = 4096;
 constexpr uint32_t BIG_KEYS = 1u << 16;  // k-mers above which many CTAs share a group (k_big)
 constexpr uint64_t WAVE_KEYS = 1u << 22; // k-mers of a wave of the first counting pass (P2Overlap)
-constexpr uint32_t BIG_CHUNK = 4096;     // packed records of such a group that a CTA takes at a time
+constexpr uint32_t MAX_SPLIT = 32;       // parts that split_group makes of a group
+constexpr uint64_t SPLIT_MIN = 1u << 20; // k-mers of a job that has room for that
+// Packed records of such a group that a CTA takes at a time (counting 155 Mbp of the
+// assembly, k=31 m=23: 1.61 ms against 1.92 with 4,096; 12.8 Mbp of reads, k=15 m=9:
+// 0.63 ms, 0.72 with 1,024).
+constexpr uint32_t BIG_CHUNK = 512;
 
 struct __align__(16) U128 {
     unsigned long long lo, hi;
@@ -422,6 +427,7 @@ struct CountSmem {
     Group grp[3];               // groups g, g + 1, g + 2
     unsigned long long pending;
     uint32_t staged;
+    uint32_t part_end[MAX_SPLIT];  // split_group: keys, cursors, then ends of the parts
     uint32_t dedup, firsts;     // groups until equal records are looked for again; first ones found
     static_assert(CAP <= IDX_MASK && CAP < SLOTS, "places and free slots");
 };
@@ -740,6 +746,60 @@ __global__ void __maxnreg__(56) k_count(const __grid_constant__ CountParams P) {
 }
 
 // ---------------------------------------------------------------- larger groups
+// Inserts the staged keys of places [n, m); those that another came before are holes.
+template <int W>
+__device__ __forceinline__ void insert_staged(CountSmem<W>& S, uint32_t n, uint32_t m, uint32_t& newm) {
+    using O = KeyOps<W>;
+    using Key = typename O::Key;
+    constexpr uint32_t SLOTS = CountSmem<W>::SLOTS;
+    const uint32_t tid = threadIdx.x;
+    for (uint32_t u = n / COUNT_THREADS; u * COUNT_THREADS < m; ++u) {
+        const uint32_t i = u * COUNT_THREADS + tid;
+        if (i < n || i >= m) continue;
+        const Key key = S.keys[i];
+        uint32_t h, en;
+        place_of<W>(slot_hash(key), i, h, en);
+        for (uint32_t p = 0; p < SLOTS; ++p) {
+            const uint32_t e = atomicCAS(&S.table[h], NO_ENTRY, en);
+            if (e == NO_ENTRY) { newm |= 1u << u; break; }
+            if (((e ^ en) >> IDX_BITS) == 0 && O::eq(S.keys[e & IDX_MASK], key)) {
+                // only this thread reads or clears the count of a place that is in no entry
+                atomicAdd(&S.cnt[e & IDX_MASK], S.cnt[i] + 1);
+                S.cnt[i] = 0;
+                break;
+            }
+            h = next_slot<W>(h, en);
+        }
+    }
+}
+
+// True, and the key's count up by weight, if the store holds the key.
+template <int W>
+__device__ __forceinline__ bool count_known(CountSmem<W>& S, const typename KeyOps<W>::Key& key, uint32_t weight) {
+    uint32_t h, en;
+    place_of<W>(slot_hash(key), 0, h, en);
+    for (uint32_t p = 0; p < CountSmem<W>::SLOTS; ++p) {
+        const uint32_t e = *(const volatile uint32_t*)&S.table[h];
+        if (e == NO_ENTRY) return false;
+        if (((e ^ en) >> IDX_BITS) == 0 && KeyOps<W>::eq(S.keys[e & IDX_MASK], key)) {
+            atomicAdd(&S.cnt[e & IDX_MASK], weight);
+            return true;
+        }
+        h = next_slot<W>(h, en);
+    }
+    return false;
+}
+
+// Every lane of the warp calls it: lanes with a get consecutive places from *at on.
+__device__ __forceinline__ uint32_t warp_place(uint32_t* at, bool a, unsigned peers) {
+    uint32_t base = 0;
+    const uint32_t lane = threadIdx.x & 31;
+    const int lead = __ffs(peers) - 1;
+    if (a && (int)lane == lead) base = atomicAdd(at, (uint32_t)__popc(peers));
+    base = __shfl_sync(0xffffffffu, base, lead < 0 ? 0 : lead);
+    return base + __popc(peers & ((1u << lane) - 1));
+}
+
 // The next records of a range in rounds. A round looks its keys up first: the
 // ones that the store holds are counted (equal records of a warp, a repeat's, as
 // one of their number), only the others are staged behind the store's keys and
@@ -753,9 +813,8 @@ __device__ __forceinline__ unsigned long long count_rounds(const CountParams& P,
                                                            unsigned long long lo, unsigned long long r,
                                                            unsigned long long nrec, uint32_t parts, uint32_t part,
                                                            uint32_t& n, uint32_t& newm) {
-    using O = KeyOps<W>;
-    using Key = typename O::Key;
-    constexpr uint32_t CAP = CountShape<W>::CAP, SLOTS = CountSmem<W>::SLOTS;
+    using Key = typename KeyOps<W>::Key;
+    constexpr uint32_t CAP = CountShape<W>::CAP;
     const uint32_t tid = threadIdx.x, lane = tid & 31;
     const int k = P.k;
     while (r < nrec && CAP - n >= CAP / 8) {
@@ -789,20 +848,7 @@ __device__ __forceinline__ unsigned long long count_rounds(const CountParams& P,
                     roll.step(k);
                     a = parts == 1 || key_part<W>(key, parts) == part;
                 }
-                if (a) {
-                    uint32_t h, en;
-                    place_of<W>(slot_hash(key), 0, h, en);
-                    for (uint32_t p = 0; p < SLOTS; ++p) {
-                        const uint32_t e = *(const volatile uint32_t*)&S.table[h];
-                        if (e == NO_ENTRY) break;
-                        if (((e ^ en) >> IDX_BITS) == 0 && O::eq(S.keys[e & IDX_MASK], key)) {
-                            atomicAdd(&S.cnt[e & IDX_MASK], weight);
-                            a = false;
-                            break;
-                        }
-                        h = next_slot<W>(h, en);
-                    }
-                }
+                if (a && count_known<W>(S, key, weight)) a = false;
                 const unsigned bal = __ballot_sync(0xffffffffu, a);
                 uint32_t base = 0;
                 if (lane == 0 && bal) base = atomicAdd(&S.staged, (uint32_t)__popc(bal));
@@ -815,24 +861,7 @@ __device__ __forceinline__ unsigned long long count_rounds(const CountParams& P,
         }
         __syncthreads();
         const uint32_t m = min(n + S.staged, CAP);
-        for (uint32_t u = n / COUNT_THREADS; u * COUNT_THREADS < m; ++u) {
-            const uint32_t i = u * COUNT_THREADS + tid;
-            if (i < n || i >= m) continue;
-            const Key key = S.keys[i];
-            uint32_t h, en;
-            place_of<W>(slot_hash(key), i, h, en);
-            for (uint32_t p = 0; p < SLOTS; ++p) {
-                const uint32_t e = atomicCAS(&S.table[h], NO_ENTRY, en);
-                if (e == NO_ENTRY) { newm |= 1u << u; break; }
-                if (((e ^ en) >> IDX_BITS) == 0 && O::eq(S.keys[e & IDX_MASK], key)) {
-                    // only this thread reads or clears the count of a place that is in no entry
-                    atomicAdd(&S.cnt[e & IDX_MASK], S.cnt[i] + 1);
-                    S.cnt[i] = 0;
-                    break;
-                }
-                h = next_slot<W>(h, en);
-            }
-        }
+        insert_staged<W>(S, n, m, newm);
         __syncthreads();  // the round is in the table; every thread has its size
         if (tid == 0) S.staged = 0;
         n = m;
@@ -842,11 +871,128 @@ __device__ __forceinline__ unsigned long long count_rounds(const CountParams& P,
     return r;
 }
 
+// A group of more distinct k-mers than a store holds, counted as F key-hash parts: its
+// k-mers are unpacked twice, to count each part's and to write them, part by part, to
+// this CTA's room in global memory (which stays in L2); then each part goes through the
+// store. A part that does not fit after all comes back through the retry list. (As F
+// passes over the records instead, each unpacking all and keeping its own part's:
+// 1.5 Gbp with k=27 m=15, whose hash has few values, took 264 ms to count against 40.)
+template <int W>
+__device__ __forceinline__ void split_group(const CountParams& P, CountSmem<W>& S, const Group& g, uint32_t F,
+                                            uint32_t& distinct) {
+    using Key = typename KeyOps<W>::Key;
+    constexpr uint32_t CAP = CountShape<W>::CAP;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    const int k = P.k;
+    Key* buf = static_cast<Key*>(P.split) + (size_t)blockIdx.x * BIG_KEYS;
+    const uint32_t nrec = (uint32_t)(g.hi - g.lo);
+    if (tid < MAX_SPLIT) S.part_end[tid] = 0;
+    __syncthreads();
+    for (int pass = 0; pass < 2; ++pass) {
+        for (uint32_t i0 = tid - lane; i0 < nrec; i0 += COUNT_THREADS) {
+            Rec<W> c;
+            uint32_t nk = 0;
+            if (i0 + lane < nrec) {
+                c = load_rec<W>(P.recs, g.lo + i0 + lane);
+                nk = c.n();
+            }
+            const uint32_t steps = __reduce_max_sync(0xffffffffu, nk);
+            Roll<W> roll;
+            if (nk) roll.start(c, k);
+            for (uint32_t t = 0; t < steps; ++t) {
+                const bool a = t < nk;
+                Key key;
+                uint32_t p = 0;
+                if (a) {
+                    key = roll.key(k);
+                    roll.step(k);
+                    p = key_part<W>(key, F);
+                }
+                // the warp's lanes of the same part
+                unsigned peers = __ballot_sync(0xffffffffu, a);
+                for (uint32_t b = 1; b < F; b <<= 1) {
+                    const unsigned s = __ballot_sync(0xffffffffu, p & b);
+                    peers &= p & b ? s : ~s;
+                }
+                if (pass == 0) {
+                    if (a && (int)lane == __ffs(peers) - 1) atomicAdd(&S.part_end[p], (uint32_t)__popc(peers));
+                } else {
+                    const uint32_t at = warp_place(&S.part_end[p], a, a ? peers : 0u);
+                    if (a && at < BIG_KEYS) buf[at] = key;
+                }
+            }
+        }
+        __syncthreads();
+        if (pass == 0 && tid < MAX_SPLIT) {  // the parts' first places, by a scan of one warp
+            const uint32_t v = S.part_end[tid];
+            uint32_t x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if ((int)tid >= o) x += y;
+            }
+            S.part_end[tid] = x - v;
+        }
+        __syncthreads();
+    }
+    for (uint32_t p = 0; p < F; ++p) {
+        const uint32_t end = min(S.part_end[p], BIG_KEYS);
+        uint32_t r = p ? S.part_end[p - 1] : 0, n = 0, newm = 0;
+        while (r < end && CAP - n >= CAP / 8) {
+            // all of the part if its k-mers fit; else few at first, since all of those take places
+            const uint32_t take = min(n ? CAP - n : (end - r <= CAP ? CAP : 512u), end - r);
+            uint32_t m = take;
+            if (n == 0) {  // the store is empty
+                for (uint32_t i = tid; i < take; i += COUNT_THREADS) S.keys[i] = buf[r + i];
+                __syncthreads();
+            } else {
+                for (uint32_t i0 = tid - lane; i0 < take; i0 += COUNT_THREADS) {
+                    bool a = i0 + lane < take;
+                    Key key;
+                    if (a) {
+                        key = buf[r + i0 + lane];
+                        a = !count_known<W>(S, key, 1);
+                    }
+                    const unsigned bal = __ballot_sync(0xffffffffu, a);
+                    const uint32_t at = n + warp_place(&S.staged, a, bal);
+                    if (a && at < CAP) S.keys[at] = key;
+                }
+                __syncthreads();
+                m = min(n + S.staged, CAP);
+            }
+            insert_staged<W>(S, n, m, newm);
+            __syncthreads();
+            if (tid == 0) S.staged = 0;
+            n = m;
+            r += take;
+            __syncthreads();
+        }
+        if (r < end) {
+            if (tid == 0) {
+                Group f = g;
+                f.parts = 2 * F;
+                const unsigned long long i = atomicAdd(P.n_retry, 2ull);
+                if (i + 1 < P.retry_cap)
+                    for (uint32_t q = 0; q < 2; ++q) {
+                        f.part = p + q * F;
+                        P.retry[i + q] = f;
+                    }
+            }
+            for (uint32_t i = tid; i < n; i += COUNT_THREADS) S.cnt[i] = 0;
+            clear_table<W>(S);
+        } else if (n) {
+            write_out<W>(P, S, n, newm, g.sample, distinct, [] {});
+        }
+        __syncthreads();
+    }
+}
+
 // Groups of more than CAP and at most BIG_KEYS k-mers (one bin each), and key-hash parts
-// of such groups, one CTA each. A group whose distinct keys do not fit comes back as F
-// key-hash parts, F the power of two that gives half-full stores for the places
-// estimated from the share of the group seen; past MAX_PARTS parts it goes to the
-// global-memory table.
+// of such groups, one CTA each. A group whose distinct keys do not fit is split
+// (split_group) or, without room for that (a job below SPLIT_MIN, one with a memory
+// budget), comes back as F key-hash parts, F the power of two that gives half-full
+// stores for the places estimated from the share of the group seen; past MAX_PARTS
+// parts it goes to the global-memory table.
 template <int W>
 __global__ void __launch_bounds__(COUNT_THREADS, COUNT_PER_SM) k_rounds(const __grid_constant__ CountParams P) {
     constexpr uint32_t CAP = CountShape<W>::CAP;
@@ -857,13 +1003,33 @@ __global__ void __launch_bounds__(COUNT_THREADS, COUNT_PER_SM) k_rounds(const __
     const unsigned long long g_end = list_end(P);
     if (P.g_begin + blockIdx.x >= g_end) return;
     start_store<W>(S);
-    __syncthreads();
-    for (unsigned long long gi = P.g_begin + blockIdx.x; gi < g_end; gi += gridDim.x) {
+    // groups differ in size by more than ten: taken from a counter, the first of each CTA aside
+    for (unsigned long long gi = P.g_begin + blockIdx.x; gi < g_end; gi = S.pending) {
+        __syncthreads();
+        if (tid == 0) S.pending = P.g_begin + gridDim.x + atomicAdd(P.work, 1ull);
         const Group g = P.list[gi];
         const unsigned long long nrec = g.hi - g.lo;
         uint32_t n = 0, newm = 0;
-        const unsigned long long r = count_rounds<W>(P, S, g.lo, 0, nrec, g.parts, g.part, n, newm);
-        if (r < nrec) {  // too many distinct keys
+        // a group that may be split: its first eighth tells whether that is needed
+        const bool may = P.split && g.parts == 1 && g.keys > CAP && g.keys <= BIG_KEYS;
+        const unsigned long long probe = may ? nrec / 8 + 1 : nrec;
+        unsigned long long r = 0, to = probe;
+        uint64_t est = 0;
+        for (;;) {
+            r = count_rounds<W>(P, S, g.lo, r, to, g.parts, g.part, n, newm);
+            est = (uint64_t)n * nrec / r;
+            if (r < to || to == nrec || est > CAP) break;
+            to = nrec;
+        }
+        if (r < nrec && may) {  // too many distinct keys
+            for (uint32_t i = tid; i < n; i += COUNT_THREADS) S.cnt[i] = 0;
+            clear_table<W>(S);
+            uint32_t F = 2;
+            while (F < MAX_SPLIT && (uint64_t)F * (CAP / 4 * 3) < est) F <<= 1;
+            split_group<W>(P, S, g, F, distinct);  // ends with a barrier
+            continue;
+        }
+        if (r < nrec) {
             if (tid == 0) {
                 Group f = g;
                 if (g.parts < MAX_PARTS) {
@@ -1118,7 +1284,7 @@ P2Plan make_plan(const P2Input& in) {
 struct P2Regions {
     unsigned long long* ctr;
     unsigned long long* aux;  // [0..1] retry counters
-    unsigned long long* work; // [0..15] group counters of k_count's launches
+    unsigned long long* work; // [0..15] group counters of k_count's launches, [16] k_rounds'
     unsigned long long* kofs;
     unsigned long long* rofs;
     uint32_t* gfirst;
@@ -1132,13 +1298,20 @@ struct P2Regions {
     unsigned long long* scur;  // [n_samples] cursors of the sample-major copy
     uint32_t* stot;            // [n_samples] pairs of each sample
     uint8_t* recs;
+    uint8_t* split;            // [k_rounds' CTAs][BIG_KEYS] keys, or null
 };
+
+// CTAs of k_rounds with room for splitting: as many as there can be groups for.
+uint64_t split_ctas(const P2Input& in) {
+    if (!in.roomy || in.n_kmers < SPLIT_MIN) return 0;
+    return std::min<uint64_t>((uint64_t)in.n_sm * COUNT_PER_SM, in.n_kmers / CountShape<2>::CAP + 1);
+}
 
 P2Regions carve(Carve& c, const P2Input& in, const P2Plan& L) {
     P2Regions R;
     R.ctr = c.take<unsigned long long>(P2C_COUNT);
     R.aux = c.take<unsigned long long>(2);
-    R.work = c.take<unsigned long long>(16);
+    R.work = c.take<unsigned long long>(17);
     R.kofs = c.take<unsigned long long>((size_t)in.all_bins + 1);
     R.rofs = c.take<unsigned long long>((size_t)in.all_bins + 1);
     R.gfirst = c.take<uint32_t>(in.all_bins);
@@ -1153,6 +1326,8 @@ P2Regions carve(Carve& c, const P2Input& in, const P2Plan& L) {
     R.scur = c.take<unsigned long long>(in.n_samples + 1);
     R.stot = c.take<uint32_t>(in.n_samples + 1);
     R.recs = c.take<uint8_t>((in.n_recs + 1) * 16 * (size_t)in.W);
+    const uint64_t sc = split_ctas(in);
+    R.split = sc ? c.take<uint8_t>(sc * BIG_KEYS * key_bytes(in.W)) : nullptr;
     return R;
 }
 }  // namespace
@@ -1397,10 +1572,12 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
         Q.list = list;
         Q.g_begin = 0;
         Q.g_end = n;
-        const unsigned grid = (unsigned)std::min<unsigned long long>(n, cgrid);
+        const unsigned grid = (unsigned)std::min<unsigned long long>(n, R.split ? split_ctas(in) : cgrid);
         if (!grid) return cudaSuccess;
         cudaError_t e = W == 1 ? set_smem_cap(k_rounds<1>, sm) : set_smem_cap(k_rounds<2>, sm);
+        if (e == cudaSuccess) e = cudaMemsetAsync(R.work + 16, 0, 8, st);
         if (e != cudaSuccess) return e;
+        Q.work = R.work + 16;
         if (W == 1) k_rounds<1><<<grid, COUNT_THREADS, sm, st>>>(Q);
         else k_rounds<2><<<grid, COUNT_THREADS, sm, st>>>(Q);
         ++*launches;
@@ -1443,6 +1620,7 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
         if (failed) { err = "fallback table overflow"; return TG_ERR_TABLE; }
         return TG_OK;
     };
+    Q.split = R.split;
     Q.retry = R.retry[0];
     Q.n_retry = R.aux;
     // ---- the largest groups, one table for those of a sample (of few MB for a group of a
