@@ -91,10 +91,10 @@ typedef struct {
 } tg_ctx_opts;
 
 /* tg_ctx_opts.flags: the first job of each key width (k <= 31, k >= 32) with at
- * least 2^26 k-mers times its counting pass with several group sizes (the load
- * of the shared-memory table when a group's keys are all distinct) on its own
- * keys and keeps the fastest for itself and every later job of the context
- * (tg_stats.group_load_pct). Without it the group size is half the table. */
+ * least 2^26 k-mers times its counting pass with several group sizes (k-mers per
+ * group, at most the shared-memory store's 4,096 or, for k >= 32, 3,072) on its own
+ * records and keeps the fastest for itself and every later job of the context
+ * (tg_stats.group_load_pct). Without it a group is as large as the store. */
 #define TG_CTX_AUTOTUNE 1u
 
 typedef struct {
@@ -120,8 +120,8 @@ typedef struct {
     uint32_t heavy_groups;    /* phase-2 groups larger than one table's target */
     uint64_t fallback_groups; /* key ranges counted in a global-memory table */
     double h2d_ms;            /* host->device copy time of the input */
-    double pack_ms;           /* device time: 2-bit packing */
-    double phase1_ms;         /* device time: minimizers, superkmers, bin histogram */
+    double pack_ms;           /* device time: 2-bit packing (its part past the copy, where it runs along with that) */
+    double phase1_ms;         /* device time: minimizers, superkmers, bin histogram (likewise) */
     double phase2_ms;         /* device time: counting, filter, compaction */
     double d2h_ms;            /* device->host time of results (copy / drain) */
     double phase1_cut_ms;     /* part of phase1_ms: the superkmer cut kernel */
@@ -136,7 +136,7 @@ typedef struct {
     uint64_t host_parsed_bytes; /* of those, bytes parsed on the host (see tg_job_feed_fastx) */
     uint64_t phase2_passes;   /* phase-2 passes over ranges of bins (more than 1 when the keys and
                                  pairs of a job exceed the context's memory budget, hbm_budget_bytes) */
-    uint32_t group_load_pct;  /* keys per counting group, % of the shared-memory table's slots */
+    uint32_t group_load_pct;  /* keys per counting group, % of 8,192 (at most the store's) */
     uint32_t autotune_trials; /* counting passes this job timed for TG_CTX_AUTOTUNE */
 } tg_stats;
 

@@ -2215,9 +2215,8 @@ static void add_run_stats(tg_stats& t, const tg_stats& r) {
 // bytes (a job of several samples is not counted in passes, so each run must
 // fit; a sample is never split), each run's result copy left running while the
 // next run counts. Cutting batches that fit into runs as well, only to overlap
-// the copies, was measured slower: the copy kernels cannot sit beside the cut
-// and key kernels on an SM (registers), so little overlapped, and smaller jobs
-// cost more (2,000 samples, 1.23 Gbp: 40 -> 73 ms in four runs).
+// the copies, gains little: 400 samples of 250 Mbp took 7.26 ms in one run, 6.93 in
+// two and 7.45 in three, and 6.75 in one since phase 1 runs along with the copy in.
 constexpr uint64_t BATCH_BYTES_PER_BASE = 40;  // keys, pairs and their sample-major copy, records, stream
 
 // The one-call entry points.

@@ -20,10 +20,11 @@
 //   k_count     persistent: each group's records are read with coalesced loads
 //               and unpacked into canonical keys in shared memory, counted in an
 //               open-addressing table there, then filtered and compacted.
-//               A group with more distinct keys than the table holds comes back
-//               as key-hash parts in the next launch (as many as its distinct
-//               keys need, estimated); past MAX_PARTS parts it goes to the
-//               global-memory table (k_fb_*).
+//   k_rounds    larger groups (one bin), a CTA each: in rounds when their distinct
+//               keys fit in the store, else as key-hash parts written to global
+//               memory first or, without room for that, read again in the next
+//               launch; past MAX_PARTS parts they go to the global table (k_fb_*)
+//   k_big       the largest, each shared by many CTAs, into one global table
 #include <algorithm>
 #include <vector>
 
@@ -43,6 +44,10 @@ constexpr uint64_t SPLIT_MIN = 1u << 20; // k-mers of a job that has room for th
 // assembly, k=31 m=23: 1.61 ms against 1.92 with 4,096; 12.8 Mbp of reads, k=15 m=9:
 // 0.63 ms, 0.72 with 1,024).
 constexpr uint32_t BIG_CHUNK = 512;
+// k-mers of such groups that share a table: larger tables leave L2 (100 Mbp, k=21 m=9,
+// nearly all of whose k-mers are in such groups: 10.5 ms of counting, 11.8 with one table).
+constexpr uint64_t BIG_TABLE_KEYS = 1u << 23;
+
 
 struct __align__(16) U128 {
     unsigned long long lo, hi;
@@ -1125,45 +1130,63 @@ __global__ void k_fb_init(void* keys, uint32_t* cnt, uint64_t S) {
     }
 }
 
-// Write the occupied slots that pass ci/cx (warp-aggregated output atomics).
+// Write the occupied slots that pass ci/cx. A warp takes EXTRACT slots of each lane at a
+// time, with one output atomic for them: with one per 32 slots the counter was what
+// bound it (2^28 slots: 6.4 ms, 2.2 now).
+constexpr int EXTRACT = 8;
 template <int W>
 __global__ void __launch_bounds__(256) k_fb_extract(const void* keys, const uint32_t* cnt, uint64_t S,
                                                     CountParams P, uint32_t sample) {
-    using O = KeyOps<W>;
-    const auto* kk = reinterpret_cast<const typename O::Key*>(keys);
-    const int lane = threadIdx.x & 31;
+    using Key = typename KeyOps<W>::Key;
+    const Key* kk = static_cast<const Key*>(keys);
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
+    const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     unsigned long long distinct = 0;
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < S; i0 += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t i = i0 + threadIdx.x;
-        bool occ = false, keep = false;
-        typename O::Key key;
-        uint32_t c = 0;
-        if (i < S) {
-            key = kk[i];
-            occ = !O::is_empty(key);
-            if (occ) {
-                c = cnt[i];
-                keep = (uint64_t)c >= P.ci && (uint64_t)c <= P.cx;
+    for (uint64_t s0 = warp * (32 * EXTRACT); s0 < S; s0 += warps * (32 * EXTRACT)) {  // S: a multiple of 256
+        Key key[EXTRACT];
+        uint32_t c[EXTRACT], kept = 0, mine = 0;
+#pragma unroll
+        for (int u = 0; u < EXTRACT; ++u) {
+            key[u] = kk[s0 + u * 32 + lane];
+            c[u] = cnt[s0 + u * 32 + lane];
+        }
+#pragma unroll
+        for (int u = 0; u < EXTRACT; ++u) {
+            const bool has = !KeyOps<W>::is_empty(key[u]);
+            distinct += has;
+            if (has && c[u] >= P.ci && c[u] <= P.cx) {
+                kept |= 1u << u;
+                ++mine;
             }
         }
-        distinct += occ ? 1 : 0;
-        const unsigned bal = __ballot_sync(0xffffffffu, keep);
-        if (!bal) continue;
+        uint32_t at = mine;  // exclusive scan over the lanes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, at, o);
+            if ((int)lane >= o) at += y;
+        }
+        const uint32_t all = __shfl_sync(0xffffffffu, at, 31);
+        if (!all) continue;
+        at -= mine;
         unsigned long long base = 0;
         if (lane == 0) {
-            base = atomicAdd(&P.ctr[P2C_OUT], (unsigned long long)__popc(bal));
-            if (P.sample_tot) atomicAdd(&P.sample_tot[sample], (uint32_t)__popc(bal));
+            base = atomicAdd(&P.ctr[P2C_OUT], (unsigned long long)all);
+            if (P.sample_tot) atomicAdd(&P.sample_tot[sample], all);
         }
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (keep) {
-            const uint64_t o = base + __popc(bal & ((1u << lane) - 1));
-            if (o < P.out_cap) {
-                O::store(P.out_keys, o, key);
-                P.out_counts[o] = c;
-                if (P.out_sample) P.out_sample[o] = sample;
+        base = __shfl_sync(0xffffffffu, base, 0) + at;
+#pragma unroll
+        for (int u = 0; u < EXTRACT; ++u)
+            if ((kept >> u) & 1u) {
+                if (base < P.out_cap) {
+                    KeyOps<W>::store(P.out_keys, base, key[u]);
+                    P.out_counts[base] = c[u];
+                    if (P.out_sample) P.out_sample[base] = sample;
+                }
+                ++base;
             }
-        }
     }
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) distinct += __shfl_down_sync(0xffffffffu, distinct, o);
     if (lane == 0 && distinct) atomicAdd(&P.ctr[P2C_DISTINCT], distinct);
 }
@@ -1623,7 +1646,7 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     Q.split = R.split;
     Q.retry = R.retry[0];
     Q.n_retry = R.aux;
-    // ---- the largest groups, one table for those of a sample (of few MB for a group of a
+    // ---- the largest groups, some of a sample to a table (of few MB for a group of a
     // million k-mers; without room for it, they are counted like the other large ones)
     uint64_t n_big = 0;
     auto count_big = [&]() -> tg_status {
@@ -1637,7 +1660,8 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
         for (size_t a = 0; a < big.size();) {
             size_t b = a;
             uint64_t nk = 0, most = 0;
-            while (b < big.size() && big[b].sample == big[a].sample && b - a < 32768) {
+            while (b < big.size() && big[b].sample == big[a].sample && b - a < 32768 &&
+                   (b == a || nk + big[b].keys <= BIG_TABLE_KEYS)) {
                 nk += big[b].keys;
                 most = std::max<uint64_t>(most, big[b].hi - big[b].lo);
                 ++b;
