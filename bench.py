@@ -8,7 +8,7 @@ divergence, 3% microsatellites — the largest single-GPU workload of the
 benchmark set. Inputs (3.1 GB) are larger than L2, so no flush is needed.
 
   value   Gbases/s with the input already resident in HBM: k_pack -> k_cut_fixed/k_cut_seq
-          -> k_scan -> k_plan -> k_keys -> k_count, results left on the device
+          -> k_scan -> k_plan -> k_recs -> k_count, results left on the device
           (stats also give distinct k-mers/s and k-mer updates/s)
   e2e     the same through the public C ABI from the FASTA file's bytes
           (tg_count_fastx) with pinned host buffers: H2D of the FASTA, lexing
@@ -855,14 +855,14 @@ def main():
     rec_bases = st["kmers"] + recs * (K - 1)
     alg = {
         "cut": n_stream / 4 + n_stream / 8 + 8 * recs,            # packed + validity in, descriptors out
-        "keys": 8 * recs + rec_bases / 4 + 8 * st["kmers"],       # descriptors + record bases in, keys out
-        "count": 8 * st["kmers"] + st["out"] * 12,                # keys in, (key, count) out
+        "keys": 8 * recs + rec_bases / 4 + 16 * recs,             # descriptors + record bases in, packed records out
+        "count": 16 * recs + st["out"] * 12,                      # packed records in, (key, count) out
         "pack": n_stream + n_stream / 4 + n_stream / 8,           # ASCII in, packed + validity out
     }
     dom = max(("cut", "keys", "count", "pack"), key=lambda x: avg[x])
     achieved = alg[dom] / (avg[dom] / 1e3) / 1e9
     cut_name = "k_cut_fixed" if (K, M) in ((31, 21), (31, 23), (21, 17), (25, 21)) else "k_cut_seq"
-    kernel_names = {"cut": cut_name, "keys": "k_scan+k_plan+k_keys", "count": "k_count", "pack": "k_pack"}
+    kernel_names = {"cut": cut_name, "keys": "k_scan+k_plan+k_recs", "count": "k_count", "pack": "k_pack"}
     # phase 1 against the reference's algorithmic bytes B1 = N/4 + record bytes (~1.82 B/base)
     ref_record_bytes = 2 * recs + (st["kmers"] + recs * (K - 1)) / 4
     b1 = bases / 4 + ref_record_bytes
