@@ -888,8 +888,10 @@ k_cut_seq(CutParams P, const HashTables* __restrict__ gT) {
 //    a run-AND of k validity bits, a chain starts at a valid k-mer that is the
 //    first of its run or whose minimizer changed, a run ends at the first
 //    invalid k-mer after a valid one;
-//  * records that close inside the batch get their slots from one warp scan and
-//    one shared atomic per warp and batch.
+//  * records that close inside the batch get their slots from one shared atomic per
+//    warp and batch and a ballot per step, so that a step's records of all lanes are
+//    written next to each other (3.1 Gbp: 16.0 -> 9.9 ms; each lane's own run of
+//    slots, from a warp scan, made every store a sector of its own).
 // The bases that leave and enter the m-mer during a batch come from two 64-bit
 // windows of the staged packed words, read once per batch and shifted by one
 // base per roll. The ntHash roll terms CTF/CTR are interleaved (one 16-byte
