@@ -1,0 +1,47 @@
+// host_bounds_check.cu — bounds that the host code relies on where a run's buffers
+// are sized before its counts are known, checked without a GPU.
+#include <algorithm>
+#include <cstdio>
+
+#include "tg_launch.h"
+
+using namespace tg;
+
+static int fails = 0;
+#define CHECK(cond, ...)                                           \
+    do {                                                           \
+        if (!(cond)) {                                             \
+            if (++fails <= 20) {                                   \
+                std::printf("FAIL line %d: ", __LINE__);           \
+                std::printf(__VA_ARGS__);                          \
+                std::printf("\n");                                 \
+            }                                                      \
+        }                                                          \
+    } while (0)
+
+// Records of the first list when every position of its chunk starts one and the last
+// of them is a chain to the stream's end, split every L positions.
+static void check_cut_lists() {
+    for (int k = 2; k <= 63; ++k)
+        for (int m = 1; m < k && m <= 32; ++m)
+            for (uint64_t n : {1ull, 1000ull, 524288ull, 3000000ull, 4194304ull, 4600000ull, 3100000000ull}) {
+                const uint32_t L = 256 - (uint32_t)k;
+                const uint64_t chunk = cut_layout(k - m, k, 1, false, n, 152).chunk;
+                const uint64_t in_chunk = std::min(chunk, n), behind = n - in_chunk;
+                const uint64_t most = cut_list_most(chunk, n, L);
+                CHECK(most >= in_chunk + (behind + L - 1) / L, "k=%d m=%d n=%llu: a list of %llu", k, m,
+                      (unsigned long long)n, (unsigned long long)most);
+                CHECK(most <= chunk + n / L + 64, "k=%d m=%d n=%llu: a list of %llu", k, m, (unsigned long long)n,
+                      (unsigned long long)most);
+            }
+}
+
+int main() {
+    check_cut_lists();
+    if (fails) {
+        std::printf("%d checks failed\n", fails);
+        return 1;
+    }
+    std::printf("OK\n");
+    return 0;
+}

@@ -697,7 +697,8 @@ static CutParams cut_params(tg_job* j, int seg, const CutSamples& cs) {
 }
 
 // deferred: the cut is launched and not waited for; its descriptor lists have
-// room for a record at every position.
+// room for all records that there can be (cut_list_most). Else they have room for the
+// usual number and, if that does not do, for as many as the cut found.
 static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, const CutSamples& cs = CutSamples(),
                          P1Counts* counts = nullptr, bool deferred = false) {
     tg_ctx* ctx = j->ctx;
@@ -713,9 +714,9 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
     j->chunk = chunk;
     j->p1_bits = p1_bits;
     // descriptors: about 2/(w+2) records per k-mer for random minimizers; grow on overflow
-    double factor = deferred ? 1.0 : std::min(1.0, 3.0 / (j->w + 2));
+    uint64_t cap = deferred ? cut_list_most(chunk, n, j->L)
+                            : (uint64_t)(lay.tiles * tile * std::min(1.0, 3.0 / (j->w + 2))) + 2ull * tile + j->L + 64;
     for (int attempt = 0; attempt < 2; ++attempt) {
-        const uint64_t cap = (uint64_t)(lay.tiles * tile * factor) + 2ull * tile + j->L + 64;
         j->desc_cap = cap;
         CK(ctx->ensure(ctx->desc, (size_t)C * cap * 8), "alloc descriptors");
         if (exp) CK(ctx->ensure(ctx->xdesc, (size_t)C * cap * 24), "alloc export descriptors");
@@ -748,7 +749,7 @@ static tg_status run_cut(tg_job* j, bool exp, uint32_t p1_bits, int* launches, c
         if (s != TG_OK) return s;
         if (counts) *counts = r;
         if (!r.overflow) return TG_OK;
-        factor = 1.0;  // every k-mer start can open a record at most once
+        cap = r.max_desc;
     }
     return ctx->fail(TG_ERR_DEVICE, "descriptor capacity exceeded");
 }
@@ -1234,7 +1235,10 @@ static tg_status tg_job_run_impl(tg_job* j) {
         const tg_status ps = phase2_run(in, ctx->scratch.p, p2_bytes, out, fallback_table, ctx->st, ctx->ev[7],
                                         &launches, msg, j->overlap ? *j->overlap : P2Overlap());
         if (ps != TG_OK) return ctx->fail(ps, msg);
-        if (deferred) r1.c = P1Counts(out.read_back);
+        if (deferred) {
+            r1.c = P1Counts(out.read_back);
+            if (r1.c.overflow) return ctx->fail(TG_ERR_DEVICE, "descriptor capacity exceeded");
+        }
         CK(cudaEventRecord(ctx->ev[8], ctx->st), "event");
         CK(cudaEventSynchronize(ctx->ev[8]), "sync");
         j->n_out = out.n_out;

@@ -132,7 +132,7 @@ struct CutParams {
     uint64_t* desc;          // [n_cta][desc_cap] record descriptors
     uint64_t desc_cap;
     uint32_t* n_desc;        // [n_cta]
-    uint32_t* max_desc;      // counting cut: the most of them
+    uint32_t* max_desc;      // the most of them, those past desc_cap too
     uint32_t* hist;          // export cut: u32 [P][n_cta] records, then u64 [P] k-mers per bucket
     unsigned long long* binhist;  // counting cut: [bins] k-mers + 2^32 x packed records per bin
     int desc_sb;             // counting cut: start bits of a descriptor (desc_start_bits)

@@ -21,6 +21,10 @@ size_t cut_smem_bytes(int w, int k, uint32_t p1, bool exp, int seg = 128);
 uint64_t cut_tile(int w, bool exp, int seg = 128);  // k-mer start positions per tile of a cut CTA
 uint32_t cut_ctas_per_sm(int w, int k, uint32_t p1, bool exp, int seg = 128);
 CutLayout cut_layout(int w, int k, uint32_t p1, bool exp, uint64_t n, uint32_t n_sm);
+// The most records that one list of a cut of n positions can get (L: CutParams::L): one
+// per position of its chunk, and the forced splits, L positions apart, of the chain
+// that is open at the chunk's end, wherever that ends (a homopolymer's: the whole stream).
+uint64_t cut_list_most(uint64_t chunk, uint64_t n, uint32_t L);
 cudaError_t launch_prepare(const PrepareParams& P, cudaStream_t st);
 // Packed words (a multiple of 4) for a stream of n bytes, padding included.
 uint64_t packed_words_for(uint64_t n);

@@ -155,7 +155,7 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     const uint64_t pw = packed_words_for(n);
     uint32_t* packed = cv.take<uint32_t>(pw);
     uint32_t* valid = cv.take<uint32_t>(pw / 2 + 16);
-    // phase-1 layout: as tg_job_run, with room for one record per k-mer start
+    // phase-1 layout: as tg_job_run of a short stream, with room for all records there can be
     uint32_t p1 = o.gpu_parts ? o.gpu_parts : std::min<uint32_t>(1024, std::max<uint32_t>(16, (uint32_t)(n / 32768)));
     uint32_t p1_bits = 0;
     while ((1u << p1_bits) < p1) ++p1_bits;
@@ -163,7 +163,7 @@ static tg_status count_noalloc(const tg_job_opts* opts, const uint8_t* d_seq, si
     const CutLayout lay = cut_layout(w, k, p1, false, n, (uint32_t)n_sm);
     const uint32_t C = lay.n_cta;
     const uint64_t chunk = lay.chunk;
-    const uint64_t desc_cap = lay.tiles * lay.tile + 2ull * lay.tile + L + 64;
+    const uint64_t desc_cap = cut_list_most(chunk, n, L);
     uint64_t* desc = cv.take<uint64_t>((size_t)C * desc_cap);
     uint32_t* n_desc = cv.take<uint32_t>(C);
     const int bin_bits = job_bin_bits(n, 1, p1_bits);

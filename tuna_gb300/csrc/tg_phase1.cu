@@ -477,7 +477,10 @@ k_cut(CutParams P, const HashTables* __restrict__ gT) {
         if (s_hk[i]) atomicAdd(reinterpret_cast<unsigned long long*>(P.hist + hist_kmers_offset(p1, P.n_cta)) + i,
                                (unsigned long long)s_hk[i]);
     }
-    if (tid == 0) P.n_desc[c] = s_ndesc;
+    if (tid == 0) {
+        P.n_desc[c] = s_ndesc;
+        atomicMax(P.max_desc, s_ndesc);
+    }
     if (overflowed) atomicExch(P.overflow, 1u);
     // block-reduce the counters
     for (int o = 16; o > 0; o >>= 1) {
@@ -1481,6 +1484,8 @@ CutLayout cut_layout(int w, int k, uint32_t p1, bool exp, uint64_t n, uint32_t n
     }
     return best;
 }
+
+uint64_t cut_list_most(uint64_t chunk, uint64_t n, uint32_t L) { return chunk + n / L + 2; }
 
 cudaError_t launch_prepare(const PrepareParams& P, cudaStream_t st) {
     const uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>(P.n_bins / 2 / 256, 1024));
