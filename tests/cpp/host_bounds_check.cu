@@ -36,8 +36,24 @@ static void check_cut_lists() {
             }
 }
 
+// A global table's slots against its k-mers, and the probes that a mask of 32 bits allows.
+static void check_tables() {
+    for (int k : {16, 31, 32, 63})
+        for (uint64_t n : {0ull, 1ull, 511ull, 65537ull, (1ull << 30) - 1, 1ull << 30, (1ull << 31) - 1}) {
+            const uint64_t S = table_slots(n, k);
+            CHECK(S >= 2 * n + 1 && S <= 1ull << 32 && (S & (S - 1)) == 0, "%llu slots for %llu k-mers",
+                  (unsigned long long)S, (unsigned long long)n);
+            CHECK((uint32_t)(S - 1) > n, "%u probes among %llu k-mers", (uint32_t)(S - 1), (unsigned long long)n);
+        }
+    for (uint64_t n : {1ull << 31, 1ull << 32, 1ull << 40}) CHECK(table_slots(n, 31) == 0, "no table");
+    // few k-mers differ, however many there are
+    CHECK(table_slots(1ull << 40, 9) >= 2ull << 18 && table_slots(1ull << 40, 9) <= 4ull << 18, "4^9 k-mers");
+    CHECK(table_slots(1ull << 40, 2) == 1024 && table_slots(100, 9) == 1024, "small tables");
+}
+
 int main() {
     check_cut_lists();
+    check_tables();
     if (fails) {
         std::printf("%d checks failed\n", fails);
         return 1;

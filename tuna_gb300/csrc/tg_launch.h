@@ -105,6 +105,9 @@ cudaError_t launch_spill_write(const uint32_t* packed, const uint64_t* desc, uin
 cudaError_t launch_rebase(uint64_t* desc, uint64_t n, uint64_t add, int n_sm, cudaStream_t st);
 size_t key_bytes(int W);
 uint32_t count_slots(int W);
+// Slots of a table in global memory for n k-mers of length k, of which at most 4^k
+// differ: a power of two, more than half of them free. 0: more than 2^32.
+uint64_t table_slots(uint64_t n, int k);
 
 // Phase 2 of one job, shared by the entry points: the phase-1 descriptor lists
 // and the k-mer counts per bin in, distinct keys and counts (and their

@@ -95,7 +95,9 @@ __device__ __forceinline__ uint32_t key_part(const typename KeyOps<W>::Key& key,
     return (uint32_t)(KeyOps<W>::hash(key) >> 8) & (parts - 1);
 }
 
-// Insert n instances of one k-mer: count += n. False if `limit` slots were taken.
+// Insert n instances of one k-mer: count += n. False if `limit` slots were taken. (A
+// table of global memory takes its mask for that, one less than its slots, 2^32 of which
+// have no number of 32 bits; more than half of them are free.)
 // 64-bit keys are probed with a plain load and claimed with a CAS. A 128-bit
 // key cannot be read in one single-copy-atomic load, and a read torn against a
 // concurrent claim could skip the slot that holds the same k-mer, so 128-bit
@@ -1089,7 +1091,7 @@ __global__ void __launch_bounds__(COUNT_THREADS, COUNT_PER_SM)
             for (uint32_t u = 0; u * COUNT_THREADS < n; ++u) {
                 const uint32_t i = u * COUNT_THREADS + tid;
                 if ((newm >> u) & 1u)
-                    if (!tbl_add<W>(static_cast<Key*>(F.tkeys), F.tcnt, F.mask, S.keys[i], S.cnt[i] + 1, F.mask + 1))
+                    if (!tbl_add<W>(static_cast<Key*>(F.tkeys), F.tcnt, F.mask, S.keys[i], S.cnt[i] + 1, F.mask))
                         atomicExch(F.fail, 1u);
                 if (i < n) S.cnt[i] = 0;
             }
@@ -1115,7 +1117,7 @@ __global__ void k_fb_insert(FallbackParams F) {
         for (uint32_t t = 0; t < n; ++t, roll.step(F.k)) {
             const typename O::Key key = roll.key(F.k);
             if (key_part<W>(key, F.parts) != F.part) continue;
-            if (!tbl_add<W>(tk, F.tcnt, F.mask, key, 1, F.mask + 1)) atomicExch(F.fail, 1u);
+            if (!tbl_add<W>(tk, F.tcnt, F.mask, key, 1, F.mask)) atomicExch(F.fail, 1u);
         }
     }
 }
@@ -1249,6 +1251,14 @@ __global__ void __launch_bounds__(256) k_samp_scatter(const void* __restrict__ k
 
 // ---------------------------------------------------------------- host side
 size_t key_bytes(int W) { return W == 1 ? 8 : 16; }
+
+uint64_t table_slots(uint64_t n, int k) {
+    if (k < 32) n = std::min<uint64_t>(n, 1ull << (2 * k));
+    if (n >= 1ull << 31) return 0;
+    uint64_t S = 1024;
+    while (S < 2 * n + 2) S <<= 1;
+    return S;
+}
 
 // The unit of a group's planned size (group_pct).
 uint32_t count_slots(int) { return 8192; }
@@ -1609,9 +1619,8 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     // a global table with room for n keys: count() launches what fills it, then its pairs are written
     auto in_table = [&](uint64_t n, uint32_t sample, const std::function<cudaError_t(const FallbackParams&)>& count,
                         bool may_lack_room) -> tg_status {
-        uint64_t S = 1024;
-        while (S < 2 * n + 2) S <<= 1;
-        if (S > (1ull << 32)) {
+        const uint64_t S = table_slots(n, in.k);
+        if (!S) {
             if (!may_lack_room) err = "fallback table too large";
             return TG_ERR_TABLE;
         }
