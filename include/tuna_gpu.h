@@ -82,7 +82,8 @@ typedef struct tg_job tg_job;
 
 typedef struct {
     int device;                 /* CUDA device ordinal */
-    uint64_t hbm_budget_bytes;  /* device memory phase 2 may hold at once (keys, pairs, groups);
+    uint64_t hbm_budget_bytes;  /* device memory phase 2 may hold at once (records, pairs, groups,
+                                   tables of large bins);
                                    0 = free HBM minus a reserve. A job whose keys and pairs do
                                    not fit is counted in passes over ranges of bins, each pass's
                                    pairs copied to host memory (results then stay on the host) */

@@ -1056,6 +1056,25 @@ static tg_status lex_append(tg_job* j, const uint8_t* draw, size_t len, const ui
 
 static tg_status run_spill(tg_job* j);
 
+// The table in global memory of a run of phase 2 (ctx->fbtab). One that several bins
+// share takes at most 0.7 GB and is kept for the next run; a larger one, a single bin's,
+// is given back when the run ends.
+struct RunTable {
+    static constexpr size_t KEEP = 1u << 30;
+    tg_ctx* ctx;
+    ~RunTable() {
+        if (ctx->fbtab.cap <= KEEP) return;
+        cudaFree(ctx->fbtab.p);
+        ctx->fbtab = DevBuf{};
+    }
+    void* operator()(size_t bytes) const { return ctx->ensure(ctx->fbtab, bytes) == cudaSuccess ? ctx->fbtab.p : nullptr; }
+};
+
+// What a memory budget leaves for tables beside `used` bytes of phase 2.
+static uint64_t table_room(const tg_ctx* ctx, uint64_t used) {
+    return !ctx->hbm_budget ? ~0ull : ctx->hbm_budget > used ? ctx->hbm_budget - used : 0;
+}
+
 static tg_status tg_job_run_impl(tg_job* j) {
     if (!j) return TG_ERR_ARG;
     const TraceRange tr("tuna.job_run");
@@ -1176,9 +1195,8 @@ static tg_status tg_job_run_impl(tg_job* j) {
     }
     CK(cudaEventRecord(ctx->ev[6], ctx->st), "event");
     std::string msg;
-    auto fallback_table = [&](size_t bytes) -> void* {
-        return ctx->ensure(ctx->fbtab, bytes) == cudaSuccess ? ctx->fbtab.p : nullptr;
-    };
+    const RunTable table{ctx};
+    const std::function<void*(size_t)> fallback_table = [&table](size_t bytes) { return table(bytes); };
     P2Output out{};
     tg_stats& S = j->st;
     float ms = 0;
@@ -1203,6 +1221,7 @@ static tg_status tg_job_run_impl(tg_job* j) {
             out.reorder_after = j->reorder_after;
         }
         out.cap = out_cap;
+        const uint64_t pair_bytes = out_cap * (ns > 1 ? 2 * key_bytes(W) + 12 : key_bytes(W) + 4);
         // group size: the context's tuned one, else half the table; with
         // TG_CTX_AUTOTUNE the first large job of a key width times the counting
         // pass at each candidate on its own keys and keeps the fastest
@@ -1215,6 +1234,7 @@ static tg_status tg_job_run_impl(tg_job* j) {
                 ti.group_pct = cp;
                 const size_t tb = phase2_scratch_bytes(ti);
                 CK(ctx->ensure(ctx->scratch, tb), "alloc phase-2 scratch");
+                ti.table_room = table_room(ctx, tb + pair_bytes);
                 P2Output to = out;
                 const tg_status ts = phase2_run(ti, ctx->scratch.p, tb, to, fallback_table, ctx->st, ctx->ev[7],
                                                 &launches, msg, P2Overlap());
@@ -1231,6 +1251,7 @@ static tg_status tg_job_run_impl(tg_job* j) {
         S.group_load_pct = pct;
         const size_t p2_bytes = phase2_scratch_bytes(in);
         CK(ctx->ensure(ctx->scratch, p2_bytes), "alloc phase-2 scratch");
+        in.table_room = table_room(ctx, p2_bytes + pair_bytes);
         CK(cudaEventRecord(ctx->ev[6], ctx->st), "event");
         const tg_status ps = phase2_run(in, ctx->scratch.p, p2_bytes, out, fallback_table, ctx->st, ctx->ev[7],
                                         &launches, msg, j->overlap ? *j->overlap : P2Overlap());
@@ -1276,6 +1297,7 @@ static tg_status tg_job_run_impl(tg_job* j) {
         CK(ctx->ensure(ctx->okeys, out_cap * key_bytes(W)), "alloc output keys");
         CK(ctx->ensure(ctx->ocnt, out_cap * 4), "alloc output counts");
         CK(ctx->ensure(ctx->scratch, p2_bytes), "alloc phase-2 scratch");
+        for (P2Input& ip : pin) ip.table_room = table_room(ctx, p2_bytes + out_cap * (key_bytes(W) + 4));
         j->spilled = true;
         j->host_keys.clear();
         j->host_counts.clear();
@@ -1543,9 +1565,8 @@ static tg_status run_spill(tg_job* j) {
     }
     tg_stats& T = j->st;
     T.group_load_pct = ctx->tuned_pct[W - 1] ? ctx->tuned_pct[W - 1] : 50;
-    auto fallback_table = [&](size_t bytes) -> void* {
-        return ctx->ensure(ctx->fbtab, bytes) == cudaSuccess ? ctx->fbtab.p : nullptr;
-    };
+    const RunTable table{ctx};
+    const std::function<void*(size_t)> fallback_table = [&table](size_t bytes) { return table(bytes); };
     j->spilled = true;
     j->host_keys.clear();
     j->host_counts.clear();
@@ -1619,6 +1640,7 @@ static tg_status run_spill(tg_job* j) {
         CK(ctx->ensure(ctx->ocnt, out_cap * 4), "alloc output counts");
         const size_t p2_bytes = phase2_scratch_bytes(in);
         CK(ctx->ensure(ctx->scratch, p2_bytes), "alloc phase-2 scratch");
+        in.table_room = table_room(ctx, p2_bytes + out_cap * (key_bytes(W) + 4));
         P2Output po{};
         po.keys = ctx->okeys.p;
         po.counts = ctx->ocnt.as<uint32_t>();

@@ -143,6 +143,7 @@ struct P2Input {
     uint64_t n_recs;                   // packed records in all
     uint64_t ci, cx;
     bool roomy = false;                // scratch for splitting large groups may be taken
+    uint64_t table_room = ~0ull;       // bytes that a table for the largest groups may take
     uint32_t n_samples = 1;
     // the bins counted by this run (all by default); segs must lie inside, and
     // n_kmers and n_recs count only theirs

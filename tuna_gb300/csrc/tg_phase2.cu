@@ -1625,7 +1625,8 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
             return TG_ERR_TABLE;
         }
         const size_t kbytes = (size_t)S * key_bytes(W);
-        uint8_t* tab = static_cast<uint8_t*>(fallback_table(kbytes + (size_t)S * 4 + 16));
+        const size_t bytes = kbytes + (size_t)S * 4 + 16;
+        uint8_t* tab = may_lack_room && bytes > in.table_room ? nullptr : static_cast<uint8_t*>(fallback_table(bytes));
         if (!tab) {
             if (!may_lack_room) err = "no room for the fallback table";
             return TG_ERR_OOM;
