@@ -51,9 +51,23 @@ static void check_tables() {
     CHECK(table_slots(1ull << 40, 2) == 1024 && table_slots(100, 9) == 1024, "small tables");
 }
 
+// Bin counts as the cut adds them up, records of 225 k-mers in 15 pieces: the sum tells
+// a bin of 2^32 k-mers or more.
+static void check_bin_counts() {
+    for (uint64_t in_one : {(1ull << 32) / 225 - 1, (1ull << 32) / 225 + 1, (3ull << 32) / 225 + 7}) {
+        uint64_t hist[2] = {0, 0}, kmers = 0, sum = 0;
+        for (uint64_t r = 0; r < in_one + 1000; ++r, kmers += 225)
+            hist[r >= in_one] += ((uint64_t)rec_pieces(225) << 32) | 225;
+        for (uint64_t h : hist) sum += h & 0xFFFFFFFFull;
+        CHECK(kmers_per_bin_ok(sum, kmers) == (in_one * 225 < 1ull << 32), "%llu k-mers of one bin",
+              (unsigned long long)in_one * 225);
+    }
+}
+
 int main() {
     check_cut_lists();
     check_tables();
+    check_bin_counts();
     if (fails) {
         std::printf("%d checks failed\n", fails);
         return 1;

@@ -61,3 +61,17 @@ def test_table_under_a_budget(k, tight):
             assert np.array_equal(got.keys, want.keys) and np.array_equal(got.counts, want.counts)
         want = got
     assert len(want) == 5
+
+
+def test_bin_of_2_32_kmers():
+    """More k-mers of one bin than its counter holds: refused, in one run, of a shard, in
+    passes and with the records in host memory."""
+    import torch
+    import tuna_gb300 as T
+    if torch.cuda.mem_get_info()[0] < 200 << 30:
+        pytest.skip("the pairs take 53 GB")
+    seq = _satellite(4_400_000_000)
+    for budget, kw in ((0, {}), (0, dict(shard=(1, 2))), (8 << 30, {}), (0, dict(spill=(1 << 33,)))):
+        with T.Context(0, hbm_budget=budget) as ctx:
+            with pytest.raises(T.GpuError, match=r"more than 2\^32"):
+                ctx.run(31, 21, seq=seq, **kw)

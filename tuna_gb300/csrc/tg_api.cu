@@ -1070,6 +1070,13 @@ struct RunTable {
     void* operator()(size_t bytes) const { return ctx->ensure(ctx->fbtab, bytes) == cudaSuccess ? ctx->fbtab.p : nullptr; }
 };
 
+// A downloaded bin histogram against the job's k-mers.
+static tg_status check_bins(tg_ctx* ctx, const std::vector<uint64_t>& hist, uint64_t n_kmers) {
+    uint64_t sum = 0;
+    for (uint64_t h : hist) sum += h & 0xFFFFFFFFull;
+    return kmers_per_bin_ok(sum, n_kmers) ? TG_OK : ctx->fail(TG_ERR_UNSUPPORTED, bin_too_large());
+}
+
 // What a memory budget leaves for tables beside `used` bytes of phase 2.
 static uint64_t table_room(const tg_ctx* ctx, uint64_t used) {
     return !ctx->hbm_budget ? ~0ull : ctx->hbm_budget > used ? ctx->hbm_budget - used : 0;
@@ -1106,17 +1113,19 @@ static tg_status tg_job_run_impl(tg_job* j) {
     // the segments this run counts: all of them, or the job's shard of them
     std::vector<Segment> segs = B.segs;
     std::vector<uint64_t> hist;  // k-mers and packed records per bin, downloaded when a shard or the passes need it
-    auto load_hist = [&]() -> cudaError_t {
-        if (!hist.empty()) return cudaSuccess;
+    auto load_hist = [&]() -> tg_status {
+        if (!hist.empty()) return TG_OK;
         hist.resize((size_t)1 << j->bin_bits);
-        return cudaMemcpy(hist.data(), ctx->hist.p, hist.size() * 8, cudaMemcpyDeviceToHost);
+        CK(cudaMemcpy(hist.data(), ctx->hist.p, hist.size() * 8, cudaMemcpyDeviceToHost), "d2h");
+        return check_bins(ctx, hist, r1.c.kmers);
     };
     // deferred: at most one k-mer, and one record, per position
     uint64_t n_kmers = deferred ? j->n : r1.c.kmers, n_recs = deferred ? j->n : r1.c.records + r1.c.extra_recs;
     if (j->n_shards > 1) {  // one sample: 2^p1_bits >= n_shards segments of consecutive bins
         const size_t P = B.segs.size();
         segs.assign(B.segs.begin() + P * j->shard / j->n_shards, B.segs.begin() + P * (j->shard + 1) / j->n_shards);
-        CK(load_hist(), "d2h");
+        const tg_status hs = load_hist();
+        if (hs != TG_OK) return hs;
         n_kmers = n_recs = 0;
         for (const Segment& g : segs)
             for (uint32_t b = g.bin_lo; b < g.bin_hi; ++b) {
@@ -1171,7 +1180,8 @@ static tg_status tg_job_run_impl(tg_job* j) {
             budget = have > reserve ? have - reserve : 0;
         }
         if (n_kmers * per_key > budget) {
-            CK(load_hist(), "d2h");
+            const tg_status hs = load_hist();
+            if (hs != TG_OK) return hs;
             const uint64_t max_keys = std::max<uint64_t>(1, budget / per_key);
             uint32_t s0 = 0;
             uint64_t acc = 0;
@@ -1452,6 +1462,8 @@ static tg_status spill_flush(tg_job* j) {
     {  // k-mers per bin
         std::vector<uint64_t> h((size_t)1 << BIN_BITS);
         CK(cudaMemcpy(h.data(), ctx->hist.p, h.size() * 8, cudaMemcpyDeviceToHost), "d2h");
+        s = check_bins(ctx, h, r.c.kmers);
+        if (s != TG_OK) return s;
         for (size_t b = 0; b < h.size(); ++b) {
             S.hist[b] += h[b] & 0xFFFFFFFFull;
             S.rec_hist[b] += h[b] >> 32;
@@ -1540,7 +1552,7 @@ static tg_status run_spill(tg_job* j) {
     std::vector<uint64_t> hu(S.hist.size());
     std::vector<uint64_t> bk(nb, 0), br(nb, 0);
     for (size_t b = 0; b < S.hist.size(); ++b) {
-        if (S.hist[b] > 0xFFFFFFFFull) return ctx->fail(TG_ERR_UNSUPPORTED, "a bin holds more than 2^32 k-mers");
+        if (S.hist[b] > 0xFFFFFFFFull) return ctx->fail(TG_ERR_UNSUPPORTED, bin_too_large());
         hu[b] = S.hist[b] | (S.rec_hist[b] << 32);
         bk[b / seg_bins] += S.hist[b];
         br[b / seg_bins] += S.rec_hist[b];

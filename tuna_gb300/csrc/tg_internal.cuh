@@ -134,7 +134,10 @@ struct CutParams {
     uint32_t* n_desc;        // [n_cta]
     uint32_t* max_desc;      // the most of them, those past desc_cap too
     uint32_t* hist;          // export cut: u32 [P][n_cta] records, then u64 [P] k-mers per bucket
-    unsigned long long* binhist;  // counting cut: [bins] k-mers + 2^32 x packed records per bin
+    // counting cut: [bins] k-mers + 2^32 x packed records per bin. A bin of 2^32 k-mers
+    // or more carries into its records: where there are that many k-mers in all, the
+    // bins' sum is compared with theirs (kmers_per_bin_ok)
+    unsigned long long* binhist;
     int desc_sb;             // counting cut: start bits of a descriptor (desc_start_bits)
     // samples of the job (counting cut): sample i is positions [start[i], start[i+1])
     const unsigned long long* sample_start;  // [n_samples + 1]

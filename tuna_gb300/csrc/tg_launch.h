@@ -109,6 +109,11 @@ uint32_t count_slots(int W);
 // differ: a power of two, more than half of them free. 0: more than 2^32.
 uint64_t table_slots(uint64_t n, int k);
 
+// Whether no bin of a job of n_kmers k-mers, whose bins' k-mers add up to sum, holds
+// 2^32 of them or more: each such bin is short by a multiple of 2^32.
+inline bool kmers_per_bin_ok(uint64_t sum, uint64_t n_kmers) { return sum == n_kmers; }
+inline const char* bin_too_large() { return "a bin holds more than 2^32 k-mers"; }
+
 // Phase 2 of one job, shared by the entry points: the phase-1 descriptor lists
 // and the k-mer counts per bin in, distinct keys and counts (and their
 // samples) out.

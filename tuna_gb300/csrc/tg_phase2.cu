@@ -1521,6 +1521,11 @@ tg_status phase2_run(const P2Input& in, void* scratch, size_t scratch_cap, P2Out
     P2_CK(launch_bin_scan(in.binhist + in.bin_lo, in.bin_hi - in.bin_lo, R.kofs + in.bin_lo, R.rofs + in.bin_lo,
                           R.sums, st, launches),
           "scan");
+    if (!in.deferred && in.n_kmers >> 32) {
+        unsigned long long sum = 0;
+        P2_CK(read_counters(ov, {R.kofs + in.bin_hi, 1}, {}, {}, &sum, st), "scan");
+        if (!kmers_per_bin_ok(sum, in.n_kmers)) { err = bin_too_large(); return TG_ERR_UNSUPPORTED; }
+    }
 
     KeysParams K{};
     K.packed = in.packed;
