@@ -240,9 +240,35 @@ def _copy_bytes(src: int, n: int, pool: ThreadPoolExecutor) -> bytes:
     """n bytes at address src, copied by the pool's threads (memmove releases the GIL)."""
     out = _bytes_new(None, n)
     dst, step = _bytes_at(out), -(-n // _COPY_THREADS // 65536) * 65536
-    for _ in pool.map(lambda o: ctypes.memmove(dst + o, src + o, min(step, n - o)) and None, range(0, n, step)):
-        pass
+    try:
+        for _ in pool.map(lambda o: ctypes.memmove(dst + o, src + o, min(step, n - o)) and None, range(0, n, step)):
+            pass
+    except BaseException:  # a thread that did not start, an interrupt
+        pool.shutdown(cancel_futures=True)  # waits: nothing writes to the bytes once they are gone
+        raise
     return out
+
+
+class _DrainSink:
+    """The bytes that tg_job_drain hands over. An exception cannot pass a ctypes callback (it
+    is printed, and the status returned is undefined): it stops the drain and is raised
+    by result()."""
+
+    def __init__(self, ctx: "Context"):
+        self.ctx, self.chunks, self.error = ctx, [], None
+
+    def __call__(self, data, nbytes, _npairs, _user) -> int:
+        try:
+            self.chunks.append(self.ctx._drained(data, nbytes))
+            return 0
+        except BaseException as e:
+            self.error = e
+            return 1
+
+    def result(self) -> bytes:
+        if self.error is not None:
+            raise self.error
+        return self.chunks[0] if len(self.chunks) == 1 else b"".join(self.chunks)
 
 
 class Context:
@@ -309,6 +335,19 @@ class Context:
         self.check(self._L.tg_fastx_to_stream(self.h, a.ctypes.data if a.size else None, a.size, out.ctypes.data,
                                               out.size, ctypes.byref(n)))
         return out[: n.value].tobytes()
+
+    def _drained(self, data: int, nbytes: int) -> bytes:
+        if nbytes >= _COPY_MIN:
+            try:
+                if self._pool is None:
+                    self._pool = ThreadPoolExecutor(_COPY_THREADS)
+                return _copy_bytes(data, nbytes, self._pool)
+            except RuntimeError:  # no thread to be had: copied here
+                self._pool = None
+            except BaseException:
+                self._pool = None
+                raise
+        return ctypes.string_at(data, nbytes)
 
     def run(self, k: int, m: int, *, seq=None, dev_seq=None, dev_len: int = 0, fastx=None, files=(),
             dev_fastx=None, samples=None, n_parts: int = 16, ci: int = 1, cx: int = _U64_MAX, gpu_parts: int = 0,
@@ -384,20 +423,12 @@ class Context:
                         sdg.append(d.as_dict())
             formatted = None
             if drain is not None:
-                chunks = []
-
-                def dsink(data, nbytes, _npairs, _u):
-                    if nbytes < _COPY_MIN:
-                        chunks.append(ctypes.string_at(data, nbytes))
-                    else:
-                        if self._pool is None:
-                            self._pool = ThreadPoolExecutor(_COPY_THREADS)
-                        chunks.append(_copy_bytes(data, nbytes, self._pool))
-                    return 0
-
+                dsink = _DrainSink(self)
                 dcb = _SINK(dsink)
-                self.check(L.tg_job_drain(j, int(drain), dcb, None))
-                formatted = chunks[0] if len(chunks) == 1 else b"".join(chunks)
+                rc = L.tg_job_drain(j, int(drain), dcb, None)
+                if dsink.error is None:
+                    self.check(rc)
+                formatted = dsink.result()
             parts = None
             if export:
                 parts = [b""] * n_parts
