@@ -64,8 +64,21 @@ static void check_bin_counts() {
     }
 }
 
+// The group sizes of a tuned context: all different, the default's the largest.
+static void check_group_sizes() {
+    for (int W = 1; W <= 2; ++W) {
+        uint32_t before = 0;
+        for (uint32_t pct : TUNE_PCT) {
+            CHECK(group_keys(W, pct) > before, "%u %% gives %u k-mers again (W=%d)", pct, group_keys(W, pct), W);
+            before = group_keys(W, pct);
+        }
+        CHECK(before == group_keys(W, P2Input{}.group_pct) && before == group_keys(W, 100), "W=%d: %u", W, before);
+    }
+}
+
 int main() {
     check_cut_lists();
+    check_group_sizes();
     check_tables();
     check_bin_counts();
     if (fails) {

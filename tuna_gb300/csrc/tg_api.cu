@@ -1232,14 +1232,13 @@ static tg_status tg_job_run_impl(tg_job* j) {
         }
         out.cap = out_cap;
         const uint64_t pair_bytes = out_cap * (ns > 1 ? 2 * key_bytes(W) + 12 : key_bytes(W) + 4);
-        // group size: the context's tuned one, else half the table; with
+        // group size: the context's tuned one, else a full store; with
         // TG_CTX_AUTOTUNE the first large job of a key width times the counting
-        // pass at each candidate on its own keys and keeps the fastest
+        // pass at each candidate on its own records and keeps the fastest
         uint32_t pct = ctx->tuned_pct[W - 1] ? ctx->tuned_pct[W - 1] : 50;
         if ((ctx->flags & TG_CTX_AUTOTUNE) && !ctx->tuned_pct[W - 1] && n_kmers >= (1ull << 26)) {
-            static const uint32_t cand[] = {35, 50, 65};
             float best = 0;
-            for (uint32_t cp : cand) {
+            for (uint32_t cp : TUNE_PCT) {
                 P2Input ti = in;
                 ti.group_pct = cp;
                 const size_t tb = phase2_scratch_bytes(ti);

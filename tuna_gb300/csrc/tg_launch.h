@@ -104,7 +104,13 @@ cudaError_t launch_spill_write(const uint32_t* packed, const uint64_t* desc, uin
                                const long long* host_shift, uint64_t* out_desc, uint8_t* out_bytes, cudaStream_t st);
 cudaError_t launch_rebase(uint64_t* desc, uint64_t n, uint64_t add, int n_sm, cudaStream_t st);
 size_t key_bytes(int W);
-uint32_t count_slots(int W);
+uint32_t count_slots(int W);  // the unit of P2Input::group_pct
+// K-mers of a group that takes pct % of the unit: at most what a CTA's store holds
+// (4,096 or, of two words, 3,072).
+uint32_t group_keys(int W, uint32_t pct);
+// The group sizes that a tuned context tries (TG_CTX_AUTOTUNE), the store's among them:
+// 2,048, 2,867 and 4,096 or 3,072 k-mers (155 Mbp, k=31 m=21: 1.57, 1.42, 1.35 ms of counting).
+constexpr uint32_t TUNE_PCT[] = {25, 35, 50};
 // Slots of a table in global memory for n k-mers of length k, of which at most 4^k
 // differ: a power of two, more than half of them free. 0: more than 2^32.
 uint64_t table_slots(uint64_t n, int k);
@@ -155,7 +161,7 @@ struct P2Input {
     uint32_t bin_lo = 0, bin_hi = 1u << BIN_BITS;
     uint32_t all_bins = 1u << BIN_BITS;  // bins of the job
     int desc_sb = DESC_START_BITS;       // start bits of a descriptor
-    uint32_t group_pct = 50;  // keys per group, % of the table's slots
+    uint32_t group_pct = 50;  // k-mers per group (group_keys)
     // Phase 1 may still run: n_kmers, n_recs and max_desc are upper bounds, the
     // counts are read on the device, and the host waits once, at the end; read_back
     // (n_read u64, device) then goes to P2Output::read_back.

@@ -1260,13 +1260,16 @@ uint64_t table_slots(uint64_t n, int k) {
     return S;
 }
 
-// The unit of a group's planned size (group_pct).
 uint32_t count_slots(int) { return 8192; }
 
-// Keys that k_plan puts in a group: group_pct of the unit, at most a store full.
+uint32_t group_keys(int W, uint32_t pct) {
+    const uint32_t cap = W == 1 ? CountShape<1>::CAP : CountShape<2>::CAP;
+    return std::max<uint32_t>(1, std::min(count_slots(W) * pct / 100, cap));
+}
+
+// Keys that k_plan puts in a group.
 static uint32_t group_target(const P2Input& in) {
-    const uint32_t cap = in.W == 1 ? CountShape<1>::CAP : CountShape<2>::CAP;
-    const uint32_t t = std::max<uint32_t>(1, std::min(count_slots(in.W) * in.group_pct / 100, cap));
+    const uint32_t t = group_keys(in.W, in.group_pct);
     // jobs too small for a full group per CTA: smaller groups, so that more SMs count
     const uint64_t share = in.n_kmers / (COUNT_PER_SM * (uint64_t)std::max<uint32_t>(1, in.n_sm));
     return (uint32_t)std::min<uint64_t>(t, std::max<uint64_t>(COUNT_THREADS, share));
