@@ -1004,8 +1004,8 @@ def main():
                     "stands in for the reference's genome assemblies",
             "config": main_config(bases, n_stream, world),
             "gpu_config": {"gpu_parts": int(st["gpu_parts"]), "group_load_pct": int(st["group_load_pct"]),
-                           "autotune": "off (--no-autotune): half the table" if args.no_autotune else
-                           "TG_CTX_AUTOTUNE: group size timed on the first warm-up step (35/50/65 % of the table)"},
+                           "autotune": "off (--no-autotune): a full store" if args.no_autotune else
+                           "TG_CTX_AUTOTUNE: group size timed on the first warm-up step (25/35/50 % of 8,192 k-mers, at most a store)"},
             "stats": {"kmers": int(st["kmers"]), "superkmers": int(st["superkmers"]),
                       "distinct": int(st["distinct"]), "fallback_groups": int(st["fallback_groups"]),
                       "distinct_kmers_per_s": int(st["distinct"]) / (ms / 1e3),

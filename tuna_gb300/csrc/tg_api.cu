@@ -2,16 +2,20 @@
 // jobs, the device pipeline driver and result access.
 //
 // A job runs, on the context's stream:
-//   k_pack      ASCII stream -> 2-bit codes + validity bits
 //   (k_lex_*    FASTA/FASTQ bytes -> the stream, when fed as files)
-//   k_cut_seq   minimizers, chain starts, forced splits -> record descriptors
-//               per CTA, k-mers and packed records per bin (one host sync here)
+//   k_prepare   counters, bins, hash tables of m, a one-sample job's layout
+//   k_pack      ASCII stream -> 2-bit codes + validity bits
+//   k_cut_*     minimizers, chain starts, forced splits -> record descriptors
+//               per CTA, k-mers and packed records per bin (then the host reads
+//               their numbers, but for short jobs, which go on with bounds)
+//   k_setup     phase 2's counters and segments
 //   k_scan*     bin counts -> k-mer and packed record offsets
 //   k_plan      groups of whole bins per segment (a run of bins of one sample)
 //   k_recs      every record with its bases at its group's cursor
 //   k_count     per group: keys into a shared-memory table, ci/cx, compaction
-//               (again for groups split by key hash)
-//   k_fb_*      (rare) key ranges that overflowed shared memory, global tables
+//   k_rounds    a bin larger than a group: in rounds or by key-hash parts
+//   k_big       the largest bins, many CTAs each, into a global table (k_fb_*)
+//   k_fb_*      (rare) also key ranges that overflowed the parts
 //   k_fmt*      (tg_job_drain / tg_job_write) pairs -> TSV / KFF / raw bytes
 // The export of partition files runs the tile cut k_cut<true> instead, which
 // also yields each record's exact minimizer position.

@@ -128,7 +128,7 @@ struct CutParams {
     uint32_t p1_bits;        // log2 internal bucket count
     uint32_t n_cta;
     int seg;                 // counting cut: k-mer start positions per thread and tile (cut_layout)
-    uint64_t chunk;          // k-mer start positions per CTA (multiple of CUT_TILE)
+    uint64_t chunk;          // k-mer start positions per CTA (cut_layout: whole tiles less 64, export cut whole tiles)
     uint64_t* desc;          // [n_cta][desc_cap] record descriptors
     uint64_t desc_cap;
     uint32_t* n_desc;        // [n_cta]

@@ -8,8 +8,8 @@
 // pre-reserved pool), or a latency-critical loop where an allocation would
 // synchronise the device. tg_count_seq_device_noalloc takes the input and the
 // output buffers from the caller and keeps every intermediate array (packed
-// bases, superkmer descriptors, the bin histogram and key offsets,
-// k-mer keys, group lists, fallback table) in one file-scope device array of
+// bases, superkmer descriptors, the bin histogram and offsets, packed
+// records, group lists, fallback table) in one file-scope device array of
 // TG_NOALLOC_SCRATCH_BYTES that stays reserved until the process exits. The CUDA
 // runtime loads this file's module, and so reserves the array, on a device the
 // first time the array's address is looked up there, which is the first call on

@@ -441,7 +441,9 @@ struct CountSmem {
 
 // Home slot and entry of a key at place i: both the top bits of a multiply-add
 // hash. They share bits, so one in 32 keys that meet at a home slot are compared in
-// full without being equal; a second mixing step costs more than that.
+// full without being equal; a second mixing step costs more than that. The odd
+// multipliers here and in rec_hash are xxHash's 32-bit primes (well-mixed constants;
+// nothing else of it is used, and no result depends on them).
 __device__ __forceinline__ uint32_t slot_hash(unsigned long long k) {
     return (uint32_t)k * 0x9E3779B1u + (uint32_t)(k >> 32) * 0x85EBCA77u;
 }
