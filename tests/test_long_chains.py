@@ -54,7 +54,7 @@ def test_pinned_input():
 def test_export():
     """The export cut's lists grow to what it found too; records [len][min_pos][bases]."""
     import tuna_gb300 as T
-    n, k = 4_600_000, 63
+    n, k = 700_000, 63  # 3,627 records, in lists of 2,514 at first
     with T.Context(0) as ctx:
         got, parts = ctx.run(k, 21, seq=_seq(b"A", n, 0), n_parts=4, export=True)
     kmers = recs = 0
